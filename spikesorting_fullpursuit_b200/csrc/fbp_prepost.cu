@@ -571,73 +571,130 @@ __global__ void k_zca_mask(const T *__restrict__ v, u32 C, u64 n, const double *
     }
 }
 
-// Per channel: count, sum and centred sum of squares of unmasked samples.
+// Per channel: count and sum (pass 0) or centred sum of squares (pass 1) of
+// unmasked samples; blocks (channel, sample range) add their parts.  Bound by
+// reading v and the mask; with one block per channel, 32 channels x 1.2 M
+// samples took 4.1 ms a pass on 32 of the SMs.
 template <typename T>
-__global__ void k_zca_diag(const T *__restrict__ v, const u8 *__restrict__ mask, u32 C, u64 n,
+__global__ void k_zca_diag(const T *__restrict__ v, const u8 *__restrict__ mask, u32 C, u64 n, u64 chunk,
                            double *__restrict__ cnt, double *__restrict__ sum, int pass, double *__restrict__ ssq) {
     __shared__ double red[2][32];
-    for (u32 c = blockIdx.x; c < C; c += gridDim.x) {
-        double a = 0.0, b = 0.0;
-        const double mu = pass ? sum[c] / cnt[c] : 0.0;
-        for (u64 s = threadIdx.x; s < n; s += blockDim.x) {
-            if (mask[(u64)c * n + s]) continue;
-            const double x = (double)v[(u64)c * n + s];
-            if (pass) { a += (x - mu) * (x - mu); } else { a += 1.0; b += x; }
+    const u32 c = blockIdx.x;
+    const u64 sb = blockIdx.y * chunk, se = min(n, sb + chunk);
+    double a = 0.0, b = 0.0;
+    const double mu = pass ? sum[c] / cnt[c] : 0.0;
+    for (u64 s0 = sb + threadIdx.x; s0 < se; s0 += 4ull * blockDim.x) {
+        T x[4];
+        u8 mk[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const u64 s = s0 + (u64)u * blockDim.x;
+            mk[u] = s < se ? mask[(u64)c * n + s] : (u8)1;
+            x[u] = s < se ? v[(u64)c * n + s] : (T)0;
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_xor_sync(0xffffffffu, a, o);
-            b += __shfl_xor_sync(0xffffffffu, b, o);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            if (mk[u]) continue;
+            const double d = (double)x[u];
+            if (pass) { a += (d - mu) * (d - mu); } else { a += 1.0; b += d; }
         }
-        if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = a; red[1][threadIdx.x >> 5] = b; }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double A = 0, B = 0;
-            for (u32 w = 0; w < blockDim.x / 32; w++) { A += red[0][w]; B += red[1][w]; }
-            if (pass) ssq[c] = A; else { cnt[c] = A; sum[c] = B; }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = a; red[1][threadIdx.x >> 5] = b; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double A = 0, B = 0;
+        for (u32 w = 0; w < blockDim.x / 32; w++) { A += red[0][w]; B += red[1][w]; }
+        if (pass) {
+            atomicAdd(&ssq[c], A);
+        } else {
+            atomicAdd(&cnt[c], A);
+            atomicAdd(&sum[c], B);
         }
-        __syncthreads();
     }
 }
 
 // Off-diagonal: G[i][j] = sum of v_i v_j and P[i][j] = count over samples
-// that neither channel masks; 16x16 channel tiles, samples split over blocks.
+// that neither channel masks; 32x32 channel tiles of the upper triangle, 2x2
+// pairs per thread, samples split over blocks.  Masked samples are staged as
+// 0 and the masks as 64-bit words, so that the inner step is one product and
+// the count one population count per 64 samples; a stretch with a value that
+// is not finite takes the loop that tests the masks (0 times it is not 0).
+// Bound by shared-memory reads (four 8-byte reads per four products); one pair
+// per thread over 16x16 tiles on 57 blocks took 8.8 ms for 32 channels x
+// 1.2 M samples.
+constexpr u32 kGramTile = 32, kGramStep = 64;
 template <typename T>
-__global__ void k_zca_gram(const T *__restrict__ v, const u8 *__restrict__ mask, u32 C, u64 n, u32 chunk,
-                           double *__restrict__ G, double *__restrict__ P) {
-    __shared__ double xs[16][65];
-    __shared__ double ys[16][65];
-    __shared__ u8 mx[16][64], my[16][64];
-    const u32 tc = ceil_div(C, 16);
+__global__ void __launch_bounds__(256)
+k_zca_gram(const T *__restrict__ v, const u8 *__restrict__ mask, u32 C, u64 n, u64 chunk, double *__restrict__ G,
+           double *__restrict__ P) {
+    __shared__ double sh[2][kGramTile][kGramStep + 1];
+    __shared__ u32 okw[2][kGramTile][2];             // unmasked samples, one bit each
+    const u32 tc = ceil_div(C, kGramTile);
     const u32 ti = blockIdx.x / tc, tj = blockIdx.x % tc;
     if (tj < ti) return;                             // upper triangle of tiles
-    const u32 li = threadIdx.x / 16, lj = threadIdx.x % 16;   // 256 threads
-    const u32 ci = ti * 16 + li, cj = tj * 16 + lj;
-    double g = 0.0, p = 0.0;
+    const u32 li = threadIdx.x / 16, lj = threadIdx.x % 16, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const u32 sides = ti == tj ? 1u : 2u, yb = sides - 1;
+    double g[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    u32 p[2][2] = {{0, 0}, {0, 0}};                  // at most `chunk` samples
     const u64 sb = (u64)blockIdx.y * chunk, se = min(n, sb + chunk);
-    for (u64 s0 = sb; s0 < se; s0 += 64) {
-        for (u32 q = threadIdx.x; q < 16 * 64; q += blockDim.x) {
-            const u32 r = q / 64, k = q % 64;
-            const u64 s = s0 + k;
-            const u32 a = ti * 16 + r, b = tj * 16 + r;
-            const bool in = s < se;
-            xs[r][k] = (in && a < C) ? (double)v[(u64)a * n + s] : 0.0;
-            mx[r][k] = (in && a < C) ? mask[(u64)a * n + s] : (u8)1;
-            ys[r][k] = (in && b < C) ? (double)v[(u64)b * n + s] : 0.0;
-            my[r][k] = (in && b < C) ? mask[(u64)b * n + s] : (u8)1;
+    for (u64 s0 = sb; s0 < se; s0 += kGramStep) {
+        bool odd = false;
+#pragma unroll 4
+        for (u32 q = warp; q < sides * kGramTile * 2; q += 8) {      // (side, row, half of the step)
+            const u32 side = q / (kGramTile * 2), row = (q / 2) % kGramTile, half = q & 1u;
+            const u32 c = (side ? tj : ti) * kGramTile + row;
+            const u64 s = s0 + half * 32 + lane;
+            const bool in = s < se && c < C;
+            const bool ok = in && !mask[(u64)c * n + s];
+            const double x = ok ? (double)v[(u64)c * n + s] : 0.0;
+            odd |= !(fabs(x) <= 1.7976931348623157e308);
+            sh[side][row][half * 32 + lane] = x;
+            const u32 w = __ballot_sync(0xffffffffu, ok);
+            if (lane == 0) okw[side][row][half] = w;
         }
-        __syncthreads();
+        const bool masked_loop = __syncthreads_or(odd);
+        u32 wx[2][2], wy[2][2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            wx[k][0] = okw[0][li + 16 * k][0]; wx[k][1] = okw[0][li + 16 * k][1];
+            wy[k][0] = okw[yb][lj + 16 * k][0]; wy[k][1] = okw[yb][lj + 16 * k][1];
+        }
+#pragma unroll
+        for (int a = 0; a < 2; a++)
+#pragma unroll
+            for (int b = 0; b < 2; b++) p[a][b] += __popc(wx[a][0] & wy[b][0]) + __popc(wx[a][1] & wy[b][1]);
+        if (!masked_loop) {
 #pragma unroll 8
-        for (u32 k = 0; k < 64; k++) {
-            const bool ok = !mx[li][k] && !my[lj][k];
-            g += ok ? xs[li][k] * ys[lj][k] : 0.0;
-            p += ok ? 1.0 : 0.0;
+            for (u32 k = 0; k < kGramStep; k++) {
+                const double x0 = sh[0][li][k], x1 = sh[0][li + 16][k], y0 = sh[yb][lj][k], y1 = sh[yb][lj + 16][k];
+                g[0][0] = fma(x0, y0, g[0][0]);
+                g[0][1] = fma(x0, y1, g[0][1]);
+                g[1][0] = fma(x1, y0, g[1][0]);
+                g[1][1] = fma(x1, y1, g[1][1]);
+            }
+        } else {
+            for (u32 k = 0; k < kGramStep; k++)
+                for (int a = 0; a < 2; a++)
+                    for (int b = 0; b < 2; b++)
+                        if ((wx[a][k >> 5] & wy[b][k >> 5]) >> (k & 31) & 1u)
+                            g[a][b] = fma(sh[0][li + 16 * a][k], sh[yb][lj + 16 * b][k], g[a][b]);
         }
         __syncthreads();
     }
-    if (ci < C && cj < C && cj > ci) {
-        atomicAdd(&G[(u64)ci * C + cj], g);
-        atomicAdd(&P[(u64)ci * C + cj], p);
-    }
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+        for (int b = 0; b < 2; b++) {
+            const u32 ci = ti * kGramTile + li + 16 * a, cj = tj * kGramTile + lj + 16 * b;
+            if (ci < C && cj < C && cj > ci) {
+                atomicAdd(&G[(u64)ci * C + cj], g[a][b]);
+                atomicAdd(&P[(u64)ci * C + cj], (double)p[a][b]);
+            }
+        }
 }
 
 __global__ void k_zca_sigma(u32 C, const double *__restrict__ G, const double *__restrict__ P,
@@ -658,43 +715,59 @@ template <> __device__ __forceinline__ short cast_out<short>(double x) { return 
 
 // out = Z @ v tile by tile: a block computes 32 output channels x 256
 // samples, the channel sum in ascending order in float64 (16 channels of
-// the voltage staged at a time).
+// the voltage staged at a time).  A thread holds 8 outputs x 4 samples, so
+// that 32 products take 8 shared-memory reads (32 outputs x 1 sample took 33
+// and were bound by them: 435 us for 32 channels x 1.2 M samples).
 template <typename T>
-__global__ void k_zca_apply(const double *__restrict__ Z, const T *__restrict__ v, u32 C, u64 n, T *__restrict__ out) {
-    __shared__ double zs[32][17];
+__global__ void __launch_bounds__(256)
+k_zca_apply(const double *__restrict__ Z, const T *__restrict__ v, u32 C, u64 n, T *__restrict__ out) {
+    __shared__ __align__(16) double zs[16][32];      // [channel][output]
     __shared__ double vs[16][256];
     const u32 tio = ceil_div(C, 32);
     const u64 tis = (n + 255) / 256;
+    const u32 og = (threadIdx.x >> 6) * 8, sx = threadIdx.x & 63;
     for (u64 t = blockIdx.x; t < tio * tis; t += gridDim.x) {
         const u32 i0 = (u32)(t % tio) * 32;
         const u64 s0 = (t / tio) * 256;
-        double acc[32];
+        double acc[8][4];
 #pragma unroll
-        for (int k = 0; k < 32; k++) acc[k] = 0.0;
+        for (int r = 0; r < 8; r++)
+#pragma unroll
+            for (int x = 0; x < 4; x++) acc[r][x] = 0.0;
         for (u32 c0 = 0; c0 < C; c0 += 16) {
             for (u32 q = threadIdx.x; q < 32 * 16; q += blockDim.x) {
                 const u32 r = q / 16, k = q % 16;
-                zs[r][k] = (i0 + r < C && c0 + k < C) ? Z[(u64)(i0 + r) * C + c0 + k] : 0.0;
+                zs[k][r] = (i0 + r < C && c0 + k < C) ? Z[(u64)(i0 + r) * C + c0 + k] : 0.0;
             }
-            for (u32 q = threadIdx.x; q < 16 * 256; q += blockDim.x) {
-                const u32 k = q / 256, x = q % 256;
-                vs[k][x] = (c0 + k < C && s0 + x < n) ? (double)v[(u64)(c0 + k) * n + s0 + x] : 0.0;
-            }
+#pragma unroll
+            for (u32 k = 0; k < 16; k++)
+                vs[k][threadIdx.x] = (c0 + k < C && s0 + threadIdx.x < n)
+                                         ? (double)v[(u64)(c0 + k) * n + s0 + threadIdx.x] : 0.0;
             __syncthreads();
             const u32 kmax = min(16u, C - c0);
             for (u32 k = 0; k < kmax; k++) {
-                const double x = vs[k][threadIdx.x];
+                double x[4];
 #pragma unroll
-                for (int r = 0; r < 32; r++) acc[r] = fma(zs[r][k], x, acc[r]);
+                for (int i = 0; i < 4; i++) x[i] = vs[k][sx + 64 * i];
+#pragma unroll
+                for (int r = 0; r < 8; r += 2) {
+                    const double2 z = *reinterpret_cast<const double2 *>(&zs[k][og + r]);
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        acc[r][i] = fma(z.x, x[i], acc[r][i]);
+                        acc[r + 1][i] = fma(z.y, x[i], acc[r + 1][i]);
+                    }
+                }
             }
             __syncthreads();
         }
-        const u64 s = s0 + threadIdx.x;
-        if (s < n) {
 #pragma unroll
-            for (int r = 0; r < 32; r++)
-                if (i0 + r < C) out[(u64)(i0 + r) * n + s] = cast_out<T>(acc[r]);
-        }
+        for (int r = 0; r < 8; r++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const u64 s = s0 + sx + 64 * i;
+                if (i0 + og + r < C && s < n) out[(u64)(i0 + og + r) * n + s] = cast_out<T>(acc[r][i]);
+            }
     }
 }
 
@@ -967,27 +1040,35 @@ int fbp_zca_covariance(const void *voltage, int dtype, uint32_t C, uint64_t n, c
     if (scratch_bytes < fbp_zca_scratch_bytes(C)) return fail(FBP_ERR_BAD_ARG, "fbp_zca_covariance: scratch too small");
     cudaStream_t st = (cudaStream_t)stream;
     double *G = (double *)scratch, *P = G + (size_t)C * C, *cnt = P + (size_t)C * C, *sum = cnt + C, *ssq = sum + C;
-    PP_CUDA(cudaMemsetAsync(G, 0, (size_t)2 * C * C * 8, st));
+    PP_CUDA(cudaMemsetAsync(G, 0, fbp_zca_scratch_bytes(C), st));
     const u32 mthreads = kMaskThreads;
     const size_t msmem = ((size_t)kMaskTile + 2 * (size_t)cushion + 2) * 4;
     if (msmem > 200 * 1024) return fail(FBP_ERR_BAD_ARG, "fbp_zca_covariance: cushion too large");
     const u64 mtiles = (n + kMaskTile - 1) / kMaskTile * C;
-    const u32 tcs = ceil_div(C, 16);
-    const u32 chunk = 1u << 16;
-    const dim3 gg(tcs * tcs, (u32)((n + chunk - 1) / chunk));
+    // sample ranges of the sums: about four blocks per SM of the gram tiles
+    // that do work (a multiple of its step, at most 2^30 samples, at most
+    // 65535 ranges), and eight of the channels
+    const u32 tcs = ceil_div(C, kGramTile);
+    auto range = [n](u64 want) {
+        const u64 c = std::max<u64>((n + want - 1) / std::max<u64>(want, 1), 4096);
+        return std::min<u64>((std::max<u64>(c, (n + 65534) / 65535) + 63) / 64 * 64, 1ull << 30);
+    };
+    const u64 chunk = range(std::max<u64>(1, 148 * 4 / std::max(1u, tcs * (tcs + 1) / 2)));
+    const u64 dchunk = range(std::max<u64>(1, 148 * 8 / C));
+    const dim3 gg(tcs * tcs, (u32)((n + chunk - 1) / chunk)), dg(C, (u32)((n + dchunk - 1) / dchunk));
     if (dtype == FBP_F32) {
         const float *v = (const float *)voltage;
         if (msmem > 48 * 1024) PP_CUDA(cudaFuncSetAttribute(k_zca_mask<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem));
         k_zca_mask<float><<<(int)std::min<u64>(mtiles, 148 * 8), mthreads, msmem, st>>>(v, C, n, thr, cushion, mask);
-        k_zca_diag<float><<<std::min<u32>(C, 148 * 4), 256, 0, st>>>(v, mask, C, n, cnt, sum, 0, ssq);
-        k_zca_diag<float><<<std::min<u32>(C, 148 * 4), 256, 0, st>>>(v, mask, C, n, cnt, sum, 1, ssq);
+        k_zca_diag<float><<<dg, 256, 0, st>>>(v, mask, C, n, dchunk, cnt, sum, 0, ssq);
+        k_zca_diag<float><<<dg, 256, 0, st>>>(v, mask, C, n, dchunk, cnt, sum, 1, ssq);
         k_zca_gram<float><<<gg, 256, 0, st>>>(v, mask, C, n, chunk, G, P);
     } else if (dtype == FBP_I16) {
         const short *v = (const short *)voltage;
         if (msmem > 48 * 1024) PP_CUDA(cudaFuncSetAttribute(k_zca_mask<short>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msmem));
         k_zca_mask<short><<<(int)std::min<u64>(mtiles, 148 * 8), mthreads, msmem, st>>>(v, C, n, thr, cushion, mask);
-        k_zca_diag<short><<<std::min<u32>(C, 148 * 4), 256, 0, st>>>(v, mask, C, n, cnt, sum, 0, ssq);
-        k_zca_diag<short><<<std::min<u32>(C, 148 * 4), 256, 0, st>>>(v, mask, C, n, cnt, sum, 1, ssq);
+        k_zca_diag<short><<<dg, 256, 0, st>>>(v, mask, C, n, dchunk, cnt, sum, 0, ssq);
+        k_zca_diag<short><<<dg, 256, 0, st>>>(v, mask, C, n, dchunk, cnt, sum, 1, ssq);
         k_zca_gram<short><<<gg, 256, 0, st>>>(v, mask, C, n, chunk, G, P);
     } else {
         return fail(FBP_ERR_BAD_ARG, "fbp_zca_covariance: dtype must be FBP_F32 or FBP_I16");
