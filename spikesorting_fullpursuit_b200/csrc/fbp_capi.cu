@@ -189,7 +189,7 @@ struct Workspace {
 bool fast_overlap_fits(u32 K, u32 L, u32 nmax) {
     const u64 S = 2 * (u64)nmax + 1;
     if (S > 4 * (u64)L + 1 || S > 65535) return false;
-    if (xm_smem_bytes(L) > 227 * 1024 || scan_smem_bytes((u32)S) > 227 * 1024) return false;
+    if (pair_smem_bytes(L, 0) > 227 * 1024 || scan_smem_bytes((u32)S) > 227 * 1024) return false;
     if (tables_smem_bytes((u32)S, K, L) > 227 * 1024) return false;
     return true;
 }
@@ -569,16 +569,26 @@ OvArgs ov_args(const Workspace &w, const float *v, u32 n, u32 C, const float *T,
 
 // Per-chunk tables of the fast overlap recheck (templates are fixed).
 int ov_chunk_setup(const Workspace &w, const float *T, u32 K, u32 C, u32 L, u32 nmax, cudaStream_t st) {
-    const u32 S = 2 * nmax + 1;
-    k_ov_chunk_tables<<<grid_for((u64)K * S, 256), 256, 0, st>>>(T, K, C, L, nmax, w.NT, w.sNT, w.tnorm, w.oc,
-                                                                  w.tsup);
-    const u64 rows = (u64)K * K * (2 * L - 1);
-    k_ov_q_table<<<grid_for(rows, 128, 16), 128, 0, st>>>(T, K, C, L, w.Q, w.tsup);
-    const size_t xm_smem = (size_t)(2 * L - 1) * (L + 1) * 4;
-    if (xm_smem > 48 * 1024)
-        FBP_ALLOW_SMEM(k_ov_xm);
-    k_ov_xm<<<(int)std::min<u64>((u64)K * K, (u64)sm_count() * 2), 256, xm_smem, st>>>(w.Q, K, L, nmax, w.oc, w.XMr,
-                                                                                        w.XM);
+    FBP_CUDA(cudaMemsetAsync(w.oc, 0, sizeof(OvConst), st));
+    if ((size_t)L * 8 > 48 * 1024)
+        FBP_ALLOW_SMEM(k_ov_chunk_tables);
+    k_ov_chunk_tables<<<(int)std::min(K, 65535u), kChunkTabThreads, (size_t)L * 8, st>>>(T, K, C, L, nmax, w.NT, w.sNT,
+                                                                                     w.tnorm, w.oc, w.tsup);
+    k_ov_const<<<1, 1, 0, st>>>(C, L, w.oc);
+    // both templates' shared channels in shared memory: two blocks per SM
+    // where the widest support allows it, else as many channels as fit
+    auto channels = [&](size_t budget) {
+        const size_t q = pair_smem_bytes(L, 0);
+        return q >= budget ? 0u : (u32)((budget - q) / ((size_t)16 * L));
+    };
+    const u32 want = w.tc_nz;
+    u32 stage_ch = std::min(want, channels(112 * 1024));
+    if (stage_ch < want) stage_ch = std::min(want, channels(226 * 1024));
+    const size_t smem = pair_smem_bytes(L, stage_ch);
+    if (smem > 48 * 1024)
+        FBP_ALLOW_SMEM(k_ov_pairs);
+    k_ov_pairs<<<(int)std::min<u64>((u64)K * K, (u64)sm_count() * 8), kPairThreads, smem, st>>>(
+        T, K, C, L, nmax, w.tsup, stage_ch, w.oc, w.Q, w.XMr, w.XM);
     FBP_LAUNCH_CHECK();
     return FBP_OK;
 }
@@ -964,7 +974,7 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
     FBP_CUDA(cudaMemsetAsync(w.umax, 0, (size_t)W * K * 4, st));
     FBP_CUDA(cudaMemsetAsync(w.wpos, 0, (size_t)W, st));
     k_iota_windows<<<grid_for(W, 256), 256, 0, st>>>(w.win, w.active, W, w.cnt);
-    k_template_ranges<<<grid_for((u64)K * 32, 256), 256, 0, st>>>(templates, K, C, L, w.tsup);
+    k_template_ranges<<<(int)std::min(K, 65535u), 256, 0, st>>>(templates, K, C, L, w.tsup);
     k_template_support<<<1, 256, 0, st>>>(templates, K, C, L, w.tsup, w.tperm, w.grange, kLikTplPerBlock,
                                           w.grange32, kTabMGroup);
     FBP_LAUNCH_CHECK();
@@ -977,17 +987,17 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
         FBP_CUDA(cudaMemcpyAsync(tperm.data(), w.tperm, tperm.size() * 4, cudaMemcpyDeviceToHost, st));
         FBP_CUDA(cudaMemcpyAsync(gr.data(), w.grange32, gr.size() * 4, cudaMemcpyDeviceToHost, st));
         FBP_CUDA(cudaStreamSynchronize(st));
+        // the widest support: adding an exact zero product is exact (in the
+        // reference's sum and in any accumulation order), so the tensor-core
+        // rounding bounds count its products, not C*L
+        w.tc_nz = 1;
+        for (u32 t = 0; t < K; t++)
+            if (tsup[2 * t + 1] > tsup[2 * t]) w.tc_nz = std::max(w.tc_nz, tsup[2 * t + 1] - tsup[2 * t]);
         if (w.tc) {
             if (!plan_tc_groups(tsup, tperm, K, C, L, w.tc_gmax, w.tcg)) {
                 w.tc = false;                        // no group fits: the FP32 kernel
             } else {
                 w.tc_cg2max = w.tc_cmax = 0;
-                // adding an exact zero product is exact (in the reference's
-                // sum and in any accumulation order), so the rounding bounds
-                // count the widest support's products, not C*L
-                w.tc_nz = 1;
-                for (u32 t = 0; t < K; t++)
-                    if (tsup[2 * t + 1] > tsup[2 * t]) w.tc_nz = std::max(w.tc_nz, tsup[2 * t + 1] - tsup[2 * t]);
                 std::vector<u32> gdesc(3 * w.tcg.size()), tgrp(K);
                 for (u32 gi = 0; gi < (u32)w.tcg.size(); gi++) {
                     const TcGroup &g = w.tcg[gi];

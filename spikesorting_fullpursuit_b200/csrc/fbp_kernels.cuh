@@ -123,22 +123,31 @@ constexpr int kLikThreads = 128;
 // Per chunk: each template's non-zero channel range [lo, hi) (tsup), the
 // template order sorted by (lo, id) (tperm), and per group of kLikTplPerBlock
 // consecutive slots the union of their ranges (grange).  One block.
-// Non-zero channel range of each template: one warp per template.
+// Non-zero channel range of each template: one block per template, warps
+// over channels.
 __global__ void k_template_ranges(const float *__restrict__ T, u32 K, u32 C, u32 L, u32 *__restrict__ tsup) {
+    __shared__ u32 slo, shi;
     const u32 lane = threadIdx.x & 31;
-    for (u32 t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < K; t += gridDim.x * (blockDim.x >> 5)) {
+    for (u32 t = blockIdx.x; t < K; t += gridDim.x) {
+        if (threadIdx.x == 0) { slo = C; shi = 0; }
+        __syncthreads();
         u32 lo = C, hi = 0;
-        for (u32 c = 0; c < C; c++) {
+        for (u32 c = threadIdx.x >> 5; c < C; c += blockDim.x >> 5) {
             const float *tp = T + ((size_t)t * C + c) * L;
             bool nz = false;
             for (u32 i = lane; i < L; i += 32) nz |= tp[i] != 0.0f;
             if (__any_sync(0xffffffffu, nz)) { lo = min(lo, c); hi = c + 1; }
         }
-        if (hi == 0) lo = 0;                         // all-zero template: empty range
-        if (lane == 0) {
-            tsup[2 * t] = lo;
-            tsup[2 * t + 1] = hi;
+        if (lane == 0 && hi > 0) {
+            atomicMin(&slo, lo);
+            atomicMax(&shi, hi);
         }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            tsup[2 * t] = shi == 0 ? 0u : slo;       // all-zero template: empty range
+            tsup[2 * t + 1] = shi;
+        }
+        __syncthreads();
     }
 }
 

@@ -97,87 +97,71 @@ __device__ __forceinline__ float warp_max_f(float x) {
 // ---------------------------------------------------------------- per chunk
 
 // NT[t][b] = sum_c sum_{j in J(db)} T[t][c][j-db]^2 (clipped energy), sNT its
-// square root, tnorm[t] = ||t||; kappa from the number of non-zero channels.
-__global__ void k_ov_chunk_tables(const float *__restrict__ T, u32 K, u32 C, u32 L, u32 nmax,
-                                  float *__restrict__ NT, float *__restrict__ sNT,
-                                  float *__restrict__ tnorm, OvConst *oc, const u32 *__restrict__ tsup) {
-    const u32 S = 2 * nmax + 1;
-    for (u32 e = blockIdx.x * blockDim.x + threadIdx.x; e < K * S; e += gridDim.x * blockDim.x) {
-        const u32 t = e / S, b = e % S;
-        const int d = (int)b - (int)nmax;
-        const int j0 = max(0, d), j1 = min((int)L, (int)L + d);
-        double acc = 0.0;
+// square root, tnorm[t] = ||t||, and the widest count of non-zero channels.
+// One block per template: the energy of every lag over the template's
+// channels once, in shared memory, then each shift adds its own lags (a
+// thread per (template, shift) that read every channel and lag again took
+// 4.6 ms for 300 templates on 384 channels, 0.03 ms now).
+constexpr int kChunkTabThreads = 128;
+__global__ void __launch_bounds__(kChunkTabThreads)
+k_ov_chunk_tables(const float *__restrict__ T, u32 K, u32 C, u32 L, u32 nmax, float *__restrict__ NT,
+                  float *__restrict__ sNT, float *__restrict__ tnorm, OvConst *oc, const u32 *__restrict__ tsup) {
+    extern __shared__ double lag_e[];                // [L]
+    __shared__ u32 nz;
+    const u32 S = 2 * nmax + 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (u32 t = blockIdx.x; t < K; t += gridDim.x) {
         const u32 clo = tsup ? tsup[2 * t] : 0u, chi = tsup ? tsup[2 * t + 1] : C;
-        for (u32 c = clo; c < chi; c++) {
-            const float *tp = T + ((size_t)t * C + c) * L;
-            for (int j = j0; j < j1; j++) {
-                const double x = tp[j - d];
-                acc += x * x;
+        const float *tt = T + (size_t)t * C * L;
+        __syncthreads();                             // the previous template's readers are done
+        if (threadIdx.x == 0) nz = 0;
+        for (u32 m = threadIdx.x; m < L; m += blockDim.x) {
+            double e = 0.0;
+            for (u32 c = clo; c < chi; c++) {
+                const double x = tt[(size_t)c * L + m];
+                e += x * x;
             }
-        }
-        NT[e] = (float)(acc * (1.0 + 1e-6));
-        sNT[e] = (float)(sqrt(acc) * (1.0 + 1e-6));
-    }
-    if (blockIdx.x == 0) {
-        __shared__ u32 cmax;
-        if (threadIdx.x == 0) cmax = 0;
-        __syncthreads();
-        for (u32 t = threadIdx.x; t < K; t += blockDim.x) {
-            double ss = 0.0;
-            u32 nz = 0;
-            for (u32 c = 0; c < C; c++) {
-                const float *tp = T + ((size_t)t * C + c) * L;
-                bool any = false;
-                for (u32 j = 0; j < L; j++) {
-                    ss += (double)tp[j] * tp[j];
-                    any |= tp[j] != 0.0f;
-                }
-                nz += any;
-            }
-            tnorm[t] = (float)(sqrt(ss) * (1.0 + 1e-6));
-            atomicMax(&cmax, nz);
+            lag_e[m] = e;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            oc->cnz_max = cmax;
-            // gamma_n with n the reference's non-zero terms: products of two
-            // templates' channels, the per-channel subtractions and sums of
-            // squares, each product carrying two roundings
-            const double u = (double)kUnitRoundoff;
-            const double n_ref = 2.0 * cmax * L + C + 2.0 * L + 16.0;
-            const double n_mine = (double)cmax * L + 8.0;
-            oc->kappa_ref = (float)(1.05 * n_ref * u / (1.0 - n_ref * u));
-            oc->kappa_mine = (float)(1.05 * n_mine * u / (1.0 - n_mine * u));
+        for (u32 c = clo + warp; c < chi; c += blockDim.x >> 5) {
+            bool any = false;
+            for (u32 m = lane; m < L; m += 32) any |= tt[(size_t)c * L + m] != 0.0f;
+            if (__any_sync(0xffffffffu, any) && lane == 0) atomicAdd(&nz, 1u);
         }
+        for (u32 b = threadIdx.x; b <= S; b += blockDim.x) {   // b == S: the whole template
+            const int d = b < S ? (int)b - (int)nmax : 0;
+            const int m0 = max(0, -d), m1 = min((int)L, (int)L - d);
+            double acc = 0.0;
+            for (int m = m0; m < m1; m++) acc += lag_e[m];
+            if (b < S) {
+                NT[(size_t)t * S + b] = (float)(acc * (1.0 + 1e-6));
+                sNT[(size_t)t * S + b] = (float)(sqrt(acc) * (1.0 + 1e-6));
+            } else {
+                tnorm[t] = (float)(sqrt(acc) * (1.0 + 1e-6));
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) atomicMax(&oc->cnz_max, nz);
     }
 }
 
-// Q[k0][t][ri][m] = sum_{m' < m} sum_c T[k0][c][m'] * T[t][c][m'+r], r = ri-(L-1).
-// One thread per (k0, t, ri) row, accumulated in double, stored in float.
-__global__ void k_ov_q_table(const float *__restrict__ T, u32 K, u32 C, u32 L, float *__restrict__ Q,
-                             const u32 *__restrict__ tsup) {
-    const u32 R = 2 * L - 1;
-    const u64 rows = (u64)K * K * R;
-    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < rows; e += (u64)gridDim.x * blockDim.x) {
-        const u32 ri = (u32)(e % R);
-        const u32 t = (u32)((e / R) % K);
-        const u32 k0 = (u32)(e / ((u64)R * K));
-        // channels where both templates can be non-zero (tsup: [lo, hi) per template)
-        const u32 clo = tsup ? max(tsup[2 * k0], tsup[2 * t]) : 0u;
-        const u32 chi = tsup ? min(tsup[2 * k0 + 1], tsup[2 * t + 1]) : C;
-        const int r = (int)ri - (int)(L - 1);
-        float *q = Q + e * (L + 1);
-        double acc = 0.0;
-        q[0] = 0.0f;
-        for (u32 m = 0; m < L; m++) {
-            const int mt = (int)m + r;
-            if (mt >= 0 && mt < (int)L) {
-                for (u32 c = clo; c < chi; c++)
-                    acc += (double)T[((size_t)k0 * C + c) * L + m] * (double)T[((size_t)t * C + c) * L + mt];
-            }
-            q[m + 1] = (float)acc;
-        }
-    }
+// The rounding bounds from the widest template (cnz_max, k_ov_chunk_tables).
+__global__ void k_ov_const(u32 C, u32 L, OvConst *oc) {
+    // gamma_n with n the reference's non-zero terms: products of two
+    // templates' channels, the per-channel subtractions and sums of
+    // squares, each product carrying two roundings
+    const u32 cmax = oc->cnz_max;
+    const double u = (double)kUnitRoundoff;
+    const double n_ref = 2.0 * cmax * L + C + 2.0 * L + 16.0;
+    const double n_mine = (double)cmax * L + 8.0;
+    oc->kappa_ref = (float)(1.05 * n_ref * u / (1.0 - n_ref * u));
+    oc->kappa_mine = (float)(1.05 * n_mine * u / (1.0 - n_mine * u));
+}
+
+// Whether no channel lies in both templates' supports: their cross term is 0
+// for every shift, and the pair has no entry in Q and XMr.
+__device__ __forceinline__ bool ov_disjoint(const u32 *__restrict__ tsup, u32 a, u32 b) {
+    return tsup && max(tsup[2 * a], tsup[2 * b]) >= min(tsup[2 * a + 1], tsup[2 * b + 1]);
 }
 
 // ---------------------------------------------------------------- per pass
@@ -398,15 +382,13 @@ __host__ __device__ inline size_t sweep_warp_bytes(u32 S) {
 __host__ __device__ inline size_t scan_smem_bytes(u32 S) {
     return (size_t)(kScanThreads / 32) * sweep_warp_bytes(S);
 }
-// k_ov_xm stages one template pair's prefix table.
-__host__ __device__ inline size_t xm_smem_bytes(u32 L) { return (size_t)(2 * L - 1) * (L + 1) * 4; }
 __host__ __device__ inline size_t tables_smem_bytes(u32 S, u32 K, u32 L) {
     const size_t Lp = (L + 7) & ~7u, Sp = (size_t)(S + 7) / 8 * 8, Kp = (size_t)(K + 7) / 8 * 8;
     return (Sp + Lp + 8 + Lp * Kp) * 4;
 }
 constexpr int kSeedThreads = 256;
 
-// Interval of one item from its row-invariant and moving parts.
+// Cross term X of one item from the pair's prefix table.
 __device__ __forceinline__ float ov_x(const float *__restrict__ q, u32 L, int a_minus_nmax, int r) {
     float X = 0.0f;
     if (r > -(int)L && r < (int)L) {
@@ -419,15 +401,6 @@ __device__ __forceinline__ float ov_x(const float *__restrict__ q, u32 L, int a_
     }
     return X;
 }
-__device__ __forceinline__ void ov_item_bounds(const float *__restrict__ q, u32 L, int a_minus_nmax, int r,
-                                               float loA, float hiA, float loB, float hiB, float kx,
-                                               float &lo, float &hi) {
-    const float X = ov_x(q, L, a_minus_nmax, r);
-    const float ex = kx * fabsf(X);
-    hi = hiA + hiB - X + ex;
-    lo = loA + loB - X - ex;
-}
-
 // Interval of a row term: G(a) = H[k0][a] (extra = 0) or H[t][b] (extra =
 // the cross term's own rounding), with the fp16 subnormal terms of
 // tensor-core tables (sub0 / sub1 scaled by the tile's voltage exponent).
@@ -480,41 +453,95 @@ __device__ __forceinline__ float ov_krm(const OvArgs &A) {
 // Slack for the float roundings of the pruning sums (2^-18 relative).
 constexpr float kPruneSlack = 3.814697265625e-06f;
 
-// Per chunk: XMr[k0][t][r + L] = an upper bound of -X + kx|X| over every
-// shift a of an item with lag r = a - b (X = 0 where the clipped templates
-// do not overlap), and XM[k0][t] = its maximum over r.  Then
-//     hi(a, b) <= hiA(a) + hiB(b) + XMr[a - b]
-// bounds every item's interval without its cross term.
-__global__ void __launch_bounds__(256)
-k_ov_xm(const float *__restrict__ Q, u32 K, u32 L, u32 nmax, const OvConst *__restrict__ oc,
-        float *__restrict__ XMr, float *__restrict__ XM) {
-    extern __shared__ float xm_sm[];                 // Q[k0][t]: [2L-1][L+1]
+// Per chunk and template pair (k0, t) with a channel in common:
+//   Q[k0][t][ri][m] = sum_{m' < m} sum_c T[k0][c][m'] * T[t][c][m'+r], r = ri-(L-1),
+//     accumulated in double, stored in float;
+//   XMr[k0][t][r + L] = an upper bound of -X + kx|X| over every shift a of an
+//     item with lag r = a - b (X = 0 where the clipped templates do not
+//     overlap), and XM[k0][t] = its maximum over r.  Then
+//         hi(a, b) <= hiA(a) + hiB(b) + XMr[a - b]
+//     bounds every item's interval without its cross term.
+// Pairs without a common channel only get XM = 0; readers take X = 0 and
+// XMr = 0 for them (ov_disjoint).  One block per pair: the shared channels of
+// both templates in shared memory as doubles (stage_ch of them at most,
+// otherwise global reads), one thread per lag accumulating down its row of Q
+// in shared memory, the bounds from there (a warp per lag, lanes over the
+// shifts), and one coalesced copy of Q to global memory.  Bound by double
+// conversions and the accumulation; a thread per row writing Q with a stride
+// of L + 1 and a second kernel reading it back took 13.6 ms for 300 templates
+// on 384 channels (92 % of the pairs disjoint) and 1.9 ms for 64 on 16.
+constexpr int kPairThreads = 256;
+__host__ __device__ inline size_t pair_smem_bytes(u32 L, u32 stage_ch) {
+    return align_up((size_t)(2 * L - 1) * (L + 1) * 4, 8) + (size_t)2 * stage_ch * L * 8;
+}
+__global__ void __launch_bounds__(kPairThreads)
+k_ov_pairs(const float *__restrict__ T, u32 K, u32 C, u32 L, u32 nmax, const u32 *__restrict__ tsup, u32 stage_ch,
+           const OvConst *__restrict__ oc, float *__restrict__ Q, float *__restrict__ XMr, float *__restrict__ XM) {
+    extern __shared__ __align__(16) unsigned char psm[];
     const u32 R = 2 * L - 1, S = 2 * nmax + 1, NR = 2 * L + 1;
+    float *qs = (float *)psm;                        // [R][L+1]
+    double *sk = (double *)(psm + align_up((size_t)R * (L + 1) * 4, 8)), *st = sk + (size_t)stage_ch * L;
     const float kx = 2.0f * oc->kappa_ref + 4.0f * kUnitRoundoff;
-    __shared__ float red[8];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+    __shared__ float red[kPairThreads / 32];
     for (u32 pair = blockIdx.x; pair < K * K; pair += gridDim.x) {
-        const float *qg = Q + (size_t)pair * R * (L + 1);
+        const u32 k0 = pair / K, t = pair % K;
+        const u32 clo = tsup ? max(tsup[2 * k0], tsup[2 * t]) : 0u;
+        const u32 chi = tsup ? min(tsup[2 * k0 + 1], tsup[2 * t + 1]) : C;
+        if (clo >= chi) {
+            if (threadIdx.x == 0) XM[pair] = 0.0f;
+            continue;
+        }
+        const u32 nch = chi - clo;
+        const bool staged = nch <= stage_ch;
+        const float *ta = T + ((size_t)k0 * C + clo) * L, *tb = T + ((size_t)t * C + clo) * L;
+        __syncthreads();                             // the previous pair's readers are done
+        if (staged) {
+            for (u32 e = threadIdx.x; e < nch * L; e += blockDim.x) {
+                sk[e] = (double)ta[e];
+                st[e] = (double)tb[e];
+            }
+        }
         __syncthreads();
-        for (u32 e = threadIdx.x; e < R * (L + 1); e += blockDim.x) xm_sm[e] = qg[e];
+        for (u32 ri = threadIdx.x; ri < R; ri += blockDim.x) {
+            const int r = (int)ri - (int)(L - 1);
+            float *q = qs + (size_t)ri * (L + 1);
+            double acc = 0.0;
+            q[0] = 0.0f;
+            for (u32 m = 0; m < L; m++) {
+                const int mt = (int)m + r;
+                if (mt >= 0 && mt < (int)L) {
+                    if (staged) {
+                        for (u32 c = 0; c < nch; c++) acc += sk[c * L + m] * st[c * L + mt];
+                    } else {
+                        for (u32 c = 0; c < nch; c++)
+                            acc += (double)__ldg(ta + (size_t)c * L + m) * (double)__ldg(tb + (size_t)c * L + mt);
+                    }
+                }
+                q[m + 1] = (float)acc;
+            }
+        }
         __syncthreads();
         float pm = -INFINITY;
-        for (u32 ri = threadIdx.x; ri < NR; ri += blockDim.x) {
+        for (u32 ri = warp; ri < NR; ri += nwarp) {
             const int r = (int)ri - (int)L;
             float m = -INFINITY;
-            for (u32 a = 0; a < S; a++) {
-                const float X = ov_x(xm_sm, L, (int)a - (int)nmax, r);
+            for (u32 a = lane; a < S; a += 32) {
+                const float X = ov_x(qs, L, (int)a - (int)nmax, r);
                 m = fmaxf(m, -X + kx * fabsf(X));
             }
+            m = warp_max_f(m);
             m += kPruneSlack * fabsf(m);
-            XMr[(size_t)pair * NR + ri] = m;
+            if (lane == 0) XMr[(size_t)pair * NR + ri] = m;
             pm = fmaxf(pm, m);
         }
-        pm = warp_max_f(pm);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = pm;
+        if (lane == 0) red[warp] = pm;
+        float *qg = Q + (size_t)pair * R * (L + 1);
+        for (u32 e = threadIdx.x; e < R * (L + 1); e += blockDim.x) qg[e] = qs[e];
         __syncthreads();
         if (threadIdx.x == 0) {
             float v = red[0];
-            for (u32 w = 1; w < blockDim.x / 32; w++) v = fmaxf(v, red[w]);
+            for (u32 w = 1; w < nwarp; w++) v = fmaxf(v, red[w]);
             XM[pair] = v;
         }
     }
@@ -636,7 +663,8 @@ k_ov_seed(OvArgs A) {
                 const bool sp = !(A.Lk[(size_t)t * n + c.bidx + b - nmax] <= 0.0f);
                 if (fp || sp) {                          // .cl:572-576
                     const float *q = A.Q + ((size_t)c.k0 * K + t) * R * (L + 1);
-                    const float X = ov_x(q, L, (int)a - (int)nmax, (int)a - (int)b);
+                    const float X = ov_disjoint(A.tsup, c.k0, t) ? 0.0f
+                                                                 : ov_x(q, L, (int)a - (int)nmax, (int)a - (int)b);
                     seed = lb_a + lb_b - X - kx * fabsf(X);
                 }
             }
@@ -745,6 +773,7 @@ k_ov_scan(OvArgs A) {
         __syncwarp();
         const float *xmr = A.XMr + pair * NR;
         const float *q = A.Q + pair * R * (L + 1);
+        const bool apart = ov_disjoint(A.tsup, c.k0, t);   // no cross term, no table
         const u32 P = na * nb;
         float lbmax = -INFINITY;
         // pair p = ai * nb + bi; each lane steps its (ai, bi) by 32 pairs
@@ -763,7 +792,7 @@ k_ov_scan(OvArgs A) {
                 valid = (a > b ? a - b : b - a) <= L &&                                    // .cl:543-556
                         (((abits[a >> 5] >> (a & 31)) | (bbits[b >> 5] >> (b & 31))) & 1u);  // .cl:572-576
                 if (valid) {
-                    const float xr = __ldg(xmr + (int)a - (int)b + (int)L);
+                    const float xr = apart ? 0.0f : __ldg(xmr + (int)a - (int)b + (int)L);
                     valid = ga_hi[a] + hb_hi[b] + xr + slack + kPruneSlack * fabsf(xr) >= TH;
                 }
             }
@@ -772,8 +801,10 @@ k_ov_scan(OvArgs A) {
             if (bi >= nb) { bi -= nb; ai++; }
             float lo = -INFINITY, hi = -INFINITY;
             if (valid) {
-                ov_item_bounds(q, L, (int)a - (int)nmax, (int)a - (int)b, ga_lo[a], ga_hi[a], hb_lo[b], hb_hi[b],
-                               kx, lo, hi);
+                const float X = apart ? 0.0f : ov_x(q, L, (int)a - (int)nmax, (int)a - (int)b);
+                const float ex = kx * fabsf(X);
+                hi = ga_hi[a] + hb_hi[b] - X + ex;
+                lo = ga_lo[a] + hb_lo[b] - X - ex;
                 evaluated++;
             }
             lbmax = fmaxf(lbmax, lo);
