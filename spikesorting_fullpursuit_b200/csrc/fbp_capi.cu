@@ -143,7 +143,6 @@ struct Workspace {
     u32 *pool_slot, *pool_item, *fb_slots, *fb_list;
     u64 *best_key;
     u32 pool_cap;
-    float *ua;
     int *kexp_tile;
     u32 stiles;
     // tensor-core likelihood (present when `tc`)
@@ -364,7 +363,6 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
         w.pool_hi = (float *)take((size_t)w.pool_cap * 4);
         w.fb_slots = (u32 *)take(sl * 4);
         w.fb_list = (u32 *)take(sl * 4);
-        w.ua = (float *)take(sl * 4);
         w.stiles = (S + kTcM - 1) / kTcM;
         w.kexp_tile = (int *)take(sl * w.stiles * 4 * (want_tc ? std::max(1u, ceil_div(K, 16)) : 1u));
     }
@@ -553,7 +551,6 @@ OvArgs ov_args(const Workspace &w, const float *v, u32 n, u32 C, const float *T,
     A.best_key = w.best_key; A.fallback = w.fallback;
     A.items_evaluated = &cnt->ov_items;
     A.pool_total = &cnt->pool_total;
-    A.ua = w.ua;
     A.lazy = lazy_ctx(w, v, T, tss, C, L, 0);   // read only: the tag is not used
     if (w.tc) {                      // H from the tensor cores
         A.km_override = tc_kappa(w.tc_nz, L, ceil_div(w.tc_nz, 8));
@@ -633,13 +630,16 @@ int ov_fast_tables(const Workspace &w, const OvArgs &A, Counters *cnt, cudaStrea
 int ov_fast_pass(const Workspace &w, const OvArgs &A, Counters *cnt, cudaStream_t st, int *launches) {
     const u32 slots = w.slots;
     const u32 S = A.S;
-    k_ov_rows<<<grid_for((u64)slots * 32, kSeedThreads, 8), kSeedThreads, 0, st>>>(A);
+    const size_t rows_smem = rows_smem_bytes(A.L);
+    if (rows_smem > 48 * 1024)
+        FBP_ALLOW_SMEM(k_ov_rows);
+    k_ov_rows<<<grid_for((u64)slots * kRowsThreads, kRowsThreads, 12), kRowsThreads, rows_smem, st>>>(A);
     k_ov_seed<<<grid_for((u64)slots * A.K * 32, kSeedThreads, 8), kSeedThreads, 0, st>>>(A);
     const size_t scan_smem = scan_smem_bytes(S);
     if (scan_smem > 48 * 1024)
         FBP_ALLOW_SMEM(k_ov_scan);
     k_ov_scan<<<grid_for((u64)slots * A.K * 32, kScanThreads, 8), kScanThreads, scan_smem, st>>>(A);
-    k_ov_refine<<<(int)sm_count() * 16, kRefineThreads, 0, st>>>(A);
+    k_ov_refine<<<(int)sm_count() * 4, kRefineThreads, ov_refine_smem_bytes(), st>>>(A);   // four blocks fit an SM
     k_ov_finalize<<<grid_for((u64)slots * 32, kRefineThreads, 8), kRefineThreads, 0, st>>>(A);
     FBP_LAUNCH_CHECK();
     int rc = compact(w.fallback, slots, w.fb_slots, &cnt->fb_count, w.tile_counts, st);

@@ -38,6 +38,7 @@ constexpr float kUnitRoundoff = 5.9604644775390625e-08f;   // 2^-24
 struct OvConst {
     float kappa_ref;      // bound of the reference's rounding, per unit of sum|terms|
     float kappa_mine;     // bound of this approximation's rounding
+    float kappa_rows;     // bound of the rounding of the best template's own rows (k_ov_rows)
     u32 cnz_max;          // max non-zero channels of a template
 };
 
@@ -55,7 +56,7 @@ struct OvArgs {
     float *best_ll;
     u8 *ovr;
     float *H;                        // [slot][K][S]
-    float *vn;                       // [slot]
+    float *vn;                       // [slot]     ||window|| over all channels (FP32 path)
     u8 *cskip;                       // [slot]
     float *cand_lb;                  // [slot]     largest lower bound of an item (atomic max, >= 0)
     float *ga_lo, *ga_hi;            // [slot][S]  interval of G(a) = H[k0][a]
@@ -84,7 +85,6 @@ struct OvArgs {
     const u32 *tgrp;                 // [K] template group of the tensor-core tables (NULL: one group)
     u32 kt_slots;                    // slots per group in kexp_tile
     u32 stiles;
-    float *ua;                       // [slot] ||window||_1
     LazyLk lazy;                     // approximate likelihood entries (tensor-core path)
 };
 
@@ -156,6 +156,7 @@ __global__ void k_ov_const(u32 C, u32 L, OvConst *oc) {
     const double n_mine = (double)cmax * L + 8.0;
     oc->kappa_ref = (float)(1.05 * n_ref * u / (1.0 - n_ref * u));
     oc->kappa_mine = (float)(1.05 * n_mine * u / (1.0 - n_mine * u));
+    oc->kappa_rows = (float)(1.05 * ((double)L + cmax + 8.0) * u);   // a channel's lags, then the channels
 }
 
 // Whether no channel lies in both templates' supports: their cross term is 0
@@ -166,33 +167,32 @@ __device__ __forceinline__ bool ov_disjoint(const u32 *__restrict__ tsup, u32 a,
 
 // ---------------------------------------------------------------- per pass
 
-// One warp per candidate slot: skip rules of .cl:518-527, window energy,
-// label histogram.
+// Skip rules of .cl:518-527 and the per-candidate state.  The norms of the
+// candidate's window come from the tensor-core likelihood, per template group
+// (ov_window_norms); the FP32 path, which keeps none, sums the window over all
+// channels (one warp per candidate).
 __global__ void k_ov_prep(OvArgs A) {
     const u32 nc = *A.n_cand;
-    const u32 lane = threadIdx.x & 31;
-    for (u32 g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < nc;
-         g += gridDim.x * (blockDim.x >> 5)) {
+    const bool sum = A.lazy.wn == nullptr;
+    const u32 lane = sum ? threadIdx.x & 31 : 0u, per = sum ? 32u : 1u;
+    for (u32 g = (blockIdx.x * blockDim.x + threadIdx.x) / per; g < nc; g += gridDim.x * blockDim.x / per) {
         const u32 id = A.cand[g];
         const u32 lab = A.best_lab[id], bidx = A.best_idx[id];
         const float bll = A.Lk[(size_t)lab * A.n + bidx];
         const bool skip = (bll < A.thr[lab]) || (bidx >= A.n - A.L);
-        double e = 0.0, e1 = 0.0;
-        if (!skip)
-            for (u32 q = lane; q < A.C * A.L; q += 32) {
-                const double x = A.v[(size_t)(q / A.L) * A.n + bidx + q % A.L];
-                e += x * x;
-                e1 += fabs(x);
-            }
+        if (sum) {
+            double e = 0.0;
+            if (!skip)
+                for (u32 q = lane; q < A.C * A.L; q += 32) {
+                    const double x = A.v[(size_t)(q / A.L) * A.n + bidx + q % A.L];
+                    e += x * x;
+                }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            e += __shfl_xor_sync(0xffffffffu, e, o);
-            e1 += __shfl_xor_sync(0xffffffffu, e1, o);
+            for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+            if (lane == 0) A.vn[g] = (float)(sqrt(e) * (1.0 + 1e-6));
         }
         if (lane == 0) {
             A.cskip[g] = skip;
-            A.vn[g] = (float)(sqrt(e) * (1.0 + 1e-6));
-            if (A.ua) A.ua[g] = (float)(e1 * (1.0 + 1e-6));
             A.best_key[g] = 0ull;
             A.cand_lb[g] = 0.0f;
         }
@@ -401,19 +401,51 @@ __device__ __forceinline__ float ov_x(const float *__restrict__ q, u32 L, int a_
     }
     return X;
 }
-// Interval of a row term: G(a) = H[k0][a] (extra = 0) or H[t][b] (extra =
-// the cross term's own rounding), with the fp16 subnormal terms of
-// tensor-core tables (sub0 / sub1 scaled by the tile's voltage exponent).
-__device__ __forceinline__ void ov_row_interval(const OvArgs &A, u32 g, u32 tmpl, u32 x, float Hv, float nt,
-                                                float snt, float vn, float krm, float extra, float sub0, float sub1,
+// L2 (and, for tensor-core tables, L1) norm of a candidate's window over
+// channels that hold template t's support: the likelihood's own norms of the
+// sample the window starts at, over t's template group (written this pass: a
+// candidate's window is listed), or the FP32 path's over all channels.  On
+// the 384-channel probe the group's norm is about a third of the whole.
+__device__ __forceinline__ void ov_window_norms(const OvArgs &A, u32 g, u32 bidx, u32 t, float &l2, float &l1) {
+    if (A.lazy.wn) {
+        const size_t i = (A.lazy.tgrp ? (size_t)A.lazy.tgrp[t] * A.lazy.gstride : 0) + bidx;
+        l2 = A.lazy.wn[i];
+        l1 = A.lazy.wa[i];
+    } else {
+        l2 = A.vn[g];
+        l1 = 0.0f;
+    }
+}
+
+// Interval of a row term H[t][b], the rounding of the cross term (eqt)
+// included, with the fp16 subnormal terms of tensor-core tables (sub0 / sub1
+// scaled by the tile's voltage exponent).
+struct OvRowB {
+    float vn, krm, eqt, sub0, sub1;
+};
+__device__ __forceinline__ OvRowB ov_row_b(const OvArgs &A, u32 g, u32 bidx, u32 k0, u32 t, float krm) {
+    OvRowB r;
+    float l1;
+    ov_window_norms(A, g, bidx, t, r.vn, l1);
+    r.krm = krm;
+    r.eqt = 4.0f * kUnitRoundoff * A.tnorm[k0] * A.tnorm[t];
+    r.sub0 = r.sub1 = 0.0f;
+    if (A.kexp_tile) {
+        r.sub1 = 2.98023224e-08f * 1.001f * ldexpf(l1, -A.texp[t]);
+        r.sub0 = 2.98023224e-08f * 1.001f * A.tabs[t];
+    }
+    return r;
+}
+__device__ __forceinline__ void ov_row_interval(const OvArgs &A, u32 g, u32 tmpl, u32 x, float Hv, const OvRowB &r,
                                                 float &lo, float &hi) {
+    const float nt = A.NT[(size_t)tmpl * A.S + x], snt = A.sNT[(size_t)tmpl * A.S + x];
     float sx = 0.0f;
     if (A.kexp_tile) {
         // scale exponent of the table tile: per template group, candidate, tile of 128 shifts
         const size_t grp = A.tgrp ? (size_t)A.tgrp[tmpl] * A.kt_slots : 0;
-        sx = sub0 * ldexpf(1.0f, -A.kexp_tile[(grp + g) * A.stiles + x / 128]) + sub1;
+        sx = r.sub0 * ldexpf(1.0f, -A.kexp_tile[(grp + g) * A.stiles + x / 128]) + r.sub1;
     }
-    const float e = krm * (snt * vn + nt) + 4.0f * kUnitRoundoff * fabsf(Hv) + extra + sx;
+    const float e = r.krm * (snt * r.vn + nt) + 4.0f * kUnitRoundoff * fabsf(Hv) + r.eqt + sx;
     lo = Hv - e;
     hi = Hv + e;
 }
@@ -421,7 +453,7 @@ __device__ __forceinline__ void ov_row_interval(const OvArgs &A, u32 g, u32 tmpl
 // Per-candidate constants of the row intervals.
 struct OvCand {
     u32 id, k0, bidx, xlo, xhi_ex;
-    float lbest, vn, subA0, subA1;
+    float lbest;
 };
 __device__ __forceinline__ OvCand ov_cand(const OvArgs &A, u32 g) {
     OvCand c;
@@ -429,22 +461,9 @@ __device__ __forceinline__ OvCand ov_cand(const OvArgs &A, u32 g) {
     c.k0 = A.best_lab[c.id];
     c.bidx = A.best_idx[c.id];
     c.lbest = A.best_ll[c.id];
-    c.vn = A.vn[g];
     c.xlo = c.bidx >= A.nmax ? 0u : A.nmax - c.bidx;          // in-bounds shifts (.cl:534-541)
     c.xhi_ex = A.n - A.L + A.nmax - c.bidx;                    // first out-of-bounds shift
-    c.subA0 = c.subA1 = 0.0f;
-    if (A.kexp_tile) {
-        c.subA1 = 2.98023224e-08f * 1.001f * ldexpf(A.ua[g], -A.texp[c.k0]);
-        c.subA0 = 2.98023224e-08f * 1.001f * A.tabs[c.k0];
-    }
     return c;
-}
-__device__ __forceinline__ void ov_sub_b(const OvArgs &A, u32 g, u32 t, float &subB0, float &subB1) {
-    subB0 = subB1 = 0.0f;
-    if (A.kexp_tile) {
-        subB1 = 2.98023224e-08f * 1.001f * ldexpf(A.ua[g], -A.texp[t]);
-        subB0 = 2.98023224e-08f * 1.001f * A.tabs[t];
-    }
 }
 __device__ __forceinline__ float ov_kx(const OvArgs &A) { return 2.0f * A.oc->kappa_ref + 4.0f * kUnitRoundoff; }
 __device__ __forceinline__ float ov_krm(const OvArgs &A) {
@@ -557,49 +576,129 @@ __device__ __forceinline__ void warp_argmax(float &v, u32 &i) {
     }
 }
 
-// Rows a of each candidate (one warp per candidate): the intervals of
-// G(a) = H[k0][a], the L[k0][afix] > 0 bits, the largest in-bounds upper
+// Rows a of each candidate (one block per candidate): G(a) = H[k0][a] in
+// FP32, the intervals, the L[k0][afix] > 0 bits, the largest in-bounds upper
 // bound and |upper bound|, and the row of largest lower bound (a1), for the
-// seed and the scan.
-__global__ void __launch_bounds__(kSeedThreads)
+// seed and the scan.  Every item of a candidate carries the error of its row
+// a, and the best template's rows have the largest: from the 16-bit tables it
+// was several times the reference's own rounding, and items whose second
+// template is nearly clipped away (b near the ends) could not be told apart
+// -- 566 contenders per candidate on 17 channels with 23 templates.  Warps
+// take the template's channels in turn; a lane holds 8 consecutive shifts and
+// 8 lags of the window at a time, so 64 FMAs take four 16-byte shared reads.
+// Channels are summed apart and then together: the rounding is that of
+// L + channels terms.
+constexpr int kRowsThreads = 128, kRowsWarps = kRowsThreads / 32;
+constexpr u32 kRowsShifts = 256;                 // shifts of a block's pass (8 per lane)
+__host__ __device__ inline u32 rows_warp_floats(u32 L) {
+    const u32 Lp = (L + 7) & ~7u;
+    return kRowsShifts + Lp + 8 + Lp;            // window strip, template row
+}
+__host__ __device__ inline size_t rows_smem_bytes(u32 L) {
+    return (size_t)kRowsWarps * (rows_warp_floats(L) + kRowsShifts) * 4;
+}
+__global__ void __launch_bounds__(kRowsThreads)
 k_ov_rows(OvArgs A) {
+    extern __shared__ __align__(16) float rsm_rows[];
+    __shared__ float red_v[kRowsWarps], red_m[kRowsWarps], red_abs[kRowsWarps];
+    __shared__ u32 red_i[kRowsWarps];
     const u32 nc = *A.n_cand;
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const u32 S = A.S, n = A.n, nmax = A.nmax, NB = (S + 31) / 32;
-    const float krm = ov_krm(A);
-    for (u32 g = blockIdx.x * (kSeedThreads / 32) + warp; g < nc; g += gridDim.x * (kSeedThreads / 32)) {
+    const u32 S = A.S, n = A.n, nmax = A.nmax, L = A.L, Lp = (L + 7) & ~7u, NB = (S + 31) / 32;
+    float *strip = rsm_rows + (size_t)warp * rows_warp_floats(L), *trow = strip + kRowsShifts + Lp + 8;
+    float *part = rsm_rows + (size_t)kRowsWarps * rows_warp_floats(L);   // [warp][kRowsShifts]
+    const float ka = A.oc->kappa_ref + A.oc->kappa_rows;
+    for (u32 g = blockIdx.x; g < nc; g += gridDim.x) {
         if (A.cskip[g]) continue;
         const OvCand c = ov_cand(A, g);
-        const float *Hg = A.H + ((size_t)g * A.K + c.k0) * S;
+        float vn, l1;
+        ov_window_norms(A, g, c.bidx, c.k0, vn, l1);
+        const u32 clo = A.tsup ? A.tsup[2 * c.k0] : 0u, chi = A.tsup ? A.tsup[2 * c.k0 + 1] : A.C;
         float va = -INFINITY, mA = -INFINITY, mabs = 0.0f;
         u32 a1 = 0;
-        for (u32 x0 = 0; x0 < S; x0 += 32) {
-            const u32 x = x0 + lane;
-            bool ap = false;
-            if (x < S) {
-                float lo, hi;
-                ov_row_interval(A, g, c.k0, x, Hg[x], A.NT[(size_t)c.k0 * S + x], A.sNT[(size_t)c.k0 * S + x], c.vn,
-                                krm, 0.0f, c.subA0, c.subA1, lo, hi);
-                A.ga_lo[(size_t)g * S + x] = lo;
-                A.ga_hi[(size_t)g * S + x] = hi;
-                if (x >= c.xlo && x < c.xhi_ex) {
-                    ap = !(A.Lk[(size_t)c.k0 * n + c.bidx + x - nmax] <= 0.0f);
-                    if (lo > va) { va = lo; a1 = x; }
-                    mA = fmaxf(mA, hi);
-                    mabs = fmaxf(mabs, fabsf(hi));
+        for (u32 x0 = 0; x0 < S; x0 += kRowsShifts) {
+            float tot[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) tot[i] = 0.0f;
+            for (u32 ch = clo + warp; ch < chi; ch += kRowsWarps) {
+                __syncwarp();
+                // strip[x]: the window at lag x0 + x - n_max (zero outside [0, L))
+                const float *v = A.v + (size_t)ch * n + c.bidx;
+                for (u32 x = lane; x < kRowsShifts + Lp + 8; x += 32) {
+                    const int rel = (int)(x0 + x) - (int)nmax;
+                    strip[x] = (rel >= 0 && rel < (int)L) ? __ldg(v + rel) : 0.0f;
                 }
+                const float *tp = A.T + ((size_t)c.k0 * A.C + ch) * L;
+                for (u32 m = lane; m < Lp; m += 32) trow[m] = m < L ? __ldg(tp + m) : 0.0f;
+                __syncwarp();
+                float acc[8], w[16];
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[i] = 0.0f;
+                if (x0 + 8 * lane < S) {
+                    const float *sp = strip + 8 * lane;
+                    *reinterpret_cast<float4 *>(w) = *reinterpret_cast<const float4 *>(sp);
+                    *reinterpret_cast<float4 *>(w + 4) = *reinterpret_cast<const float4 *>(sp + 4);
+                    for (u32 m = 0; m < Lp; m += 8) {
+                        float t[8];
+                        *reinterpret_cast<float4 *>(w + 8) = *reinterpret_cast<const float4 *>(sp + m + 8);
+                        *reinterpret_cast<float4 *>(w + 12) = *reinterpret_cast<const float4 *>(sp + m + 12);
+                        *reinterpret_cast<float4 *>(t) = *reinterpret_cast<const float4 *>(trow + m);
+                        *reinterpret_cast<float4 *>(t + 4) = *reinterpret_cast<const float4 *>(trow + m + 4);
+#pragma unroll
+                        for (int mm = 0; mm < 8; mm++)
+#pragma unroll
+                            for (int i = 0; i < 8; i++) acc[i] = fmaf(t[mm], w[i + mm], acc[i]);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) w[i] = w[i + 8];
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++) tot[i] += acc[i];
             }
-            const u32 m = __ballot_sync(0xffffffffu, ap);
-            if (lane == 0) A.ga_bits[(size_t)g * NB + x0 / 32] = m;
+            __syncthreads();                         // the previous shifts' readers of part are done
+#pragma unroll
+            for (int i = 0; i < 8; i++) part[warp * kRowsShifts + 8 * lane + i] = tot[i];
+            __syncthreads();
+            for (u32 y = 32 * warp; y < kRowsShifts && x0 + y < S; y += kRowsThreads) {
+                const u32 x = x0 + y + lane;
+                bool ap = false;
+                if (x < S) {
+                    float h = 0.0f;
+#pragma unroll
+                    for (int w8 = 0; w8 < kRowsWarps; w8++) h += part[w8 * kRowsShifts + y + lane];
+                    const float nt = A.NT[(size_t)c.k0 * S + x], snt = A.sNT[(size_t)c.k0 * S + x];
+                    h -= 0.5f * nt;
+                    const float e = ka * (snt * vn + nt) + 4.0f * kUnitRoundoff * fabsf(h);
+                    const float lo = h - e, hi = h + e;
+                    A.ga_lo[(size_t)g * S + x] = lo;
+                    A.ga_hi[(size_t)g * S + x] = hi;
+                    if (x >= c.xlo && x < c.xhi_ex) {
+                        ap = !(A.Lk[(size_t)c.k0 * n + c.bidx + x - nmax] <= 0.0f);
+                        if (lo > va) { va = lo; a1 = x; }
+                        mA = fmaxf(mA, hi);
+                        mabs = fmaxf(mabs, fabsf(hi));
+                    }
+                }
+                const u32 m = __ballot_sync(0xffffffffu, ap);
+                if (lane == 0) A.ga_bits[(size_t)g * NB + (x0 + y) / 32] = m;
+            }
         }
         warp_argmax(va, a1);
         mA = warp_max_f(mA);
         mabs = warp_max_f(mabs);
-        if (lane == 0) {
+        if (lane == 0) { red_v[warp] = va; red_i[warp] = a1; red_m[warp] = mA; red_abs[warp] = mabs; }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w8 = 1; w8 < kRowsWarps; w8++) {
+                if (red_v[w8] > va || (red_v[w8] == va && red_i[w8] < a1)) { va = red_v[w8]; a1 = red_i[w8]; }
+                mA = fmaxf(mA, red_m[w8]);
+                mabs = fmaxf(mabs, red_abs[w8]);
+            }
             A.ga_max[g] = mA;
             A.ga_abs[g] = mabs;
             A.seed_a1[g] = a1;
         }
+        __syncthreads();                             // red_* are read before the next candidate writes them
     }
 }
 
@@ -625,16 +724,13 @@ k_ov_seed(OvArgs A) {
         const float *ga_lo = A.ga_lo + (size_t)g * S;
         const float va = ga_lo[a1];
         const float *Hg = A.H + ((size_t)g * K + t) * S;
-        float subB0, subB1;
-        ov_sub_b(A, g, t, subB0, subB1);
-        const float eqt = 4.0f * kUnitRoundoff * A.tnorm[c.k0] * A.tnorm[t];
+        const OvRowB rb = ov_row_b(A, g, c.bidx, c.k0, t, krm);
         const u32 xend = min(S, c.xhi_ex);
         float v1 = -INFINITY, v2 = -INFINITY, mB = -INFINITY, mabs = 0.0f;
         u32 b1 = 0, b2 = 0;
         for (u32 x = c.xlo + lane; x < xend; x += 32) {
             float lo, hi;
-            ov_row_interval(A, g, t, x, Hg[x], A.NT[(size_t)t * S + x], A.sNT[(size_t)t * S + x], c.vn, krm, eqt,
-                            subB0, subB1, lo, hi);
+            ov_row_interval(A, g, t, x, Hg[x], rb, lo, hi);
             if (lo > v1) { v1 = lo; b1 = x; }
             if ((x > a1 ? x - a1 : a1 - x) <= L && lo > v2) { v2 = lo; b2 = x; }
             mB = fmaxf(mB, hi);
@@ -725,9 +821,7 @@ k_ov_scan(OvArgs A) {
             if (!(mA + mB0 + XM + slack0 >= TH)) continue;
         }
         const float *Hg = A.H + ((size_t)g * K + t) * S;
-        float subB0, subB1;
-        ov_sub_b(A, g, t, subB0, subB1);
-        const float eqt = 4.0f * kUnitRoundoff * A.tnorm[c.k0] * A.tnorm[t];
+        const OvRowB rb = ov_row_b(A, g, c.bidx, c.k0, t, krm);
         // rows b: intervals and the L[t][ashift] > 0 bits; rows a: copied
         float mB = -INFINITY, mabs = A.ga_abs[g];
         for (u32 x0 = 0; x0 < S; x0 += 32) {
@@ -737,8 +831,7 @@ k_ov_scan(OvArgs A) {
                 ga_lo[x] = A.ga_lo[(size_t)g * S + x];
                 ga_hi[x] = A.ga_hi[(size_t)g * S + x];
                 float lo, hi;
-                ov_row_interval(A, g, t, x, Hg[x], A.NT[(size_t)t * S + x], A.sNT[(size_t)t * S + x], c.vn, krm, eqt,
-                                subB0, subB1, lo, hi);
+                ov_row_interval(A, g, t, x, Hg[x], rb, lo, hi);
                 hb_lo[x] = lo;
                 hb_hi[x] = hi;
                 if (x >= c.xlo && x < c.xhi_ex) {
@@ -899,25 +992,177 @@ __device__ float overlap_item_exact_global(const OvArgs &A, u32 lab, u32 bidx, u
 }
 
 constexpr int kRefineThreads = 256;
+constexpr u32 kRefRows = 16;             // product rows (chunks of 32 lags) a warp stages at once
+constexpr u32 kRefWarpMax = 24576;       // pool entries up to which a warp shares the terms of its contenders
+constexpr u32 kRefStride = 33;           // row stride: lanes walk 32 rows without bank conflicts
+struct RefItem {                         // one contender, in shared memory
+    u32 lab, t, bidx, r0, n1, r2, nch, e;
+    int fa, sa;
+};
+__host__ __device__ inline size_t ov_refine_smem_bytes() {
+    return (size_t)(kRefineThreads / 32) * (2 * kRefRows * kRefStride * 4 + kRefRows * sizeof(RefItem)) +
+           2 * kRefineThreads * 4;
+}
 
 // Exact values of the pooled contenders whose upper bound reaches their
-// candidate's final lower bound, one thread each (the sums are sequential,
-// so many items in flight hide them best); each candidate keeps the largest
-// value above its current best, lowest item id on ties (the parse kernel's
-// strict-greater scan over single-item groups, .cl:699-706).
+// candidate's final lower bound (overlap_recheck_indices, .cl:583-646), each
+// by the reference's own sequence of operations; each candidate keeps the
+// largest value above its current best, lowest item id on ties (the parse
+// kernel's strict-greater scan over single-item groups, .cl:699-706).
+//
+// An item is two float chains (the likelihood and the channel's sum of
+// squares) over channels x lags that must be added in order, of terms that
+// are independent.  With many contenders one thread each hides its loads
+// behind the others'.  With few (most passes: the last contenders of a
+// recording take as many passes as the first) nothing hides them: 276 us a
+// pass on the 384-channel probe however few contenders there were.  Up to
+// kRefWarpMax pool entries a block therefore gathers the contenders still in
+// question, and a warp takes up to 16 of them: its lanes form the terms of 32
+// lags of one channel of one contender at a time (coalesced loads, each
+// product rounded as in the reference) into a row of shared memory, then lane
+// i adds contender i's rows in order; few contenders get several rows each, so
+// that they wait for global memory once per eight rows (48 us a pass).  That
+// costs 84 instructions per 32 terms against about 22 of a thread's: the line
+// lies where both take about 250 us (17 channels x 77 lags).
 __global__ void __launch_bounds__(kRefineThreads)
 k_ov_refine(OvArgs A) {
+    extern __shared__ float refsm[];
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *pr = refsm + (size_t)warp * 2 * kRefRows * kRefStride;    // sum * voltage
+    float *qr = pr + kRefRows * kRefStride;                          // sum * sum
+    RefItem *items = (RefItem *)(refsm + (size_t)(kRefineThreads / 32) * 2 * kRefRows * kRefStride) + kRefRows * warp;
+    const u32 L = A.L, C = A.C, K = A.K, S = A.S;
     const u32 m = min(*A.pool_total, A.pool_cap);
-    for (u32 e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
-        const u32 g = A.pool_slot[e];
-        if (A.fallback[g]) continue;
-        if (A.pool_hi[e] < A.cand_lb[g]) continue;      // below another item's lower bound
-        atomicAdd(A.refined, 1u);
-        const u32 it = A.pool_item[e];
-        const u32 id = A.cand[g];
-        const u32 t = it % A.K, a = (it / A.K) % A.S, b = it / (A.K * A.S);
-        const float ll = overlap_item_exact_global(A, A.best_lab[id], A.best_idx[id], t, a, b);
-        if (ll > A.best_ll[id]) atomicMax(&A.best_key[g], ov_pack(ll, it));
+    if (m > kRefWarpMax) {
+        for (u32 e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
+            const u32 g = A.pool_slot[e];
+            if (A.fallback[g] || A.pool_hi[e] < A.cand_lb[g]) continue;   // below another item's lower bound
+            atomicAdd(A.refined, 1u);
+            const u32 it = A.pool_item[e], id = A.cand[g];
+            const float ll = overlap_item_exact_global(A, A.best_lab[id], A.best_idx[id], it % K, (it / K) % S,
+                                                       it / (K * S));
+            if (ll > A.best_ll[id]) atomicMax(&A.best_key[g], ov_pack(ll, it));
+        }
+        return;
+    }
+    u32 *list = (u32 *)((RefItem *)(refsm + (size_t)(kRefineThreads / 32) * 2 * kRefRows * kRefStride) +
+                        kRefRows * (kRefineThreads / 32));
+    __shared__ u32 cnt;
+    const u32 part = (m + gridDim.x - 1) / gridDim.x;
+    const u32 e0 = min(m, part * blockIdx.x), e1 = min(m, e0 + part);
+    const u32 ncl = (L + 31) / 32;                   // rows of a channel
+    if (threadIdx.x == 0) cnt = 0;
+    __syncthreads();
+    for (u32 eb = e0; eb < e1; eb += kRefineThreads) {
+      const u32 e = eb + threadIdx.x;
+      if (e < e1) {
+          const u32 g = A.pool_slot[e];
+          // the others lie below another item's lower bound
+          if (!A.fallback[g] && !(A.pool_hi[e] < A.cand_lb[g])) list[atomicAdd(&cnt, 1u)] = e;
+      }
+      __syncthreads();
+      const u32 held = cnt;                          // < 2 * kRefineThreads
+      if (held < kRefineThreads && eb + kRefineThreads < e1) continue;   // gather more
+      if (threadIdx.x == 0 && held) atomicAdd(A.refined, held);
+      const u32 per = min(kRefRows, max(1u, (held + kRefineThreads / 32 - 1) / (kRefineThreads / 32)));
+      for (u32 base = warp * per; base < held; base += (kRefineThreads / 32) * per) {
+        const u32 nact = min(per, held - base);
+        const bool act = lane < nact;
+        u32 nq = 0;                                  // this lane's contender: rows
+        if (act) {
+            RefItem it;
+            it.e = list[base + lane];
+            const u32 id = A.cand[A.pool_slot[it.e]], item = A.pool_item[it.e];
+            it.lab = A.best_lab[id];
+            it.bidx = A.best_idx[id];
+            it.t = item % K;
+            it.fa = (int)A.nmax - (int)((item / K) % S);
+            it.sa = (int)A.nmax - (int)(item / (K * S));
+            // channels where either template is non-zero, in channel order: the
+            // two supports as one range when they meet, else one after the other
+            // (elsewhere both terms are 0 and the reference's sums do not change)
+            it.r0 = 0; it.n1 = C; it.r2 = C; it.nch = C;
+            if (A.tsup) {
+                u32 al = A.tsup[2 * it.lab], ah = A.tsup[2 * it.lab + 1], bl = A.tsup[2 * it.t], bh = A.tsup[2 * it.t + 1];
+                if (ah <= al) { al = bl; ah = bh; }
+                if (bh <= bl) { bl = al; bh = ah; }
+                if (bl < al) { u32 x = al; al = bl; bl = x; x = ah; ah = bh; bh = x; }
+                it.r0 = al;
+                if (bl <= ah) { it.n1 = max(ah, bh) - al; it.r2 = al + it.n1; it.nch = it.n1; }
+                else { it.n1 = ah - al; it.r2 = bl; it.nch = it.n1 + (bh - bl); }
+            }
+            nq = it.nch * ncl;
+            items[lane] = it;
+        }
+        u32 nqmax = nq;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) nqmax = max(nqmax, __shfl_xor_sync(0xffffffffu, nqmax, o));
+        __syncwarp();
+        const u32 sh = nact <= 2 ? 3u : nact <= 4 ? 2u : nact <= 8 ? 1u : 0u;   // log2(rows of a contender per stage)
+        const u32 nrows = nact << sh;
+        float cml = 0.0f, ss = 0.0f;
+        for (u32 q0 = 0; q0 < nqmax; q0 += 1u << sh) {
+            const u32 my_ci = (q0 + (lane & 7u)) / ncl;              // channel and chunk of row q0 + (lane & 7)
+            const u32 my_lc = (q0 + (lane & 7u)) - my_ci * ncl;
+            for (u32 rb = 0; rb < nrows; rb += 8) {
+                float fv[8], sv[8], wv[8];
+#pragma unroll
+                for (u32 u = 0; u < 8; u++) {
+                    const u32 r = rb + u, k = r & ((1u << sh) - 1u);
+                    const u32 ci = __shfl_sync(0xffffffffu, my_ci, k), j = __shfl_sync(0xffffffffu, my_lc, k) * 32 + lane;
+                    fv[u] = sv[u] = wv[u] = 0.0f;
+                    const RefItem &it = items[min(r >> sh, nact - 1)];
+                    if (r < nrows && ci < it.nch && j < L) {
+                        const u32 c = ci < it.n1 ? it.r0 + ci : it.r2 + (ci - it.n1);
+                        const int jf = it.fa + (int)j, js = it.sa + (int)j;
+                        if (jf >= 0 && jf < (int)L) fv[u] = __ldg(A.T + ((size_t)it.lab * C + c) * L + jf);
+                        if (js >= 0 && js < (int)L) sv[u] = __ldg(A.T + ((size_t)it.t * C + c) * L + js);
+                        wv[u] = __ldg(A.v + (size_t)c * A.n + it.bidx + j);
+                    }
+                }
+#pragma unroll
+                for (u32 u = 0; u < 8; u++) {
+                    if (rb + u >= nrows) break;      // uniform in the warp
+                    const float sum = __fadd_rn(fv[u], sv[u]);
+                    pr[(rb + u) * kRefStride + lane] = __fmul_rn(sum, wv[u]);
+                    qr[(rb + u) * kRefStride + lane] = __fmul_rn(sum, sum);
+                }
+            }
+            __syncwarp();
+            for (u32 k = 0; k < (1u << sh); k++) {
+                const u32 lc = __shfl_sync(0xffffffffu, my_lc, k);
+                if (q0 + k < nq) {
+                    const float *p = pr + ((lane << sh) + k) * kRefStride, *q = qr + ((lane << sh) + k) * kRefStride;
+                    const u32 cnt = min(32u, L - lc * 32);
+                    u32 j = 0;
+                    for (; j + 8 <= cnt; j += 8) {
+#pragma unroll
+                        for (u32 x = 0; x < 8; x++) {
+                            ss = __fadd_rn(ss, q[j + x]);
+                            cml = __fadd_rn(cml, p[j + x]);
+                        }
+                    }
+                    for (; j < cnt; j++) {
+                        ss = __fadd_rn(ss, q[j]);
+                        cml = __fadd_rn(cml, p[j]);
+                    }
+                    if (lc == ncl - 1) {             // the channel's last lag (.cl:627-630)
+                        if ((double)ss > 0.0) cml = __double2float_rn(__dsub_rn((double)cml, __dmul_rn(0.5, (double)ss)));
+                        ss = 0.0f;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        if (lane < nact) {
+            const u32 pe = items[lane].e, pg = A.pool_slot[pe];
+            if (cml > A.best_ll[A.cand[pg]]) atomicMax(&A.best_key[pg], ov_pack(cml, A.pool_item[pe]));
+        }
+        __syncwarp();
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) cnt = 0;
+      __syncthreads();
     }
 }
 
