@@ -18,6 +18,7 @@
 #include "fbp_overlap_fast.cuh"
 #include "fbp_lik_tc.cuh"
 #include "fbp_lik_tcw.cuh"
+#include "fbp_ov_tcw.cuh"
 
 using namespace fbp;
 
@@ -134,6 +135,10 @@ struct Workspace {
     float *NT, *sNT, *tnorm, *Q, *XMr, *XM, *H, *vn, *cand_lb, *ga_lo, *ga_hi, *ga_max, *ga_abs, *pool_hi;
     u32 *ga_bits, *seed_a1;
     float *pair_mb, *pair_mabs;
+    u16 *pair_b1;                    // wide overlap tables: rows of the pairs' largest lower bounds
+    uint4 *slot_tab;                 //                      candidates of a pass
+    bool ovw = false;                // this chunk's overlap tables use k_ov_tcw
+    OvtPlan ovt;
     Counters *snap;                  // counts of the last pass
     u32 *tsup, *tperm, *grange;      // template channel supports, order, group ranges
     u32 *grange32;                   // group ranges of 32 slots (masked overlap tables)
@@ -354,7 +359,11 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
         w.ga_abs = (float *)take(sl * 4);
         w.seed_a1 = (u32 *)take(sl * 4);
         w.pair_mb = (float *)take(sl * K * 4);
-        w.pair_mabs = (float *)take(sl * K * 4);
+        w.pair_mabs = (float *)take(sl * K * 4);     // with wide tables: the largest lower bounds
+        if (want_tc) {
+            w.pair_b1 = (u16 *)take(sl * K * 2);
+            w.slot_tab = (uint4 *)take(sl * sizeof(uint4));
+        }
         w.cand_lb = (float *)take(sl * 4);
         w.best_key = (u64 *)take(sl * 8);
         w.pool_cap = (u32)std::min<u64>(0x7fffffffull, std::max<u64>(1u << 22, (u64)sl * 128));
@@ -543,7 +552,11 @@ OvArgs ov_args(const Workspace &w, const float *v, u32 n, u32 C, const float *T,
     A.cand_lb = w.cand_lb;
     A.ga_lo = w.ga_lo; A.ga_hi = w.ga_hi; A.ga_bits = w.ga_bits; A.ga_max = w.ga_max; A.ga_abs = w.ga_abs;
     A.seed_a1 = w.seed_a1;
-    A.pair_mb = w.pair_mb; A.pair_mabs = w.pair_mabs;
+    A.pair_mb = w.pair_mb; A.pair_mabs = w.ovw ? nullptr : w.pair_mabs;
+    if (w.ovw) {
+        A.pair_v1 = w.pair_mabs; A.pair_b1 = w.pair_b1;
+        A.slot_tab = w.slot_tab; A.vwmax = w.vwmax;
+    }
     A.tsup = w.tsup;
     A.pool_slot = w.pool_slot; A.pool_item = w.pool_item; A.pool_hi = w.pool_hi; A.pool_cap = w.pool_cap;
     A.refined = &cnt->ov_ref;
@@ -558,7 +571,7 @@ OvArgs ov_args(const Workspace &w, const float *v, u32 n, u32 C, const float *T,
         A.kt_slots = w.slots;
         A.tabs = w.tc_tabs;
         A.texp = w.tc_texp;
-        A.kexp_tile = w.kexp_tile;
+        A.kexp_tile = w.ovw ? nullptr : w.kexp_tile;
         A.stiles = w.stiles;
     }
     return A;
@@ -601,7 +614,18 @@ int ov_fast_tables(const Workspace &w, const OvArgs &A, Counters *cnt, cudaStrea
     FBP_CUDA(cudaMemsetAsync(&cnt->scan_next, 0, 8, st));
     k_ov_prep<<<grid_for((u64)slots * 32, 256), 256, 0, st>>>(A);
     FBP_LAUNCH_CHECK();
-    if (w.tc) {
+    if (w.ovw) {
+        FBP_ALLOW_SMEM(k_ov_tcw);
+        OvtArgs P{};
+        P.o = A;
+        P.groups = w.tcw_args; P.ngroups = (u32)w.tcwg.size();
+        P.ncol = w.ovt.ncol; P.spt = w.ovt.spt; P.N = w.ovt.N; P.ns = w.ovt.ns; P.px = w.ovt.px;
+        P.stage = (u32)w.ovt.stage;
+        P.err = &cnt->tc_err;
+        P.wait_polls = g_lim_wait.load();
+        k_ov_tcw<<<sm_count(), kTcThreads, w.ovt.smem, st>>>(P);
+        FBP_LAUNCH_CHECK();
+    } else if (w.tc) {
         FBP_ALLOW_SMEM(k_lik_tc<1>);
         const u32 G = (u32)w.tcg.size();
         k_lik_tc<1><<<std::max<u32>(sm_count(), G), kTcThreads, w.tc_smem, st>>>(w.tc_args1, G);
@@ -634,7 +658,10 @@ int ov_fast_pass(const Workspace &w, const OvArgs &A, Counters *cnt, cudaStream_
     if (rows_smem > 48 * 1024)
         FBP_ALLOW_SMEM(k_ov_rows);
     k_ov_rows<<<grid_for((u64)slots * kRowsThreads, kRowsThreads, 12), kRowsThreads, rows_smem, st>>>(A);
-    k_ov_seed<<<grid_for((u64)slots * A.K * 32, kSeedThreads, 8), kSeedThreads, 0, st>>>(A);
+    if (w.ovw)
+        k_ov_seed_pairs<<<grid_for((u64)slots * A.K, kSeedThreads, 8), kSeedThreads, 0, st>>>(A);
+    else
+        k_ov_seed<<<grid_for((u64)slots * A.K * 32, kSeedThreads, 8), kSeedThreads, 0, st>>>(A);
     const size_t scan_smem = scan_smem_bytes(S);
     if (scan_smem > 48 * 1024)
         FBP_ALLOW_SMEM(k_ov_scan);
@@ -1015,6 +1042,10 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
                     // the stream table marks tail outputs in bit 31 of a sample
                     w.tcw = w.tcw_ns > 0 && n < 0x80000000u;
                 }
+                // the overlap tables' layout: wide tiles beside a wide likelihood
+                // (its norms are per wide group) where a candidate's shifts fit a tile
+                w.ovt = ovt_plan(L, nmax);
+                w.ovw = w.tcw && w.fast && do_overlap_recheck && w.ovt.spt > 0;
                 std::vector<u32> gdesc_w(3 * w.tcwg.size()), tgrp_w(K);
                 if (w.tcw) {
                     for (u32 gi = 0; gi < (u32)w.tcwg.size(); gi++) {

@@ -65,7 +65,13 @@ struct OvArgs {
     unsigned long long *scan_next;   // next (candidate, template) pair of the scan
     u32 *seed_a1;                    // [slot]     in-bounds row a of largest lower bound
     float *pair_mb, *pair_mabs;      // [slot][K]  per (candidate, template): largest in-bounds upper
-                                     //            bound of a row b and of its magnitude (from the seed)
+                                     //            bound of a row b and of its magnitude (from the seed;
+                                     //            NULL with k_ov_tcw's tables, which keep the first)
+    float *pair_v1;                  // [slot][K]  k_ov_tcw: largest lower bound of an in-bounds row b
+    u16 *pair_b1;                    // [slot][K]  and its row
+    uint4 *slot_tab;                 // [slot]     k_ov_tcw: window start (~0: skipped), fp16 scale exponent,
+                                     //            ||k0|| (float bits)
+    const float *vwmax;              // [W + 2]    bound on |v| of each window (k_ov_tcw's scale)
     const u32 *tsup;                 // [K][2] non-zero channel range of each template (may be NULL)
     u32 *pool_total;                 // appended entries this pass
     u32 pool_cap;
@@ -81,7 +87,7 @@ struct OvArgs {
     float km_override;               // > 0: bound of the tensor-core tables
     const float *tabs;               // [K] ||t||_1
     const int *texp;                 // [K] template scale exponents
-    const int *kexp_tile;            // [group][slot][stiles] window scale exponents
+    const int *kexp_tile;            // [group][slot][stiles] window scale exponents of k_lik_tc<1>'s tables
     const u32 *tgrp;                 // [K] template group of the tensor-core tables (NULL: one group)
     u32 kt_slots;                    // slots per group in kexp_tile
     u32 stiles;
@@ -195,6 +201,17 @@ __global__ void k_ov_prep(OvArgs A) {
             A.cskip[g] = skip;
             A.best_key[g] = 0ull;
             A.cand_lb[g] = 0.0f;
+            if (A.slot_tab) {
+                // the window's samples lie in its recording window and the next
+                const float mm = fmaxf(A.vwmax[id], A.vwmax[id + 1]);
+                int kexp = 0;
+                if (mm > 0.0f) {
+                    int e;
+                    frexpf(mm, &e);                  // mm < 2^e
+                    kexp = max(-126, min(126, 14 - e));      // scaled magnitudes < 2^14
+                }
+                A.slot_tab[g] = make_uint4(skip ? 0xffffffffu : bidx, (u32)kexp, __float_as_uint(A.tnorm[lab]), 0u);
+            }
         }
     }
 }
@@ -430,20 +447,21 @@ __device__ __forceinline__ OvRowB ov_row_b(const OvArgs &A, u32 g, u32 bidx, u32
     r.krm = krm;
     r.eqt = 4.0f * kUnitRoundoff * A.tnorm[k0] * A.tnorm[t];
     r.sub0 = r.sub1 = 0.0f;
-    if (A.kexp_tile) {
+    if (A.texp) {
         r.sub1 = 2.98023224e-08f * 1.001f * ldexpf(l1, -A.texp[t]);
         r.sub0 = 2.98023224e-08f * 1.001f * A.tabs[t];
+        if (A.slot_tab) r.sub1 += ldexpf(r.sub0, -(int)A.slot_tab[g].y);   // one scale per candidate
     }
     return r;
 }
 __device__ __forceinline__ void ov_row_interval(const OvArgs &A, u32 g, u32 tmpl, u32 x, float Hv, const OvRowB &r,
                                                 float &lo, float &hi) {
     const float nt = A.NT[(size_t)tmpl * A.S + x], snt = A.sNT[(size_t)tmpl * A.S + x];
-    float sx = 0.0f;
+    float sx = r.sub1;
     if (A.kexp_tile) {
         // scale exponent of the table tile: per template group, candidate, tile of 128 shifts
         const size_t grp = A.tgrp ? (size_t)A.tgrp[tmpl] * A.kt_slots : 0;
-        sx = r.sub0 * ldexpf(1.0f, -A.kexp_tile[(grp + g) * A.stiles + x / 128]) + r.sub1;
+        sx += r.sub0 * ldexpf(1.0f, -A.kexp_tile[(grp + g) * A.stiles + x / 128]);
     }
     const float e = r.krm * (snt * r.vn + nt) + 4.0f * kUnitRoundoff * fabsf(Hv) + r.eqt + sx;
     lo = Hv - e;
@@ -812,16 +830,18 @@ k_ov_scan(OvArgs A) {
         const float TH = fmaxf(LB, c.lbest);
         const size_t pair = (size_t)c.k0 * K + t;
         const float XM = A.XM[pair];
+        const OvRowB rb = ov_row_b(A, g, c.bidx, c.k0, t, krm);
         {
             // the pair test below with the seed's row maxima (the same values
             // the row pass computes): a pair that fails it needs no row pass
             const float mB0 = A.pair_mb[e];
-            const float mabs0 = fmaxf(A.ga_abs[g], A.pair_mabs[e]);
+            // without the stored magnitude, a bound: |H| + its error is below 1.02 (||t|| ||window|| + ||t||^2)
+            const float mabs0 = fmaxf(A.ga_abs[g], A.pair_mabs ? A.pair_mabs[e]
+                                                               : 1.02f * A.tnorm[t] * (rb.vn + A.tnorm[t]) + rb.eqt + rb.sub1);
             const float slack0 = kPruneSlack * (2.0f * mabs0 + fabsf(TH) + fabsf(XM));
             if (!(mA + mB0 + XM + slack0 >= TH)) continue;
         }
         const float *Hg = A.H + ((size_t)g * K + t) * S;
-        const OvRowB rb = ov_row_b(A, g, c.bidx, c.k0, t, krm);
         // rows b: intervals and the L[t][ashift] > 0 bits; rows a: copied
         float mB = -INFINITY, mabs = A.ga_abs[g];
         for (u32 x0 = 0; x0 < S; x0 += 32) {
