@@ -132,7 +132,7 @@ struct Workspace {
     // fast overlap recheck (present when `fast`)
     bool fast;
     u32 slots;
-    float *NT, *sNT, *tnorm, *Q, *XMr, *XM, *H, *vn, *cand_lb, *ga_lo, *ga_hi, *ga_max, *ga_abs, *pool_hi;
+    float *NT, *sNT, *tnorm, *Q, *XMr, *XMw, *XM, *H, *vn, *cand_lb, *ga_lo, *ga_hi, *ga_max, *ga_abs, *pool_hi;
     u32 *ga_bits, *seed_a1;
     float *pair_mb, *pair_mabs;
     u16 *pair_b1;                    // wide overlap tables: rows of the pairs' largest lower bounds
@@ -347,6 +347,7 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
         w.tnorm = (float *)take((size_t)K * 4);
         w.Q = (float *)take((size_t)K * K * (2 * L - 1) * (L + 1) * 4);
         w.XMr = (float *)take((size_t)K * K * (2 * L + 1) * 4);
+        w.XMw = (float *)take((size_t)K * K * (2 * L + 32) * 4);
         w.XM = (float *)take((size_t)K * K * 4);
         w.H = (float *)take(sl * K * S * 4);
         w.vn = (float *)take(sl * 4);
@@ -544,7 +545,7 @@ OvArgs ov_args(const Workspace &w, const float *v, u32 n, u32 C, const float *T,
     OvArgs A{};
     A.n = n; A.C = C; A.K = K; A.L = L; A.nmax = nmax; A.S = 2 * nmax + 1;
     A.v = v; A.T = T; A.Lk = Lk; A.thr = thr;
-    A.NT = w.NT; A.sNT = w.sNT; A.tnorm = w.tnorm; A.Q = w.Q; A.XMr = w.XMr; A.XM = w.XM; A.oc = w.oc;
+    A.NT = w.NT; A.sNT = w.sNT; A.tnorm = w.tnorm; A.Q = w.Q; A.XMr = w.XMr; A.XMw = w.XMw; A.XM = w.XM; A.oc = w.oc;
     A.cand = cand; A.n_cand = n_cand;
     A.best_idx = s.best_idx; A.best_lab = s.best_lab; A.ov_idx = s.ov_idx; A.ov_lab = s.ov_lab;
     A.best_ll = s.best_ll; A.ovr = s.overlap_recheck;
@@ -598,7 +599,7 @@ int ov_chunk_setup(const Workspace &w, const float *T, u32 K, u32 C, u32 L, u32 
     if (smem > 48 * 1024)
         FBP_ALLOW_SMEM(k_ov_pairs);
     k_ov_pairs<<<(int)std::min<u64>((u64)K * K, (u64)sm_count() * 8), kPairThreads, smem, st>>>(
-        T, K, C, L, nmax, w.tsup, stage_ch, w.oc, w.Q, w.XMr, w.XM);
+        T, K, C, L, nmax, w.tsup, stage_ch, w.oc, w.Q, w.XMr, w.XMw, w.XM);
     FBP_LAUNCH_CHECK();
     return FBP_OK;
 }
@@ -623,7 +624,7 @@ int ov_fast_tables(const Workspace &w, const OvArgs &A, Counters *cnt, cudaStrea
         P.stage = (u32)w.ovt.stage;
         P.err = &cnt->tc_err;
         P.wait_polls = g_lim_wait.load();
-        k_ov_tcw<<<sm_count(), kTcThreads, w.ovt.smem, st>>>(P);
+        k_ov_tcw<<<sm_count(), kOvtThreads, w.ovt.smem, st>>>(P);
         FBP_LAUNCH_CHECK();
     } else if (w.tc) {
         FBP_ALLOW_SMEM(k_lik_tc<1>);

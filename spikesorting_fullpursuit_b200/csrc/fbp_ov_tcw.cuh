@@ -8,10 +8,10 @@
 // slot, zeros elsewhere, so position b of a slot is shift b and no other
 // candidate's sample is within its lags (ST >= max(2 n_max + 1, n_max + L)).
 //
-// Persistent, one CTA per SM, 17 warps.  An item is (tile of spt candidates,
+// Persistent, one CTA per SM, 16 warps.  An item is (tile of spt candidates,
 // template group); consecutive items are the groups of one tile, so that
 // concurrent CTAs read the same windows.  Producer warps take whole channels
-// in turn, one warp per ring stage (at most 8): the channel's samples come by coalesced 4-byte loads (16
+// in turn, one warp per ring stage (at most 7): the channel's samples come by coalesced 4-byte loads (16
 // in flight per lane, issued before the wait for a free ring stage), are
 // scaled by their candidate's power of two and written as fp16 into the stage
 // beside the template tiles, which one bulk copy brings.  No barrier joins the
@@ -32,6 +32,10 @@
 
 namespace fbp {
 
+// Sixteen warps (four to a scheduler, so that a thread may hold 128 registers).
+constexpr int kOvtProdWarps = 7, kOvtMmaWarp = kOvtProdWarps, kOvtEpiWarp0 = 8, kOvtEpiWarps = 8;
+constexpr int kOvtThreads = 512, kOvtProdThreads = 32 * kOvtProdWarps;
+
 // Slots of a tile: columns per slot, slots, MMA N, staged positions.
 struct OvtPlan {
     u32 ncol, spt, N, px, ns;
@@ -50,7 +54,7 @@ __host__ __device__ inline OvtPlan ovt_plan(u32 L, u32 nmax) {
     p.px = 8 * p.N + 16 * tcw_nkc(L);
     p.stage = align_up((size_t)tcw_nkc(L) * kWATile + align_up((size_t)p.px * 2, 16), 128);
     const size_t tail = 1024;                        // barriers, fill counts, flags
-    for (p.ns = kTcProdWarps; p.ns >= 2; p.ns--)     // a stage for each producer warp at most
+    for (p.ns = kOvtProdWarps; p.ns >= 2; p.ns--)     // a stage for each producer warp at most
         if (p.ns * p.stage + tail <= 227 * 1024) break;
     if (p.ns < 2) p.spt = 0;
     p.smem = p.ns * p.stage + tail;
@@ -66,11 +70,14 @@ struct OvtArgs {
     u32 wait_polls;
 };
 
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(kOvtThreads, 1)
 k_ov_tcw(const __grid_constant__ OvtArgs P) {
     const OvArgs &A = P.o;
     const u32 nc = *A.n_cand;
-    const u32 G = P.ngroups, spt = P.spt, ns = P.ns;
+    // with few candidates, fewer to a tile: every CTA gets an item
+    const u32 G = P.ngroups, ns = P.ns;
+    const u32 spt = (u32)min((u64)P.spt, max((u64)1, ((u64)nc * G + gridDim.x - 1) / gridDim.x));
+    const u32 N = min(P.N, ((spt - 1) * P.ncol + (P.ncol + 7) / 8 * 8 + 15) / 16 * 16);
     const u64 nitems = (u64)((nc + spt - 1) / spt) * G;
     if ((u64)blockIdx.x >= nitems) return;           // no item for this CTA: no set-up at all
     extern __shared__ __align__(128) unsigned char osm[];
@@ -94,7 +101,7 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
         }
         for (u32 b = 0; b < 2; b++) {
             mbar_init(bar_afull(b), 1);
-            mbar_init(bar_aempty(b), kTcEpiWarps);
+            mbar_init(bar_aempty(b), kOvtEpiWarps);
         }
         mbar_init(bar_fin, 1);
         *abort_flag = 0;
@@ -116,7 +123,7 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const u32 tmem = *tmem_slot;
 
-    if (warp < kTcProdWarps) {
+    if (warp < kOvtProdWarps) {
         // =========================== producers ===========================
         const u32 ncl = (L + 31) / 32;               // loads of a slot's channel per lane
         u32 gs0 = 0;                                 // ring uses before this item
@@ -185,14 +192,14 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
         }
         // every copy into the ring has landed before the CTA exits (a warp
         // that issued one has also arrived)
-        named_bar(1, kTcProdThreads);
+        named_bar(1, kOvtProdThreads);
         if (tid == 0) {
             for (u32 s = 0; s < ns; s++)
                 if (fills[s] > 0) mbar_wait_bounded(bar_sfull(s), (fills[s] - 1) & 1u, kTcDrainPolls);
         }
-    } else if (warp == kTcMmaWarp) {
+    } else if (warp == kOvtMmaWarp) {
         // =========================== MMA issue ===========================
-        const u32 idesc = (1u << 4) | ((P.N >> 3) << 17) | ((u32)(kTcM >> 4) << 24);
+        const u32 idesc = (1u << 4) | ((N >> 3) << 17) | ((u32)(kTcM >> 4) << 24);
         const u64 a0 = umma_desc(smem_u32(osm), kWATile / 2, 128);        // K halves 2048 B apart
         const u64 b0 = umma_desc(smem_u32(osm) + a_bytes, 16, 128);       // rows 8 positions apart
         const u64 sstep = (u64)(P.stage >> 4);
@@ -247,7 +254,7 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
         __syncwarp();
     } else {
         // =========================== epilogue ===========================
-        const u32 ew_ = warp - kTcEpiWarp0;          // 0..7
+        const u32 ew_ = warp - kOvtEpiWarp0;         // 0..7
         const u32 quad = warp & 3u;                  // TMEM lanes [32 quad, 32 quad + 32)
         const u32 half = ew_ >> 2;                   // slots half, half + 2, ...
         const u32 row = quad * 32 + lane, tl = row >> 3, d = row & 7u;
@@ -261,7 +268,20 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
             const u32 gt = real ? T.trow[tl] : 0u;
             const int texp_t = A.texp[gt];
             const float tn = A.tnorm[gt], tab = A.tabs[gt];
-            const float *NTt = A.NT + (size_t)gt * S, *sNTt = A.sNT + (size_t)gt * S;
+            // clipped norms of the template at this lane's shifts, the same for
+            // every slot (the clipped energy is their square: its rounding is
+            // far inside the tables' bound); 32 columns in registers
+            const float *sNTt = A.sNT + (size_t)gt * S;
+            auto norms = [&](u32 c0, float (&sn)[8]) {
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const u32 x = 8 * (c0 + q) + d;
+                    sn[q] = (x < S && real) ? __ldg(sNTt + x) : 0.0f;
+                }
+            };
+            float snt[4][8];
+#pragma unroll
+            for (int q = 0; q < 4; q++) norms(8 * q, snt[q]);
             // lane k: slot k's candidate, its window norms over this group's channels
             uint4 sl = make_uint4(0xffffffffu, 0u, 0u, 0u);
             float wn = 0.0f, wa = 0.0f;
@@ -299,30 +319,31 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
                 float *Hg = A.H + ((size_t)g * K + gt) * S;
                 float mb = -INFINITY, v1 = -INFINITY;
                 u32 b1 = 0;
-                for (u32 c0 = 0; c0 < P.ncol; c0 += 8) {
+                auto chunk = [&](u32 c0, const float (&sn)[8]) {
                     u32 r[8];
-                    float nt[8], snt[8];
                     __syncwarp();
                     tmem_ld<8>(r, acc0 + k * P.ncol + c0);
 #pragma unroll
                     for (int q = 0; q < 8; q++) {
                         const u32 x = 8 * (c0 + q) + d;
-                        nt[q] = snt[q] = 0.0f;
-                        if (x < S && real) { nt[q] = __ldg(NTt + x); snt[q] = __ldg(sNTt + x); }
-                    }
-#pragma unroll
-                    for (int q = 0; q < 8; q++) {
-                        const u32 x = 8 * (c0 + q) + d;
                         if (x >= S || !real || c0 + q >= P.ncol) continue;
-                        const float a = __uint_as_float(r[q]);
-                        const float h = (plain ? __fmul_rn(a, sc) : ldexpf(a, ex)) - 0.5f * nt[q];
+                        const float a = __uint_as_float(r[q]), nt = sn[q] * sn[q];
+                        const float h = (plain ? __fmul_rn(a, sc) : ldexpf(a, ex)) - 0.5f * nt;
                         Hg[x] = h;
-                        const float e = krm * (snt[q] * vn + nt[q]) + 4.0f * kUnitRoundoff * fabsf(h) + cst;
+                        const float e = krm * (sn[q] * vn + nt) + 4.0f * kUnitRoundoff * fabsf(h) + cst;
                         if (x >= xlo && x < xhi) {
                             mb = fmaxf(mb, h + e);
                             if (h - e > v1) { v1 = h - e; b1 = x; }
                         }
                     }
+                };
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (8u * q < P.ncol) chunk(8 * q, snt[q]);
+                for (u32 c0 = 32; c0 < P.ncol; c0 += 8) {
+                    float sn[8];
+                    norms(c0, sn);
+                    chunk(c0, sn);
                 }
 #pragma unroll
                 for (int o = 1; o < 8; o <<= 1) {            // the template's 8 sample shifts

@@ -49,6 +49,7 @@ struct OvArgs {
     const float *NT, *sNT, *tnorm;   // [K][S], [K][S], [K]
     const float *Q;                  // [K][K][2L-1][L+1]
     const float *XMr;                // [K][K][2L+1] upper bound of -X + kx|X| per lag r = a - b
+    const float *XMw;                // [K][K][2L+32] XMr's largest value over the 32 lags from i - L - 31
     const float *XM;                 // [K][K]       its largest value over the lags
     const OvConst *oc;
     const u32 *cand, *n_cand;
@@ -390,11 +391,11 @@ k_ov_tables_m(OvArgs A, const u32 *__restrict__ tperm, const u32 *__restrict__ t
 }
 
 constexpr int kScanThreads = 256;
-// Per-warp scratch of the scan: ga_lo, ga_hi, hb_lo, hb_hi (S floats each),
-// the a and b row lists (S u16 each), and the bitmasks of rows a with
-// L[k0][afix] not <= 0 and rows b with L[t][ashift] not <= 0 (S bits each).
+// Per-warp scratch of the scan: hb_lo, hb_hi (S floats each), and per block
+// of 32 rows b the bits of rows with L[t][ashift] not <= 0 and the largest
+// upper bound.
 __host__ __device__ inline size_t sweep_warp_bytes(u32 S) {
-    return align_up((size_t)20 * S + (size_t)(S + 31) / 32 * 8, 16);
+    return align_up((size_t)8 * S + (size_t)(S + 31) / 32 * 8, 16);
 }
 __host__ __device__ inline size_t scan_smem_bytes(u32 S) {
     return (size_t)(kScanThreads / 32) * sweep_warp_bytes(S);
@@ -497,7 +498,9 @@ constexpr float kPruneSlack = 3.814697265625e-06f;
 //     item with lag r = a - b (X = 0 where the clipped templates do not
 //     overlap), and XM[k0][t] = its maximum over r.  Then
 //         hi(a, b) <= hiA(a) + hiB(b) + XMr[a - b]
-//     bounds every item's interval without its cross term.
+//     bounds every item's interval without its cross term;
+//   XMw[k0][t][i] = the maximum of XMr over the lags i - L - 31 .. i - L, for the
+//     32 rows b of a block against one row a.
 // Pairs without a common channel only get XM = 0; readers take X = 0 and
 // XMr = 0 for them (ov_disjoint).  One block per pair: the shared channels of
 // both templates in shared memory as doubles (stage_ch of them at most,
@@ -513,7 +516,8 @@ __host__ __device__ inline size_t pair_smem_bytes(u32 L, u32 stage_ch) {
 }
 __global__ void __launch_bounds__(kPairThreads)
 k_ov_pairs(const float *__restrict__ T, u32 K, u32 C, u32 L, u32 nmax, const u32 *__restrict__ tsup, u32 stage_ch,
-           const OvConst *__restrict__ oc, float *__restrict__ Q, float *__restrict__ XMr, float *__restrict__ XM) {
+           const OvConst *__restrict__ oc, float *__restrict__ Q, float *XMr, float *__restrict__ XMw,
+           float *__restrict__ XM) {
     extern __shared__ __align__(16) unsigned char psm[];
     const u32 R = 2 * L - 1, S = 2 * nmax + 1, NR = 2 * L + 1;
     float *qs = (float *)psm;                        // [R][L+1]
@@ -573,6 +577,12 @@ k_ov_pairs(const float *__restrict__ T, u32 K, u32 C, u32 L, u32 nmax, const u32
             pm = fmaxf(pm, m);
         }
         if (lane == 0) red[warp] = pm;
+        __syncthreads();
+        for (u32 i = threadIdx.x; i < 2 * L + 32; i += blockDim.x) {
+            float m = -INFINITY;                     // XMr index of lag r: r + L
+            for (int q = max(0, (int)i - 31); q <= min((int)i, (int)(NR - 1)); q++) m = fmaxf(m, XMr[(size_t)pair * NR + q]);
+            XMw[(size_t)pair * (2 * L + 32) + i] = m;
+        }
         float *qg = Q + (size_t)pair * R * (L + 1);
         for (u32 e = threadIdx.x; e < R * (L + 1); e += blockDim.x) qg[e] = qs[e];
         __syncthreads();
@@ -792,156 +802,172 @@ k_ov_seed(OvArgs A) {
 // evaluates (.cl:534-576) either gets its interval here or is shown to have
 // hi < TH, TH = max(best lower bound so far, current best likelihood):
 //   - the whole pair is skipped when max hiA + max hiB + XM < TH;
-//   - rows a / b whose bound with the other side's maximum is below TH drop;
-//   - of the remaining pairs, those that pass the skip rules and
-//     hiA + hiB + XMr[a-b] >= TH get their interval from the prefix table.
+//   - a row a against a block of 32 rows b is skipped when
+//     hiA + max hiB of the block + XMw of its lags < TH (lanes over the rows a);
+//   - of a row and a block that remain, lanes over the rows b, the items that
+//     pass the skip rules and hiA + hiB + XMr[a-b] >= TH get their interval
+//     from the prefix table.
 // An item that is never enumerated can neither be the best item (whose value
 // is >= every lower bound) nor beat the current best.  Items with
 // hi >= TH and hi > current best go to the contender pool with their hi;
-// their lower bounds raise the candidate's best lower bound.
+// their lower bounds raise the candidate's best lower bound, and TH with it
+// after every block (the block of largest upper bound goes first).  Testing
+// rows against blocks leaves about 50 warp steps of a pair with 201 shifts;
+// lists of single rows a and b were crossed pair by pair, up to 1,250 steps.
 __global__ void __launch_bounds__(kScanThreads)
 k_ov_scan(OvArgs A) {
     extern __shared__ float sm[];
     const u32 S = A.S, K = A.K, L = A.L, nmax = A.nmax, n = A.n;
-    const u32 R = 2 * L - 1, NR = 2 * L + 1, NB = (S + 31) / 32;
+    const u32 R = 2 * L - 1, NR = 2 * L + 1, NW = 2 * L + 32, NB = (S + 31) / 32;
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float *ga_lo = (float *)((char *)sm + (size_t)warp * sweep_warp_bytes(S));
-    float *ga_hi = ga_lo + S, *hb_lo = ga_hi + S, *hb_hi = hb_lo + S;
-    u16 *alist = (u16 *)(hb_hi + S);
-    u16 *blist = alist + S;
-    u32 *abits = (u32 *)((char *)ga_lo + (size_t)20 * S);
-    u32 *bbits = abits + NB;
+    float *hb_lo = (float *)((char *)sm + (size_t)warp * sweep_warp_bytes(S)), *hb_hi = hb_lo + S;
+    u32 *bbits = (u32 *)(hb_hi + S);
+    float *bmax = (float *)(bbits + NB);             // largest in-bounds upper bound of each block of rows b
     const u32 nc = *A.n_cand;
     const u64 total = (u64)nc * K;
+    // a warp's share of a small pass is spread over two turns at least
+    const u32 per = (u32)max(1ull, min(32ull, total / ((u64)gridDim.x * (kScanThreads / 32) * 2)));
     const float krm = ov_krm(A), kx = ov_kx(A);
     u32 evaluated = 0;
     for (;;) {
-        // pairs are taken dynamically: their cost varies by orders of magnitude
-        u64 e = 0;
-        if (lane == 0) e = atomicAdd(A.scan_next, 1ull);
-        e = __shfl_sync(0xffffffffu, e, 0);
-        if (e >= total) break;
-        const u32 g = (u32)(e / K), t = (u32)(e % K);
-        if (A.cskip[g]) continue;
-        const float mA = A.ga_max[g];
-        if (mA == -INFINITY) continue;                  // no in-bounds row
-        const OvCand c = ov_cand(A, g);
-        const float LB = *(volatile const float *)(A.cand_lb + g);
-        const float TH = fmaxf(LB, c.lbest);
-        const size_t pair = (size_t)c.k0 * K + t;
-        const float XM = A.XM[pair];
-        const OvRowB rb = ov_row_b(A, g, c.bidx, c.k0, t, krm);
-        {
-            // the pair test below with the seed's row maxima (the same values
-            // the row pass computes): a pair that fails it needs no row pass
-            const float mB0 = A.pair_mb[e];
-            // without the stored magnitude, a bound: |H| + its error is below 1.02 (||t|| ||window|| + ||t||^2)
-            const float mabs0 = fmaxf(A.ga_abs[g], A.pair_mabs ? A.pair_mabs[e]
-                                                               : 1.02f * A.tnorm[t] * (rb.vn + A.tnorm[t]) + rb.eqt + rb.sub1);
-            const float slack0 = kPruneSlack * (2.0f * mabs0 + fabsf(TH) + fabsf(XM));
-            if (!(mA + mB0 + XM + slack0 >= TH)) continue;
-        }
-        const float *Hg = A.H + ((size_t)g * K + t) * S;
-        // rows b: intervals and the L[t][ashift] > 0 bits; rows a: copied
-        float mB = -INFINITY, mabs = A.ga_abs[g];
-        for (u32 x0 = 0; x0 < S; x0 += 32) {
-            const u32 x = x0 + lane;
-            bool bp = false;
-            if (x < S) {
-                ga_lo[x] = A.ga_lo[(size_t)g * S + x];
-                ga_hi[x] = A.ga_hi[(size_t)g * S + x];
-                float lo, hi;
-                ov_row_interval(A, g, t, x, Hg[x], rb, lo, hi);
-                hb_lo[x] = lo;
-                hb_hi[x] = hi;
-                if (x >= c.xlo && x < c.xhi_ex) {
-                    bp = !(A.Lk[(size_t)t * n + c.bidx + x - nmax] <= 0.0f);
-                    mB = fmaxf(mB, hi);
-                    mabs = fmaxf(mabs, fabsf(hi));
+        // pairs are taken dynamically, up to 32 at a time: their cost varies by
+        // orders of magnitude, and most fail the pair test (lanes over pairs)
+        u64 e32 = 0;
+        if (lane == 0) e32 = atomicAdd(A.scan_next, (unsigned long long)per);
+        e32 = __shfl_sync(0xffffffffu, e32, 0);
+        if (e32 >= total) break;
+        // the pair test with the seed's row maxima: a pair that fails it needs no row pass
+        bool go = false;
+        if (lane < per && e32 + lane < total) {
+            const u64 e = e32 + lane;
+            const u32 g = (u32)(e / K), t = (u32)(e - (u64)g * K);
+            const float mA = A.cskip[g] ? -INFINITY : A.ga_max[g];
+            if (mA != -INFINITY) {                   // else skipped, or no in-bounds row
+                const u32 id = A.cand[g], k0 = A.best_lab[id];
+                const float TH = fmaxf(*(volatile const float *)(A.cand_lb + g), A.best_ll[id]);
+                const float XM = A.XM[(size_t)k0 * K + t];
+                // without the stored magnitude, a bound: |H| + its error is below 1.02 (||t|| ||window|| + ||t||^2)
+                float mabs;
+                if (A.pair_mabs) {
+                    mabs = A.pair_mabs[e];
+                } else {
+                    const OvRowB rb = ov_row_b(A, g, A.best_idx[id], k0, t, krm);
+                    mabs = 1.02f * A.tnorm[t] * (rb.vn + A.tnorm[t]) + rb.eqt + rb.sub1;
                 }
-            }
-            const u32 mb = __ballot_sync(0xffffffffu, bp);
-            if (lane == 0) {
-                bbits[x0 / 32] = mb;
-                abits[x0 / 32] = A.ga_bits[(size_t)g * NB + x0 / 32];
+                const float slack = kPruneSlack * (2.0f * fmaxf(A.ga_abs[g], mabs) + fabsf(TH) + fabsf(XM));
+                go = mA + A.pair_mb[e] + XM + slack >= TH;
             }
         }
-        mB = warp_max_f(mB);
-        mabs = warp_max_f(mabs);
-        const float slack = kPruneSlack * (2.0f * mabs + fabsf(TH) + fabsf(XM));
-        if (!(mA + mB + XM + slack >= TH)) continue;
-        // rows that can reach TH with the other side's best
-        u32 na = 0, nb = 0;
-        for (u32 x0 = 0; x0 < S; x0 += 32) {
-            const u32 x = x0 + lane;
-            const bool inb = x < S && x >= c.xlo && x < c.xhi_ex;
-            const bool ka = inb && ga_hi[x] + mB + XM + slack >= TH;
-            const bool kb = inb && hb_hi[x] + mA + XM + slack >= TH;
-            const u32 ma = __ballot_sync(0xffffffffu, ka), mb = __ballot_sync(0xffffffffu, kb);
-            if (ka) alist[na + __popc(ma & ((1u << lane) - 1u))] = (u16)x;
-            if (kb) blist[nb + __popc(mb & ((1u << lane) - 1u))] = (u16)x;
-            na += __popc(ma);
-            nb += __popc(mb);
-        }
-        __syncwarp();
-        const float *xmr = A.XMr + pair * NR;
-        const float *q = A.Q + pair * R * (L + 1);
-        const bool apart = ov_disjoint(A.tsup, c.k0, t);   // no cross term, no table
-        const u32 P = na * nb;
-        float lbmax = -INFINITY;
-        // pair p = ai * nb + bi; each lane steps its (ai, bi) by 32 pairs
-        u32 ai = 0, bi = lane, dq = 0, dr = 32;
-        if (nb) {
-            ai = lane / nb; bi = lane - ai * nb;
-            dq = 32 / nb; dr = 32 - dq * nb;
-        }
-        for (u32 p0 = 0; p0 < P; p0 += 32) {
-            const u32 p = p0 + lane;
-            bool valid = false;
-            u32 a = 0, b = 0;
-            if (p < P) {
-                a = alist[ai];
-                b = blist[bi];
-                valid = (a > b ? a - b : b - a) <= L &&                                    // .cl:543-556
-                        (((abits[a >> 5] >> (a & 31)) | (bbits[b >> 5] >> (b & 31))) & 1u);  // .cl:572-576
-                if (valid) {
-                    const float xr = apart ? 0.0f : __ldg(xmr + (int)a - (int)b + (int)L);
-                    valid = ga_hi[a] + hb_hi[b] + xr + slack + kPruneSlack * fabsf(xr) >= TH;
-                }
-            }
-            ai += dq;
-            bi += dr;
-            if (bi >= nb) { bi -= nb; ai++; }
-            float lo = -INFINITY, hi = -INFINITY;
-            if (valid) {
-                const float X = apart ? 0.0f : ov_x(q, L, (int)a - (int)nmax, (int)a - (int)b);
-                const float ex = kx * fabsf(X);
-                hi = ga_hi[a] + hb_hi[b] - X + ex;
-                lo = ga_lo[a] + hb_lo[b] - X - ex;
-                evaluated++;
-            }
-            lbmax = fmaxf(lbmax, lo);
-            const bool keep = valid && hi >= TH && hi > c.lbest;
-            const u32 mk = __ballot_sync(0xffffffffu, keep);
-            if (mk) {
-                u32 base = 0;
-                if (lane == 0) base = atomicAdd(A.pool_total, (u32)__popc(mk));
-                base = __shfl_sync(0xffffffffu, base, 0);
-                if (keep) {
-                    const u32 pp = base + __popc(mk & ((1u << lane) - 1u));
-                    if (pp < A.pool_cap) {
-                        A.pool_slot[pp] = g;
-                        A.pool_item[pp] = t + K * (a + S * b);
-                        A.pool_hi[pp] = hi;
-                    } else {
-                        A.fallback[g] = 1;
+        u32 todo = __ballot_sync(0xffffffffu, go);
+        while (todo) {
+            const u64 e = e32 + (u32)(__ffs(todo) - 1);
+            todo &= todo - 1;
+            const u32 g = (u32)(e / K), t = (u32)(e - (u64)g * K);
+            const OvCand c = ov_cand(A, g);
+            const float mA = A.ga_max[g];
+            float TH = fmaxf(*(volatile const float *)(A.cand_lb + g), c.lbest);
+            const size_t pair = (size_t)c.k0 * K + t;
+            const float XM = A.XM[pair];
+            const OvRowB rb = ov_row_b(A, g, c.bidx, c.k0, t, krm);
+            const float *Hg = A.H + ((size_t)g * K + t) * S;
+            const float *ga_lo = A.ga_lo + (size_t)g * S, *ga_hi = A.ga_hi + (size_t)g * S;
+            const u32 *abits = A.ga_bits + (size_t)g * NB;
+            // rows b: intervals and the L[t][ashift] > 0 bits
+            float mB = -INFINITY, mabs = A.ga_abs[g];
+            u32 kbest = 0;
+            __syncwarp();                            // the previous pair's readers are done
+            for (u32 x0 = 0; x0 < S; x0 += 32) {
+                const u32 x = x0 + lane;
+                bool bp = false;
+                float up = -INFINITY;
+                if (x < S) {
+                    float lo, hi;
+                    ov_row_interval(A, g, t, x, Hg[x], rb, lo, hi);
+                    hb_lo[x] = lo;
+                    hb_hi[x] = hi;
+                    if (x >= c.xlo && x < c.xhi_ex) {
+                        bp = !(A.Lk[(size_t)t * n + c.bidx + x - nmax] <= 0.0f);
+                        up = hi;
+                        mabs = fmaxf(mabs, fabsf(hi));
                     }
                 }
+                const u32 mb = __ballot_sync(0xffffffffu, bp);
+                up = warp_max_f(up);
+                if (lane == 0) { bbits[x0 / 32] = mb; bmax[x0 / 32] = up; }
+                if (up > mB) { mB = up; kbest = x0 / 32; }
+            }
+            mabs = warp_max_f(mabs);
+            __syncwarp();
+            float slack = kPruneSlack * (2.0f * mabs + fabsf(TH) + fabsf(XM));
+            if (!(mA + mB + XM + slack >= TH)) continue;
+            const bool apart = ov_disjoint(A.tsup, c.k0, t);   // no cross term, no table
+            const float *xmr = A.XMr + pair * NR, *xmw = A.XMw + pair * NW;
+            const float *q = A.Q + pair * R * (L + 1);
+            for (u32 kk = 0; kk < NB; kk++) {
+                const u32 k = kk == 0 ? kbest : kk <= kbest ? kk - 1 : kk;   // kbest, then the others in order
+                const float mBk = bmax[k];
+                if (!(mA + mBk + XM + slack >= TH)) continue;                // uniform
+                const u32 b = 32 * k + lane;
+                const bool inb = b < S && b >= c.xlo && b < c.xhi_ex;
+                const float lo_b = b < S ? hb_lo[b] : 0.0f, hi_b = b < S ? hb_hi[b] : 0.0f;
+                const bool bp = (bbits[k] >> lane) & 1u;
+                float lbmax = -INFINITY;
+                for (u32 a0 = 0; a0 < S; a0 += 32) {
+                    // lags of row a against the block: a - 32 k - 31 .. a - 32 k
+                    const u32 al = a0 + lane;
+                    const int wi = (int)al - (int)(32 * k) + (int)L;        // XMw index
+                    bool ka = al < S && al >= c.xlo && al < c.xhi_ex && wi >= 0 && wi < (int)NW;
+                    if (ka) {
+                        const float xw = apart ? 0.0f : __ldg(xmw + wi);
+                        ka = ga_hi[al] + mBk + xw + slack + kPruneSlack * fabsf(xw) >= TH;
+                    }
+                    u32 rows = __ballot_sync(0xffffffffu, ka);
+                    while (rows) {
+                        const u32 a = a0 + __ffs(rows) - 1;
+                        rows &= rows - 1;
+                        const float hi_a = ga_hi[a];
+                        bool valid = inb && (a > b ? a - b : b - a) <= L &&              // .cl:543-556
+                                     (bp || ((abits[a >> 5] >> (a & 31)) & 1u));         // .cl:572-576
+                        if (valid) {
+                            const float xr = apart ? 0.0f : __ldg(xmr + (int)a - (int)b + (int)L);
+                            valid = hi_a + hi_b + xr + slack + kPruneSlack * fabsf(xr) >= TH;
+                        }
+                        if (!__any_sync(0xffffffffu, valid)) continue;
+                        float hi = -INFINITY;
+                        if (valid) {
+                            const float X = apart ? 0.0f : ov_x(q, L, (int)a - (int)nmax, (int)a - (int)b);
+                            const float ex = kx * fabsf(X);
+                            hi = hi_a + hi_b - X + ex;
+                            lbmax = fmaxf(lbmax, ga_lo[a] + lo_b - X - ex);
+                            evaluated++;
+                        }
+                        const bool keep = valid && hi >= TH && hi > c.lbest;
+                        const u32 mk = __ballot_sync(0xffffffffu, keep);
+                        if (mk) {
+                            u32 base = 0;
+                            if (lane == 0) base = atomicAdd(A.pool_total, (u32)__popc(mk));
+                            base = __shfl_sync(0xffffffffu, base, 0);
+                            if (keep) {
+                                const u32 pp = base + __popc(mk & ((1u << lane) - 1u));
+                                if (pp < A.pool_cap) {
+                                    A.pool_slot[pp] = g;
+                                    A.pool_item[pp] = t + K * (a + S * b);
+                                    A.pool_hi[pp] = hi;
+                                } else {
+                                    A.fallback[g] = 1;
+                                }
+                            }
+                        }
+                    }
+                }
+                lbmax = warp_max_f(lbmax);
+                if (lbmax > TH) {
+                    if (lane == 0) atomicMax(reinterpret_cast<int *>(A.cand_lb) + g, __float_as_int(lbmax));   // > 0
+                    TH = lbmax;
+                    slack = kPruneSlack * (2.0f * mabs + fabsf(TH) + fabsf(XM));
+                }
             }
         }
-        lbmax = warp_max_f(lbmax);
-        if (lane == 0 && lbmax > 0.0f) atomicMax(reinterpret_cast<int *>(A.cand_lb) + g, __float_as_int(lbmax));
-        __syncwarp();
     }
     if (A.items_evaluated) {
 #pragma unroll
