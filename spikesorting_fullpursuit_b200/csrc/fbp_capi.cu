@@ -166,9 +166,11 @@ struct Workspace {
     float *tc_tnorm, *tc_tabs;
     int *tc_texp;
     u8 *apx;
-    float *wn_s, *wa_s, *bm_s, *wlb;
+    float *wn_s, *wa_s, *wlb;
     float *umax;                     // [W][K] largest upper bound of a template's entries per window
-    u8 *wpos;                        // [W] some entry of the window is > 0
+    u8 *wpos;                        // [W][G16] some entry of the (window, group) is > 0
+    u32 G16, GW;                     // groups of 16 templates, words of their bits
+    u32 *dirty;                      // [W][GW] (window, group) pairs to recompute when the window is listed
     signed char *kx_s;
     u32 *tc_ref_t, *tc_ref_s, *tc_seg_s0, *tc_seg_base, *tc_seg_cnt;
     u32 tc_seg_cap;
@@ -177,8 +179,8 @@ struct Workspace {
     u32 tcw_ns = 0;                  // ring stages
     std::vector<TcGroup> tcwg;       // wide groups (tb_off: offset of its A tiles, 4 KB units)
     float *vwmax;                    // [W + 2] bound on |v| per window (all channels)
-    u8 *ws_brk;                      // [window bytes] run starts of the pass's list
-    u32 *ws_runs, *ws_pos, *ws_first;
+    u32 wl_stride, wf_stride;        // the groups' window lists and streams of a pass
+    u32 *wl_win, *wl_pos, *wl_first, *wl_nwin, *wl_nst, *wl_counts;
     unsigned char *Aw;               // packed A tiles of every wide group
     u32 *tgrp_w;                     // [K] wide group of each template
     u32 *tcw_gdesc;                  // [group][3]: t0, clo, Cg (device)
@@ -269,7 +271,7 @@ u32 plan_tcw_groups(const std::vector<u32> &tsup, const std::vector<u32> &tperm,
     out.clear();
     if (L < kWMinL || L > 1024) return 0;
     u32 ns = 0;
-    for (u32 s = kWMaxStages; s >= 2; s--)
+    for (u32 s = kWProdWarps; s >= 2; s--)
         if (tcw_smem_layout(L, s).total <= 227 * 1024) { ns = s; break; }
     if (ns == 0) return 0;
     size_t off = 0;
@@ -307,9 +309,12 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
     };
     w.cnt = (Counters *)take(sizeof(Counters));
     w.snap = (Counters *)take(sizeof(Counters));
-    w.wlb = (float *)take((size_t)W * 4);
+    w.G16 = ceil_div(K, 16);
+    w.GW = ceil_div(w.G16, 32);
+    w.wlb = (float *)take((size_t)W * w.G16 * 4);
     w.umax = (float *)take((size_t)W * K * 4);
-    w.wpos = (u8 *)take((size_t)W);
+    w.wpos = (u8 *)take((size_t)W * w.G16);
+    w.dirty = (u32 *)take((size_t)W * w.GW * 4);
     w.tsup = (u32 *)take((size_t)K * 8);
     w.tperm = (u32 *)take((size_t)K * 4);
     w.grange = (u32 *)take((size_t)ceil_div(K, kLikTplPerBlock) * 8);
@@ -385,7 +390,6 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
         w.Tb = (uint4 *)take((size_t)L * cg2all * (2 * (size_t)K + 16) * 16);
         w.apx = (u8 *)take((size_t)K * n);
         w.wn_s = (float *)take((size_t)w.tc_gmax * n * 4);
-        w.bm_s = (float *)take((size_t)n * 4);
         w.wa_s = (float *)take((size_t)w.tc_gmax * n * 4);
         w.kx_s = (signed char *)take((size_t)w.tc_gmax * n);
         w.tc_tnorm = (float *)take((size_t)K * 4);
@@ -406,10 +410,14 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
         // wide tiles: per-window |v| bound, the pass's stream, A tiles of
         // every group of 16 templates (at most all C channels each)
         w.vwmax = (float *)take(((size_t)W + 2) * 4);
-        w.ws_brk = (u8 *)take(window_bytes_u8(W));
-        w.ws_runs = (u32 *)take(Wp * 4);
-        w.ws_pos = (u32 *)take(Wp * 4);
-        w.ws_first = (u32 *)take(((size_t)W * (2 * (size_t)L) / kWPos + 4) * 4);
+        w.wl_stride = W;
+        w.wf_stride = (u32)((size_t)W * (2 * (size_t)L) / kWPos + 4);
+        w.wl_win = (u32 *)take((size_t)w.G16 * W * 4);
+        w.wl_pos = (u32 *)take((size_t)w.G16 * W * 4);
+        w.wl_first = (u32 *)take((size_t)w.G16 * w.wf_stride * 4);
+        w.wl_nwin = (u32 *)take((size_t)w.G16 * 4);
+        w.wl_nst = (u32 *)take((size_t)w.G16 * 4);
+        w.wl_counts = (u32 *)take((size_t)w.G16 * ceil_div(W, kCompactTile) * 4);
         w.Aw = (unsigned char *)take((size_t)w.tc_gmax * C * tcw_nkc(L) * kWATile);
         w.tgrp_w = (u32 *)take((size_t)K * 4);
         w.tcw_gdesc = (u32 *)take((size_t)w.tc_gmax * 12);
@@ -501,7 +509,8 @@ int launch_check_overlap(u32 n, u32 L, const u32 *cand, const u32 *n_cand_dev, u
 int launch_accept(u32 n, u32 C, u32 L, const float *thr, const u32 *win, const u32 *n_win_dev,
                   u32 max_windows, const fbp_window_state &s, const u8 *active, u8 *has, u8 *flags_out,
                   u32 *acc_list, u32 *spk_idx, u32 *spk_lab, u32 *spk_win, u32 *n_spk_dev,
-                  u32 *tile_counts, cudaStream_t st) {
+                  u32 *tile_counts, cudaStream_t st, const WinBounds &wb = WinBounds{}, const u32 *grange = nullptr,
+                  const u32 *tsup = nullptr, u32 K = 0) {
     const u32 W = ceil_div(n, L);
     const int threads = 256;
     FBP_CUDA(cudaMemsetAsync(has, 0, window_bytes_u8(W), st));
@@ -513,7 +522,8 @@ int launch_accept(u32 n, u32 C, u32 L, const float *thr, const u32 *win, const u
     int rc = compact(has, W, acc_list, n_spk_dev, tile_counts, st);
     if (rc) return rc;
     k_gather_spikes<<<grid_for(W, threads), threads, 0, st>>>(n, C, L, acc_list, n_spk_dev, s.best_idx,
-                                                              s.best_lab, spk_idx, spk_lab, spk_win);
+                                                              s.best_lab, spk_idx, spk_lab, spk_win, wb, grange,
+                                                              tsup, K);
     FBP_LAUNCH_CHECK();
     return FBP_OK;
 }
@@ -523,18 +533,24 @@ float tc_kappa_s(u32 C, u32 L);
 TcArgs tc_group_args(const Workspace &w, u32 gi, const float *v, u32 n, u32 C, const float *T, u32 K, u32 L,
                      const float *tss, float *Lk, Counters *cnt);
 
+// The window bounds; the 128-sample tiles recompute every group of a listed
+// window, the other likelihood kernels those whose voltage changed.
+WinBounds win_bounds(const Workspace &w) {
+    return WinBounds{w.wlb, w.umax, w.wpos, w.G16, w.tc && !w.tcw ? nullptr : w.dirty, w.GW};
+}
+
 // Context for likelihood entries the tensor-core path left approximate.
 LazyLk lazy_ctx(const Workspace &w, const float *v, const float *T, const float *tss, u32 C, u32 L, u32 pass) {
     LazyLk z{};
     if (!w.tc) return z;
-    z.apx = w.apx; z.wn = w.wn_s; z.wa = w.wa_s; z.kx = w.kx_s;
+    z.apx = w.apx; z.wn = w.wn_s; z.wa = w.tcw ? nullptr : w.wa_s; z.kx = w.kx_s;
+    z.wa_f = tcw_l1_factor(w.tc_cmax, L);
     z.tnorm = w.tc_tnorm; z.tabs = w.tc_tabs; z.tss = tss; z.texp = w.tc_texp;
     z.v = v; z.T = T; z.C = C; z.L = L;
     z.kappa_b = tc_kappa(w.tc_nz, L, ceil_div(w.tc_nz, 8));
     z.kappa_s = tc_kappa_s(w.tc_nz, L);
     z.tgrp = w.tcw ? w.tgrp_w : w.tgrp; z.gstride = w.n; z.tsup = w.tsup;
     z.refined = &w.cnt->lazy_ref;
-    z.wlb = w.wlb; z.bm = w.bm_s;
     z.tag = 2u + (pass & 1u);
     return z;
 }
@@ -743,28 +759,24 @@ int tc_chunk_setup(const Workspace &w, const float *v, u32 n, const float *T, u3
     return FBP_OK;
 }
 
-// Launch arguments of one wide-tile group.
-TcwArgs tcw_group_args(const Workspace &w, u32 gi, const float *v, u32 n, u32 C, u32 K, u32 L, const float *tss,
-                       float *Lk, Counters *cnt) {
-    const TcGroup &g = w.tcwg[gi];
-    TcwArgs A{};
-    A.n = n; A.Cg = g.Cg; A.nt = g.nt; A.L = L;
-    A.nkc = tcw_nkc(L); A.ns = w.tcw_ns; A.px = tcw_px(L); A.Kall = K; A.W = ceil_div(n, L);
-    A.trow = w.tperm + g.t0;
+// Launch arguments of the wide tiles over every group of a pass.
+TcwParams tcw_params(const Workspace &w, u32 n, u32 K, u32 L, const float *tss, float *Lk, Counters *cnt,
+                     float *dbg_bound) {
+    TcwParams A{};
+    A.n = n; A.L = L; A.ns = w.tcw_ns; A.G = (u32)w.tcwg.size(); A.Kall = K; A.W = ceil_div(n, L);
+    A.wstride = w.wl_stride; A.fstride = w.wf_stride;
+    A.groups = w.tcw_args;
     A.kappa_b = tc_kappa(w.tc_nz, L, ceil_div(w.tc_nz, 8));
     A.kappa_s = tc_kappa_s(w.tc_nz, L);
-    A.v = v + (size_t)g.clo * n;
     A.tss = tss; A.tnorm = w.tc_tnorm; A.tabs = w.tc_tabs; A.texp = w.tc_texp;
-    A.Aw = w.Aw + g.tb_off * kWATile;
     A.vwmax = w.vwmax;
-    A.win = w.win; A.n_win = &cnt->n_win;
-    A.pos = w.ws_pos; A.first = w.ws_first; A.n_stiles = &cnt->n_stiles;
-    A.Lk = Lk; A.apx = w.apx;
-    A.wn_s = w.wn_s + (size_t)gi * n; A.wa_s = w.wa_s + (size_t)gi * n; A.kx_s = w.kx_s + (size_t)gi * n;
-    A.bm_s = w.bm_s; A.wlb = w.wlb; A.umax = w.umax; A.wpos = w.wpos;
+    A.win = w.wl_win; A.pos = w.wl_pos; A.first = w.wl_first; A.n_win = w.wl_nwin; A.n_stiles = w.wl_nst;
+    A.Lk = Lk; A.apx = w.apx; A.dbgE = dbg_bound;
+    A.wn_s = w.wn_s; A.kx_s = w.kx_s;
+    A.wa_f = tcw_l1_factor(w.tc_cmax, L);
+    A.wlb = w.wlb; A.umax = w.umax; A.wpos = w.wpos;
     A.ref_t = w.tc_ref_t; A.ref_s = w.tc_ref_s; A.refseg = &cnt->tc_refseg; A.ref_cap = w.tc_ref_cap;
     A.seg_s0 = w.tc_seg_s0; A.seg_base = w.tc_seg_base; A.seg_cnt = w.tc_seg_cnt; A.seg_grp = w.tc_seg_grp;
-    A.grp = gi;
     A.seg_overflow = &cnt->tc_overflow; A.seg_cap = w.tc_seg_cap;
     A.err = &cnt->tc_err;
     A.wait_polls = g_lim_wait.load();
@@ -795,7 +807,8 @@ TcArgs tc_group_args(const Workspace &w, u32 gi, const float *v, u32 n, u32 C, c
     A.seg_overflow = &cnt->tc_overflow; A.seg_cap = w.tc_seg_cap;
     A.err = &cnt->tc_err;
     A.wait_polls = g_lim_wait.load();
-    A.apx = w.apx; A.bm_s = w.bm_s; A.wlb = w.wlb; A.umax = w.umax; A.wpos = w.wpos;
+    A.apx = w.apx; A.wlb = w.wlb; A.umax = w.umax; A.wpos = w.wpos;
+    A.G16 = w.G16; A.g16 = g.t0 / 16;
     A.wn_s = w.wn_s + (size_t)gi * n; A.wa_s = w.wa_s + (size_t)gi * n; A.kx_s = w.kx_s + (size_t)gi * n;
     return A;
 }
@@ -829,26 +842,21 @@ float tc_kappa_s(u32 C, u32 L) {
 // one launch per template group.
 int tc_likelihood_pass(const Workspace &w, const float *v, u32 n, u32 C, const float *T, u32 K, u32 L,
                        const float *tss, const u32 *win, const u32 *n_win, u32 max_windows, float *Lk,
-                       Counters *cnt, cudaStream_t st, int *launches) {
-    (void)max_windows;
+                       Counters *cnt, cudaStream_t st, int *launches, float *dbg_bound = nullptr) {
+    (void)max_windows; (void)v; (void)C; (void)T;
     FBP_CUDA(cudaMemsetAsync(&cnt->tc_refseg, 0, 8, st));
     FBP_CUDA(cudaMemsetAsync(&cnt->tc_overflow, 0, 4, st));   // set by the tiles when the list overflows
-    (void)v; (void)C; (void)T; (void)K; (void)tss; (void)Lk;
     if (w.tcw) {
-        // the pass's window stream: run starts, their list, stream positions
-        const u32 W = ceil_div(n, L);
-        const size_t wbb = window_bytes_u8(W);
-        k_ws_breaks<<<grid_for(wbb, 256), 256, 0, st>>>(win, n_win, (u32)wbb, w.ws_brk);
-        FBP_LAUNCH_CHECK();
-        if (int rc = compact(w.ws_brk, W, w.ws_runs, &cnt->n_runs, w.tile_counts, st)) return rc;
-        k_ws_pos<<<grid_for(W, 256), 256, 0, st>>>(n_win, w.ws_brk, w.ws_runs, &cnt->n_runs, L, w.ws_pos,
-                                                    w.ws_first, &cnt->n_stiles);
-        FBP_LAUNCH_CHECK();
+        // the groups' window lists and streams, then their tiles
+        const u32 W = ceil_div(n, L), G = (u32)w.tcwg.size();
+        const dim3 lg(ceil_div(W, kCompactTile), G);
+        k_tcw_count<<<lg, kCompactThreads, 0, st>>>(w.active, w.dirty, w.GW, W, w.wl_counts);
+        k_tcw_lists<<<lg, kCompactThreads, 0, st>>>(w.active, w.dirty, w.GW, W, L, w.wl_counts, w.wl_stride,
+                                                     w.wf_stride, w.wl_win, w.wl_pos, w.wl_first, w.wl_nwin, w.wl_nst);
         FBP_ALLOW_SMEM(k_lik_tcw);
-        const u32 G = (u32)w.tcwg.size();
-        k_lik_tcw<<<std::max<u32>(sm_count(), G), kTcThreads, w.tcw_smem, st>>>(w.tcw_args, G);
+        k_lik_tcw<<<sm_count(), kWThreads, w.tcw_smem, st>>>(tcw_params(w, n, K, L, tss, Lk, cnt, dbg_bound));
         FBP_LAUNCH_CHECK();
-        *launches = 6;
+        *launches = 3;
         return FBP_OK;
     }
     (void)win; (void)n_win;
@@ -875,11 +883,11 @@ int tc_refine_pass(const Workspace &w, const float *v, u32 n, u32 C, const float
     k_tc_refine<<<sm_count() * 8, kRefThreads, rsmem, st>>>(
         v, n, C, w.tc_cmax, T, K, L, tss, w.tc_ref_t, w.tc_ref_s, w.tc_seg_s0, w.tc_seg_base, w.tc_seg_cnt,
         w.tc_seg_grp, w.tcw ? w.tcw_gdesc : w.tc_gdesc, w.tperm, reinterpret_cast<const u32 *>(&cnt->tc_refseg), w.tc_seg_cap, Lk,
-        lazy_ctx(w, v, T, tss, C, L, 0), gamma, &cnt->tc_seq, w.wpos, &cnt->tc_overflow, w.tc_ref_cap);
+        lazy_ctx(w, v, T, tss, C, L, 0), gamma, &cnt->tc_seq, w.wpos, w.G16, &cnt->tc_overflow, w.tc_ref_cap);
     k_tc_gate<<<1, 1, 0, st>>>(cnt, w.tc_ref_cap, w.tc_seg_cap);
     FBP_LAUNCH_CHECK();
     int rc = launch_likelihood(v, n, C, T, K, L, tss, win, n_win, max_windows, Lk, st, &cnt->tc_overflow, w.apx,
-                               w.tperm, w.grange, WinBounds{w.wlb, w.umax, w.wpos});
+                               w.tperm, w.grange, win_bounds(w));
     *launches = 3;
     return rc;
 }
@@ -998,9 +1006,10 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
     FBP_CUDA(cudaMemsetAsync(w.ovr, 0, wb, st));
     FBP_CUDA(cudaMemsetAsync(w.ovr2, 0, wb, st));
     FBP_CUDA(cudaMemsetAsync(w.active, 0, wb, st));
-    FBP_CUDA(cudaMemsetAsync(w.wlb, 0, (size_t)W * 4, st));
+    FBP_CUDA(cudaMemsetAsync(w.wlb, 0, (size_t)W * w.G16 * 4, st));
     FBP_CUDA(cudaMemsetAsync(w.umax, 0, (size_t)W * K * 4, st));
-    FBP_CUDA(cudaMemsetAsync(w.wpos, 0, (size_t)W, st));
+    FBP_CUDA(cudaMemsetAsync(w.wpos, 0, (size_t)W * w.G16, st));
+    FBP_CUDA(cudaMemsetAsync(w.dirty, 0xff, (size_t)W * w.GW * 4, st));   // nothing is computed yet
     k_iota_windows<<<grid_for(W, 256), 256, 0, st>>>(w.win, w.active, W, w.cnt);
     k_template_ranges<<<(int)std::min(K, 65535u), 256, 0, st>>>(templates, K, C, L, w.tsup);
     k_template_support<<<1, 256, 0, st>>>(templates, K, C, L, w.tsup, w.tperm, w.grange, kLikTplPerBlock,
@@ -1076,7 +1085,6 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
     if (w.tc) {
         timer.begin(FBP_STAGE_LIKELIHOOD);
         FBP_CUDA(cudaMemsetAsync(w.apx, 0, (size_t)K * n, st));
-        FBP_CUDA(cudaMemsetAsync(w.bm_s, 0, (size_t)n * 4, st));
         int rc0 = tc_chunk_setup(w, voltage, n, templates, K, C, L, st);
         if (rc0) return rc0;
         // launch arguments of every template group (constant for the chunk)
@@ -1106,8 +1114,8 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
             std::vector<TcwArgs> aw(w.tcwg.size());
             if (w.tcw) {
                 for (u32 gi = 0; gi < (u32)aw.size(); gi++) {
-                    aw[gi] = tcw_group_args(w, gi, voltage, n, C, K, L, neg_half_ss, w.Lk, w.cnt);
-                    aw[gi].dbgE = dbg_bound;
+                    const TcGroup &g = w.tcwg[gi];
+                    aw[gi] = TcwArgs{g.Cg, g.nt, w.tperm + g.t0, voltage + (size_t)g.clo * n, w.Aw + g.tb_off * kWATile};
                 }
                 FBP_CUDA(cudaMemcpyAsync(w.tcw_args, aw.data(), aw.size() * sizeof(TcwArgs), cudaMemcpyHostToDevice,
                                          st));
@@ -1221,7 +1229,7 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
         } else {
             if ((rc2 = launch_likelihood(voltage, n, C, templates, K, L, neg_half_ss, w.win, &w.cnt->n_win, W,
                                          w.Lk, q, nullptr, nullptr, w.tperm, w.grange,
-                                         WinBounds{w.wlb, w.umax, w.wpos})))
+                                         win_bounds(w))))
                 return rc2;
             launched[FBP_STAGE_LIKELIHOOD] += 1;
         }
@@ -1229,7 +1237,7 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
         // 2. per-window argmax over all templates (.py:551-562)
         timer.begin(FBP_STAGE_ARGMAX);
         const LazyLk lz = lazy_ctx(w, voltage, templates, neg_half_ss, C, L, pass);
-        if ((rc2 = launch_argmax(n, L, K, w.win, &w.cnt->n_win, W, s, w.Lk, q, lz, WinBounds{w.wlb, w.umax, w.wpos})))
+        if ((rc2 = launch_argmax(n, L, K, w.win, &w.cnt->n_win, W, s, w.Lk, q, lz, win_bounds(w))))
             return rc2;
         launched[FBP_STAGE_ARGMAX] += 1;
         timer.end(FBP_STAGE_ARGMAX);
@@ -1268,7 +1276,7 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
         timer.begin(FBP_STAGE_ACCEPT);
         if ((rc2 = launch_accept(n, C, L, thresholds, w.win, &w.cnt->n_win, W, s, w.active, w.has,
                                  w.flags_out, w.acc_list, w.spk_idx, w.spk_lab, w.spk_win, &w.cnt->n_spk,
-                                 w.tile_counts, q)))
+                                 w.tile_counts, q, win_bounds(w), w.grange, w.tsup, K)))
             return rc2;
         launched[FBP_STAGE_ACCEPT] += 6;
         timer.end(FBP_STAGE_ACCEPT);
@@ -1278,8 +1286,7 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
         timer.begin(FBP_STAGE_LISTS);
         FBP_CUDA(cudaMemsetAsync(w.ovr, 0, wb, q));
         if ((rc2 = compact(w.flags_out, W, w.win, &w.cnt->n_win, w.tile_counts, q))) return rc2;
-        k_mark_active<<<grid_for(W, 256), 256, 0, q>>>(w.flags_out, w.active, W, WinBounds{w.wlb, w.umax, w.wpos},
-                                                       w.tc ? w.bm_s : nullptr, L, n, K);
+        k_mark_active<<<grid_for(W, 256), 256, 0, q>>>(w.flags_out, w.active, W, win_bounds(w), K, w.tperm);
         FBP_CUDA(cudaMemsetAsync(w.flags, 0, wb, q));
         // 8. keep the spikes (.py:702-710)
         k_append_spikes<<<grid_for(W, 256), 256, 0, q>>>(w.spk_idx, w.spk_lab, w.cnt, spike_idx, spike_lab,
@@ -1465,7 +1472,7 @@ int fbp_tc_likelihood_bounds(const float *voltage, uint32_t n, uint32_t C, const
     if (!w.tc) return fail(FBP_ERR_BAD_ARG, "fbp_tc_likelihood_bounds: no tensor-core plan for this shape");
     int nl = 0;
     if (int e = tc_likelihood_pass(w, voltage, n, C, templates, K, L, neg_half_ss, w.win, &w.cnt->n_win,
-                                   ceil_div(n, L), w.Lk, w.cnt, st, &nl))
+                                   ceil_div(n, L), w.Lk, w.cnt, st, &nl, bound))
         return e;
     FBP_CUDA(cudaMemcpyAsync(approx, w.Lk, (size_t)K * n * 4, cudaMemcpyDeviceToDevice, st));
     u32 err = 0;

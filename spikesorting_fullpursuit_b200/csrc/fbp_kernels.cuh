@@ -16,15 +16,27 @@
 namespace fbp {
 
 // Per-window bounds written by the likelihood kernels (both paths) for the
-// window argmax: wlb[w] the largest lower bound of an entry of window w,
-// umax[w][t] the largest upper bound of template t's entries there (>= 0),
-// wpos[w] whether any entry of the window is > 0.  Reset when the window is
-// listed for recomputation; entries only move inside their intervals later.
+// window argmax, per group g of 16 templates in support order (tperm):
+// wlb[w][g] the largest lower bound of an entry of window w, umax[w][t] the
+// largest upper bound of template t's entries there (>= 0), wpos[w][g]
+// whether any entry is > 0.  Reset when the (window, group) is recomputed;
+// entries only move inside their intervals later.
+// dirty: one bit per (window, group), GW words a window: the voltage the
+// group's entries of the window read has changed since they were computed
+// (k_gather_spikes), so a listed window recomputes them; the others keep the
+// values the same voltage gave.  NULL: every group of a listed window is
+// recomputed.
 struct WinBounds {
     float *wlb;
     float *umax;
     u8 *wpos;
+    u32 G;
+    u32 *dirty;
+    u32 GW;
 };
+__device__ __forceinline__ bool win_dirty(const WinBounds &wb, u32 w, u32 g) {
+    return !wb.dirty || ((wb.dirty[(size_t)w * wb.GW + (g >> 5)] >> (g & 31)) & 1u);
+}
 
 
 // ---------------------------------------------------------------------------
@@ -84,20 +96,28 @@ __global__ void k_iota_windows(u32 *__restrict__ win, u8 *__restrict__ active, u
     if (blockIdx.x == 0 && threadIdx.x == 0) cnt->n_win = W;
 }
 
-// active[j] = (flags[j] != 0) for the next pass.
-// active = flags != 0; windows about to be recomputed also drop their
-// lower bound (wlb, tensor-core path; may be NULL).
+// active = flags != 0 for the next pass; windows about to be recomputed drop
+// the bounds of the groups they recompute.  Warps take 32 windows at a time;
+// lanes then share each listed window's templates and groups.
 __global__ void k_mark_active(const u8 *__restrict__ flags, u8 *__restrict__ active, u32 W, WinBounds wb,
-                              float *__restrict__ bm, u32 L, u32 n, u32 K) {
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < W; i += gridDim.x * blockDim.x) {
-        active[i] = flags[i] != 0;
-        if (!flags[i]) continue;
-        if (wb.wlb) wb.wlb[i] = 0.0f;
-        if (wb.wpos) wb.wpos[i] = 0;
-        if (wb.umax)
-            for (u32 t = 0; t < K; t++) wb.umax[(size_t)i * K + t] = 0.0f;
-        if (bm)
-            for (u32 s = i * L; s < min((i + 1) * L, n); s++) bm[s] = 0.0f;
+                              u32 K, const u32 *__restrict__ tperm) {
+    const u32 lane = threadIdx.x & 31, step = gridDim.x * blockDim.x;
+    for (u32 i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < W; i0 += step) {
+        const u32 i = i0 + lane;
+        const bool on = i < W && flags[i] != 0;
+        if (i < W) active[i] = on;
+        u32 m = wb.umax ? __ballot_sync(0xffffffffu, on) : 0u;
+        while (m) {
+            const u32 w = i0 + __ffs(m) - 1;
+            m &= m - 1;
+            for (u32 g = lane; g < wb.G; g += 32) {
+                if (!win_dirty(wb, w, g)) continue;
+                wb.wlb[(size_t)w * wb.G + g] = 0.0f;
+                wb.wpos[(size_t)w * wb.G + g] = 0;
+            }
+            for (u32 sl = lane; sl < K; sl += 32)
+                if (win_dirty(wb, w, sl / 16)) wb.umax[(size_t)w * K + tperm[sl]] = 0.0f;
+        }
     }
 }
 
@@ -207,6 +227,7 @@ k_likelihood_fp32(const float *__restrict__ v, u32 n, u32 C, const float *__rest
     for (u64 item = blockIdx.x; item < total; item += gridDim.x) {
         const u32 w = win[item / kgroups];
         const u32 kg = (u32)(item % kgroups);
+        if (!gate && !win_dirty(wb, w, kg)) continue;   // computed from the same voltage (uniform in the block)
         const u32 sw = w * L;
         const u32 ew = min((w + 1) * L, n);
         const u32 slot0 = kg * kLikTplPerBlock + warp * kLikQ;
@@ -269,10 +290,10 @@ k_likelihood_fp32(const float *__restrict__ v, u32 n, u32 C, const float *__rest
                     anypos |= mq > 0.0f;
                     if (lane == 0 && mq > 0.0f && slot0 + q < K) {
                         atomicMax(reinterpret_cast<int *>(wb.umax) + (size_t)w * K + tq[q], __float_as_int(mq));
-                        atomicMax(reinterpret_cast<int *>(wb.wlb) + w, __float_as_int(mq));
+                        atomicMax(reinterpret_cast<int *>(wb.wlb) + (size_t)w * wb.G + kg, __float_as_int(mq));
                     }
                 }
-                if (lane == 0 && anypos) wb.wpos[w] = 1;
+                if (lane == 0 && anypos) wb.wpos[(size_t)w * wb.G + kg] = 1;
             }
 #pragma unroll
             for (int q = 0; q < kLikQ; q++) {
@@ -309,7 +330,8 @@ k_likelihood_fp32(const float *__restrict__ v, u32 n, u32 C, const float *__rest
 // other parity was written by an earlier launch and is exact.
 struct LazyLk {
     u8 *apx;                          // [K][n]; NULL: every entry is exact
-    const float *wn, *wa;             // [n] window L2 / L1 norms at computation time
+    const float *wn, *wa;             // [n] window L2 / L1 norms at computation time (wa NULL: at most wa_f wn)
+    float wa_f;
     const signed char *kx;            // [n] fp16 scale exponent of the tile
     const float *tnorm, *tabs, *tss;  // [K]
     const int *texp;                  // [K]
@@ -318,8 +340,6 @@ struct LazyLk {
     float kappa_b;                    // bound per unit of ||t|| ||window||
     float kappa_s;                    // bound per unit of |SS_t / 2| (the reference's running sum starts there)
     u64 *refined;                     // count of entries refined on demand (may be NULL)
-    const float *wlb;                 // [W] largest lower bound over each window's entries
-    const float *bm;                  // [n] largest bound of a flagged entry of each sample
     u32 tag;                          // 2 + pass % 2
     const u32 *tgrp;                  // [K] template group; wn/wa/kx are [group][n] (NULL: one group)
     u64 gstride;                      // n
@@ -329,7 +349,7 @@ struct LazyLk {
 // The bound the tensor-core epilogue used for entry (t, s) (same formula).
 __device__ __forceinline__ float lazy_bound(const LazyLk &z, u32 t, u32 s, float approx) {
     const size_t i = (z.tgrp ? (size_t)z.tgrp[t] * z.gstride : 0) + s;
-    const float sub = 2.98023223876953125e-08f * (ldexpf(z.tabs[t], -(int)z.kx[i]) + ldexpf(z.wa[i], -z.texp[t])) * 1.001f;
+    const float sub = 2.98023223876953125e-08f * (ldexpf(z.tabs[t], -(int)z.kx[i]) + ldexpf(z.wa ? z.wa[i] : z.wa_f * z.wn[i], -z.texp[t])) * 1.001f;
     return z.kappa_b * z.tnorm[t] * z.wn[i] + sub + z.kappa_s * fabsf(z.tss[t]) +
            2.384185791015625e-07f * fabsf(approx);
 }
@@ -430,6 +450,7 @@ k_lazy_freeze(u32 n, u32 L, u32 K, const u32 *__restrict__ idx, const u32 *__res
          g += gridDim.x * warps_per_block) {
         if (lab[g] >= K) continue;
         const u32 p = idx[g];
+        const u32 sup_lo = z.tsup ? z.tsup[2 * lab[g]] : 0u, sup_hi = z.tsup ? z.tsup[2 * lab[g] + 1] : z.C;
         const u32 lo = p + 1 > L ? p + 1 - L : 0;
         const u32 hi = min(n, p + L);
         u32 nref = 0;
@@ -437,7 +458,10 @@ k_lazy_freeze(u32 n, u32 L, u32 K, const u32 *__restrict__ idx, const u32 *__res
             const u32 s = s0 + lane;
             const u32 wd = s / L;
             const bool cand = s < hi && !(wd < W && next_active[wd]);   // not recomputed next pass
+            if (!__any_sync(0xffffffffu, cand)) continue;
             for (u32 t = 0; t < K; t++) {
+                // templates without a channel of the spike's read no changing sample
+                if (z.tsup && (z.tsup[2 * t] >= sup_hi || z.tsup[2 * t + 1] <= sup_lo)) continue;
                 const size_t e = (size_t)t * n + s;
                 u32 nm = __ballot_sync(0xffffffffu, cand && z.apx[e] == 1);
                 while (nm) {
@@ -485,6 +509,9 @@ k_window_argmax(u32 n, u32 L, u32 K, const u32 *__restrict__ win,
         const u32 sw = id * L, ew = (id + 1) * L;
         const u32 start = (L > sw) ? 0 : sw - L;
         const u32 stop = (ew + L) > n ? n : ew + L;
+        // the window's groups have just been computed
+        if (wb.dirty)
+            for (u32 k = lane; k < wb.GW; k += 32) wb.dirty[(size_t)id * wb.GW + k] = 0;
         if (ew >= n - L) continue;                       // .cl:380-383
         // Approximate entries (tensor-core path): lb = the largest lower
         // bound over windows id-1..id+1, which is the range [start, stop).
@@ -492,10 +519,12 @@ k_window_argmax(u32 n, u32 L, u32 K, const u32 *__restrict__ win,
         // cannot hold it, so only entries that reach lb need their
         // reference value; every other one is read as stored (< lb).
         float lb = 0.0f;
+        bool check = false;
         if (wb.wlb) {
-            lb = wb.wlb[id];
-            if (id > 0) lb = fmaxf(lb, wb.wlb[id - 1]);
-            if (id + 1 < W) lb = fmaxf(lb, wb.wlb[id + 1]);
+            const u32 glo = (id > 0 ? id - 1 : 0) * wb.G, ghi = min(id + 2, W) * wb.G;
+            for (u32 k = glo + lane; k < ghi; k += 32) lb = fmaxf(lb, wb.wlb[k]);
+            for (u32 k = lane; k < wb.G; k += 32) check |= wb.wpos[(size_t)id * wb.G + k] != 0;
+            lb = warp_max_float(lb);
         }
         // With window bounds only templates whose upper bound over windows
         // id-1..id+1 reaches lb (and 0) can hold the maximum or tie it: the
@@ -504,7 +533,6 @@ k_window_argmax(u32 n, u32 L, u32 K, const u32 *__restrict__ win,
         u32 nref = 0;
         float bl = 0.0f;                                 // .cl:389-393 (template 0 resets)
         u32 blab = best_lab[id], bidx = best_idx[id];
-        bool check = bounded && wb.wpos[id] != 0;
         for (u32 t0 = 0; t0 < K; t0 += 32) {
           bool cand = t0 + lane < K;
           if (bounded && cand) {
@@ -527,7 +555,8 @@ k_window_argmax(u32 n, u32 L, u32 K, const u32 *__restrict__ win,
                 float cur = in ? row[s] : -INFINITY;
                 check |= in && cur > 0.0f && s >= sw && s < ew;   // a flagged entry is > 0 either way
                 bool need = false;
-                if (z.apx && in && cur + z.bm[s] >= lb) {
+                // a flagged entry is certainly > 0, so its value is below twice its approximation
+                if (z.apx && in && cur > 0.0f && 2.001f * cur >= lb) {
                     const u32 f = z.apx[(size_t)t * n + s];
                     need = (f == 1 || f == z.tag) && cur + lazy_bound(z, t, s, cur) >= lb;
                 }
@@ -849,18 +878,37 @@ __global__ void k_accept_flags(AcceptView a, u8 *__restrict__ flags_out) {
     }
 }
 
-// Spike payload of an accepting window (.cl:971-976, 1057-1061).
+// Spike payload of an accepting window (.cl:971-976, 1057-1061), and the
+// (window, template group) pairs whose likelihoods the spike's subtraction
+// will change.
 __global__ void k_gather_spikes(u32 n, u32 C, u32 L, const u32 *__restrict__ list,
                                 const u32 *__restrict__ n_list_dev, const u32 *__restrict__ best_idx,
                                 const u32 *__restrict__ best_lab, u32 *__restrict__ out_idx,
-                                u32 *__restrict__ out_lab, u32 *__restrict__ out_win) {
+                                u32 *__restrict__ out_lab, u32 *__restrict__ out_win, WinBounds wb,
+                                const u32 *__restrict__ grange, const u32 *__restrict__ tsup, u32 K) {
     const u32 m = *n_list_dev;
     for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < m; g += gridDim.x * blockDim.x) {
         const u32 id = list[g];
         const bool valid = ((id + 1) * L < n - L) && C > 0;
-        out_idx[g] = valid ? best_idx[id] : 0;
-        out_lab[g] = valid ? best_lab[id] : 0;
+        const u32 p = valid ? best_idx[id] : 0, lab = valid ? best_lab[id] : 0;
+        out_idx[g] = p;
+        out_lab[g] = lab;
         if (out_win) out_win[g] = id;
+        if (wb.dirty && lab < K) {
+            // the subtraction changes samples [p, p + L) on the template's
+            // channels: entries of outputs p - L + 1 .. p + L - 1 of the groups
+            // whose channels meet them
+            const u32 w0 = (p + 1 > L ? p + 1 - L : 0) / L, w1 = min((p + L - 1) / L, (n + L - 1) / L - 1);
+            const u32 lo = tsup[2 * lab], hi = tsup[2 * lab + 1];
+            for (u32 k = 0; k < wb.GW; k++) {
+                u32 bits = 0;
+                for (u32 b = 0; b < 32 && 32 * k + b < wb.G; b++) {
+                    const u32 q = 32 * k + b;
+                    bits |= (grange[2 * q] < hi && grange[2 * q + 1] > lo ? 1u : 0u) << b;
+                }
+                for (u32 w = w0; bits && w <= w1; w++) atomicOr(wb.dirty + (size_t)w * wb.GW + k, bits);
+            }
+        }
     }
 }
 

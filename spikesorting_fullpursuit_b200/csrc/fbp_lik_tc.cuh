@@ -97,10 +97,11 @@ struct TcArgs {
     float *dbgE;                     // MODE 0, testing: when set, the bound E of every entry ([K][n])
     u8 *apx;                         // [K][n] approximate-entry flags
     float *wn_s, *wa_s;              // [n] per-sample window norms
-    float *bm_s;                     // [n] largest bound of a flagged entry of the sample
-    float *wlb;                      // [W] largest lower bound over a window's entries
+    float *wlb;                      // [W][G16] largest lower bound over a window's entries (this group's
+                                     // first 16 templates stand for all of them)
+    u32 G16, g16;                    // groups of 16 templates, this group's first
     float *umax;                     // [W][Kall] largest upper bound of a template's entries in a window
-    u8 *wpos;                        // [W] some entry of the window is > 0
+    u8 *wpos;                        // [W][G16] some entry of the window is > 0
     signed char *kx_s;               // [n] per-sample fp16 scale exponent
     // overlap-table tiles (MODE 1): rows are the shifts b of a candidate window
     u32 S, nmax, stiles;
@@ -113,7 +114,7 @@ struct TcArgs {
 
 // Shared memory of the tensor-core kernel (nbuf strip buffers).
 struct TcSmem {
-    size_t Bs, As, rowsq, rowab, tsc, tsa, ctk, ctb, ctss, cta, ctrow, tinfo, bars, misc, tcnt, bmh, total;
+    size_t Bs, As, rowsq, rowab, tsc, tsa, ctk, ctb, ctss, cta, ctrow, tinfo, bars, misc, tcnt, total;
 };
 __host__ __device__ inline TcSmem tc_smem_layout(u32 L, u32 Cg2, u32 Np, u32 nbuf) {
     const size_t rows_pad = (kTcM + L - 1 + 7) / 8 * 8;
@@ -135,7 +136,6 @@ __host__ __device__ inline TcSmem tc_smem_layout(u32 L, u32 Cg2, u32 Np, u32 nbu
     m.bars = o;  o += 8 * 8;                                // full[2], empty[2], staged[2], templates
     m.misc = o;  o += 64;                                   // tmem slot, segment info, reductions, abort
     m.tcnt = o;  o += (size_t)Np * 4;                       // per-template counters of the tile
-    m.bmh = o;   o += (size_t)kTcM * 4;                     // second half's largest flagged bound per row
     m.total = o;
     return m;
 }
@@ -300,7 +300,6 @@ k_lik_tc(const TcArgs *__restrict__ gargs, u32 ngroups) {
     u32 *misc = (u32 *)(tsm + lay.misc);
     u32 *tmem_slot = misc, *seg_info = misc + 1, *pred = misc + 4, *abort_flag = misc + 12;
     u32 *tcnt = (u32 *)(tsm + lay.tcnt);
-    float *bmh = (float *)(tsm + lay.bmh);
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const u32 wlim = A.wait_polls;                   // pipeline waits (a test may shorten them)
     // MODE 0 tiles: one listed window (L > 64 may take several tiles), or
@@ -663,7 +662,7 @@ k_lik_tc(const TcArgs *__restrict__ gargs, u32 ngroups) {
             // overwrites them before anything reads them).  Branch-free, and
             // every index is known at compile time (no local memory).
             u32 wantbits[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // Np <= 256: word k holds chunks k of both halves
-            float lomax = 0.0f, bmax = 0.0f;
+            float lomax = 0.0f;
             const bool tail = s + L >= n;                // .cl:231-234
             // this warp's rows lie in windows wlo..whi (one window per tile
             // when wpt == 1; with block tiles L >= 32, so at most two)
@@ -704,7 +703,6 @@ k_lik_tc(const TcArgs *__restrict__ gargs, u32 ngroups) {
                     const bool pos = approx - E > 0.0f;      // certainly > 0: refined when a decision needs it
                     const bool neg = approx + E <= 0.0f;     // certainly <= 0: only its sign is read
                     lomax = real ? fmaxf(lomax, approx - E) : lomax;
-                    bmax = (real && pos) ? fmaxf(bmax, E) : bmax;
                     cw |= (real && !tail && !pos && !neg) ? (1u << q) : 0u;
                     if (real) {
                         *dst = tail ? 0.0f : approx;
@@ -714,7 +712,7 @@ k_lik_tc(const TcArgs *__restrict__ gargs, u32 ngroups) {
                     uq[q] = (real && !tail) ? fmaxf(0.0f, approx + E) : 0.0f;
                     anypos |= real && !tail && pos;
                 }
-                if (tail) lomax = 0.0f, bmax = 0.0f;
+                if (tail) lomax = 0.0f;
                 word |= cw << shift;
                 }
                 // per (window, template): the largest upper bound over the
@@ -752,24 +750,18 @@ k_lik_tc(const TcArgs *__restrict__ gargs, u32 ngroups) {
                     chunk(ColW<16>{}, c0, wantbits[k], 16 * half);
                 }
             }
-            if (__any_sync(0xffffffffu, anypos && myw == wlo) && lane == 0) A.wpos[wlo] = 1;
-            if (whi != wlo && __any_sync(0xffffffffu, anypos && myw == whi) && lane == 0) A.wpos[whi] = 1;
+            if (__any_sync(0xffffffffu, anypos && myw == wlo) && lane == 0) A.wpos[(size_t)wlo * A.G16 + A.g16] = 1;
+            if (whi != wlo && __any_sync(0xffffffffu, anypos && myw == whi) && lane == 0) A.wpos[(size_t)whi * A.G16 + A.g16] = 1;
             // accumulator b and the row sums are no longer needed
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_empty(b));
-            if (in_win && lomax > 0.0f) atomicMax(reinterpret_cast<int *>(A.wlb) + s / L, __float_as_int(lomax));
-            if (half == 1) bmh[row] = bmax;
+            if (in_win && lomax > 0.0f) 
+                atomicMax(reinterpret_cast<int *>(A.wlb) + (size_t)(s / L) * A.G16 + A.g16, __float_as_int(lomax));
             u32 nwant = 0;
 #pragma unroll
             for (int wd = 0; wd < 8; wd++) nwant += __popc(wantbits[wd]);
-            const bool anywant = named_bar_or(2, kTcEpiThreads, nwant != 0);   // also publishes bmh
-            // largest flagged bound of the sample over every template group
-            // (reset when its window is listed for recomputation)
-            if (half == 0 && in_win) {
-                const float bmv = fmaxf(bmax, bmh[row]);
-                if (bmv > 0.0f) atomicMax(reinterpret_cast<int *>(A.bm_s) + s, __float_as_int(bmv));
-            }
+            const bool anywant = named_bar_or(2, kTcEpiThreads, nwant != 0);
             if (anywant) {
                 // phase 2: one contiguous segment of (template, sample)
                 // entries per tile, ordered by template so the refinement
@@ -908,7 +900,7 @@ k_tc_refine(const float *__restrict__ vall, u32 n, u32 Call, u32 Cmax, const flo
             const u32 *__restrict__ seg_s0, const u32 *__restrict__ seg_base, const u32 *__restrict__ seg_cnt,
             const u32 *__restrict__ seg_grp, const u32 *__restrict__ gdesc, const u32 *__restrict__ tperm,
             const u32 *__restrict__ seg_count, u32 seg_cap, float *__restrict__ Lk, LazyLk z, double gamma,
-            u64 *__restrict__ n_seq, u8 *__restrict__ wpos, const u32 *__restrict__ overflow, u32 ref_cap) {
+            u64 *__restrict__ n_seq, u8 *__restrict__ wpos, u32 G16, const u32 *__restrict__ overflow, u32 ref_cap) {
     extern __shared__ float rsm[];
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float *wbuf = rsm + (size_t)warp * kWarpChunk;
@@ -954,10 +946,7 @@ k_tc_refine(const float *__restrict__ vall, u32 n, u32 Call, u32 Cmax, const flo
                     Lk[idx] = xf;
                     if (X - bnd > 0.0) {                 // certainly > 0: refined on demand
                         z.apx[idx] = 1;
-                        wpos[(s0 + so) / L] = 1;
-                        const u32 s = s0 + so;
-                        atomicMax(reinterpret_cast<int *>(const_cast<float *>(z.bm)) + s,
-                                  __float_as_int(lazy_bound(z, t, s, xf)));
+                        wpos[(size_t)((s0 + so) / L) * G16 + t0 / 16] = 1;
                     }
                 }
                 continue;
@@ -976,7 +965,7 @@ k_tc_refine(const float *__restrict__ vall, u32 n, u32 Call, u32 Cmax, const flo
             }
             if (lane == 0) {
                 Lk[idx] = acc;
-                if (acc > 0.0f) wpos[(s0 + so) / L] = 1;
+                if (acc > 0.0f) wpos[(size_t)((s0 + so) / L) * G16 + t0 / 16] = 1;
                 nseq++;
             }
         }

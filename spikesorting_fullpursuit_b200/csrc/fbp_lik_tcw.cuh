@@ -16,13 +16,21 @@
 // sample-major kernel (fbp_lik_tc.cuh) does 128 x (templates in a group) x 16.
 // A (the shifted templates) is packed once per chunk (k_tcw_pack) and
 // streamed per channel into a ring of shared-memory stages with one bulk
-// asynchronous copy.  The channel's fp32 voltage reaches a staging slot by
-// coalesced 4-byte asynchronous copies, kWDepth - 1 channels ahead, and the
-// producers convert it to fp16 into the stage.  Accumulators are FP32 in
-// tensor memory (two tiles of 256 columns).
+// asynchronous copy.  Accumulators are FP32 in tensor memory (two tiles of
+// 256 columns).
 //
-// The stream.  A pass lists windows w (ascending).  Their outputs are laid
-// end to end: listed window i of the list starts at stream position
+// What a pass computes.  A window's likelihoods under a template change only
+// when a spike's subtraction touches samples the window's outputs read, on the
+// template's channels.  Per window, a bit per group of 16 templates says
+// whether that has happened since the group's last computation (dirty;
+// k_gather_spikes sets it, the window argmax clears it), and a group computes
+// the listed windows with its bit set: the others hold the values a
+// recomputation from the same voltage would give.  On the 384-channel probe,
+// whose templates cover 16 channels, that leaves about a fifth of the (window,
+// group) pairs of a pursuit.
+//
+// The stream.  A group's windows w of a pass (ascending) are laid end to end:
+// window i of its list starts at stream position
 //     pos_i = i * L + R_i * (L - 1),
 // R_i = the number of runs of consecutive windows before it, so a run is
 // contiguous and every run is followed by L - 1 positions that continue its
@@ -51,75 +59,98 @@ constexpr u32 kWN = 256;                 // MMA N: blocks of 8 samples per tile
 constexpr u32 kWPos = 8 * kWN;           // 2048 stream positions per tile
 constexpr u32 kWTwMax = 136;             // listed windows a tile can touch (L >= kWMinL)
 constexpr u32 kWMinL = 16;
-constexpr u32 kWMaxStages = 8;
 constexpr u32 kWATile = 4096;            // one A tile: 128 rows x 16 lags x fp16
-constexpr u32 kWDepth = 3;               // channels of voltage in flight (fp32 staging slots)
-constexpr u32 kWTail = 0x80000000u;      // stream table: a kept output in the zeroed tail (n < 2^31)
-
 __host__ __device__ inline u32 tcw_nkc(u32 L) { return (L + 7 + 15) / 16; }
 __host__ __device__ inline u32 tcw_px(u32 L) { return kWPos + 16 * tcw_nkc(L); }   // staged positions
 
+// One template group (16 templates in support order).
 struct TcwArgs {
-    u32 n, Cg, nt, L, nkc, ns, px, Kall, W;
+    u32 Cg, nt;                      // channels of the union of its supports, templates
     const u32 *trow;                 // [nt] template of each group column
-    float kappa_b, kappa_s;
     const float *v;                  // channel clo of the recording ([Cg][n] from there)
+    const unsigned char *Aw;         // [Cg][nkc] A tiles
+};
+struct TcwParams {
+    u32 n, L, ns, G, Kall, W, wstride, fstride;
+    const TcwArgs *groups;           // [G]
+    float kappa_b, kappa_s;
     const float *tss, *tnorm, *tabs;
     const int *texp;
-    const unsigned char *Aw;         // [Cg][nkc] A tiles of this group
     const float *vwmax;              // [W + 2] largest |v| of each window over all channels
-    const u32 *win, *n_win;          // the pass's window list
-    const u32 *pos, *first, *n_stiles;   // stream position of each listed window; first listed
-                                         // window of each tile; tiles of the stream
+    const u32 *win, *pos;            // [G][wstride] the group's windows of this pass, their stream positions
+    const u32 *first;                // [G][fstride] first window of each tile of the group's stream
+    const u32 *n_win, *n_stiles;     // [G] windows, tiles of the stream
     float *Lk;                       // [Kall][n]
     u8 *apx;                         // [Kall][n]
     float *dbgE;                     // testing: when set, the bound E of every entry ([Kall][n])
-    float *wn_s, *wa_s;              // [n] this group's window norms
-    signed char *kx_s;               // [n] this group's fp16 scale exponents
-    float *bm_s, *wlb, *umax;
-    u8 *wpos;
+    float *wn_s;                     // [G][n] window norms
+    float wa_f;                      // a window's L1 norm is at most wa_f times its L2 norm
+    signed char *kx_s;               // [G][n] fp16 scale exponents
+    float *wlb, *umax;               // [W][G], [W][Kall]
+    u8 *wpos;                        // [W][G]
     u32 *ref_t, *ref_s;
     unsigned long long *refseg;
     u32 ref_cap;
     u32 *seg_s0, *seg_base, *seg_cnt, *seg_grp;
-    u32 grp;
     u32 *seg_overflow;
     u32 seg_cap;
     u32 *err;
     u32 wait_polls;
 };
 
-static_assert(sizeof(TcwArgs) % 4 == 0, "TcwArgs is copied as 32-bit words");
+// Warp roles: 4 table warps (the tile's table, position map and window
+// norms), up to 7 producer warps (one per ring stage), 1 MMA warp, 8 epilogue
+// warps.
+constexpr int kWTabWarps = 4, kWTabThreads = 32 * kWTabWarps;
+constexpr int kWProdWarp0 = kWTabWarps, kWProdWarps = 7;
+constexpr int kWMmaWarp = kWProdWarp0 + kWProdWarps;
+constexpr int kWEpiWarp0 = kWMmaWarp + 1, kWEpiWarps = 8, kWEpiThreads = 32 * kWEpiWarps;
+constexpr int kWThreads = 32 * (kWEpiWarp0 + kWEpiWarps);
+static_assert(kWEpiWarp0 % 4 == 0, "epilogue warp w reads TMEM lanes 32 (w % 4)..");
+// ||window||_1 <= sqrt(terms) ||window||_2: it only scales the subnormal term of
+// the bound, 2^-13 of the main one at most.
+__host__ __device__ inline float tcw_l1_factor(u32 Cmax, u32 L) { return 1.001f * sqrtf((float)Cmax * (float)L); }
+// Windows a tile's table can hold for this L (kWTwMax at L = kWMinL).
+__host__ __device__ inline u32 tcw_entries(u32 L) {
+    const u32 e = tcw_px(L) / L + 3;
+    return e < kWTwMax ? e : kWTwMax;
+}
+constexpr u32 kWMaps = 3;                // position maps in flight: built, read by producers, by the epilogue
+constexpr u32 kWLoads = 24;              // voltage loads of a producer lane in flight
+
+struct TcwInfo {                         // per map: the tile
+    u32 g, Cg;
+    int kexp;
+    float kscale;
+    u32 gt[16];                          // template of each group column
+    float ck[16], cb[16], css[16], ca[16], tsc[16], tsa[16];
+    int texp[16];
+};
 struct TcwSmem {
-    size_t args, ring, stage, a_bytes, vst, spos, wnwa, wrel, tw, cw, tf, ti, psq, pab, tpos, twin, xs, xe, ct, bars,
-        misc, tcnt, total;
+    size_t ring, stage, a_bytes, map, map_bytes, smap, wrel, tw, es, info, tpos, twin, nrm, um, wl, bars, misc, tcnt, total;
 };
 __host__ __device__ inline TcwSmem tcw_smem_layout(u32 L, u32 ns) {
-    const size_t nkc = tcw_nkc(L), px = tcw_px(L);
+    const size_t nkc = tcw_nkc(L), px = tcw_px(L), rows = px / 8;
     TcwSmem m;
     m.a_bytes = nkc * kWATile;
     m.stage = align_up(m.a_bytes + align_up(px * 2, 16), 128);
     size_t o = 0;
-    m.args = o;  o += align_up(sizeof(TcwArgs), 128);     // the launch arguments (shared-memory copy)
+    m.smap = o;  o += px * 4;                             // sample of every staged position, ~0 past the recording
+    m.es = o;    o += rows * 4;                           // energies of the blocks of 8
+    m.info = o;  o += sizeof(TcwInfo);
+    m.tw = o;    o += (size_t)kWTwMax * 4;                // window of each table entry
+    m.wrel = o;  o += kWPos;                              // table entry of a kept output, else 0xff
+    m.map_bytes = align_up(o, 16);
+    o = 0;
     m.ring = o;  o += ns * m.stage;                       // A tiles + voltage stream per channel
-    m.vst = o;   o += (size_t)kWDepth * px * 4;            // producers: fp32 voltage of the next channels
-    m.spos = o;  o += 2 * (size_t)kWPos * 4;               // per tile: sample of a kept output, else ~0
-    m.wnwa = o;  o += 2 * (size_t)kWPos * 8;               // per tile: window L2 / L1 norms
-    m.wrel = o;  o += 2 * (size_t)kWPos;                   // per tile: table entry of a kept output, else 0xff
-    m.tw = o;    o += 2 * (size_t)kWTwMax * 4;             // per tile: window of each table entry
-    m.cw = o;    o += 2 * 16 * 4;                          // per tile, per 128 positions: first | last entry << 16
-    m.tf = o;    o += 2 * 32 * 4;                          // per tile: tsc[16], tsa[16]
-    m.ti = o;    o += 2 * 16;                              // per tile: kexp
+    m.map = o;   o += kWMaps * m.map_bytes;
+    m.tpos = o;  o += (size_t)(kWTwMax + 1) * 4;          // table warps: stream position and window of each entry
+    m.twin = o;  o += (size_t)(kWTwMax + 1) * 4;
+    m.nrm = o;   o += 2 * (size_t)kWN * 4;                // epilogue: window norms per block of 8, two spans
+    m.um = o;    o += (size_t)16 * tcw_entries(L) * 4;    //           upper bounds per (template, window)
+    m.wl = o;    o += (size_t)tcw_entries(L) * 4;         //           lower bounds per window
     o = align_up(o, 8);
-    m.psq = o;   o += (px + 1) * 8;                        // producers: prefix sums of row energies
-    m.pab = o;   o += (px + 1) * 8;                        //            and of row absolute sums
-    m.tpos = o;  o += (size_t)(kWTwMax + 1) * 4;           //            tile table: stream position
-    m.twin = o;  o += (size_t)(kWTwMax + 1) * 4;           //            and window of each entry
-    m.xs = o;    o += (px - kWPos) * 4;                    //            samples of the positions past 2048
-    m.xe = o;    o += 2 * (px - kWPos) * 4;                //            and their energy / absolute sums
-    m.ct = o;    o += 16 * 4 * 5;                          // template constants
-    o = align_up(o, 8);
-    m.bars = o;  o += (size_t)(2 * ns + 9) * 8;
+    m.bars = o;  o += (size_t)(2 * ns + 5 + 3 * kWMaps) * 8;
     m.misc = o;  o += 256;
     m.tcnt = o;  o += 16 * 4;
     m.total = o;
@@ -146,96 +177,93 @@ __device__ __forceinline__ double warp_incl_scan_d(double v, u32 lane) {
     }
     return v;
 }
-// 4-byte asynchronous copy global -> shared; src_bytes 0 writes a zero
-// (nothing is read)
-__device__ __forceinline__ void cp_async4(u32 dst, const float *src, u32 src_bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ u16 half_bits_clamped(float f) {
     return __half_as_ushort(__float2half_rn(fminf(fmaxf(f, -65504.0f), 65504.0f)));
 }
 
-// Persistent, one CTA per SM, 17 warps: 8 producers (tile tables, voltage
-// stream per channel, window norms), 1 MMA warp, 8 epilogue warps (two per
-// TMEM lane quadrant, one half of the 256 columns each).  The launch
-// arguments are copied into shared memory first.  Barriers:
-//   stage_full[s]  producers wrote the stream (one arrive) and the A copy landed (tx);
-//   stage_empty[s] the MMAs that read stage s are done (tcgen05.commit);
+// Persistent, one CTA per SM, 20 warps.  The tiles of all groups' streams form
+// one sequence; CTA b takes tiles b, b + gridDim, ...
+//   Table warps, per tile, one tile ahead: the windows that meet it, the sample
+//     of every position, the tile's fp16 scale and per-template factors; then,
+//     as each channel of the tile is staged, the energy of every block of 8
+//     positions from the fp16 values themselves (their rounding is bounded and
+//     added).
+//   Producer warp s fills ring stage s: a channel's voltage by coalesced 4-byte
+//     loads (24 in flight per lane, the first ones issued before the wait for
+//     the stage), scaled, rounded to fp16; one bulk copy brings the channel's A
+//     tiles.  No barrier joins the producers.
+//   The MMA warp issues nkc MMAs per channel.
+//   Epilogue warps (two per TMEM lane quadrant, one half of the columns each)
+//     bound every output's window norm by the blocks that hold its lags,
+//     classify and store; the entries that are not certainly <= 0 update the
+//     per-(window, template) and per-window bounds of the tile in shared
+//     memory, which go to global memory once per tile (global atomics per
+//     entry took 110,000 of 135,000 cycles a tile).
+// Producers that shared every channel over 256 threads with two barriers a
+// channel and built the tables and norms between tiles took 144,000 cycles a
+// tile of 34 channels, against 31,000 of MMA issue.
+// Barriers:
+//   stage_full[s]  the producer arrived and the A copy landed (tx);
+//   stage_empty[s] the MMAs that read stage s are done (tcgen05.commit) and the
+//                  table warps have read it (one arrive each);
 //   acc_full[b]    the tile's MMAs are done (commit);
-//   acc_empty[b]   the epilogue read accumulator b (one arrive per epilogue warp);
-//   info_full[b]   the producers wrote tile b's tables and norms (one arrive);
-//   buf_empty[b]   the epilogue is done with tile b's tables (one arrive per warp).
+//   acc_empty[b]   the epilogue read accumulator b (one arrive per warp);
+//   map_full[k], norm_full[k]  map k is built, its norms are (one arrive each);
+//   map_empty[k]   producers and epilogue are done with map k (one arrive per warp).
 // Every wait is bounded; a wait that gives up sets err and the abort flag.
-__global__ void __launch_bounds__(kTcThreads, 1)
-k_lik_tcw(const TcwArgs *__restrict__ gargs, u32 ngroups) {
-    u32 gi, bi, cnt;
-    {
-        const u32 b = blockIdx.x, base = gridDim.x / ngroups, rem = gridDim.x % ngroups;
-        if (base == 0) {
-            gi = b; bi = 0; cnt = 1;
-        } else if (b < rem * (base + 1)) {
-            gi = b / (base + 1); bi = b % (base + 1); cnt = base + 1;
-        } else {
-            const u32 b2 = b - rem * (base + 1);
-            gi = rem + b2 / base; bi = b2 % base; cnt = base;
-        }
-        if (gi >= ngroups) return;
-    }
-    const TcwArgs &Ag = gargs[gi];
-    const u32 ntiles = *Ag.n_stiles;
-    if (bi >= ntiles) return;                        // no tile for this CTA: no set-up at all
+__global__ void __launch_bounds__(kWThreads, 1)
+k_lik_tcw(const __grid_constant__ TcwParams P) {
+    const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const u32 G = P.G;
+    u32 total = 0;                                   // tiles of all groups
+    for (u32 g = lane; g < G; g += 32) total += P.n_stiles[g];
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (blockIdx.x >= total) return;                 // no tile for this CTA: no set-up at all
     extern __shared__ __align__(128) unsigned char wsm[];
-    // the roles read their arguments from a shared-memory copy (a reload
-    // costs a shared-memory access, not a global one)
-    for (u32 i = threadIdx.x; i < (u32)(sizeof(TcwArgs) / 4); i += blockDim.x)
-        reinterpret_cast<u32 *>(wsm)[i] = reinterpret_cast<const u32 *>(&Ag)[i];
-    const TcwArgs &A = *reinterpret_cast<const TcwArgs *>(wsm);   // valid after the first __syncthreads
-    const u32 L = Ag.L, nkc = Ag.nkc, ns = Ag.ns, px = Ag.px, n = Ag.n, Cg = Ag.Cg;
+    const u32 L = P.L, ns = P.ns, n = P.n, nkc = tcw_nkc(L), px = tcw_px(L);
     const TcwSmem lay = tcw_smem_layout(L, ns);
     unsigned char *ring = wsm + lay.ring;
-    u32 *spos_all = (u32 *)(wsm + lay.spos);
-    float2 *wnwa_all = (float2 *)(wsm + lay.wnwa);
-    u8 *wrel_all = wsm + lay.wrel;
-    u32 *tw_all = (u32 *)(wsm + lay.tw);
-    u32 *cw_all = (u32 *)(wsm + lay.cw);
-    float *tf_all = (float *)(wsm + lay.tf);
-    int *ti_all = (int *)(wsm + lay.ti);
-    double *psq = (double *)(wsm + lay.psq), *pab = (double *)(wsm + lay.pab);
-    int *tpos = (int *)(wsm + lay.tpos);
-    u32 *twin = (u32 *)(wsm + lay.twin);
-    u32 *xs = (u32 *)(wsm + lay.xs);
-    float *xe2 = (float *)(wsm + lay.xe), *xab = xe2 + (px - kWPos);
-    float *ctk = (float *)(wsm + lay.ct), *ctb = ctk + 16, *ctss = ctk + 32, *cta = ctk + 48;
-    u32 *ctrow = (u32 *)(ctk + 64);
+    auto map_of = [&](u32 k) { return wsm + lay.map + (size_t)k * lay.map_bytes; };
     u64 *bars = (u64 *)(wsm + lay.bars);
     u32 *misc = (u32 *)(wsm + lay.misc);
-    u32 *tmem_slot = misc, *seg_info = misc + 1, *abort_flag = misc + 4;
-    float *pred = (float *)(misc + 8);               // [8] producer warp maxima
-    double *dsum = (double *)(misc + 16);            // [16] producer warp sums (two arrays)
+    u32 *tmem_slot = misc, *seg_info = misc + 1, *abort_flag = misc + 4, *fills = misc + 8;   // fills: [ns]
+    float *pred = (float *)(misc + 16);              // [4] table warps' maxima
     u32 *tcnt = (u32 *)(wsm + lay.tcnt);
-    const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const u32 wlim = Ag.wait_polls;
+    const u32 wlim = P.wait_polls;
     auto bar_sfull = [&](u32 s) { return smem_u32(&bars[s]); };
     auto bar_sempty = [&](u32 s) { return smem_u32(&bars[ns + s]); };
     auto bar_afull = [&](u32 b) { return smem_u32(&bars[2 * ns + b]); };
     auto bar_aempty = [&](u32 b) { return smem_u32(&bars[2 * ns + 2 + b]); };
-    auto bar_ifull = [&](u32 b) { return smem_u32(&bars[2 * ns + 4 + b]); };
-    auto bar_bempty = [&](u32 b) { return smem_u32(&bars[2 * ns + 6 + b]); };
-    const u32 bar_fin = smem_u32(&bars[2 * ns + 8]);
+    auto bar_mfull = [&](u32 k) { return smem_u32(&bars[2 * ns + 4 + k]); };
+    auto bar_nfull = [&](u32 k) { return smem_u32(&bars[2 * ns + 4 + kWMaps + k]); };
+    auto bar_mempty = [&](u32 k) { return smem_u32(&bars[2 * ns + 4 + 2 * kWMaps + k]); };
+    const u32 bar_fin = smem_u32(&bars[2 * ns + 4 + 3 * kWMaps]);
+    auto aborted = [&]() { return *(volatile u32 *)abort_flag != 0; };
+    // a wait of one warp: false when it gave up or another role has
+    auto wait_warp = [&](u32 bar, u32 parity, u32 code) -> bool {
+        bool ok = !aborted();
+        if (ok && !mbar_wait_bounded(bar, parity, wlim)) {
+            if (lane == 0) atomicExch(P.err, code);
+            atomicExch(abort_flag, 1u);
+            ok = false;
+        }
+        return __all_sync(0xffffffffu, ok);
+    };
 
     if (tid == 0) {
         for (u32 s = 0; s < ns; s++) {
             mbar_init(bar_sfull(s), 1);
-            mbar_init(bar_sempty(s), 1);
+            mbar_init(bar_sempty(s), 1 + kWTabWarps);
+            fills[s] = 0;
         }
         for (u32 b = 0; b < 2; b++) {
             mbar_init(bar_afull(b), 1);
-            mbar_init(bar_aempty(b), kTcEpiWarps);
-            mbar_init(bar_ifull(b), 1);
-            mbar_init(bar_bempty(b), kTcEpiWarps);
+            mbar_init(bar_aempty(b), kWEpiWarps);
+        }
+        for (u32 k = 0; k < kWMaps; k++) {
+            mbar_init(bar_mfull(k), 1);
+            mbar_init(bar_nfull(k), 1);
+            mbar_init(bar_mempty(k), ns + kWEpiWarps);
         }
         mbar_init(bar_fin, 1);
         *abort_flag = 0;
@@ -246,365 +274,275 @@ k_lik_tcw(const TcwArgs *__restrict__ gargs, u32 ngroups) {
                      ::"r"(smem_u32(tmem_slot)), "r"(2 * kWN));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    for (u32 t = tid; t < 16; t += blockDim.x) {
-        tcnt[t] = 0;
-        const bool real = t < Ag.nt;
-        const u32 gt = real ? Ag.trow[t] : 0u;
-        ctrow[t] = gt;
-        ctk[t] = real ? Ag.kappa_b * Ag.tnorm[gt] : 0.0f;
-        ctb[t] = real ? 2.98023223876953125e-08f * 1.001f * ldexpf(1.0f, -Ag.texp[gt]) : 0.0f;
-        ctss[t] = real ? Ag.tss[gt] : 0.0f;
-        cta[t] = real ? Ag.kappa_s * fabsf(Ag.tss[gt]) : 0.0f;
-    }
+    if (tid < 16) tcnt[tid] = 0;
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const u32 tmem = *tmem_slot;
-    u32 gstage = 0;                                  // producers / MMA: stages used so far
 
-    if (warp < kTcProdWarps) {
-        // =========================== producers ===========================
-        const u32 pt = tid;                          // 0..255
-        const u32 m = *A.n_win;
-        const u32 nB = px - kWPos;                   // staged positions past 2048
-        const bool hasB = 8 * pt < nB;               // this thread packs 8 of them
-        float *vst = (float *)(wsm + lay.vst);       // [kWDepth][px] fp32 voltage (cp.async)
-        u32 use0 = 0u, use1 = 0u;
-        u32 it = 0;
-        for (u32 q = bi; q < ntiles; q += cnt, it++) {
-            const u32 b = it & 1u;
-            const u32 ub = b ? use1 : use0;
-            if (ub > 0 && !mbar_wait_bounded(bar_bempty(b), (ub - 1) & 1u, wlim)) {
-                atomicExch(A.err, 13u);
-                atomicExch(abort_flag, 1u);
+    if (warp < kWTabWarps) {
+        // ======================= tables and norms ========================
+        const u32 tt = tid;                          // 0..127
+        const u32 rows = px / 8;                     // blocks of 8 positions
+        int *tpos = (int *)(wsm + lay.tpos);
+        u32 *twin = (u32 *)(wsm + lay.twin);
+        // builds the map of the CTA's it-th tile; false when a role gave up
+        auto build = [&](u32 f, u32 it) -> bool {
+            const u32 k = it % kWMaps, use = it / kWMaps;
+            unsigned char *mp = map_of(k);
+            u32 *smap = (u32 *)(mp + lay.smap), *tw = (u32 *)(mp + lay.tw);
+            u8 *wrel = mp + lay.wrel;
+            TcwInfo &I = *(TcwInfo *)(mp + lay.info);
+            const bool free_map = use == 0 || wait_warp(bar_mempty(k), (use - 1) & 1u, 13u);
+            if (named_bar_or(3, kWTabThreads, !free_map)) return false;
+            // the tile's group and its place in the group's stream.  Group after
+            // group: tiles computed together write the rows of 16 templates and
+            // read one group's channels (taking every group's tile 0, then tile
+            // 1, ... spreads them over all rows, 1,000 pages of 2 MB on the
+            // 384-channel probe: 17.9 against 10.6 ms for its first pass of 100 s)
+            u32 g = 0, q = f;
+            for (u32 g0 = 0; g0 < G; g0 += 32) {
+                const u32 t = g0 + lane < G ? P.n_stiles[g0 + lane] : 0u;
+                const u32 incl = warp_incl_scan(t);
+                const u32 m = __ballot_sync(0xffffffffu, q < incl);
+                if (m) {
+                    const u32 src = __ffs(m) - 1;
+                    g = g0 + src;
+                    q -= __shfl_sync(0xffffffffu, incl - t, src);
+                    break;
+                }
+                q -= __shfl_sync(0xffffffffu, incl, 31);
             }
-            if (named_bar_or(1, kTcProdThreads, *(volatile u32 *)abort_flag != 0)) break;
-            u32 *spos = spos_all + (size_t)b * kWPos;
-            float2 *wnwa = wnwa_all + (size_t)b * kWPos;
-            u8 *wrel = wrel_all + (size_t)b * kWPos;
-            u32 *tw = tw_all + (size_t)b * kWTwMax;
-            u32 *cw = cw_all + b * 16;
-            float *tsc = tf_all + b * 32, *tsa = tsc + 16;
-            // ---- the tile's table: listed windows whose outputs or lags meet
-            //      stream positions [Q0, Q0 + px)
+            const TcwArgs &T = P.groups[g];
+            // the windows whose outputs or lags meet positions [Q0, Q0 + px)
             const long long Q0 = (long long)q * kWPos;
-            const u32 i_lo = A.first[q];
-            bool in = false;
-            if (pt <= kWTwMax) {
-                const u32 i = i_lo + pt;
-                in = i < m && (long long)A.pos[i] < Q0 + (long long)px;
-                if (in && pt < kWTwMax) {
-                    tpos[pt] = (int)((long long)A.pos[i] - Q0);
-                    twin[pt] = A.win[i];
-                    tw[pt] = A.win[i];
-                }
-                if (in && pt == kWTwMax) {           // cannot happen for L >= kWMinL
-                    atomicExch(A.err, 15u);
+            const u32 m = P.n_win[g], i_lo = P.first[(size_t)g * P.fstride + q];
+            const u32 *gpos = P.pos + (size_t)g * P.wstride, *gwin = P.win + (size_t)g * P.wstride;
+            u32 nw = 0;
+            float mx = 0.0f;
+            for (u32 b0 = 0; b0 < kWTwMax + 1; b0 += kWTabThreads) {
+                const u32 e = b0 + tt, i = i_lo + e;
+                bool in = e <= kWTwMax && i < m && (long long)gpos[i] < Q0 + (long long)px;
+                if (in && e == kWTwMax) {            // cannot happen for L >= kWMinL
+                    atomicExch(P.err, 15u);
                     atomicExch(abort_flag, 1u);
+                    in = false;
                 }
+                if (in) {
+                    const u32 w = gwin[i];
+                    tpos[e] = (int)((long long)gpos[i] - Q0);
+                    twin[e] = w;
+                    tw[e] = w;
+                    // every sample a kept output multiplies by a non-zero
+                    // template value lies in its window or the next
+                    mx = fmaxf(mx, fmaxf(P.vwmax[w], P.vwmax[w + 1]));
+                }
+                nw += named_bar_popc(3, kWTabThreads, in);          // also publishes the table
             }
-            const u32 nw = named_bar_popc(1, kTcProdThreads, in && pt < kWTwMax);   // also publishes the table
-            if (nw == 0 || tpos[0] > 0) {            // the stream kernels guarantee an entry at or before Q0
-                if (pt == 0) { atomicExch(A.err, 16u); atomicExch(abort_flag, 1u); }
-                break;
+            if (nw == 0 || tpos[0] > 0) {            // the list kernels guarantee an entry at or before Q0
+                if (tt == 0) { atomicExch(P.err, 16u); atomicExch(abort_flag, 1u); }
+                nw = 0;
             }
-            // ---- positions -> samples (this thread: 8pt.. in registers and,
-            //      past 2048, 2048 + 8pt.. in shared memory)
-            u32 smpA[8], smpB[8];
-            auto map8 = [&](u32 x0, u32 (&smp)[8], bool kept_out) -> u32 {
-                // last entry with tpos <= x0 (binary search), then step
-                u32 lo = 0, hi = nw - 1;
+            mx = warp_max_float(mx);
+            if (lane == 0) pred[warp] = mx;
+            if (named_bar_or(3, kWTabThreads, nw == 0 || aborted())) return false;
+            float mm = 0.0f;
+            for (int w4 = 0; w4 < kWTabWarps; w4++) mm = fmaxf(mm, pred[w4]);
+            int kexp = 0;
+            if (mm > 0.0f) {
+                int e;
+                frexpf(mm, &e);                      // mm < 2^e
+                kexp = max(-126, min(126, 14 - e));  // scaled magnitudes < 2^14
+            }
+            if (tt == 0) {
+                I.g = g;
+                I.Cg = T.Cg;
+                I.kexp = kexp;
+                I.kscale = ldexpf(1.0f, kexp);       // exact: |kexp| <= 126
+            }
+            if (tt < 16) {
+                const bool real = tt < T.nt;
+                const u32 gt = real ? T.trow[tt] : 0u;
+                const int te = real ? P.texp[gt] : 0, ex = -(kexp + te);
+                I.gt[tt] = real ? gt : 0xffffffffu;
+                I.texp[tt] = te;
+                I.ck[tt] = real ? P.kappa_b * P.tnorm[gt] : 0.0f;
+                I.cb[tt] = real ? 2.98023223876953125e-08f * 1.001f * ldexpf(1.0f, -te) : 0.0f;
+                I.css[tt] = real ? P.tss[gt] : 0.0f;
+                I.ca[tt] = real ? P.kappa_s * fabsf(P.tss[gt]) : 0.0f;
+                I.tsc[tt] = (real && ex >= -149 && ex <= 127) ? ldexpf(1.0f, ex) : 0.0f;   // exact power of two
+                I.tsa[tt] = real ? 2.98023223876953125e-08f * 1.001f * ldexpf(P.tabs[gt], -kexp) : 0.0f;
+            }
+            for (u32 r = tt; r < rows; r += kWTabThreads) {          // 8 positions of a block
+                const u32 x0 = 8 * r;
+                u32 lo = 0, hi = nw - 1;             // last entry with tpos <= x0
                 while (lo < hi) {
                     const u32 mid = (lo + hi + 1) >> 1;
                     if (tpos[mid] <= (int)x0) lo = mid; else hi = mid - 1;
                 }
-                u32 j = lo, kept = 0;
+                u32 j = lo, sv[8], wv[2] = {0u, 0u};
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
                     const u32 x = x0 + e;
                     while (j + 1 < nw && tpos[j + 1] <= (int)x) j++;
                     const u32 o = (u32)((int)x - tpos[j]);
                     const u32 s = twin[j] * L + o;
-                    smp[e] = s;
-                    if (kept_out) {
-                        const bool k = o < L && s < n;
-                        // bit 31: the output is the reference's zeroed tail (.cl:231-234)
-                        spos[x] = k ? (s | (s + L >= n ? kWTail : 0u)) : 0xffffffffu;
-                        wrel[x] = k ? (u8)j : (u8)0xff;
-                        kept |= k ? (1u << e) : 0u;
-                    }
+                    sv[e] = s < n ? s : 0xffffffffu;
+                    wv[e >> 2] |= ((o < L && s < n) ? j : 0xffu) << (8 * (e & 3));
                 }
-                return kept;
-            };
-            map8(8 * pt, smpA, true);              // spos / wrel of this thread's positions
-            if (hasB) {
-                map8(kWPos + 8 * pt, smpB, false);
+                *reinterpret_cast<uint4 *>(smap + x0) = make_uint4(sv[0], sv[1], sv[2], sv[3]);
+                *reinterpret_cast<uint4 *>(smap + x0 + 4) = make_uint4(sv[4], sv[5], sv[6], sv[7]);
+                if (x0 < kWPos) *reinterpret_cast<uint2 *>(wrel + x0) = make_uint2(wv[0], wv[1]);
+            }
+            named_bar(3, kWTabThreads);
+            if (tt == 0) mbar_arrive(bar_mfull(k));  // release: the barrier ordered every write
+            return true;
+        };
+        u32 gs0 = 0, it = 0;                         // ring uses before this tile
+        bool ok = build(blockIdx.x, 0);
+        for (u32 f = blockIdx.x; ok && f < total; f += gridDim.x, it++) {
+            if (f + gridDim.x < total && !build(f + gridDim.x, it + 1)) break;
+            const u32 k = it % kWMaps;
+            unsigned char *mp = map_of(k);
+            const TcwInfo &I = *(const TcwInfo *)(mp + lay.info);
+            const u32 Cg = I.Cg;
+            float e2[3][2];
 #pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    xs[8 * pt + e] = smpB[e];
-                    xe2[8 * pt + e] = 0.0f;
-                    xab[8 * pt + e] = 0.0f;
-                }
-            }
-            // per 128-position chunk: the table entries whose outputs meet it
-            if (pt < 16) {
-                const int c0 = 128 * (int)pt, c1 = c0 + 128;
-                u32 lo = 0, hi = nw - 1;             // last entry starting at or before c0
-                while (lo < hi) {
-                    const u32 mid = (lo + hi + 1) >> 1;
-                    if (tpos[mid] <= c0) lo = mid; else hi = mid - 1;
-                }
-                const u32 wf = (tpos[lo] + (int)L > c0) ? lo : lo + 1;
-                u32 wl = lo;                         // last entry starting before c1
-                while (wl + 1 < nw && tpos[wl + 1] < c1) wl++;
-                cw[pt] = wf | (wl << 16);
-            }
-            // ---- the tile's fp16 scale: every sample a kept output multiplies
-            //      by a non-zero template value lies in its window or the next
-            float mx = 0.0f;
-            if (pt < nw) mx = fmaxf(A.vwmax[twin[pt]], A.vwmax[twin[pt] + 1]);
-            mx = warp_max_float(mx);
-            if (lane == 0) pred[warp] = mx;
-            named_bar(1, kTcProdThreads);
-            int kexp = 0;
-            {
-                float mm = 0.0f;
-                for (int w8 = 0; w8 < kTcProdWarps; w8++) mm = fmaxf(mm, pred[w8]);
-                if (mm > 0.0f) {
-                    int e;
-                    frexpf(mm, &e);                  // mm < 2^e
-                    kexp = max(-126, min(126, 14 - e));   // scaled magnitudes < 2^14
-                }
-            }
-            if (pt == 0) ti_all[b * 4] = kexp;
-            if (pt < 16) {
-                float sc = 0.0f, sa = 0.0f;
-                if (pt < A.nt) {
-                    const u32 gt = ctrow[pt];
-                    const int ex = -(kexp + A.texp[gt]);
-                    if (ex >= -149 && ex <= 127) sc = ldexpf(1.0f, ex);   // exact power of two
-                    sa = 2.98023223876953125e-08f * 1.001f * ldexpf(A.tabs[gt], -kexp);
-                }
-                tsc[pt] = sc;
-                tsa[pt] = sa;
-            }
-            // ---- the voltage stream, one channel per ring stage.  Each channel
-            //      is copied (fp32) into a staging slot by coalesced 4-byte
-            //      asynchronous copies -- thread pt copies positions pt + 256 e --
-            //      kWDepth - 1 channels ahead of the one being packed; a thread
-            //      packs positions 8 pt .. 8 pt + 7 (and 2048 + 8 pt .. when hasB).
-            u32 lidx[8];                             // sample of position pt + 256 e, ~0 past the recording
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                const int x = (int)(pt + 256u * e);
-                u32 lo = 0, hi = nw - 1;             // last entry with tpos <= x
-                while (lo < hi) {
-                    const u32 mid = (lo + hi + 1) >> 1;
-                    if (tpos[mid] <= x) lo = mid; else hi = mid - 1;
-                }
-                const u32 sx = twin[lo] * L + (u32)(x - tpos[lo]);
-                lidx[e] = sx < n ? sx : 0xffffffffu;
-            }
-            auto issue = [&](u32 c) {
-                float *dst = vst + (size_t)(c % kWDepth) * px;
-                const float *vc = A.v + (size_t)c * n;
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const bool ok = lidx[e] != 0xffffffffu;
-                    cp_async4(smem_u32(dst + pt + 256u * e), vc + (ok ? lidx[e] : 0u), ok ? 4u : 0u);
-                }
-                for (u32 x = pt; x < nB; x += kTcProdThreads) {
-                    const u32 sb = xs[x];
-                    cp_async4(smem_u32(dst + kWPos + x), vc + (sb < n ? sb : 0u), sb < n ? 4u : 0u);
-                }
-            };
-            const float kscale = ldexpf(1.0f, kexp);     // exact: |kexp| <= 126
-            float e2A[8], abA[8];
-#pragma unroll
-            for (int e = 0; e < 8; e++) e2A[e] = abA[e] = 0.0f;
-#pragma unroll
-            for (u32 j = 0; j + 1 < kWDepth; j++) {
-                if (j < Cg) issue(j);
-                cp_async_commit();
-            }
-            cp_async_wait<kWDepth - 2>();            // channel 0: this thread's copies
-            named_bar(1, kTcProdThreads);            // and every thread's
-            bool stop = false;
+            for (int r = 0; r < 3; r++) e2[r][0] = e2[r][1] = 0.0f;
             for (u32 c = 0; c < Cg; c++) {
-                if (c + kWDepth - 1 < Cg) issue(c + kWDepth - 1);
-                cp_async_commit();                   // one group per channel (empty past the last)
-                const float *src = vst + (size_t)(c % kWDepth) * px;
-                uint4 qa, qb = make_uint4(0u, 0u, 0u, 0u);
-                {
-                    const float4 f0 = *reinterpret_cast<const float4 *>(src + 8 * pt);
-                    const float4 f1 = *reinterpret_cast<const float4 *>(src + 8 * pt + 4);
-                    const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
-                    u16 h[8];
+                const u32 gs = gs0 + c, s = gs % ns, u = gs / ns;
+                if (!wait_warp(bar_sfull(s), u & 1u, 17u)) break;    // the barrier below sees the abort flag
+                const unsigned char *B = ring + (size_t)s * lay.stage + lay.a_bytes;
 #pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        e2A[e] = fmaf(f[e], f[e], e2A[e]);
-                        abA[e] += fabsf(f[e]);
-                        h[e] = half_bits_clamped(__fmul_rn(f[e], kscale));
-                    }
-                    qa.x = ((u32)h[1] << 16) | h[0];
-                    qa.y = ((u32)h[3] << 16) | h[2];
-                    qa.z = ((u32)h[5] << 16) | h[4];
-                    qa.w = ((u32)h[7] << 16) | h[6];
-                }
-                if (hasB) {
-                    const float4 f0 = *reinterpret_cast<const float4 *>(src + kWPos + 8 * pt);
-                    const float4 f1 = *reinterpret_cast<const float4 *>(src + kWPos + 8 * pt + 4);
-                    const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
-                    u16 h[8];
+                for (int r = 0; r < 3; r++) {
+                    const u32 row = tt + 128u * r;
+                    if (row >= rows) continue;
+                    const uint4 h = *reinterpret_cast<const uint4 *>(B + 16 * (size_t)row);
+                    const u32 hw[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
-                    for (int e = 0; e < 8; e++) {
-                        xe2[8 * pt + e] = fmaf(f[e], f[e], xe2[8 * pt + e]);
-                        xab[8 * pt + e] += fabsf(f[e]);
-                        h[e] = half_bits_clamped(__fmul_rn(f[e], kscale));
+                    for (int e = 0; e < 4; e++) {
+                        const float2 x = __half22float2(*reinterpret_cast<const __half2 *>(&hw[e]));
+                        e2[r][0] = fmaf(x.x, x.x, e2[r][0]);
+                        e2[r][1] = fmaf(x.y, x.y, e2[r][1]);
                     }
-                    qb.x = ((u32)h[1] << 16) | h[0];
-                    qb.y = ((u32)h[3] << 16) | h[2];
-                    qb.z = ((u32)h[5] << 16) | h[4];
-                    qb.w = ((u32)h[7] << 16) | h[6];
                 }
-                const u32 s = gstage % ns, u = gstage / ns;
-                if (u > 0 && !mbar_wait_bounded(bar_sempty(s), (u - 1) & 1u, wlim)) {
-                    atomicExch(A.err, 11u);
-                    atomicExch(abort_flag, 1u);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_sempty(s));
+            }
+            gs0 += Cg;
+            float *es = (float *)(mp + lay.es);
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                const u32 row = tt + 128u * r;
+                if (row < rows) es[row] = e2[r][0] + e2[r][1];
+            }
+            if (named_bar_or(3, kWTabThreads, aborted())) break;
+            if (tt == 0) mbar_arrive(bar_nfull(k));
+        }
+    } else if (warp < kWMmaWarp) {
+        // =========================== producers ===========================
+        const u32 s = warp - kWProdWarp0;            // this warp's ring stage
+        u32 gs0 = 0, it = 0;
+        unsigned char *stg = ring + (size_t)s * lay.stage;
+        u16 *B = reinterpret_cast<u16 *>(stg + lay.a_bytes);
+        bool stop = s >= ns;
+        for (u32 f = blockIdx.x; !stop && f < total; f += gridDim.x, it++) {
+            const u32 k = it % kWMaps;
+            if (!wait_warp(bar_mfull(k), (it / kWMaps) & 1u, 18u)) break;
+            const unsigned char *mp = map_of(k);
+            const u32 *smap = (const u32 *)(mp + lay.smap);
+            const TcwInfo &I = *(const TcwInfo *)(mp + lay.info);
+            const TcwArgs &T = P.groups[I.g];
+            const float kscale = I.kscale;
+            const float *v = T.v;
+            const unsigned char *Aw = T.Aw;
+            const u32 Cg = I.Cg;
+            for (u32 c = (s + ns - gs0 % ns) % ns; c < Cg; c += ns) {
+                const u32 u = (gs0 + c) / ns;
+                const float *vc = v + (size_t)c * n;
+                for (u32 x0 = lane; x0 < px; x0 += 32 * kWLoads) {
+                    float fv[kWLoads];
+#pragma unroll
+                    for (u32 i = 0; i < kWLoads; i++) {
+                        const u32 x = x0 + 32 * i;
+                        // unconditional, so that the loads do not wait for one another; a
+                        // position past the recording reads its last sample, which no
+                        // output that is not in the zeroed tail multiplies
+                        fv[i] = __ldg(vc + min(smap[min(x, px - 1)], n - 1));
+                    }
+                    if (x0 == lane) {                // the first loads are in flight
+                        if (u > 0 && !wait_warp(bar_sempty(s), (u - 1) & 1u, 11u)) { stop = true; break; }
+                        if (lane == 0) {
+                            fills[s] = u + 1;
+                            mbar_expect_tx(bar_sfull(s), (u32)lay.a_bytes);
+                            asm volatile(
+                                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                                ::"r"(smem_u32(stg)), "l"(Aw + (size_t)c * lay.a_bytes), "r"((u32)lay.a_bytes),
+                                  "r"(bar_sfull(s)) : "memory");
+                        }
+                    }
+#pragma unroll
+                    for (u32 i = 0; i < kWLoads; i++) {
+                        const u32 x = x0 + 32 * i;
+                        if (x < px) B[x] = half_bits_clamped(__fmul_rn(fv[i], kscale));
+                    }
                 }
-                if (named_bar_or(1, kTcProdThreads, *(volatile u32 *)abort_flag != 0)) { stop = true; break; }
-                gstage++;
-                unsigned char *stg = ring + (size_t)s * lay.stage;
-                if (pt == 0) {
-                    const u32 bytes = nkc * kWATile;
-                    mbar_expect_tx(bar_sfull(s), bytes);
-                    asm volatile(
-                        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                        ::"r"(smem_u32(stg)), "l"(A.Aw + (size_t)c * bytes), "r"(bytes), "r"(bar_sfull(s))
-                        : "memory");
-                }
-                *reinterpret_cast<uint4 *>(stg + lay.a_bytes + 16 * (size_t)pt) = qa;
-                if (hasB) *reinterpret_cast<uint4 *>(stg + lay.a_bytes + 16 * (size_t)(kWN + pt)) = qb;
+                if (stop) break;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                cp_async_wait<kWDepth - 2>();        // channel c + 1: this thread's copies
-                named_bar(1, kTcProdThreads);        // every thread's; the stage is written
-                if (pt == 0) mbar_arrive(bar_sfull(s));  // release: the barrier ordered every write
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_sfull(s));
             }
-            cp_async_wait<0>();                      // no copy lands after the loop (abort path)
             if (stop) break;
-            // ---- window norms: prefix sums (double) over the staged positions
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                psq[8 * pt + e] = e2A[e];
-                pab[8 * pt + e] = abA[e];
-                if (hasB) {
-                    psq[kWPos + 8 * pt + e] = xe2[8 * pt + e];
-                    pab[kWPos + 8 * pt + e] = xab[8 * pt + e];
-                }
-            }
-            named_bar(1, kTcProdThreads);
-            {
-                const u32 per = (px + kTcProdThreads - 1) / kTcProdThreads;
-                const u32 lo = min(px, pt * per), hi = min(px, lo + per);
-                double a = 0.0, bb = 0.0;
-                for (u32 x = lo; x < hi; x++) { a += psq[x]; bb += pab[x]; }
-                const double ia = warp_incl_scan_d(a, lane), ib = warp_incl_scan_d(bb, lane);
-                if (lane == 31) { dsum[warp] = ia; dsum[8 + warp] = ib; }
-                named_bar(1, kTcProdThreads);
-                double ca = ia - a, cb = ib - bb;
-                for (u32 w8 = 0; w8 < warp; w8++) { ca += dsum[w8]; cb += dsum[8 + w8]; }
-                for (u32 x = lo; x < hi; x++) {
-                    ca += psq[x]; cb += pab[x];
-                    psq[x] = ca; pab[x] = cb;
-                }
-            }
-            named_bar(1, kTcProdThreads);
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                const u32 x = 8 * pt + e, hi_x = x + L - 1;    // < px
-                const u32 sp = spos[x];              // the sample of a kept output
-                if (sp == 0xffffffffu) continue;
-                const u32 smp = sp & ~kWTail;
-                const double pa = psq[hi_x], pb = pab[hi_x];
-                const double da = pa - (x ? psq[x - 1] : 0.0), db = pb - (x ? pab[x - 1] : 0.0);
-                // the double sums' own rounding (< 2 px 2^-53 of the prefix) is added back
-                const float wn = (float)sqrt(fmax(da, 0.0) + 1e-12 * pa) * 1.0001f + 1e-30f;
-                const float wa = (float)(fmax(db, 0.0) + 1e-12 * pb) * 1.0001f + 1e-30f;
-                wnwa[x] = make_float2(wn, wa);
-                A.wn_s[smp] = wn;
-                A.wa_s[smp] = wa;
-                A.kx_s[smp] = (signed char)kexp;
-            }
-            named_bar(1, kTcProdThreads);
-            if (pt == 0) mbar_arrive(bar_ifull(b));
-            if (b) use1++; else use0++;
+            gs0 += Cg;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_mempty(k));
         }
-        // the last copies into the ring land before the CTA exits
-        if (pt == 0) {
-            for (u32 s = 0; s < ns; s++) {
-                const u32 uses = gstage / ns + (s < gstage % ns ? 1u : 0u);
-                if (uses > 0) mbar_wait_bounded(bar_sfull(s), (uses - 1) & 1u, kTcDrainPolls);
-            }
-        }
-    } else if (warp == kTcMmaWarp) {
+        // every copy into the ring has landed before the CTA exits (a warp
+        // that issued one has also arrived)
+        __syncwarp();
+        if (lane == 0 && s < ns && fills[s] > 0) mbar_wait_bounded(bar_sfull(s), (fills[s] - 1) & 1u, kTcDrainPolls);
+    } else if (warp == kWMmaWarp) {
         // =========================== MMA issue ===========================
         // D f32, A/B f16, both K-major, M = 128, N = 256
         const u32 idesc = (1u << 4) | ((kWN >> 3) << 17) | ((u32)(kTcM >> 4) << 24);
         const u64 a0 = umma_desc(smem_u32(ring), kWATile / 2, 128);       // K halves 2048 B apart
         const u64 b0 = umma_desc(smem_u32(ring) + (u32)lay.a_bytes, 16, 128);   // rows 8 samples apart
         const u64 sstep = (u64)(lay.stage >> 4);
-        u32 use0 = 0u, use1 = 0u;
-        u32 it = 0;
+        u32 gs = 0, it = 0;
         bool issued = false;
-        for (u32 q = bi; q < ntiles; q += cnt, it++) {
-            const u32 b = it & 1u;
-            const u32 ub = b ? use1 : use0;
-            u32 ok = 1;
-            if (lane == 0) {
-                if (ub > 0 && !mbar_wait_bounded(bar_aempty(b), (ub - 1) & 1u, wlim)) {
-                    atomicExch(A.err, 12u);
-                    ok = 0;
-                }
-                if (!ok) atomicExch(abort_flag, 1u);
-                if (*(volatile u32 *)abort_flag) ok = 0;
-            }
-            if (!__shfl_sync(0xffffffffu, ok, 0)) break;
+        for (u32 f = blockIdx.x; f < total; f += gridDim.x, it++) {
+            const u32 b = it & 1u, ub = it >> 1, k = it % kWMaps;
+            if (!wait_warp(bar_mfull(k), (it / kWMaps) & 1u, 19u)) break;
+            const u32 Cg = ((const TcwInfo *)(map_of(k) + lay.info))->Cg;
+            if (ub > 0 && !wait_warp(bar_aempty(b), (ub - 1) & 1u, 12u)) break;
             const u32 dst = tmem + b * kWN;
-            for (u32 c = 0; c < Cg && ok; c++) {
-                const u32 s = gstage % ns, u = gstage / ns;
-                gstage++;
-                if (lane == 0) {
-                    if (!mbar_wait_bounded(bar_sfull(s), u & 1u, wlim)) {
-                        atomicExch(A.err, 14u);
-                        ok = 0;
+            bool ok = true;
+            for (u32 c = 0; c < Cg && ok; c++, gs++) {
+                const u32 s = gs % ns, u = gs / ns;
+                ok = wait_warp(bar_sfull(s), u & 1u, 14u);
+                if (ok && lane == 0) {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    u64 da = a0 + s * sstep, db = b0 + s * sstep;
+                    for (u32 q = 0; q < nkc; q++) {
+                        const u32 acc = (c | q) != 0 ? 1u : 0u;   // the first MMA overwrites
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\t"
+                            "setp.ne.b32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                            ::"r"(dst), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
+                        da += (u64)(kWATile >> 4);           // next A tile
+                        db += 2u;                            // 16 samples (32 bytes) later
                     }
-                    if (!ok) atomicExch(abort_flag, 1u);
-                    if (*(volatile u32 *)abort_flag) ok = 0;
-                    if (ok) {
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        u64 da = a0 + s * sstep, db = b0 + s * sstep;
-                        for (u32 k = 0; k < nkc; k++) {
-                            const u32 acc = (c | k) != 0 ? 1u : 0u;   // the first MMA overwrites
-                            asm volatile(
-                                "{\n\t.reg .pred p;\n\t"
-                                "setp.ne.b32 p, %4, 0;\n\t"
-                                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                                ::"r"(dst), "l"(da), "l"(db), "r"(idesc), "r"(acc) : "memory");
-                            da += (u64)(kWATile >> 4);           // next A tile
-                            db += 2u;                            // 16 samples (32 bytes) later
-                        }
-                        issued = true;
-                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                                     ::"r"(bar_sempty(s)) : "memory");
-                    }
+                    issued = true;
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                                 ::"r"(bar_sempty(s)) : "memory");
                 }
-                ok = __shfl_sync(0xffffffffu, ok, 0);
+                __syncwarp();
             }
             if (!ok) break;
             if (lane == 0)
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                              ::"r"(bar_afull(b)) : "memory");
             __syncwarp();
-            if (b) use1++; else use0++;
         }
         // every MMA issued here is done before TMEM and the ring are released
         if (lane == 0 && issued) {
@@ -615,172 +553,212 @@ k_lik_tcw(const TcwArgs *__restrict__ gargs, u32 ngroups) {
         __syncwarp();
     } else {
         // =========================== epilogue ===========================
-        const u32 ew_ = warp - kTcEpiWarp0;          // 0..7
+        const u32 ew_ = warp - kWEpiWarp0;           // 0..7
         const u32 quad = warp & 3u;                  // TMEM lanes [32 quad, 32 quad + 32)
         const u32 half = ew_ >> 2;                   // columns [128 half, 128 half + 128)
         const u32 row = quad * 32 + lane;
         const u32 tl = row >> 3, d = row & 7u;       // template column, sample shift
-        const bool real = tl < A.nt;
-        const u32 gt = ctrow[tl];
-        const float ck = ctk[tl], cb = ctb[tl], css = ctss[tl], ca = cta[tl];
-        const int texp_t = real ? A.texp[gt] : 0;
-        // this lane's template row of the likelihood and flag buffers
-        float *const Lk_t = A.Lk + (size_t)gt * n;
-        u8 *const apx_t = A.apx + (size_t)gt * n;
-        float *const dbg_t = A.dbgE ? A.dbgE + (size_t)gt * n : nullptr;
-        int *const bm_i = reinterpret_cast<int *>(A.bm_s);
-        u32 use0 = 0u, use1 = 0u;
+        const u32 span = d + (L - 1) % 8 >= 8 ? kWN : 0u;    // which of the two norm spans
+        const u32 et = tid - 32 * kWEpiWarp0;        // 0..255
+        const u32 TW = tcw_entries(L);
+        float *nrm_all = (float *)(wsm + lay.nrm);
+        int *um = (int *)(wsm + lay.um), *wl = (int *)(wsm + lay.wl);    // [16][TW], [TW]
+        for (u32 q = et; q < 16 * TW; q += kWEpiThreads) um[q] = 0;
+        for (u32 q = et; q < TW; q += kWEpiThreads) wl[q] = 0;
         u32 it = 0;
-        for (u32 q = bi; q < ntiles; q += cnt, it++) {
-            const u32 b = it & 1u;
-            const u32 ub = b ? use1 : use0;
-            bool ok = mbar_wait_bounded(bar_afull(b), ub & 1u, wlim);
-            ok = ok && mbar_wait_bounded(bar_ifull(b), ub & 1u, wlim);
-            if (!ok) { atomicExch(A.err, 10u); atomicExch(abort_flag, 1u); }
-            if (named_bar_or(2, kTcEpiThreads, *(volatile u32 *)abort_flag != 0)) break;
+        for (u32 f = blockIdx.x; f < total; f += gridDim.x, it++) {
+            const u32 b = it & 1u, ub = it >> 1, k3 = it % kWMaps;
+            bool ok = wait_warp(bar_mfull(k3), (it / kWMaps) & 1u, 20u) &&
+                      wait_warp(bar_nfull(k3), (it / kWMaps) & 1u, 20u) && wait_warp(bar_afull(b), ub & 1u, 10u);
+            if (named_bar_or(2, kWEpiThreads, !ok || aborted())) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const u32 *spos = spos_all + (size_t)b * kWPos;
-            const float2 *wnwa = wnwa_all + (size_t)b * kWPos;
-            const u8 *wrel = wrel_all + (size_t)b * kWPos;
-            const u32 *tw = tw_all + (size_t)b * kWTwMax;
-            const u32 *cw = cw_all + b * 16;
-            const int kexp = ti_all[b * 4];
-            const float tsc = tf_all[b * 32 + tl], tsa = tf_all[b * 32 + 16 + tl];
+            const unsigned char *mp = map_of(k3);
+            const u32 *smap = (const u32 *)(mp + lay.smap), *tw = (const u32 *)(mp + lay.tw);
+            const u8 *wrel = mp + lay.wrel;
+            const TcwInfo &I = *(const TcwInfo *)(mp + lay.info);
+            const u32 gi = I.g;
+            {
+                // norms of the blocks that hold an output's lags: output 8 u + d
+                // reads blocks u .. u + (L - 1) / 8, one more when d + (L - 1) % 8
+                // reaches 8.  The fp16 values round the scaled samples by 2^-11
+                // (2^-25 below the normal range, added as such); the sums' own
+                // rounding (Cg * 4 terms and (L + 14) / 8 blocks in float) is
+                // inside the factor.
+                const float *es = (const float *)(mp + lay.es);
+                const float add = ldexpf(2.98023223876953125e-08f * 1.001f * sqrtf((float)I.Cg * (float)(L + 14)), -I.kexp) +
+                                  1e-30f;
+                float e = 0.0f;
+                const u32 nb = (L - 1) / 8 + 1;
+                for (u32 q = 0; q < nb; q++) e += es[et + q];
+                nrm_all[et] = ldexpf(sqrtf(e) * 1.001f, -I.kexp) + add;
+                nrm_all[kWN + et] = ldexpf(sqrtf(e + es[et + nb]) * 1.001f, -I.kexp) + add;
+            }
+            named_bar(2, kWEpiThreads);
+            const float *nrm = nrm_all + span;
+            // interval data of the kept outputs (read by later kernels)
+            for (u32 x = et; x < kWPos; x += kWEpiThreads) {
+                if (wrel[x] == 0xffu) continue;
+                const size_t o = (size_t)gi * n + smap[x];
+                P.wn_s[o] = nrm_all[(x >> 3) + ((x & 7u) + (L - 1) % 8 >= 8 ? kWN : 0u)];
+                P.kx_s[o] = (signed char)I.kexp;
+            }
+            const bool real = I.gt[tl] != 0xffffffffu;
+            const u32 gt = real ? I.gt[tl] : 0u;
+            const float ck = fmaf(I.cb[tl], P.wa_f, I.ck[tl]), css = I.css[tl], tsc = I.tsc[tl];
+            const float cst = I.tsa[tl] + I.ca[tl];
+            const int ex = -(I.kexp + I.texp[tl]);
+            // this lane's template row of the likelihood and flag buffers
+            float *const Lk_t = P.Lk + (size_t)gt * n;
+            u8 *const apx_t = P.apx + (size_t)gt * n;
+            float *const dbg_t = P.dbgE ? P.dbgE + (size_t)gt * n : nullptr;
             const u32 acc0 = tmem + ((quad * 32u) << 16) + b * kWN;
             // the rare cases (a scale outside the float range, the testing
             // output of E) take a separate, warp-uniform copy of the loop
-            const bool rare = __any_sync(0xffffffffu, tsc == 0.0f) || dbg_t != nullptr;
-            u32 want[8];
-            // one 16-column chunk: classify and store its entries; per
-            // (window, template) the largest upper bound, per window the
-            // largest lower bound and whether some entry is > 0
+            const bool rare = __any_sync(0xffffffffu, real && tsc == 0.0f) || dbg_t != nullptr;
+            u32 curw = 0xffu;                        // table entry the lane's running bounds belong to
+            float mu = 0.0f, ml = 0.0f;
+            auto flush = [&]() {
+                if (mu > 0.0f) atomicMax(um + tl * TW + curw, __float_as_int(mu));
+                if (ml > 0.0f) atomicMax(wl + curw, __float_as_int(ml));
+            };
+            u32 want[4];                             // bit 8 (k & 3) + j of word k / 4: column 8 k + j of this half
+#pragma unroll
+            for (int q = 0; q < 4; q++) want[q] = 0;
+            // one 8-column chunk: classify and store its entries.  Every shared
+            // read first, then the arithmetic, then the stores, so that a column
+            // does not wait for the one before it; the few entries that are not
+            // certainly <= 0 afterwards, column by column.
             auto chunk = [&](const int k, auto RARE) {
                 constexpr bool kRare = decltype(RARE)::value;
-                const u32 c0 = 128 * half + 16 * k;
-                u32 r[16];
-                tmem_ld<16>(r, acc0 + c0);
-                float uq[16], lq[16];
-                u32 wbits = 0, pbits = 0;
-                bool any = false;
+                const u32 c0 = 128 * half + 8 * k;
+                u32 r[8], sm[8], wr[8];
+                float ap[8], E[8];
+                float nw[8];
+                __syncwarp();
+                tmem_ld<8>(r, acc0 + c0);
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const u32 x = 8 * (c0 + j) + d;
-                    const u32 sp = spos[x];
-                    const bool kept = real && sp != 0xffffffffu;
-                    const bool tail = (sp & kWTail) != 0u;          // .cl:231-234 (kept outputs only)
-                    const u32 s = sp & ~kWTail;
-                    const float2 nwa = wnwa[x];
+                for (int j = 0; j < 8; j++) {
+                    sm[j] = smap[8 * (c0 + j) + d];
+                    wr[j] = wrel[8 * (c0 + j) + d];
+                    nw[j] = nrm[c0 + j];
+                }
+                u32 hot = 0, pos = 0;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
                     const float a = __uint_as_float(r[j]);
                     float sa = __fmul_rn(a, tsc);
-                    if (kRare && tsc == 0.0f) sa = ldexpf(a, -(kexp + texp_t));
-                    const float approx = __fadd_rn(sa, css);
+                    if (kRare && tsc == 0.0f) sa = ldexpf(a, ex);
+                    ap[j] = __fadd_rn(sa, css);
                     // E = kappa ||t|| ||w|| + 2^-25 (|t|_1 / s_v + |w|_1 / s_t) * 1.001
                     //     + kappa_s |SS/2| + 2^-22 |approx|
-                    const float E = fmaf(ck, nwa.x, fmaf(cb, nwa.y, tsa) + ca + 2.384185791015625e-07f * fabsf(approx));
-                    const bool pos = approx - E > 0.0f;        // certainly > 0: refined when a decision needs it
-                    const bool neg = approx + E <= 0.0f;       // certainly <= 0: only its sign is read
+                    E[j] = fmaf(ck, nw[j], cst + 2.384185791015625e-07f * fabsf(ap[j]));
+                    const bool kept = real && wr[j] != 0xffu;
+                    const bool tail = sm[j] + L >= n;                // .cl:231-234 (kept outputs: s < n < 2^31)
                     const bool live = kept && !tail;
+                    const bool p = live && ap[j] - E[j] > 0.0f;      // certainly > 0: refined when a decision needs it
+                    hot |= live && !(ap[j] + E[j] <= 0.0f) ? 1u << j : 0u;   // not certainly <= 0
+                    pos |= p ? 1u << j : 0u;
                     if (kept) {
-                        Lk_t[s] = tail ? 0.0f : approx;
-                        apx_t[s] = (live && pos) ? (u8)1 : (u8)0;
-                        if (kRare && dbg_t) dbg_t[s] = tail ? 0.0f : E;
+                        Lk_t[sm[j]] = tail ? 0.0f : ap[j];
+                        apx_t[sm[j]] = p ? (u8)1 : (u8)0;
+                        if (kRare && dbg_t) dbg_t[sm[j]] = tail ? 0.0f : E[j];
                     }
-                    if (live && pos) atomicMax(bm_i + s, __float_as_int(E));
-                    wbits |= (live && !pos && !neg) ? (1u << j) : 0u;
-                    pbits |= (live && pos) ? (1u << j) : 0u;
-                    uq[j] = live ? fmaxf(0.0f, approx + E) : 0.0f;
-                    lq[j] = live ? approx - E : 0.0f;
-                    any |= live && !neg;
                 }
-                want[k] = wbits;
-                if (__any_sync(0xffffffffu, any)) {
-                    const u32 cwv = cw[half * 8 + k];
-                    const u32 wf = cwv & 0xffffu, wl = cwv >> 16;
-                    for (u32 w = wf; w <= wl; w++) {
-                        float mu = 0.0f, ml = 0.0f;
-                        bool mp = false;
+                want[k >> 2] |= (hot & ~pos) << (8 * (k & 3));
+                // bounds per (window, template) and per window: a lane's columns
+                // pass through the windows in order, so it keeps the running
+                // maxima of one window and hands them over when it leaves it
+                if (!__any_sync(0xffffffffu, hot != 0)) return;
 #pragma unroll
-                        for (int j = 0; j < 16; j++) {
-                            const bool here = wrel[8 * (c0 + j) + d] == w;
-                            mu = here ? fmaxf(mu, uq[j]) : mu;
-                            ml = here ? fmaxf(ml, lq[j]) : ml;
-                            mp |= here && ((pbits >> j) & 1u);
-                        }
-#pragma unroll
-                        for (int o = 1; o < 8; o <<= 1) mu = fmaxf(mu, __shfl_xor_sync(0xffffffffu, mu, o));
-#pragma unroll
-                        for (int o = 1; o < 32; o <<= 1) ml = fmaxf(ml, __shfl_xor_sync(0xffffffffu, ml, o));
-                        const u32 wa = tw[w];
-                        if (d == 0 && real && mu > 0.0f)
-                            atomicMax(reinterpret_cast<int *>(A.umax) + (size_t)wa * A.Kall + gt, __float_as_int(mu));
-                        if (lane == 0 && ml > 0.0f) atomicMax(reinterpret_cast<int *>(A.wlb) + wa, __float_as_int(ml));
-                        if (__any_sync(0xffffffffu, mp) && lane == 0) A.wpos[wa] = 1;
+                for (int j = 0; j < 8; j++) {
+                    if (!((hot >> j) & 1u)) continue;
+                    if (wr[j] != curw) {
+                        flush();
+                        curw = wr[j];
+                        mu = ml = 0.0f;
                     }
+                    mu = fmaxf(mu, ap[j] + E[j]);
+                    if ((pos >> j) & 1u) ml = fmaxf(ml, ap[j] - E[j]);
                 }
             };
             if (rare) {
 #pragma unroll
-                for (int k = 0; k < 8; k++) chunk(k, std::true_type{});
+                for (int k = 0; k < 16; k++) chunk(k, std::true_type{});
             } else {
 #pragma unroll
-                for (int k = 0; k < 8; k++) chunk(k, std::false_type{});
+                for (int k = 0; k < 16; k++) chunk(k, std::false_type{});
             }
+            flush();
             // accumulator b is no longer needed
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_aempty(b));
             u32 nwant = 0;
 #pragma unroll
-            for (int k = 0; k < 8; k++) nwant += __popc(want[k]);
-            if (named_bar_or(2, kTcEpiThreads, nwant != 0)) {
+            for (int q = 0; q < 4; q++) nwant += __popc(want[q]);
+            const bool queue = named_bar_or(2, kWEpiThreads, nwant != 0);   // also orders the bounds in shared memory
+            // the tile's bounds to global memory (a window may lie in two tiles)
+            for (u32 q = et; q < 16 * TW; q += kWEpiThreads) {
+                const int v = um[q];
+                if (v == 0) continue;
+                um[q] = 0;
+                atomicMax(reinterpret_cast<int *>(P.umax) + (size_t)tw[q % TW] * P.Kall + I.gt[q / TW], v);
+            }
+            for (u32 q = et; q < TW; q += kWEpiThreads) {
+                const int v = wl[q];
+                if (v == 0) continue;
+                wl[q] = 0;
+                atomicMax(reinterpret_cast<int *>(P.wlb) + (size_t)tw[q] * G + gi, v);
+                P.wpos[(size_t)tw[q] * G + gi] = 1;
+            }
+            if (queue) {
                 // one contiguous segment of (template, sample) entries per
                 // tile, ordered by template (tcnt is zero here)
                 if (nwant) atomicAdd(&tcnt[tl], nwant);
-                named_bar(2, kTcEpiThreads);
+                named_bar(2, kWEpiThreads);
                 if (ew_ == 0) {
                     const u32 cnt_t = lane < 16 ? tcnt[lane] : 0u;
                     const u32 incl = warp_incl_scan(cnt_t);
                     if (lane < 16) tcnt[lane] = incl - cnt_t;
-                    const u32 total = __shfl_sync(0xffffffffu, incl, 31);
+                    const u32 tot = __shfl_sync(0xffffffffu, incl, 31);
                     if (lane == 0) {
-                        const unsigned long long old = atomicAdd(A.refseg, ((unsigned long long)total << 32) | 1ull);
+                        const unsigned long long old = atomicAdd(P.refseg, ((unsigned long long)tot << 32) | 1ull);
                         const u32 base = (u32)(old >> 32), si = (u32)old;
                         seg_info[0] = base;
                         seg_info[2] = 0;
-                        if (base + total <= A.ref_cap && si < A.seg_cap) {
-                            A.seg_s0[si] = 0;                // entries carry their absolute samples
-                            A.seg_base[si] = base;
-                            A.seg_cnt[si] = total;
-                            A.seg_grp[si] = A.grp;
+                        if (base + tot <= P.ref_cap && si < P.seg_cap) {
+                            P.seg_s0[si] = 0;                // entries carry their absolute samples
+                            P.seg_base[si] = base;
+                            P.seg_cnt[si] = tot;
+                            P.seg_grp[si] = gi;
                             seg_info[2] = 1;
                         } else {
-                            atomicExch(A.seg_overflow, 1u);
+                            atomicExch(P.seg_overflow, 1u);
                         }
                     }
                 }
-                named_bar(2, kTcEpiThreads);
+                named_bar(2, kWEpiThreads);
                 const u32 seg_base = seg_info[0];
                 if (seg_info[2] && nwant) {
 #pragma unroll
-                    for (int k = 0; k < 8; k++) {
-                        u32 bits = want[k];
+                    for (int q = 0; q < 4; q++) {
+                        u32 bits = want[q];
                         while (bits) {
                             const u32 j = __ffs(bits) - 1;
                             bits &= bits - 1;
-                            const u32 x = 8 * (128 * half + 16 * k + j) + d;
+                            const u32 x = 8 * (128 * half + 32 * q + j) + d;
                             const u32 p = seg_base + atomicAdd(&tcnt[tl], 1u);
-                            A.ref_t[p] = tl;
-                            A.ref_s[p] = spos[x] & ~kWTail;
+                            P.ref_t[p] = tl;
+                            P.ref_s[p] = smap[x];
                         }
                     }
                 }
-                named_bar(2, kTcEpiThreads);         // tcnt / seg_info are done with
+                named_bar(2, kWEpiThreads);          // tcnt / seg_info are done with
                 if (ew_ == 0 && lane < 16) tcnt[lane] = 0;
             }
-            // the tile's tables are no longer needed
+            // the tile's map is no longer needed
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_bempty(b));
-            if (b) use1++; else use0++;
+            if (lane == 0) mbar_arrive(bar_mempty(k3));
         }
     }
     __syncthreads();
@@ -827,37 +805,75 @@ __global__ void k_window_vmax(const float *__restrict__ v, u32 n, u32 C, u32 L, 
     }
 }
 
-// The stream of a pass.  brk[i] = 1 where listed window i starts a run
-// (entries past the list are 0, as the ordered compaction reads them).
-__global__ void k_ws_breaks(const u32 *__restrict__ win, const u32 *__restrict__ n_win, u32 nbytes,
-                            u8 *__restrict__ brk) {
-    const u32 m = *n_win;
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < nbytes; i += gridDim.x * blockDim.x)
-        brk[i] = (i < m && (i == 0 || win[i] != win[i - 1] + 1)) ? 1 : 0;
+// The groups' window lists and streams of a pass: a group's windows are those
+// listed (active) with the group's dirty bit set.  Two launches over (tile of
+// kCompactTile windows, group): counts of windows and of runs of consecutive
+// windows, then the lists with their stream positions, the first window of
+// every tile of the stream (the one whose stretch of positions holds the
+// tile's start: a window's own L, and after the last window of a run L - 1
+// more), and the totals.
+__device__ __forceinline__ u32 tcw_selected(const u8 *__restrict__ active, const u32 *__restrict__ dirty, u32 GW, u32 g,
+                                            u32 W, u32 w) {
+    return w < W && active[w] && ((dirty[(size_t)w * GW + (g >> 5)] >> (g & 31)) & 1u) ? 1u : 0u;
 }
-
-// pos[i] = i L + R_i (L - 1), R_i = runs before listed window i (runs[] =
-// list index of each run's first window); first[q] = the last listed window
-// with pos <= 2048 q; *n_stiles = tiles that hold kept outputs.
-__global__ void k_ws_pos(const u32 *__restrict__ n_win, const u8 *__restrict__ brk, const u32 *__restrict__ runs,
-                         const u32 *__restrict__ n_runs, u32 L, u32 *__restrict__ pos, u32 *__restrict__ first,
-                         u32 *__restrict__ n_stiles) {
-    const u32 m = *n_win, nr = *n_runs;
-    const u32 g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g == 0 && m == 0) *n_stiles = 0;
-    for (u32 i = g; i < m; i += gridDim.x * blockDim.x) {
-        u32 lo = 0, hi = nr;                         // first run starting after i
-        while (lo < hi) {
-            const u32 mid = (lo + hi) >> 1;
-            if (runs[mid] <= i) lo = mid + 1; else hi = mid;
-        }
-        const u32 R = lo - 1;                        // runs[0] = 0 <= i
-        const u32 p = i * L + R * (L - 1);
-        pos[i] = p;
-        const u64 next = i + 1 < m ? (u64)p + L + (brk[i + 1] ? L - 1 : 0) : ~0ull;
-        const u64 qt = ((u64)p + kWPos - 1) / kWPos;  // the one tile start in [p, next), if any
-        if (qt * kWPos < next && (i + 1 < m || qt * kWPos < (u64)p + L)) first[qt] = i;
-        if (i + 1 == m) *n_stiles = (u32)(((u64)p + L + kWPos - 1) / kWPos);
+// this thread's kCompactPerThread windows and their two neighbours: bit k + 1
+// is window base + k
+__device__ __forceinline__ u32 tcw_selection(const u8 *active, const u32 *dirty, u32 GW, u32 g, u32 W, u32 base) {
+    u32 m = base > 0 ? tcw_selected(active, dirty, GW, g, W, base - 1) : 0u;
+#pragma unroll
+    for (u32 k = 0; k <= kCompactPerThread; k++) m |= tcw_selected(active, dirty, GW, g, W, base + k) << (k + 1);
+    return m;
+}
+static_assert(kCompactPerThread + 2 <= 32, "a thread's windows and neighbours fit a word");
+__device__ __forceinline__ u32 tcw_counts(u32 m) {   // windows, runs started << 16
+    const u32 own = (m >> 1) & ((1u << kCompactPerThread) - 1u), prev = m & ((1u << kCompactPerThread) - 1u);
+    return __popc(own) | (__popc(own & ~prev) << 16);
+}
+__global__ void __launch_bounds__(kCompactThreads)
+k_tcw_count(const u8 *__restrict__ active, const u32 *__restrict__ dirty, u32 GW, u32 W, u32 *__restrict__ counts) {
+    const u32 g = blockIdx.y, base = blockIdx.x * kCompactTile + threadIdx.x * kCompactPerThread;
+    u32 tot;
+    block_excl_scan(tcw_counts(tcw_selection(active, dirty, GW, g, W, base)), &tot);
+    if (threadIdx.x == 0) counts[(size_t)g * gridDim.x + blockIdx.x] = tot;
+}
+__global__ void __launch_bounds__(kCompactThreads)
+k_tcw_lists(const u8 *__restrict__ active, const u32 *__restrict__ dirty, u32 GW, u32 W, u32 L,
+            const u32 *__restrict__ counts, u32 wstride, u32 fstride, u32 *__restrict__ win, u32 *__restrict__ pos,
+            u32 *__restrict__ first, u32 *__restrict__ n_win, u32 *__restrict__ n_stiles) {
+    const u32 g = blockIdx.y, base = blockIdx.x * kCompactTile + threadIdx.x * kCompactPerThread;
+    // windows and runs of the tiles before this one
+    u32 bm = 0, br = 0, tot;
+    for (u32 t = threadIdx.x; t < blockIdx.x; t += blockDim.x) {
+        const u32 c = counts[(size_t)g * gridDim.x + t];
+        bm += c & 0xffffu;
+        br += c >> 16;
+    }
+    block_excl_scan(bm, &tot);
+    bm = tot;
+    __syncthreads();
+    block_excl_scan(br, &tot);
+    br = tot;
+    __syncthreads();
+    const u32 sel = tcw_selection(active, dirty, GW, g, W, base);
+    const u32 before = block_excl_scan(tcw_counts(sel), &tot);
+    u32 i = bm + (before & 0xffffu), runs = br + (before >> 16);
+    u32 *gw = win + (size_t)g * wstride, *gp = pos + (size_t)g * wstride, *gf = first + (size_t)g * fstride;
+#pragma unroll
+    for (u32 k = 0; k < kCompactPerThread; k++) {
+        if (!((sel >> (k + 1)) & 1u)) continue;
+        if (!((sel >> k) & 1u)) runs++;
+        const u32 p = i * L + (runs - 1) * (L - 1);
+        gw[i] = base + k;
+        gp[i] = p;
+        const u32 nxt = p + L + (((sel >> (k + 2)) & 1u) ? 0u : L - 1);
+        const u32 qt = (p + kWPos - 1) / kWPos;      // the one tile start that [p, nxt) can hold
+        if (qt * kWPos < nxt) gf[qt] = i;
+        i++;
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        const u32 m = bm + (tot & 0xffffu), r = br + (tot >> 16);
+        n_win[g] = m;
+        n_stiles[g] = m ? ((m - 1) * L + (r - 1) * (L - 1) + L + kWPos - 1) / kWPos : 0u;
     }
 }
 

@@ -135,6 +135,7 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
             uint4 sl = make_uint4(0xffffffffu, 0u, 0u, 0u);
             if (lane < spt && g < nc) sl = A.slot_tab[g];
             const float scale = ldexpf(1.0f, (int)sl.y);     // exact: |kexp| <= 126
+            const u32 start = sl.x != 0xffffffffu ? sl.x : 0u;       // n >= 4 L
             const u32 Cg = T.Cg, nq = spt * ncl;
             const float *v = T.v;
             const unsigned char *Aw = T.Aw;
@@ -149,9 +150,10 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
                     u32 k = q0 / ncl, jc = q0 - k * ncl;
 #pragma unroll
                     for (int i = 0; i < 16; i++) {
-                        const u32 b0 = __shfl_sync(0xffffffffu, sl.x, min(k, 31u));
-                        const u32 j = jc * 32 + lane;
-                        f[i] = (k < spt && j < L && b0 != 0xffffffffu) ? __ldg(vc + b0 + j) : 0.0f;
+                        // unconditional, so that the loads do not wait for one another
+                        // (a slot without a candidate reads samples whose outputs are dropped)
+                        const u32 b0 = __shfl_sync(0xffffffffu, start, min(k, 31u));
+                        f[i] = __ldg(vc + b0 + min(jc * 32 + lane, L - 1));
                         if (++jc == ncl) { jc = 0; k++; }
                     }
                     if (q0 == 0) {
@@ -288,7 +290,7 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
             if (lane < spt && gbase + lane < nc) sl = A.slot_tab[gbase + lane];
             if (sl.x != 0xffffffffu) {
                 wn = A.lazy.wn[(size_t)gi * A.lazy.gstride + sl.x];
-                wa = A.lazy.wa[(size_t)gi * A.lazy.gstride + sl.x];
+                wa = A.lazy.wa_f * wn;               // at most (the wide likelihood keeps no L1 norms)
             }
             u32 ok = 1;
             if (lane == 0) {

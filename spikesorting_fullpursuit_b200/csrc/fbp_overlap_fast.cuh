@@ -428,7 +428,7 @@ __device__ __forceinline__ void ov_window_norms(const OvArgs &A, u32 g, u32 bidx
     if (A.lazy.wn) {
         const size_t i = (A.lazy.tgrp ? (size_t)A.lazy.tgrp[t] * A.lazy.gstride : 0) + bidx;
         l2 = A.lazy.wn[i];
-        l1 = A.lazy.wa[i];
+        l1 = A.lazy.wa ? A.lazy.wa[i] : A.lazy.wa_f * l2;
     } else {
         l2 = A.vn[g];
         l1 = 0.0f;
@@ -648,16 +648,28 @@ k_ov_rows(OvArgs A) {
             float tot[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) tot[i] = 0.0f;
+            __syncwarp();
+            for (u32 x = lane; x < kRowsShifts + Lp + 8; x += 32) strip[x] = 0.0f;
             for (u32 ch = clo + warp; ch < chi; ch += kRowsWarps) {
                 __syncwarp();
-                // strip[x]: the window at lag x0 + x - n_max (zero outside [0, L))
-                const float *v = A.v + (size_t)ch * n + c.bidx;
-                for (u32 x = lane; x < kRowsShifts + Lp + 8; x += 32) {
-                    const int rel = (int)(x0 + x) - (int)nmax;
-                    strip[x] = (rel >= 0 && rel < (int)L) ? __ldg(v + rel) : 0.0f;
+                // strip[x]: the window at lag x0 + x - n_max (zero outside [0, L));
+                // four loads of each row in flight
+                const float *v = A.v + (size_t)ch * n + c.bidx, *tp = A.T + ((size_t)c.k0 * A.C + ch) * L;
+                for (u32 m0 = lane; m0 < Lp; m0 += 128) {
+                    float f[4], tv[4];
+#pragma unroll
+                    for (u32 i = 0; i < 4; i++) {
+                        const u32 m = min(m0 + 32 * i, L - 1);
+                        f[i] = __ldg(v + m);
+                        tv[i] = __ldg(tp + m);
+                    }
+#pragma unroll
+                    for (u32 i = 0; i < 4; i++) {
+                        const u32 m = m0 + 32 * i, x = m + nmax - x0;
+                        if (m < L && x < kRowsShifts + Lp + 8) strip[x] = f[i];
+                        if (m < Lp) trow[m] = m < L ? tv[i] : 0.0f;
+                    }
                 }
-                const float *tp = A.T + ((size_t)c.k0 * A.C + ch) * L;
-                for (u32 m = lane; m < Lp; m += 32) trow[m] = m < L ? __ldg(tp + m) : 0.0f;
                 __syncwarp();
                 float acc[8], w[16];
 #pragma unroll
