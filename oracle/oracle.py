@@ -65,7 +65,7 @@ def pursuit_chunk(chunk_v, templates_vec, K, L, tss, thr, n_max_shift, do_overla
         out_l = np.zeros(cap, np.uint32)
         passes = U(0)
         pc = np.zeros(max_passes, np.uint32)
-        work = np.ascontiguousarray(chunk_v, dtype=np.float32)
+        work = np.array(chunk_v, dtype=np.float32, order="C")   # a retry starts from the recording again
         r = lib().bpo_pursuit_chunk(work.reshape(-1), n, C, templates_vec, K, L, tss, thr,
                                     int(n_max_shift), int(bool(do_overlap)), out_i, out_l, cap,
                                     ctypes.byref(passes), pc, max_passes, int(nthreads))
