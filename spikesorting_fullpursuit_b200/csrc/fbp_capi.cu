@@ -195,7 +195,7 @@ struct Workspace {
 bool fast_overlap_fits(u32 K, u32 L, u32 nmax) {
     const u64 S = 2 * (u64)nmax + 1;
     if (S > 4 * (u64)L + 1 || S > 65535) return false;
-    if (pair_smem_bytes(L, 0) > 227 * 1024 || scan_smem_bytes((u32)S) > 227 * 1024) return false;
+    if (pair_smem_bytes(L, 0) > 227 * 1024 || scan_smem_bytes((u32)S, L) > 227 * 1024) return false;
     if (tables_smem_bytes((u32)S, K, L) > 227 * 1024) return false;
     return true;
 }
@@ -679,7 +679,7 @@ int ov_fast_pass(const Workspace &w, const OvArgs &A, Counters *cnt, cudaStream_
         k_ov_seed_pairs<<<grid_for((u64)slots * A.K, kSeedThreads, 8), kSeedThreads, 0, st>>>(A);
     else
         k_ov_seed<<<grid_for((u64)slots * A.K * 32, kSeedThreads, 8), kSeedThreads, 0, st>>>(A);
-    const size_t scan_smem = scan_smem_bytes(S);
+    const size_t scan_smem = scan_smem_bytes(S, A.L);
     if (scan_smem > 48 * 1024)
         FBP_ALLOW_SMEM(k_ov_scan);
     k_ov_scan<<<grid_for((u64)slots * A.K * 32, kScanThreads, 8), kScanThreads, scan_smem, st>>>(A);

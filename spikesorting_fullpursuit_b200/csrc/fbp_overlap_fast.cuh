@@ -391,14 +391,17 @@ k_ov_tables_m(OvArgs A, const u32 *__restrict__ tperm, const u32 *__restrict__ t
 }
 
 constexpr int kScanThreads = 256;
-// Per-warp scratch of the scan: hb_lo, hb_hi (S floats each), and per block
-// of 32 rows b the bits of rows with L[t][ashift] not <= 0 and the largest
-// upper bound.
-__host__ __device__ inline size_t sweep_warp_bytes(u32 S) {
-    return align_up((size_t)8 * S + (size_t)(S + 31) / 32 * 8, 16);
+// Per-warp scratch of the scan: hb_lo, hb_hi (S floats each), per block of 32
+// rows b the bits of rows with L[t][ashift] not <= 0 and the largest upper
+// bound, the rows a's bits and upper bounds (blocks of 32), the lag bounds of
+// a block of rows a against one of rows b by their distance, the pair's lag
+// bounds, and a queue of items.
+__host__ __device__ inline size_t sweep_warp_bytes(u32 S, u32 L) {
+    const size_t NB = (S + 31) / 32;
+    return align_up((size_t)8 * S + NB * 12 + NB * 128 + 2 * NB * 128 + (size_t)(2 * L + 1) * 4 + 64 * 4, 16);
 }
-__host__ __device__ inline size_t scan_smem_bytes(u32 S) {
-    return (size_t)(kScanThreads / 32) * sweep_warp_bytes(S);
+__host__ __device__ inline size_t scan_smem_bytes(u32 S, u32 L) {
+    return (size_t)(kScanThreads / 32) * sweep_warp_bytes(S, L);
 }
 __host__ __device__ inline size_t tables_smem_bytes(u32 S, u32 K, u32 L) {
     const size_t Lp = (L + 7) & ~7u, Sp = (size_t)(S + 7) / 8 * 8, Kp = (size_t)(K + 7) / 8 * 8;
@@ -455,16 +458,16 @@ __device__ __forceinline__ OvRowB ov_row_b(const OvArgs &A, u32 g, u32 bidx, u32
     }
     return r;
 }
-__device__ __forceinline__ void ov_row_interval(const OvArgs &A, u32 g, u32 tmpl, u32 x, float Hv, const OvRowB &r,
-                                                float &lo, float &hi) {
-    const float nt = A.NT[(size_t)tmpl * A.S + x], snt = A.sNT[(size_t)tmpl * A.S + x];
+__device__ __forceinline__ void ov_row_interval(const OvArgs &A, u32 g, u32 tmpl, u32 x, float Hv, float snt,
+                                                const OvRowB &r, float &lo, float &hi) {
+    // the clipped energy as the square of its root: the roundings are far inside the tables' bound
     float sx = r.sub1;
     if (A.kexp_tile) {
         // scale exponent of the table tile: per template group, candidate, tile of 128 shifts
         const size_t grp = A.tgrp ? (size_t)A.tgrp[tmpl] * A.kt_slots : 0;
         sx += r.sub0 * ldexpf(1.0f, -A.kexp_tile[(grp + g) * A.stiles + x / 128]);
     }
-    const float e = r.krm * (snt * r.vn + nt) + 4.0f * kUnitRoundoff * fabsf(Hv) + r.eqt + sx;
+    const float e = r.krm * (snt * r.vn + snt * snt) + 4.0f * kUnitRoundoff * fabsf(Hv) + r.eqt + sx;
     lo = Hv - e;
     hi = Hv + e;
 }
@@ -770,7 +773,7 @@ k_ov_seed(OvArgs A) {
         u32 b1 = 0, b2 = 0;
         for (u32 x = c.xlo + lane; x < xend; x += 32) {
             float lo, hi;
-            ov_row_interval(A, g, t, x, Hg[x], rb, lo, hi);
+            ov_row_interval(A, g, t, x, Hg[x], A.sNT[(size_t)t * S + x], rb, lo, hi);
             if (lo > v1) { v1 = lo; b1 = x; }
             if ((x > a1 ? x - a1 : a1 - x) <= L && lo > v2) { v2 = lo; b2 = x; }
             mB = fmaxf(mB, hi);
@@ -817,24 +820,29 @@ k_ov_seed(OvArgs A) {
 //   - a row a against a block of 32 rows b is skipped when
 //     hiA + max hiB of the block + XMw of its lags < TH (lanes over the rows a);
 //   - of a row and a block that remain, lanes over the rows b, the items that
-//     pass the skip rules and hiA + hiB + XMr[a-b] >= TH get their interval
-//     from the prefix table.
+//     pass the skip rules and hiA + hiB + XMr[a-b] >= TH are queued, and 32 of
+//     them at a time, one per lane, get their interval from the prefix table.
 // An item that is never enumerated can neither be the best item (whose value
 // is >= every lower bound) nor beat the current best.  Items with
 // hi >= TH and hi > current best go to the contender pool with their hi;
 // their lower bounds raise the candidate's best lower bound, and TH with it
-// after every block (the block of largest upper bound goes first).  Testing
-// rows against blocks leaves about 50 warp steps of a pair with 201 shifts;
-// lists of single rows a and b were crossed pair by pair, up to 1,250 steps.
-__global__ void __launch_bounds__(kScanThreads)
+// (the block of largest upper bound goes first).  Testing rows against blocks
+// leaves about 50 warp steps of a pair with 201 shifts; lists of single rows
+// a and b were crossed pair by pair, up to 1,250 steps.  What is left is bound
+// by latency, so everything a pair needs is loaded before it is used and kept
+// in shared memory.
+__global__ void __launch_bounds__(kScanThreads, 4)
 k_ov_scan(OvArgs A) {
     extern __shared__ float sm[];
     const u32 S = A.S, K = A.K, L = A.L, nmax = A.nmax, n = A.n;
     const u32 R = 2 * L - 1, NR = 2 * L + 1, NW = 2 * L + 32, NB = (S + 31) / 32;
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float *hb_lo = (float *)((char *)sm + (size_t)warp * sweep_warp_bytes(S)), *hb_hi = hb_lo + S;
-    u32 *bbits = (u32 *)(hb_hi + S);
-    float *bmax = (float *)(bbits + NB);             // largest in-bounds upper bound of each block of rows b
+    float *hb_lo = (float *)((char *)sm + (size_t)warp * sweep_warp_bytes(S, L)), *hb_hi = hb_lo + S;
+    u32 *bbits = (u32 *)(hb_hi + S), *abits = bbits + NB;
+    float *bmax = (float *)(abits + NB);             // largest in-bounds upper bound of each block of rows b
+    float *ua = bmax + NB, *xw = ua + 32 * NB;       // rows a; lag bounds: block distance (ka - kb + NB - 1), lane
+    float *xr = xw + 64 * NB;                        // the pair's lag bounds, slack added
+    u32 *queue = (u32 *)(xr + NR);                   // items a | b << 16 that passed every bound
     const u32 nc = *A.n_cand;
     const u64 total = (u64)nc * K;
     // a warp's share of a small pass is spread over two turns at least
@@ -883,30 +891,43 @@ k_ov_scan(OvArgs A) {
             const OvRowB rb = ov_row_b(A, g, c.bidx, c.k0, t, krm);
             const float *Hg = A.H + ((size_t)g * K + t) * S;
             const float *ga_lo = A.ga_lo + (size_t)g * S, *ga_hi = A.ga_hi + (size_t)g * S;
-            const u32 *abits = A.ga_bits + (size_t)g * NB;
             // rows b: intervals and the L[t][ashift] > 0 bits
             float mB = -INFINITY, mabs = A.ga_abs[g];
             u32 kbest = 0;
             __syncwarp();                            // the previous pair's readers are done
-            for (u32 x0 = 0; x0 < S; x0 += 32) {
-                const u32 x = x0 + lane;
-                bool bp = false;
-                float up = -INFINITY;
-                if (x < S) {
-                    float lo, hi;
-                    ov_row_interval(A, g, t, x, Hg[x], rb, lo, hi);
-                    hb_lo[x] = lo;
-                    hb_hi[x] = hi;
-                    if (x >= c.xlo && x < c.xhi_ex) {
-                        bp = !(A.Lk[(size_t)t * n + c.bidx + x - nmax] <= 0.0f);
-                        up = hi;
-                        mabs = fmaxf(mabs, fabsf(hi));
-                    }
+            // (every load of 256 rows before their arithmetic)
+            for (u32 x1 = 0; x1 < S; x1 += 256) {
+                float hv[8], nt[8], lk[8];
+#pragma unroll
+                for (u32 i = 0; i < 8; i++) {
+                    const u32 x = min(x1 + 32 * i + lane, S - 1);
+                    hv[i] = __ldg(Hg + x);
+                    nt[i] = __ldg(A.sNT + (size_t)t * S + x);
+                    // in-bounds rows only: the others' positions lie outside the recording
+                    lk[i] = A.Lk[(size_t)t * n + c.bidx + max(c.xlo, min(x, c.xhi_ex - 1)) - nmax];
                 }
-                const u32 mb = __ballot_sync(0xffffffffu, bp);
-                up = warp_max_f(up);
-                if (lane == 0) { bbits[x0 / 32] = mb; bmax[x0 / 32] = up; }
-                if (up > mB) { mB = up; kbest = x0 / 32; }
+#pragma unroll
+                for (u32 i = 0; i < 8; i++) {
+                    const u32 x = x1 + 32 * i + lane;
+                    if (x1 + 32 * i >= S) break;     // uniform in the warp
+                    bool bp = false;
+                    float up = -INFINITY;
+                    if (x < S) {
+                        float lo, hi;
+                        ov_row_interval(A, g, t, x, hv[i], nt[i], rb, lo, hi);
+                        hb_lo[x] = lo;
+                        hb_hi[x] = hi;
+                        if (x >= c.xlo && x < c.xhi_ex) {
+                            bp = !(lk[i] <= 0.0f);
+                            up = hi;
+                            mabs = fmaxf(mabs, fabsf(hi));
+                        }
+                    }
+                    const u32 mb = __ballot_sync(0xffffffffu, bp);
+                    up = warp_max_f(up);
+                    if (lane == 0) { bbits[x1 / 32 + i] = mb; bmax[x1 / 32 + i] = up; }
+                    if (up > mB) { mB = up; kbest = x1 / 32 + i; }
+                }
             }
             mabs = warp_max_f(mabs);
             __syncwarp();
@@ -914,71 +935,112 @@ k_ov_scan(OvArgs A) {
             if (!(mA + mB + XM + slack >= TH)) continue;
             const bool apart = ov_disjoint(A.tsup, c.k0, t);   // no cross term, no table
             const float *xmr = A.XMr + pair * NR, *xmw = A.XMw + pair * NW;
+            // rows a (out of bounds: below everything), and for every distance of
+            // blocks the bound of the lags of a row a against 32 rows b: XMw at
+            // a - 32 k + L (no lag there: below everything)
+            for (u32 x = lane; x < NB; x += 32) abits[x] = A.ga_bits[(size_t)g * NB + x];
+            for (u32 x0 = lane; x0 < NR; x0 += 256) {
+                float y[8];
+#pragma unroll
+                for (u32 i = 0; i < 8; i++) y[i] = apart ? 0.0f : __ldg(xmr + min(x0 + 32 * i, NR - 1));
+#pragma unroll
+                for (u32 i = 0; i < 8; i++)
+                    if (x0 + 32 * i < NR) xr[x0 + 32 * i] = y[i] + kPruneSlack * fabsf(y[i]);
+            }
+            for (u32 k = 0; k < NB; k += 4) {
+                float u[4], y[8];
+#pragma unroll
+                for (u32 i = 0; i < 4; i++) u[i] = __ldg(ga_hi + min(32 * (k + i) + lane, S - 1));
+#pragma unroll
+                for (u32 i = 0; i < 8; i++) {
+                    const int wi = 32 * ((int)(2 * k + i) - (int)(NB - 1)) + (int)lane + (int)L;
+                    y[i] = apart ? 0.0f : __ldg(xmw + max(0, min((int)NW - 1, wi)));
+                    if (wi < 0 || wi >= (int)NW) y[i] = -INFINITY;
+                }
+#pragma unroll
+                for (u32 i = 0; i < 4; i++) {
+                    const u32 a = 32 * (k + i) + lane;
+                    if (k + i < NB) ua[a] = a < S && a >= c.xlo && a < c.xhi_ex ? u[i] : -INFINITY;
+                }
+#pragma unroll
+                for (u32 i = 0; i < 8; i++)
+                    if (2 * k + i < 2 * NB - 1)
+                        xw[32 * (2 * k + i) + lane] = y[i] > -INFINITY ? y[i] + kPruneSlack * fabsf(y[i]) : y[i];
+            }
+            __syncwarp();
             const float *q = A.Q + pair * R * (L + 1);
+            u32 held = 0;                            // items in the queue
+            // intervals of the first min(held, 32) queued items, one per lane
+            auto drain = [&]() {
+                __syncwarp();
+                const bool valid = lane < held;
+                const u32 it = valid ? queue[lane] : 0u, a = it & 0xffffu, b = it >> 16;
+                float hi = -INFINITY, lo = -INFINITY;
+                if (valid) {
+                    const float la = __ldg(ga_lo + a);
+                    const float X = apart ? 0.0f : ov_x(q, L, (int)a - (int)nmax, (int)a - (int)b);
+                    const float ex = kx * fabsf(X);
+                    hi = ua[a] + hb_hi[b] - X + ex;
+                    lo = la + hb_lo[b] - X - ex;
+                    evaluated++;
+                }
+                const bool keep = valid && hi >= TH && hi > c.lbest;
+                const u32 mk = __ballot_sync(0xffffffffu, keep);
+                if (mk) {
+                    u32 base = 0;
+                    if (lane == 0) base = atomicAdd(A.pool_total, (u32)__popc(mk));
+                    base = __shfl_sync(0xffffffffu, base, 0);
+                    if (keep) {
+                        const u32 pp = base + __popc(mk & ((1u << lane) - 1u));
+                        if (pp < A.pool_cap) {
+                            A.pool_slot[pp] = g;
+                            A.pool_item[pp] = t + K * (a + S * b);
+                            A.pool_hi[pp] = hi;
+                        } else {
+                            A.fallback[g] = 1;
+                        }
+                    }
+                }
+                lo = warp_max_f(lo);
+                if (lo > TH) {
+                    if (lane == 0) atomicMax(reinterpret_cast<int *>(A.cand_lb) + g, __float_as_int(lo));   // > 0
+                    TH = lo;
+                    slack = kPruneSlack * (2.0f * mabs + fabsf(TH) + fabsf(XM));
+                }
+                const u32 rest = held > 32 && lane < held - 32 ? queue[32 + lane] : 0u;
+                __syncwarp();
+                if (held > 32 && lane < held - 32) queue[lane] = rest;
+                held = held > 32 ? held - 32 : 0;
+                __syncwarp();
+            };
             for (u32 kk = 0; kk < NB; kk++) {
                 const u32 k = kk == 0 ? kbest : kk <= kbest ? kk - 1 : kk;   // kbest, then the others in order
                 const float mBk = bmax[k];
                 if (!(mA + mBk + XM + slack >= TH)) continue;                // uniform
                 const u32 b = 32 * k + lane;
                 const bool inb = b < S && b >= c.xlo && b < c.xhi_ex;
-                const float lo_b = b < S ? hb_lo[b] : 0.0f, hi_b = b < S ? hb_hi[b] : 0.0f;
+                const float hi_b = b < S ? hb_hi[b] : 0.0f;
                 const bool bp = (bbits[k] >> lane) & 1u;
-                float lbmax = -INFINITY;
                 for (u32 a0 = 0; a0 < S; a0 += 32) {
-                    // lags of row a against the block: a - 32 k - 31 .. a - 32 k
-                    const u32 al = a0 + lane;
-                    const int wi = (int)al - (int)(32 * k) + (int)L;        // XMw index
-                    bool ka = al < S && al >= c.xlo && al < c.xhi_ex && wi >= 0 && wi < (int)NW;
-                    if (ka) {
-                        const float xw = apart ? 0.0f : __ldg(xmw + wi);
-                        ka = ga_hi[al] + mBk + xw + slack + kPruneSlack * fabsf(xw) >= TH;
-                    }
+                    const float xb = xw[a0 + 32 * (NB - 1 - k) + lane], ub = ua[a0 + lane];
+                    const bool ka = xb > -INFINITY && ub > -INFINITY && ub + mBk + xb + slack >= TH;
                     u32 rows = __ballot_sync(0xffffffffu, ka);
+                    const u32 ap = abits[a0 / 32];
                     while (rows) {
-                        const u32 a = a0 + __ffs(rows) - 1;
+                        const u32 r = __ffs(rows) - 1, a = a0 + r;
                         rows &= rows - 1;
-                        const float hi_a = ga_hi[a];
-                        bool valid = inb && (a > b ? a - b : b - a) <= L &&              // .cl:543-556
-                                     (bp || ((abits[a >> 5] >> (a & 31)) & 1u));         // .cl:572-576
-                        if (valid) {
-                            const float xr = apart ? 0.0f : __ldg(xmr + (int)a - (int)b + (int)L);
-                            valid = hi_a + hi_b + xr + slack + kPruneSlack * fabsf(xr) >= TH;
-                        }
-                        if (!__any_sync(0xffffffffu, valid)) continue;
-                        float hi = -INFINITY;
-                        if (valid) {
-                            const float X = apart ? 0.0f : ov_x(q, L, (int)a - (int)nmax, (int)a - (int)b);
-                            const float ex = kx * fabsf(X);
-                            hi = hi_a + hi_b - X + ex;
-                            lbmax = fmaxf(lbmax, ga_lo[a] + lo_b - X - ex);
-                            evaluated++;
-                        }
-                        const bool keep = valid && hi >= TH && hi > c.lbest;
-                        const u32 mk = __ballot_sync(0xffffffffu, keep);
-                        if (mk) {
-                            u32 base = 0;
-                            if (lane == 0) base = atomicAdd(A.pool_total, (u32)__popc(mk));
-                            base = __shfl_sync(0xffffffffu, base, 0);
-                            if (keep) {
-                                const u32 pp = base + __popc(mk & ((1u << lane) - 1u));
-                                if (pp < A.pool_cap) {
-                                    A.pool_slot[pp] = g;
-                                    A.pool_item[pp] = t + K * (a + S * b);
-                                    A.pool_hi[pp] = hi;
-                                } else {
-                                    A.fallback[g] = 1;
-                                }
-                            }
-                        }
+                        const bool valid = inb && (a > b ? a - b : b - a) <= L &&        // .cl:543-556
+                                           (bp || ((ap >> r) & 1u)) &&                   // .cl:572-576
+                                           ua[a] + hi_b + xr[(int)a - (int)b + (int)L] + slack >= TH;
+                        const u32 m = __ballot_sync(0xffffffffu, valid);
+                        if (m == 0) continue;
+                        if (valid) queue[held + __popc(m & ((1u << lane) - 1u))] = a | (b << 16);
+                        held += __popc(m);
+                        if (held >= 32) drain();
                     }
-                }
-                lbmax = warp_max_f(lbmax);
-                if (lbmax > TH) {
-                    if (lane == 0) atomicMax(reinterpret_cast<int *>(A.cand_lb) + g, __float_as_int(lbmax));   // > 0
-                    TH = lbmax;
-                    slack = kPruneSlack * (2.0f * mabs + fabsf(TH) + fabsf(XM));
                 }
             }
+            if (held) drain();
         }
     }
     if (A.items_evaluated) {
