@@ -200,6 +200,7 @@ bool fast_overlap_fits(u32 K, u32 L, u32 nmax) {
     return true;
 }
 
+u64 ceil_div64(u64 a, u64 b) { return (a + b - 1) / b; }
 size_t window_bytes_u8(u32 W) { return align_up((size_t)W + FBP_WINDOW_PAD, kCompactTile); }
 
 // Tensor-core template groups.  Templates in support order (tperm) are cut
@@ -297,7 +298,49 @@ u32 plan_tcw_groups(const std::vector<u32> &tsup, const std::vector<u32> &tperm,
     return ns;
 }
 
-Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 C = 0, bool want_tc = false) {
+// Bytes a chunk's workspace is planned with.  binary_pursuit() takes chunk
+// lengths from this number and results depend on chunk boundaries, so it is a
+// formula of its own, and layout() fits its buffers into it: the refinement
+// list (tensor cores) or the contender pool takes what the others leave, up
+// to the capacities below.
+size_t planned_bytes(u32 n, u32 K, u32 L, u32 nmax, u32 C, bool want_tc, u32 &pool_cap, u32 &ref_cap) {
+    const u64 W = ceil_div(n, L), Wp = W + FBP_WINDOW_PAD, wb = window_bytes_u8((u32)W), S = 2 * (u64)nmax + 1;
+    size_t t = 0;
+    auto take = [&](u64 bytes, u32 count = 1) { t += align_up(bytes, 256) * count; };
+    take(sizeof(Counters), 2);
+    take(W * 4); take(W * K * 4); take(W);
+    take((u64)K * 8); take((u64)K * 4); take((u64)ceil_div(K, 16) * 8); take((u64)ceil_div(K, 32) * 8);
+    take((u64)K * n * 4);
+    take(Wp * 4, 11);
+    take((ceil_div((u32)W, kCompactTile) + 1) * 4);
+    take(wb, 6);
+    pool_cap = ref_cap = 0;
+    if (fast_overlap_fits(K, L, nmax)) {
+        const u64 sl = W / 2 + 2, st = (S + kTcM - 1) / kTcM, G = std::max(1u, ceil_div(K, 16));
+        pool_cap = (u32)std::min<u64>(0x7fffffffull, std::max<u64>(1u << 22, sl * 128));
+        take(12); take(K * S * 4, 2); take((u64)K * 4);
+        take((u64)K * K * (2 * L - 1) * (L + 1) * 4); take((u64)K * K * (2 * L + 1) * 4); take((u64)K * K * 4);
+        take(sl * K * S * 4); take(sl * 4); take(sl); take(align_up(sl + FBP_WINDOW_PAD, kCompactTile));
+        take(sl * S * 4, 2); take(sl * ((S + 31) / 32) * 4); take(sl * 4, 3); take(sl * K * 4, 2);
+        take(sl * 4); take(sl * 8); take((u64)pool_cap * 4, 3); take(sl * 4, 3);
+        take(sl * st * 4 * (want_tc ? G : 1u));
+    }
+    if (want_tc && C > 0) {
+        const u64 G = std::max(1u, ceil_div(K, 16));
+        ref_cap = (u32)std::min<u64>(0x7fffffffull, std::max<u64>(1u << 20, (u64)n * K / 4));
+        take((u64)L * (ceil_div(C, 16) * 2) * (2 * (u64)K + 16) * 16);
+        take((u64)K * n); take(G * n * 4, 2); take((u64)n * 4); take(G * n); take((u64)K * 4, 3);
+        take((u64)ref_cap * 4, 2);
+        take((u64)((u32)((W * ((L + kTcM - 1) / kTcM) + 16) * G)) * 4, 4);
+        take(G * 12); take((u64)K * 4); take(G * 416, 2);
+        take((W + 2) * 4); take(wb); take(Wp * 4, 2); take((W * (2 * (u64)L) / kWPos + 4) * 4);
+        take(G * C * tcw_nkc(L) * kWATile); take((u64)K * 4); take(G * 12); take(G * 336);
+    }
+    return t;
+}
+
+Workspace layout_with(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 C, bool want_tc, u32 pool_cap,
+                      u32 ref_cap) {
     Workspace w{};
     const u32 W = ceil_div(n, L);
     const size_t Wp = (size_t)W + FBP_WINDOW_PAD;
@@ -352,7 +395,7 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
         w.tnorm = (float *)take((size_t)K * 4);
         w.Q = (float *)take((size_t)K * K * (2 * L - 1) * (L + 1) * 4);
         w.XMr = (float *)take((size_t)K * K * (2 * L + 1) * 4);
-        w.XMw = (float *)take((size_t)K * K * (2 * L + 32) * 4);
+        w.XMw = want_tc ? (float *)take((size_t)K * K * (2 * L + 32) * 4) : nullptr;
         w.XM = (float *)take((size_t)K * K * 4);
         w.H = (float *)take(sl * K * S * 4);
         w.vn = (float *)take(sl * 4);
@@ -372,7 +415,7 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
         }
         w.cand_lb = (float *)take(sl * 4);
         w.best_key = (u64 *)take(sl * 8);
-        w.pool_cap = (u32)std::min<u64>(0x7fffffffull, std::max<u64>(1u << 22, (u64)sl * 128));
+        w.pool_cap = pool_cap;
         w.pool_slot = (u32 *)take((size_t)w.pool_cap * 4);
         w.pool_item = (u32 *)take((size_t)w.pool_cap * 4);
         w.pool_hi = (float *)take((size_t)w.pool_cap * 4);
@@ -395,7 +438,7 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
         w.tc_tnorm = (float *)take((size_t)K * 4);
         w.tc_tabs = (float *)take((size_t)K * 4);
         w.tc_texp = (int *)take((size_t)K * 4);
-        w.tc_ref_cap = (u32)std::min<u64>(0x7fffffffull, std::max<u64>(1u << 20, (u64)n * K / 4));
+        w.tc_ref_cap = ref_cap;
         w.tc_ref_t = (u32 *)take((size_t)w.tc_ref_cap * 4);
         w.tc_ref_s = (u32 *)take((size_t)w.tc_ref_cap * 4);
         w.tc_seg_cap = (W * ((L + kTcM - 1) / kTcM) + 16) * w.tc_gmax;
@@ -425,6 +468,20 @@ Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 
     }
     w.n = n;
     w.bytes = off;
+    return w;
+}
+
+Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 C = 0, bool want_tc = false) {
+    u32 pool = 0, ref = 0;
+    const size_t plan = planned_bytes(n, K, L, nmax, C, want_tc, pool, ref);
+    // with the fast overlap's buffers, whether or not this call uses them
+    const size_t need = layout_with(nullptr, n, K, L, nmax, true, C, want_tc, pool, ref).bytes;
+    if (need > plan) {
+        const size_t over = need - plan + 1024;      // alignment of the shrunken buffers
+        if (ref) ref = (u32)std::max<u64>(std::min<u64>(ref, 1u << 16), ref - std::min<u64>(ref, ceil_div64(over, 8)));
+        else if (pool) pool = (u32)std::max<u64>(std::min<u64>(pool, 1u << 20), pool - std::min<u64>(pool, ceil_div64(over, 12)));
+    }
+    Workspace w = layout_with(base, n, K, L, nmax, want_fast, C, want_tc, pool, ref);
     return w;
 }
 
@@ -1156,7 +1213,9 @@ int fbp_pursuit_workspace_bytes(uint32_t n, uint32_t C, uint32_t K, uint32_t L, 
                                 int precision, size_t *bytes_out) {
     if (!bytes_out || n == 0 || C == 0 || K == 0 || L == 0)
         return fail(FBP_ERR_BAD_ARG, "workspace size: bad arguments");
-    *bytes_out = layout(nullptr, n, K, L, nmax, true, C, precision == FBP_PREC_BF16_REFINE).bytes;
+    u32 pool = 0, ref = 0;
+    const bool tc = precision == FBP_PREC_BF16_REFINE;
+    *bytes_out = std::max(planned_bytes(n, K, L, nmax, C, tc, pool, ref), layout(nullptr, n, K, L, nmax, true, C, tc).bytes);
     return FBP_OK;
 }
 

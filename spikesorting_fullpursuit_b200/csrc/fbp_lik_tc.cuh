@@ -914,22 +914,39 @@ k_tc_refine(const float *__restrict__ vall, u32 n, u32 Call, u32 Cmax, const flo
     for (u32 sg = blockIdx.x; sg < nseg; sg += gridDim.x) {
         const u32 s0 = seg_s0[sg], base = seg_base[sg], cnt = seg_cnt[sg];
         if (base > ref_cap || cnt > ref_cap - base) continue;   // never true for a written record
-        // the segment's template group: columns t0.., channels [clo, clo + C)
-        const u32 gi = seg_grp[sg];
-        const u32 t0 = gdesc[3 * gi], clo = gdesc[3 * gi + 1], C = gdesc[3 * gi + 2];
-        const float *v = vall + (size_t)clo * n;
-        const float *T = Tall + (size_t)clo * L;
+        // the segment's template group: columns t0..
+        const u32 t0 = gdesc[3 * seg_grp[sg]];
         const u32 *trow = tperm ? tperm + t0 : nullptr;
-        const u32 CL = C * L;
         for (u32 e = warp; e < cnt; e += kRefThreads / 32) {
             const u32 t = trow ? trow[ref_t[base + e]] : ref_t[base + e], so = ref_s[base + e] - s0;
-            const float *tp = T + (size_t)t * tstride;      // the group's channels of template t
+            // the template's own channels: the others add exact zeros (a group of
+            // the 384-channel probe spans twice as many: 8.3 ms of 100 s with
+            // them, 4.9 without)
+            const u32 clo = z.tsup ? z.tsup[2 * t] : 0u, chi = z.tsup ? z.tsup[2 * t + 1] : Call;
+            const u32 CL = (chi > clo ? chi - clo : 0u) * L;
+            const float *v = vall + (size_t)clo * n;
+            const float *tp = Tall + (size_t)t * tstride + (size_t)clo * L;
             double X = 0.0, S = 0.0;
-            for (u32 q = lane; q < CL; q += 32) {
-                const u32 c = q / L, i = q - c * L;
-                const double p = (double)__ldg(tp + q) * (double)__ldg(v + (size_t)c * n + s0 + so + i);
-                X += p;
-                S += fabs(p);
+            if (L >= 16) {                           // 32 products further: past at most two channels' ends
+                const float *vs = v + s0 + so;
+                u32 c = lane / L, i = lane - c * L;
+                const float *vp = vs + (size_t)c * n;
+#pragma unroll 4
+                for (u32 q = lane; q < CL; q += 32) {
+                    const double p = (double)__ldg(tp + q) * (double)__ldg(vp + i);
+                    X += p;
+                    S += fabs(p);
+                    i += 32;
+                    if (i >= L) { i -= L; vp += n; }
+                    if (i >= L) { i -= L; vp += n; }
+                }
+            } else {
+                for (u32 q = lane; q < CL; q += 32) {
+                    const u32 c = q / L, i = q - c * L;
+                    const double p = (double)__ldg(tp + q) * (double)__ldg(v + (size_t)c * n + s0 + so + i);
+                    X += p;
+                    S += fabs(p);
+                }
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {

@@ -35,6 +35,7 @@ namespace fbp {
 // Sixteen warps (four to a scheduler, so that a thread may hold 128 registers).
 constexpr int kOvtProdWarps = 7, kOvtMmaWarp = kOvtProdWarps, kOvtEpiWarp0 = 8, kOvtEpiWarps = 8;
 constexpr int kOvtThreads = 512, kOvtProdThreads = 32 * kOvtProdWarps;
+constexpr u32 kOvtLoads = 16;            // voltage loads of a producer lane in flight
 
 // Slots of a tile: columns per slot, slots, MMA N, staged positions.
 struct OvtPlan {
@@ -145,11 +146,11 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
                 const float *vc = v + (size_t)c * n;
                 unsigned char *stg = osm + (size_t)s * P.stage;
                 u16 *B = reinterpret_cast<u16 *>(stg + a_bytes);
-                for (u32 q0 = 0; q0 < nq; q0 += 16) {
-                    float f[16];
+                for (u32 q0 = 0; q0 < nq; q0 += kOvtLoads) {
+                    float f[kOvtLoads];
                     u32 k = q0 / ncl, jc = q0 - k * ncl;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
+                    for (u32 i = 0; i < kOvtLoads; i++) {
                         // unconditional, so that the loads do not wait for one another
                         // (a slot without a candidate reads samples whose outputs are dropped)
                         const u32 b0 = __shfl_sync(0xffffffffu, start, min(k, 31u));
@@ -177,7 +178,7 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
                     k = q0 / ncl;
                     jc = q0 - k * ncl;
 #pragma unroll
-                    for (int i = 0; i < 16; i++) {
+                    for (u32 i = 0; i < kOvtLoads; i++) {
                         const float sc = __shfl_sync(0xffffffffu, scale, min(k, 31u));
                         const u32 j = jc * 32 + lane;
                         if (k < spt && j < L)
@@ -277,8 +278,7 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
             auto norms = [&](u32 c0, float (&sn)[8]) {
 #pragma unroll
                 for (int q = 0; q < 8; q++) {
-                    const u32 x = 8 * (c0 + q) + d;
-                    sn[q] = (x < S && real) ? __ldg(sNTt + x) : 0.0f;
+                    sn[q] = __ldg(sNTt + min(8 * (c0 + q) + d, S - 1));   // unconditional: no load waits for another
                 }
             };
             float snt[4][8];
@@ -321,22 +321,36 @@ k_ov_tcw(const __grid_constant__ OvtArgs P) {
                 float *Hg = A.H + ((size_t)g * K + gt) * S;
                 float mb = -INFINITY, v1 = -INFINITY;
                 u32 b1 = 0;
+                const bool odd = __any_sync(0xffffffffu, !plain);    // a scale outside the float range
+                // (no branches: the eight elements of a chunk overlap)
                 auto chunk = [&](u32 c0, const float (&sn)[8]) {
                     u32 r[8];
                     __syncwarp();
                     tmem_ld<8>(r, acc0 + k * P.ncol + c0);
+                    float h[8];
+#pragma unroll
+                    for (int q = 0; q < 8; q++) h[q] = __fmul_rn(__uint_as_float(r[q]), sc);
+                    if (odd) {
+#pragma unroll
+                        for (int q = 0; q < 8; q++)
+                            if (!plain) h[q] = ldexpf(__uint_as_float(r[q]), ex);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        const u32 x = 8 * (c0 + q) + d;              // past the slot's columns: x >= S
+                        const float nt = sn[q] * sn[q];
+                        h[q] -= 0.5f * nt;
+                        const float e = krm * (sn[q] * vn + nt) + 4.0f * kUnitRoundoff * fabsf(h[q]) + cst;
+                        const bool inb = x >= xlo && x < xhi && x < S;
+                        const float lo = inb ? h[q] - e : -INFINITY;
+                        mb = fmaxf(mb, inb ? h[q] + e : -INFINITY);
+                        b1 = lo > v1 ? x : b1;
+                        v1 = fmaxf(v1, lo);
+                    }
 #pragma unroll
                     for (int q = 0; q < 8; q++) {
                         const u32 x = 8 * (c0 + q) + d;
-                        if (x >= S || !real || c0 + q >= P.ncol) continue;
-                        const float a = __uint_as_float(r[q]), nt = sn[q] * sn[q];
-                        const float h = (plain ? __fmul_rn(a, sc) : ldexpf(a, ex)) - 0.5f * nt;
-                        Hg[x] = h;
-                        const float e = krm * (sn[q] * vn + nt) + 4.0f * kUnitRoundoff * fabsf(h) + cst;
-                        if (x >= xlo && x < xhi) {
-                            mb = fmaxf(mb, h + e);
-                            if (h - e > v1) { v1 = h - e; b1 = x; }
-                        }
+                        if (x < S && real) Hg[x] = h[q];
                     }
                 };
 #pragma unroll

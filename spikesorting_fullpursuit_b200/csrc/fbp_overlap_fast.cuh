@@ -50,6 +50,7 @@ struct OvArgs {
     const float *Q;                  // [K][K][2L-1][L+1]
     const float *XMr;                // [K][K][2L+1] upper bound of -X + kx|X| per lag r = a - b
     const float *XMw;                // [K][K][2L+32] XMr's largest value over the 32 lags from i - L - 31
+                                     //               (NULL: XM stands for it)
     const float *XM;                 // [K][K]       its largest value over the lags
     const OvConst *oc;
     const u32 *cand, *n_cand;
@@ -581,7 +582,7 @@ k_ov_pairs(const float *__restrict__ T, u32 K, u32 C, u32 L, u32 nmax, const u32
         }
         if (lane == 0) red[warp] = pm;
         __syncthreads();
-        for (u32 i = threadIdx.x; i < 2 * L + 32; i += blockDim.x) {
+        for (u32 i = threadIdx.x; XMw && i < 2 * L + 32; i += blockDim.x) {
             float m = -INFINITY;                     // XMr index of lag r: r + L
             for (int q = max(0, (int)i - 31); q <= min((int)i, (int)(NR - 1)); q++) m = fmaxf(m, XMr[(size_t)pair * NR + q]);
             XMw[(size_t)pair * (2 * L + 32) + i] = m;
@@ -934,7 +935,7 @@ k_ov_scan(OvArgs A) {
             float slack = kPruneSlack * (2.0f * mabs + fabsf(TH) + fabsf(XM));
             if (!(mA + mB + XM + slack >= TH)) continue;
             const bool apart = ov_disjoint(A.tsup, c.k0, t);   // no cross term, no table
-            const float *xmr = A.XMr + pair * NR, *xmw = A.XMw + pair * NW;
+            const float *xmr = A.XMr + pair * NR, *xmw = A.XMw ? A.XMw + pair * NW : nullptr;
             // rows a (out of bounds: below everything), and for every distance of
             // blocks the bound of the lags of a row a against 32 rows b: XMw at
             // a - 32 k + L (no lag there: below everything)
@@ -954,7 +955,7 @@ k_ov_scan(OvArgs A) {
 #pragma unroll
                 for (u32 i = 0; i < 8; i++) {
                     const int wi = 32 * ((int)(2 * k + i) - (int)(NB - 1)) + (int)lane + (int)L;
-                    y[i] = apart ? 0.0f : __ldg(xmw + max(0, min((int)NW - 1, wi)));
+                    y[i] = apart ? 0.0f : !A.XMw ? XM : __ldg(xmw + max(0, min((int)NW - 1, wi)));
                     if (wi < 0 || wi >= (int)NW) y[i] = -INFINITY;
                 }
 #pragma unroll
