@@ -930,14 +930,13 @@ int tc_likelihood_pass(const Workspace &w, const float *v, u32 n, u32 C, const f
 int tc_refine_pass(const Workspace &w, const float *v, u32 n, u32 C, const float *T, u32 K, u32 L,
                    const float *tss, const u32 *win, const u32 *n_win, u32 max_windows, float *Lk,
                    Counters *cnt, cudaStream_t st, int *launches) {
-    const size_t rsmem = tc_refine_smem_bytes(w.tc_cmax, L);
-    if (rsmem > 48 * 1024)
-        FBP_ALLOW_SMEM(k_tc_refine);
+    const size_t rsmem = tc_refine_smem_bytes(w.tc_cmax, L);   // below 48 KB
     // gamma: the reference's recursive sum of C*L + 1 terms (products
     // rounded once each), plus the double sums' own error
     const double u = 1.0 / 16777216.0, nr = (double)w.tc_nz * L + 2;
     const double gamma = 1.01 * (nr * u / (1.0 - nr * u)) + 4.0 * nr * 1.1102230246251565e-16;
-    k_tc_refine<<<sm_count() * 8, kRefThreads, rsmem, st>>>(
+    auto refine = L >= 16 ? k_tc_refine<true> : k_tc_refine<false>;
+    refine<<<sm_count() * 8, kRefThreads, rsmem, st>>>(
         v, n, C, w.tc_cmax, T, K, L, tss, w.tc_ref_t, w.tc_ref_s, w.tc_seg_s0, w.tc_seg_base, w.tc_seg_cnt,
         w.tc_seg_grp, w.tcw ? w.tcw_gdesc : w.tc_gdesc, w.tperm, reinterpret_cast<const u32 *>(&cnt->tc_refseg), w.tc_seg_cap, Lk,
         lazy_ctx(w, v, T, tss, C, L, 0), gamma, &cnt->tc_seq, w.wpos, w.G16, &cnt->tc_overflow, w.tc_ref_cap);

@@ -894,6 +894,10 @@ __host__ __device__ inline size_t tc_refine_smem_bytes(u32 C, u32 L) {
     (void)C; (void)L;
     return (size_t)(kRefThreads / 32) * kWarpChunk * 4;
 }
+// kLong: L >= 16.  Bound by the latency of its loads, so by how many the loop
+// has in flight: with the general index step in the same loop the compiler
+// keeps fewer, and it takes 39 to 47 ms where this one takes 30 (linear16 300 s).
+template <bool kLong>
 __global__ void __launch_bounds__(kRefThreads)
 k_tc_refine(const float *__restrict__ vall, u32 n, u32 Call, u32 Cmax, const float *__restrict__ Tall, u32 K,
             u32 L, const float *__restrict__ tss, const u32 *__restrict__ ref_t, const u32 *__restrict__ ref_s,
@@ -927,7 +931,7 @@ k_tc_refine(const float *__restrict__ vall, u32 n, u32 Call, u32 Cmax, const flo
             const float *v = vall + (size_t)clo * n;
             const float *tp = Tall + (size_t)t * tstride + (size_t)clo * L;
             double X = 0.0, S = 0.0;
-            if (L >= 16) {                           // 32 products further: past at most two channels' ends
+            if constexpr (kLong) {                   // 32 products further: past at most two channels' ends
                 const float *vs = v + s0 + so;
                 u32 c = lane / L, i = lane - c * L;
                 const float *vp = vs + (size_t)c * n;
