@@ -145,7 +145,7 @@ struct Workspace {
     bool masked_tables = false;      // templates occupy narrow channel ranges
     OvConst *oc;
     u8 *cskip, *fallback, *need;
-    u32 *pool_slot, *pool_item, *fb_slots, *fb_list;
+    u32 *pool_slot, *pool_item;
     u64 *best_key;
     u32 pool_cap;
     int *kexp_tile;
@@ -419,8 +419,6 @@ Workspace layout_with(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast,
         w.pool_slot = (u32 *)take((size_t)w.pool_cap * 4);
         w.pool_item = (u32 *)take((size_t)w.pool_cap * 4);
         w.pool_hi = (float *)take((size_t)w.pool_cap * 4);
-        w.fb_slots = (u32 *)take(sl * 4);
-        w.fb_list = (u32 *)take(sl * 4);
         w.stiles = (S + kTcM - 1) / kTcM;
         w.kexp_tile = (int *)take(sl * w.stiles * 4 * (want_tc ? std::max(1u, ceil_div(K, 16)) : 1u));
     }
@@ -500,6 +498,11 @@ int compact(const u8 *f, u32 W, u32 *list, u32 *count_dev, u32 *tile_counts, cud
         FBP_CUDA(cudaMemsetAsync(count_dev, 0, 4, st));
         return FBP_OK;
     }
+    if (tiles <= kCompactOneTiles) {
+        k_compact_one<<<tiles, kCompactThreads, 0, st>>>(f, W, list, count_dev);
+        FBP_LAUNCH_CHECK();
+        return FBP_OK;
+    }
     k_compact_count<<<tiles, kCompactThreads, 0, st>>>(f, W, tile_counts);
     k_compact_scan<<<1, kCompactThreads, 0, st>>>(tile_counts, tiles, count_dev);
     k_compact_write<<<tiles, kCompactThreads, 0, st>>>(f, W, tile_counts, list);
@@ -537,7 +540,8 @@ int launch_argmax(u32 n, u32 L, u32 K, const u32 *win, const u32 *n_win_dev, u32
 int launch_overlap(const float *v, u32 n, u32 C, const float *T, u32 K, u32 L, const u32 *cand,
                    const u32 *n_cand_dev, u32 max_cand, const fbp_window_state &s, float *Lk,
                    u32 nmax, const float *thr, u64 *items_evaluated, cudaStream_t st,
-                   const LazyLk &z = LazyLk{}, const u32 *tsup = nullptr) {
+                   const LazyLk &z = LazyLk{}, const u32 *tsup = nullptr, const u8 *only = nullptr,
+                   u32 *n_only = nullptr) {
     const size_t smem = (size_t)2 * C * L * sizeof(float);
     if (smem > 227 * 1024)
         return fail(FBP_ERR_BAD_ARG, "overlap recheck: C*L = %u too large for shared memory", C * L);
@@ -547,18 +551,19 @@ int launch_overlap(const float *v, u32 n, u32 C, const float *T, u32 K, u32 L, c
     const int grid = grid_for((u64)max_cand * kOvThreads, kOvThreads, 4);
     k_overlap_exact<<<grid, kOvThreads, smem, st>>>(v, n, C, T, K, L, cand, n_cand_dev, s.best_idx,
                                                     s.best_lab, s.best_ll, s.ov_idx, s.ov_lab,
-                                                    s.overlap_recheck, Lk, nmax, thr, items_evaluated, z, tsup);
+                                                    s.overlap_recheck, Lk, nmax, thr, items_evaluated, z, tsup, only,
+                                                    n_only);
     FBP_LAUNCH_CHECK();
     return FBP_OK;
 }
 
 int launch_check_overlap(u32 n, u32 L, const u32 *cand, const u32 *n_cand_dev, u32 max_cand,
-                         const fbp_window_state &s, u8 *scratch, cudaStream_t st) {
+                         const fbp_window_state &s, u8 *scratch, cudaStream_t st, bool copy = true) {
     const int threads = 256;
     const int grid = grid_for(max_cand, threads, 8);
     k_check_overlap<<<grid, threads, 0, st>>>(n, L, cand, n_cand_dev, s.best_idx, s.best_lab, s.flags,
                                               s.ov_idx, s.ov_lab, s.overlap_recheck, scratch);
-    k_copy_ovr<<<grid, threads, 0, st>>>(cand, n_cand_dev, scratch, s.overlap_recheck);
+    if (copy) k_copy_ovr<<<grid, threads, 0, st>>>(cand, n_cand_dev, scratch, s.overlap_recheck);
     FBP_LAUNCH_CHECK();
     return FBP_OK;
 }
@@ -567,12 +572,12 @@ int launch_accept(u32 n, u32 C, u32 L, const float *thr, const u32 *win, const u
                   u32 max_windows, const fbp_window_state &s, const u8 *active, u8 *has, u8 *flags_out,
                   u32 *acc_list, u32 *spk_idx, u32 *spk_lab, u32 *spk_win, u32 *n_spk_dev,
                   u32 *tile_counts, cudaStream_t st, const WinBounds &wb = WinBounds{}, const u32 *grange = nullptr,
-                  const u32 *tsup = nullptr, u32 K = 0) {
+                  const u32 *tsup = nullptr, u32 K = 0, const u8 *checked = nullptr) {
+    (void)win; (void)n_win_dev; (void)max_windows;
     const u32 W = ceil_div(n, L);
     const int threads = 256;
-    FBP_CUDA(cudaMemsetAsync(has, 0, window_bytes_u8(W), st));
-    k_accept_has<<<grid_for(max_windows, threads), threads, 0, st>>>(
-        n, C, L, thr, win, n_win_dev, s.best_idx, s.best_lab, s.best_ll, s.overlap_recheck, has);
+    k_accept_has<<<grid_for(W, threads), threads, 0, st>>>(n, C, L, W, thr, active, s.best_idx, s.best_lab, s.best_ll,
+                                                           s.overlap_recheck, checked, has);
     AcceptView a{n, C, L, W, n / L, thr, s.best_idx, s.best_lab, s.best_ll, active, has, s.flags};
     k_accept_flags<<<grid_for(W, threads), threads, 0, st>>>(a, flags_out);
     FBP_LAUNCH_CHECK();
@@ -682,11 +687,7 @@ int ov_chunk_setup(const Workspace &w, const float *T, u32 K, u32 C, u32 L, u32 
 int ov_fast_tables(const Workspace &w, const OvArgs &A, Counters *cnt, cudaStream_t st, int *launches) {
     const u32 slots = w.slots;
     const u32 S = A.S;
-    FBP_CUDA(cudaMemsetAsync(w.fallback, 0, align_up((size_t)slots + FBP_WINDOW_PAD, kCompactTile), st));
-    FBP_CUDA(cudaMemsetAsync(&cnt->pool_total, 0, 4, st));
-    FBP_CUDA(cudaMemsetAsync(&cnt->ov_ref, 0, 4, st));
-    FBP_CUDA(cudaMemsetAsync(&cnt->scan_next, 0, 8, st));
-    k_ov_prep<<<grid_for((u64)slots * 32, 256), 256, 0, st>>>(A);
+    k_ov_prep<<<grid_for((u64)slots * (w.tc ? 1 : 32), 256), 256, 0, st>>>(A, slots, &cnt->fb_count);
     FBP_LAUNCH_CHECK();
     if (w.ovw) {
         FBP_ALLOW_SMEM(k_ov_tcw);
@@ -743,14 +744,11 @@ int ov_fast_pass(const Workspace &w, const OvArgs &A, Counters *cnt, cudaStream_
     k_ov_refine<<<(int)sm_count() * 4, kRefineThreads, ov_refine_smem_bytes(), st>>>(A);   // four blocks fit an SM
     k_ov_finalize<<<grid_for((u64)slots * 32, kRefineThreads, 8), kRefineThreads, 0, st>>>(A);
     FBP_LAUNCH_CHECK();
-    int rc = compact(w.fallback, slots, w.fb_slots, &cnt->fb_count, w.tile_counts, st);
-    if (rc) return rc;
-    k_ov_fallback_list<<<grid_for(slots, 256), 256, 0, st>>>(A, w.fb_slots, &cnt->fb_count, w.fb_list);
-    FBP_LAUNCH_CHECK();
+    // candidates whose contenders did not fit the pool: every item exactly
     fbp_window_state s{A.best_idx, A.best_lab, A.best_ll, A.ov_idx, A.ov_lab, nullptr, A.ovr};
-    rc = launch_overlap(A.v, A.n, A.C, A.T, A.K, A.L, w.fb_list, &cnt->fb_count, slots, s, A.Lk, A.nmax, A.thr,
-                        A.items_evaluated, st, A.lazy, w.tsup);
-    *launches = 10;
+    const int rc = launch_overlap(A.v, A.n, A.C, A.T, A.K, A.L, A.cand, A.n_cand, slots, s, A.Lk, A.nmax, A.thr,
+                                  A.items_evaluated, st, A.lazy, w.tsup, w.fallback, &cnt->fb_count);
+    *launches = 6;
     return rc;
 }
 
@@ -901,13 +899,11 @@ int tc_likelihood_pass(const Workspace &w, const float *v, u32 n, u32 C, const f
                        const float *tss, const u32 *win, const u32 *n_win, u32 max_windows, float *Lk,
                        Counters *cnt, cudaStream_t st, int *launches, float *dbg_bound = nullptr) {
     (void)max_windows; (void)v; (void)C; (void)T;
-    FBP_CUDA(cudaMemsetAsync(&cnt->tc_refseg, 0, 8, st));
-    FBP_CUDA(cudaMemsetAsync(&cnt->tc_overflow, 0, 4, st));   // set by the tiles when the list overflows
     if (w.tcw) {
         // the groups' window lists and streams, then their tiles
         const u32 W = ceil_div(n, L), G = (u32)w.tcwg.size();
         const dim3 lg(ceil_div(W, kCompactTile), G);
-        k_tcw_count<<<lg, kCompactThreads, 0, st>>>(w.active, w.dirty, w.GW, W, w.wl_counts);
+        k_tcw_count<<<lg, kCompactThreads, 0, st>>>(w.active, w.dirty, w.GW, W, w.wl_counts, cnt);
         k_tcw_lists<<<lg, kCompactThreads, 0, st>>>(w.active, w.dirty, w.GW, W, L, w.wl_counts, w.wl_stride,
                                                      w.wf_stride, w.wl_win, w.wl_pos, w.wl_first, w.wl_nwin, w.wl_nst);
         FBP_ALLOW_SMEM(k_lik_tcw);
@@ -917,6 +913,8 @@ int tc_likelihood_pass(const Workspace &w, const float *v, u32 n, u32 C, const f
         return FBP_OK;
     }
     (void)win; (void)n_win;
+    FBP_CUDA(cudaMemsetAsync(&cnt->tc_refseg, 0, 8, st));
+    FBP_CUDA(cudaMemsetAsync(&cnt->tc_overflow, 0, 4, st));   // set by the tiles when the list overflows
     FBP_ALLOW_SMEM(k_lik_tc<0>);
     const u32 G = (u32)w.tcg.size();
     k_lik_tc<0><<<std::max<u32>(sm_count(), G), kTcThreads, w.tc_smem, st>>>(w.tc_args0, G);
@@ -1266,6 +1264,7 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
     // counts from device memory, so the same launches serve every pass.  The
     // counts of the pass are snapshotted (w.snap) before the next pass's
     // window list overwrites them.  `launched` receives the launches per stage.
+    const u32 ncompact = ceil_div(W, kCompactTile) <= kCompactOneTiles ? 1 : 3;   // launches of compact()
     auto enqueue_pass = [&](u32 pass, uint64_t *launched, cudaStream_t q) -> int {
         int rc2 = FBP_OK;
         // 1. likelihood over the listed windows (.py:538-549)
@@ -1303,7 +1302,7 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
         if (do_overlap_recheck) {
             timer.begin(FBP_STAGE_LISTS);
             if ((rc2 = compact(w.ovr, W, w.cand, &w.cnt->n_cand, w.tile_counts, q))) return rc2;
-            launched[FBP_STAGE_LISTS] += 3;
+            launched[FBP_STAGE_LISTS] += ncompact;
             timer.end(FBP_STAGE_LISTS);
             timer.begin(FBP_STAGE_OVERLAP);
             if (w.fast) {
@@ -1326,32 +1325,30 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
             }
             timer.end(FBP_STAGE_OVERLAP);
             timer.begin(FBP_STAGE_CHECK);
-            if ((rc2 = launch_check_overlap(n, L, w.cand, &w.cnt->n_cand, W, s, w.ovr2, q))) return rc2;
-            launched[FBP_STAGE_CHECK] += 2;
+            if ((rc2 = launch_check_overlap(n, L, w.cand, &w.cnt->n_cand, W, s, w.ovr2, q, false))) return rc2;
+            launched[FBP_STAGE_CHECK] += 1;
             timer.end(FBP_STAGE_CHECK);
         }
         // 5. accept (.py:663-671)
         timer.begin(FBP_STAGE_ACCEPT);
         if ((rc2 = launch_accept(n, C, L, thresholds, w.win, &w.cnt->n_win, W, s, w.active, w.has,
                                  w.flags_out, w.acc_list, w.spk_idx, w.spk_lab, w.spk_win, &w.cnt->n_spk,
-                                 w.tile_counts, q, win_bounds(w), w.grange, w.tsup, K)))
+                                 w.tile_counts, q, win_bounds(w), w.grange, w.tsup, K,
+                                 do_overlap_recheck ? w.ovr2 : nullptr)))
             return rc2;
-        launched[FBP_STAGE_ACCEPT] += 6;
+        launched[FBP_STAGE_ACCEPT] += 3 + ncompact;
         timer.end(FBP_STAGE_ACCEPT);
         // 6. the pass's counts (.py:673-676 stops when nothing was added)
         FBP_CUDA(cudaMemcpyAsync(w.snap, w.cnt, sizeof(Counters), cudaMemcpyDeviceToDevice, q));
         // 7. reset overlap flags, next list = nonzero(flags), reset flags (.py:678-700)
         timer.begin(FBP_STAGE_LISTS);
-        FBP_CUDA(cudaMemsetAsync(w.ovr, 0, wb, q));
         if ((rc2 = compact(w.flags_out, W, w.win, &w.cnt->n_win, w.tile_counts, q))) return rc2;
-        k_mark_active<<<grid_for(W, 256), 256, 0, q>>>(w.flags_out, w.active, W, win_bounds(w), K, w.tperm);
-        FBP_CUDA(cudaMemsetAsync(w.flags, 0, wb, q));
+        k_mark_active<<<grid_for(W, 256), 256, 0, q>>>(w.flags_out, w.active, W, win_bounds(w), K, w.tperm, w.ovr, w.flags);
         // 8. keep the spikes (.py:702-710)
         k_append_spikes<<<grid_for(W, 256), 256, 0, q>>>(w.spk_idx, w.spk_lab, w.cnt, spike_idx, spike_lab,
                                                            spike_cap);
-        k_commit_total<<<1, 1, 0, q>>>(w.cnt, spike_cap);
         FBP_LAUNCH_CHECK();
-        launched[FBP_STAGE_LISTS] += 6;
+        launched[FBP_STAGE_LISTS] += 2 + ncompact;
         timer.end(FBP_STAGE_LISTS);
         // 9. subtract them (.py:712-731)
         timer.begin(FBP_STAGE_RESIDUAL);
@@ -1363,7 +1360,7 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
         }
         k_residual<<<grid_for((u64)W * 256, 256, 16), 256, 0, q>>>(voltage, n, C, templates, K, L, w.spk_idx,
                                                                     w.spk_lab, &w.cnt->n_spk, 0, R, w.tsup,
-                                                                    w.tcw ? w.vwmax : nullptr);
+                                                                    w.tcw ? w.vwmax : nullptr, w.cnt, spike_cap);
         FBP_LAUNCH_CHECK();
         launched[FBP_STAGE_RESIDUAL] += 1;
         timer.end(FBP_STAGE_RESIDUAL);

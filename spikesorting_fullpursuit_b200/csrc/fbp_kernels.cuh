@@ -85,6 +85,39 @@ __global__ void k_compact_write(const u8 *__restrict__ f, u32 W, const u32 *__re
         if (base + i < W && b[i] != 0) out[off++] = base + i;
 }
 
+// The same in one launch, for at most kCompactOneTiles tiles: a block counts
+// the bytes of every tile before its own itself (on average 128 KB from L2 for
+// 64 tiles, a few microseconds, where two more launches cost four), then
+// writes its own.
+constexpr u32 kCompactOneTiles = 64;
+__global__ void __launch_bounds__(kCompactThreads)
+k_compact_one(const u8 *__restrict__ f, u32 W, u32 *__restrict__ out, u32 *__restrict__ total_out) {
+    const u32 before = blockIdx.x * kCompactTile;
+    u32 c = 0;
+#pragma unroll 4
+    for (u32 b = threadIdx.x * kCompactPerThread; b < before; b += kCompactTile) {   // whole tiles: all below W
+        const uint4 q = *reinterpret_cast<const uint4 *>(f + b);
+        const u32 w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) c += __popc(__vcmpne4(w[k], 0u)) >> 3;           // bytes that are not 0
+    }
+    u32 base_count;
+    block_excl_scan(c, &base_count);
+    __syncthreads();
+    const u32 base = before + threadIdx.x * kCompactPerThread;
+    const uint4 q = *reinterpret_cast<const uint4 *>(f + base);
+    const u8 *b = reinterpret_cast<const u8 *>(&q);
+    c = 0;
+#pragma unroll
+    for (u32 i = 0; i < kCompactPerThread; i++) c += (base + i < W && b[i] != 0);
+    u32 own;
+    u32 off = base_count + block_excl_scan(c, &own);
+#pragma unroll
+    for (u32 i = 0; i < kCompactPerThread; i++)
+        if (base + i < W && b[i] != 0) out[off++] = base + i;
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total_out = base_count + own;
+}
+
 // ---------------------------------------------------------------------------
 // Pass setup.
 // ---------------------------------------------------------------------------
@@ -100,12 +133,16 @@ __global__ void k_iota_windows(u32 *__restrict__ win, u8 *__restrict__ active, u
 // the bounds of the groups they recompute.  Warps take 32 windows at a time;
 // lanes then share each listed window's templates and groups.
 __global__ void k_mark_active(const u8 *__restrict__ flags, u8 *__restrict__ active, u32 W, WinBounds wb,
-                              u32 K, const u32 *__restrict__ tperm) {
+                              u32 K, const u32 *__restrict__ tperm, u8 *__restrict__ ovr, u8 *__restrict__ old_flags) {
     const u32 lane = threadIdx.x & 31, step = gridDim.x * blockDim.x;
     for (u32 i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < W; i0 += step) {
         const u32 i = i0 + lane;
         const bool on = i < W && flags[i] != 0;
-        if (i < W) active[i] = on;
+        if (i < W) {
+            active[i] = on;
+            ovr[i] = 0;                              // .py:679-680, :699-700
+            old_flags[i] = 0;
+        }
         u32 m = wb.umax ? __ballot_sync(0xffffffffu, on) : 0u;
         while (m) {
             const u32 w = i0 + __ffs(m) - 1;
@@ -684,7 +721,8 @@ k_overlap_exact(const float *__restrict__ v, u32 n, u32 C, const float *__restri
                 u32 *__restrict__ best_idx, u32 *__restrict__ best_lab, float *__restrict__ best_ll,
                 u32 *__restrict__ ov_idx, u32 *__restrict__ ov_lab, u8 *__restrict__ ovr,
                 const float *__restrict__ Lk, u32 nmax, const float *__restrict__ thr,
-                u64 *__restrict__ items_evaluated, LazyLk z, const u32 *__restrict__ tsup) {
+                u64 *__restrict__ items_evaluated, LazyLk z, const u32 *__restrict__ tsup,
+                const u8 *__restrict__ only, u32 *__restrict__ n_only) {
     extern __shared__ float sm[];          // vwin [C*L], tk0 [C*L]
     __shared__ float red_v[kOvThreads / 32];
     __shared__ u64 red_i[kOvThreads / 32];
@@ -693,6 +731,10 @@ k_overlap_exact(const float *__restrict__ v, u32 n, u32 C, const float *__restri
     const u64 items = (u64)S * S * K;
     float *vwin = sm, *tk0 = sm + (size_t)C * L;
     for (u32 g = blockIdx.x; g < n_cand; g += gridDim.x) {
+        if (only) {                        // the fast search's leftovers
+            if (!only[g]) continue;
+            if (threadIdx.x == 0) atomicAdd(n_only, 1u);
+        }
         const u32 id = cand[g];
         const u32 lab = best_lab[id], bidx = best_idx[id];
         const u32 lo_lab = tsup && lab < K ? tsup[2 * lab] : 0u, hi_lab = tsup && lab < K ? tsup[2 * lab + 1] : C;
@@ -807,19 +849,20 @@ __global__ void k_copy_ovr(const u32 *__restrict__ cand, const u32 *__restrict__
 // k_accept_flags: the flags after the kernel, for every window, reproducing
 // the sequential reads of the neighbours' flags in phase two.
 // ---------------------------------------------------------------------------
-__global__ void k_accept_has(u32 n, u32 C, u32 L, const float *__restrict__ thr,
-                             const u32 *__restrict__ win, const u32 *__restrict__ n_win_dev,
-                             const u32 *__restrict__ best_idx, const u32 *__restrict__ best_lab,
-                             const float *__restrict__ best_ll, const u8 *__restrict__ ovr,
-                             u8 *__restrict__ has) {
-    const u32 n_win = *n_win_dev;
-    for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < n_win; g += gridDim.x * blockDim.x) {
-        const u32 id = win[g];
+// Windows that are not listed (active) get 0.  checked: the overlap flags
+// after check_overlap_reassignments where they are kept apart (of windows with
+// ovr set; NULL: ovr holds them).
+__global__ void k_accept_has(u32 n, u32 C, u32 L, u32 W, const float *__restrict__ thr,
+                             const u8 *__restrict__ active, const u32 *__restrict__ best_idx,
+                             const u32 *__restrict__ best_lab, const float *__restrict__ best_ll,
+                             const u8 *__restrict__ ovr, const u8 *__restrict__ checked, u8 *__restrict__ has) {
+    for (u32 id = blockIdx.x * blockDim.x + threadIdx.x; id < W; id += gridDim.x * blockDim.x) {
+        if (!active[id]) { has[id] = 0; continue; }
         const u32 sw = id * L, ew = (id + 1) * L;
         u32 lab = 0, idx = 0;
         float ml = 0.0f;
         if (ew < n - L && C > 0) { ml = best_ll[id]; lab = best_lab[id]; idx = best_idx[id]; }
-        const bool o = ovr[id] == 1;
+        const bool o = ovr[id] == 1 && (!checked || checked[id] == 1);
         has[id] = ((ml > thr[lab]) || o) && ((idx >= sw && idx < ew) || o);   // .cl:982-999
     }
 }
@@ -926,10 +969,6 @@ __global__ void k_append_spikes(const u32 *__restrict__ idx, const u32 *__restri
     }
 }
 
-__global__ void k_commit_total(Counters *cnt, u32 cap) {
-    if (cnt->total + cnt->n_spk <= cap) cnt->total += cnt->n_spk;
-}
-
 // ---------------------------------------------------------------------------
 // Path (c): residual subtract, compute_residual (binary_pursuit.cl:57-102).
 // Spikes of one pass can overlap (an overlap-recheck spike may move up to
@@ -952,9 +991,12 @@ constexpr u32 kResNb = 128;
 __global__ void __launch_bounds__(256)
 k_residual(float *__restrict__ v, u32 n, u32 C, const float *__restrict__ T, u32 K, u32 L,
            const u32 *__restrict__ idx, const u32 *__restrict__ lab, const u32 *__restrict__ n_spk_dev,
-           u32 n_spk_host, u32 R, const u32 *__restrict__ tsup, float *__restrict__ vwmax = nullptr) {
+           u32 n_spk_host, u32 R, const u32 *__restrict__ tsup, float *__restrict__ vwmax = nullptr,
+           Counters *commit = nullptr, u32 cap = 0) {
     __shared__ u32 nb_p[kResNb], nb_lab[kResNb], nb_lo[kResNb], nb_hi[kResNb];
     const u32 m = n_spk_dev ? *n_spk_dev : n_spk_host;
+    // the pass's spikes, appended by an earlier launch, count from now on
+    if (commit && blockIdx.x == 0 && threadIdx.x == 0 && commit->total + m <= cap) commit->total += m;
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     for (u32 s = blockIdx.x; s < m; s += gridDim.x) {
         const u32 ls = lab[s];

@@ -830,7 +830,12 @@ __device__ __forceinline__ u32 tcw_counts(u32 m) {   // windows, runs started <<
     return __popc(own) | (__popc(own & ~prev) << 16);
 }
 __global__ void __launch_bounds__(kCompactThreads)
-k_tcw_count(const u8 *__restrict__ active, const u32 *__restrict__ dirty, u32 GW, u32 W, u32 *__restrict__ counts) {
+k_tcw_count(const u8 *__restrict__ active, const u32 *__restrict__ dirty, u32 GW, u32 W, u32 *__restrict__ counts,
+            Counters *cnt) {
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {   // the pass's refinement list
+        cnt->tc_refseg = 0;
+        cnt->tc_overflow = 0;                        // set by the tiles when the list overflows
+    }
     const u32 g = blockIdx.y, base = blockIdx.x * kCompactTile + threadIdx.x * kCompactPerThread;
     u32 tot;
     block_excl_scan(tcw_counts(tcw_selection(active, dirty, GW, g, W, base)), &tot);

@@ -179,8 +179,15 @@ __device__ __forceinline__ bool ov_disjoint(const u32 *__restrict__ tsup, u32 a,
 // candidate's window come from the tensor-core likelihood, per template group
 // (ov_window_norms); the FP32 path, which keeps none, sums the window over all
 // channels (one warp per candidate).
-__global__ void k_ov_prep(OvArgs A) {
+__global__ void k_ov_prep(OvArgs A, u32 slots, u32 *__restrict__ fb_count) {
     const u32 nc = *A.n_cand;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {       // the pass's counters
+        *A.pool_total = 0;
+        *A.refined = 0;
+        *A.scan_next = 0;
+        *fb_count = 0;
+    }
+    for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < slots; g += gridDim.x * blockDim.x) A.fallback[g] = 0;
     const bool sum = A.lazy.wn == nullptr;
     const u32 lane = sum ? threadIdx.x & 31 : 0u, per = sum ? 32u : 1u;
     for (u32 g = (blockIdx.x * blockDim.x + threadIdx.x) / per; g < nc; g += gridDim.x * blockDim.x / per) {
@@ -1321,14 +1328,6 @@ k_ov_finalize(OvArgs A) {
             overlap_parse_tail(id, bv, lab, t, afix, ashift, lf, ls, A.best_idx, A.best_lab, A.best_ll, A.ov_idx,
                                A.ov_lab, A.ovr, A.thr);
     }
-}
-
-// Window ids of the candidates that overflowed a contender list.
-__global__ void k_ov_fallback_list(OvArgs A, const u32 *__restrict__ slots, const u32 *__restrict__ n_slots,
-                                   u32 *__restrict__ out) {
-    const u32 m = *n_slots;
-    for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
-        out[i] = A.cand[slots[i]];
 }
 
 }  // namespace fbp
