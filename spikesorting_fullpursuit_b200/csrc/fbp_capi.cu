@@ -514,14 +514,17 @@ int launch_likelihood(const float *v, u32 n, u32 C, const float *T, u32 K, u32 L
                       const u32 *win, const u32 *n_win_dev, u32 max_windows, float *Lk,
                       cudaStream_t st, const u32 *gate = nullptr, u8 *apx = nullptr,
                       const u32 *tperm = nullptr, const u32 *grange = nullptr, WinBounds wb = WinBounds{}) {
-    const size_t smem = (size_t)kLikChanChunk * (kLikTile + L) * sizeof(float);
+    if (L > kLikMaxL) return fail(FBP_ERR_CUDA, "likelihood: %u samples per template, at most %u", L, kLikMaxL);
+    const int R = lik_lane_samples(L);
+    const size_t smem = lik_smem_bytes(L, (u32)R);
+    auto k = R == 2 ? k_likelihood_fp32<2> : k_likelihood_fp32<4>;
     if (smem > 48 * 1024) {
-        FBP_ALLOW_SMEM(k_likelihood_fp32);
+        FBP_ALLOW_SMEM(k_likelihood_fp32<2>);
+        FBP_ALLOW_SMEM(k_likelihood_fp32<4>);
     }
     const u64 items = (u64)max_windows * ceil_div(K, kLikTplPerBlock);
     const int grid = grid_for(items * kLikThreads, kLikThreads, 16);
-    k_likelihood_fp32<<<grid, kLikThreads, smem, st>>>(v, n, C, T, K, L, tss, win, n_win_dev, Lk, gate, apx,
-                                                       tperm, grange, wb);
+    k<<<grid, kLikThreads, smem, st>>>(v, n, C, T, K, L, tss, win, n_win_dev, Lk, gate, apx, tperm, grange, wb);
     FBP_LAUNCH_CHECK();
     return FBP_OK;
 }

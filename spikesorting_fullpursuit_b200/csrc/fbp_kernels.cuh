@@ -243,22 +243,71 @@ __global__ void k_template_support(const float *__restrict__ T, u32 K, u32 C, u3
     }
 }
 constexpr int kLikQ = 4;             // templates per warp
-constexpr int kLikR = 4;             // samples per lane
-constexpr int kLikTile = 32 * kLikR; // 128 samples
 constexpr int kLikTplPerBlock = (kLikThreads / 32) * kLikQ;   // 16
-constexpr int kLikChanChunk = 8;
+constexpr int kLikRow = kLikTplPerBlock + 4;   // floats a step's template values take: stores 4 ways into the banks, not 16
+constexpr u32 kLikMaxL = 7136;
+constexpr u32 kLikSteps = 256;       // steps of a channel staged at a time
 
+// Consecutive samples per lane: tiles of 64 samples where those of 128 would
+// cover a window with one whole half of a tile idle (L = 61: 1.9 times the
+// lanes at work), else 128, which loads half as often per product.
+inline int lik_lane_samples(u32 L) { return L % 128 >= 1 && L % 128 <= 64 ? 2 : 4; }
+
+// Channels staged at a time (as many as 20 KB hold, so that eleven blocks fit
+// an SM), and the shared memory for them.
+__host__ __device__ inline u32 lik_strip(u32 L, u32 R) { return 32 * R + (L + 3) / 4 * 4; }
+__host__ __device__ inline u32 lik_chan_floats(u32 L, u32 R) {
+    return (L < kLikSteps ? L : kLikSteps) * kLikRow + lik_strip(L, R);
+}
+__host__ __device__ inline u32 lik_chans(u32 L, u32 R) {
+    const u32 c = 5 * 1024 / lik_chan_floats(L, R);
+    return c < 1 ? 1 : c > 8 ? 8 : c;
+}
+inline size_t lik_smem_bytes(u32 L, u32 R) { return (size_t)lik_chans(L, R) * lik_chan_floats(L, R) * sizeof(float); }
+
+__device__ __forceinline__ u64 pack2(float a, float b) {
+    u64 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(u64 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+// Two products, each rounded to IEEE binary32.  The sums stay scalar: a packed
+// add after a packed multiply came back with one rounding instead of two (a
+// last bit off the oracle's), and two scalar adds cost the FP32 pipe the same.
+__device__ __forceinline__ u64 mul2_rn(u64 a, u64 b) {
+    u64 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// A block takes one listed window and 16 templates, a warp four of them, a
+// lane R consecutive samples.  The reference's order (channel by channel, step
+// by step, product and sum rounded apart) leaves the FP32 pipe as the bound: 16
+// products and 16 sums a lane and step.  So the rest is kept off the issue
+// slots: the products are packed two templates at a time, the samples slide
+// through registers (a lane loads R of them every R steps), and the templates'
+// values of a step lie together in shared memory, one 16-byte read a warp.
+// 64 templates of 16 channels x 101 samples on 400,000 samples: 4.05 ms (2.9 at
+// the pipe's rate, 27 of 128 lanes' samples past the window's end); with a
+// global read of each template value and a shared read of each sample 6.1 ms.
+template <int R>
 __global__ void __launch_bounds__(kLikThreads)
 k_likelihood_fp32(const float *__restrict__ v, u32 n, u32 C, const float *__restrict__ T, u32 K, u32 L,
                   const float *__restrict__ tss, const u32 *__restrict__ win,
                   const u32 *__restrict__ n_win_dev, float *__restrict__ Lk, const u32 *__restrict__ gate,
                   u8 *__restrict__ apx, const u32 *__restrict__ tperm, const u32 *__restrict__ grange,
                   WinBounds wb) {
-    extern __shared__ float strip[];   // kLikChanChunk x (kLikTile + L)
+    extern __shared__ __align__(16) float lik_sm[];   // template rows of every staged channel, then the strips
     if (gate && *gate == 0) return;    // only run when the gate asks for it
+    constexpr u32 kTile = 32 * R;
+    using Vec = typename std::conditional<R == 4, float4, float2>::type;
     const u32 n_win = *n_win_dev;
     const u32 kgroups = ceil_div(K, kLikTplPerBlock);
-    const u32 stride = kLikTile + L;
+    const u32 chans = lik_chans(L, R), rows = min(L, kLikSteps), stride = lik_strip(L, R);
+    float *trow = lik_sm, *strip = lik_sm + (size_t)chans * rows * kLikRow;
     const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const u64 total = (u64)n_win * kgroups;
     for (u64 item = blockIdx.x; item < total; item += gridDim.x) {
@@ -278,37 +327,71 @@ k_likelihood_fp32(const float *__restrict__ v, u32 n, u32 C, const float *__rest
         // channels where some template of the group is non-zero (the others
         // add exact zeros to the reference's sum)
         const u32 cbeg = grange ? grange[2 * kg] : 0u, cend = grange ? grange[2 * kg + 1] : C;
-        for (u32 s0 = sw; s0 < ew; s0 += kLikTile) {
-            float acc[kLikQ][kLikR];
+        for (u32 s0 = sw; s0 < ew; s0 += kTile) {
+            float acc[kLikQ][R];
 #pragma unroll
             for (int q = 0; q < kLikQ; q++)
 #pragma unroll
-                for (int r = 0; r < kLikR; r++) acc[q][r] = (slot0 + q < K) ? tss[tq[q]] : 0.0f;
-            for (u32 c0 = cbeg; c0 < cend; c0 += kLikChanChunk) {
-                const u32 cc = min((u32)kLikChanChunk, cend - c0);
-                __syncthreads();
-                for (u32 e = threadIdx.x; e < cc * stride; e += blockDim.x) {
-                    const u32 c = e / stride, x = e % stride;
-                    const u32 g = s0 + x;
-                    strip[c * stride + x] = g < n ? v[(size_t)(c0 + c) * n + g] : 0.0f;
-                }
-                __syncthreads();
-                for (u32 c = 0; c < cc; c++) {
-                    const float *sp = strip + c * stride + lane;
-                    const float *tp[kLikQ];
+                for (int r = 0; r < R; r++) acc[q][r] = (slot0 + q < K) ? tss[tq[q]] : 0.0f;
+            for (u32 c0 = cbeg; c0 < cend; c0 += chans) {
+                const u32 cc = min(chans, cend - c0);
+                for (u32 b0 = 0; b0 < L; b0 += rows) {   // more than one part: then chans is 1
+                    const u32 nb = min(rows, L - b0);
+                    __syncthreads();
+                    if (b0 == 0)
+                        for (u32 c = 0; c < cc; c++)
+                            for (u32 x = threadIdx.x; x < stride; x += kLikThreads) {
+                                const u32 g = s0 + x;
+                                strip[c * stride + x] = g < n ? v[(size_t)(c0 + c) * n + g] : 0.0f;
+                            }
+                    // each warp its own templates; lanes along the steps
+                    for (u32 c = 0; c < cc; c++)
+                        for (u32 i = lane; i < nb; i += 32) {
+                            float t[kLikQ];
 #pragma unroll
-                    for (int q = 0; q < kLikQ; q++) tp[q] = T + ((size_t)tq[q] * C + (c0 + c)) * L;
-                    for (u32 i = 0; i < L; i++) {
-                        float tv[kLikQ], vv[kLikR];
+                            for (int q = 0; q < kLikQ; q++) t[q] = __ldg(T + ((size_t)tq[q] * C + (c0 + c)) * L + b0 + i);
+                            *reinterpret_cast<float4 *>(trow + (size_t)(c * rows + i) * kLikRow + warp * kLikQ) =
+                                make_float4(t[0], t[1], t[2], t[3]);
+                        }
+                    __syncthreads();
+                    for (u32 c = 0; c < cc; c++) {
+                        const Vec *sp = reinterpret_cast<const Vec *>(strip + c * stride + b0) + lane;
+                        const float *tr = trow + (size_t)c * rows * kLikRow + warp * kLikQ;
+                        u64 d[2 * R];                    // (v, v) of samples x .. x + 2R - 1
+                        auto load = [&](int at) {
+                            const Vec x = *sp++;
+                            const float *f = reinterpret_cast<const float *>(&x);
 #pragma unroll
-                        for (int q = 0; q < kLikQ; q++) tv[q] = __ldg(tp[q] + i);
+                            for (int r = 0; r < R; r++) d[at + r] = pack2(f[r], f[r]);
+                        };
+                        auto step = [&](int k) {
+                            const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(tr);
+                            tr += kLikRow;
 #pragma unroll
-                        for (int r = 0; r < kLikR; r++) vv[r] = sp[32 * r + i];
+                            for (int r = 0; r < R; r++) {
+                                const float2 p = unpack2(mul2_rn(t.x, d[k + r])), q = unpack2(mul2_rn(t.y, d[k + r]));
+                                acc[0][r] = __fadd_rn(acc[0][r], p.x);
+                                acc[1][r] = __fadd_rn(acc[1][r], p.y);
+                                acc[2][r] = __fadd_rn(acc[2][r], q.x);
+                                acc[3][r] = __fadd_rn(acc[3][r], q.y);
+                            }
+                        };
+                        load(0);
+                        u32 i = 0;
+#pragma unroll 2
+                        for (; i + R <= nb; i += R) {
+                            load(R);
 #pragma unroll
-                        for (int q = 0; q < kLikQ; q++)
+                            for (int k = 0; k < R; k++) step(k);
 #pragma unroll
-                            for (int r = 0; r < kLikR; r++)
-                                acc[q][r] = __fadd_rn(acc[q][r], __fmul_rn(tv[q], vv[r]));
+                            for (int r = 0; r < R; r++) d[r] = d[R + r];
+                        }
+                        if (i < nb) {
+                            load(R);
+#pragma unroll
+                            for (int k = 0; k + 1 < R; k++)
+                                if (i + k < nb) step(k);
+                        }
                     }
                 }
             }
@@ -319,9 +402,9 @@ k_likelihood_fp32(const float *__restrict__ v, u32 n, u32 C, const float *__rest
                 for (int q = 0; q < kLikQ; q++) {
                     float mq = 0.0f;
 #pragma unroll
-                    for (int r = 0; r < kLikR; r++) {
-                        const u32 s = s0 + lane + 32 * r;
-                        if (s < ew && s < s0 + kLikTile && s + L < n) mq = fmaxf(mq, acc[q][r]);
+                    for (int r = 0; r < R; r++) {
+                        const u32 s = s0 + R * lane + r;
+                        if (s < ew && s + L < n) mq = fmaxf(mq, acc[q][r]);
                     }
                     mq = warp_max_float(mq);
                     anypos |= mq > 0.0f;
@@ -336,9 +419,9 @@ k_likelihood_fp32(const float *__restrict__ v, u32 n, u32 C, const float *__rest
             for (int q = 0; q < kLikQ; q++) {
                 if (slot0 + q >= K) continue;
 #pragma unroll
-                for (int r = 0; r < kLikR; r++) {
-                    const u32 s = s0 + lane + 32 * r;
-                    if (s < ew && s < s0 + kLikTile) {
+                for (int r = 0; r < R; r++) {
+                    const u32 s = s0 + R * lane + r;
+                    if (s < ew) {
                         Lk[(size_t)tq[q] * n + s] = (s + L >= n) ? 0.0f : acc[q][r];
                         if (apx) apx[(size_t)tq[q] * n + s] = 0;
                     }
