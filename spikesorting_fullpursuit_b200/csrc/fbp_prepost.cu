@@ -131,6 +131,107 @@ __device__ u32 warp_select(u32 m, u32 k, KeyOf key_of, u32 *hist) {
     return prefix;
 }
 
+// A warp's histogram of m values in 256 equal bins of [lo, hi], kept in
+// registers (lane l holds bins 8l .. 8l + 7).  A bin's index does not decrease
+// with the value, so the bins bound ranks.
+// Units of more spikes than this select by radix at once: a bin in the middle of
+// 256 over a normal sample's range holds 1 %, which has to stay below kBinGather.
+constexpr u32 kBinMax = 4096;
+constexpr u32 kBinGather = 64;         // values of one rank's bins that a warp sorts out directly
+struct WarpBins {
+    float lo, scale;
+    u32 c[8], sum, excl;
+    bool ok, all;                      // all: few values, no bins needed
+    __device__ u32 bin(float x) const { return min(255u, __float2uint_rz(__fmul_rn(__fsub_rn(x, lo), scale))); }
+};
+
+template <class ValOf>
+__device__ void bins_build(WarpBins &b, u32 m, float lo, float hi, ValOf val, u32 *hist) {
+    const u32 lane = threadIdx.x & 31;
+    const float range = __fsub_rn(hi, lo);
+    b.lo = lo;
+    b.scale = __fdiv_rn(256.0f, range);
+    b.all = m <= kBinGather;
+    b.ok = b.all || (range > 0.0f && range < 3e38f && b.scale < 3e38f);   // no NaN, no infinity
+    b.sum = b.excl = 0;
+    if (b.all || !b.ok) return;
+    for (u32 j = lane; j < 256; j += 32) hist[j] = 0;
+    __syncwarp();
+#pragma unroll 4
+    for (u32 i = lane; i < m; i += 32) atomicAdd(&hist[b.bin(val(i))], 1u);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        b.c[j] = hist[8 * lane + j];
+        b.sum += b.c[j];
+    }
+    b.excl = fbp::warp_incl_scan(b.sum) - b.sum;
+    __syncwarp();
+}
+
+// The bin that holds rank k, the values below it and in it.
+__device__ __forceinline__ void bins_find(const WarpBins &b, u32 k, u32 &bin, u32 &before, u32 &count) {
+    const u32 lane = threadIdx.x & 31;
+    const bool mine = k >= b.excl && k < b.excl + b.sum;
+    u32 acc = b.excl;
+    bin = before = count = 0;
+    if (mine) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            if (k >= acc && k < acc + b.c[j]) { bin = 8 * lane + j; before = acc; count = b.c[j]; }
+            acc += b.c[j];
+        }
+    }
+    const int src = __ffs(__ballot_sync(0xffffffffu, mine)) - 1;
+    bin = __shfl_sync(0xffffffffu, bin, src);
+    before = __shfl_sync(0xffffffffu, before, src);
+    count = __shfl_sync(0xffffffffu, count, src);
+}
+
+// The values of ranks k0 <= k1; false if their bins hold too many values.
+template <class ValOf>
+__device__ bool bins_pick(const WarpBins &b, u32 m, u32 k0, u32 k1, ValOf val, u32 *buf, float &v0, float &v1) {
+    const u32 lane = threadIdx.x & 31;
+    u32 b0 = 0, b1 = 255, before = 0, cnt = m;
+    if (!b.all) {
+        u32 c0, before1, c1;
+        bins_find(b, k0, b0, before, c0);
+        bins_find(b, k1, b1, before1, c1);
+        cnt = before1 + c1 - before;
+        if (cnt > kBinGather) return false;
+    }
+    u32 base = 0;
+#pragma unroll 4
+    for (u32 i0 = 0; i0 < m; i0 += 32) {
+        const u32 i = i0 + lane;
+        const float x = val(min(i, m - 1));
+        const u32 j = b.all ? 0u : b.bin(x);
+        const bool in = i < m && j >= b0 && j <= b1;
+        const u32 ball = __ballot_sync(0xffffffffu, in);
+        if (in) buf[base + __popc(ball & ((1u << lane) - 1u))] = fkey(x);
+        base += __popc(ball);
+    }
+    __syncwarp();
+    const bool ina = lane < cnt, inb = lane + 32 < cnt;
+    const u32 ka = ina ? buf[lane] : 0u, kb = inb ? buf[lane + 32] : 0u;
+    u32 ra = 0, rb = 0;                                  // ranks, equal keys in buffer order
+    for (u32 j = 0; j < cnt; j++) {
+        const u32 k = buf[j];
+        ra += k < ka || (k == ka && j < lane);
+        rb += k < kb || (k == kb && j < lane + 32);
+    }
+    auto key_at = [&](u32 r) {
+        const u32 at = __ballot_sync(0xffffffffu, ina && ra == r), bt = __ballot_sync(0xffffffffu, inb && rb == r);
+        const u32 x = __shfl_sync(0xffffffffu, ka, at ? __ffs(at) - 1 : 0);
+        const u32 y = __shfl_sync(0xffffffffu, kb, bt ? __ffs(bt) - 1 : 0);
+        return at ? x : y;
+    };
+    v0 = kfloat(key_at(k0 - before));
+    v1 = kfloat(key_at(k1 - before));
+    __syncwarp();
+    return true;
+}
+
 template <typename T> struct RobustArith;
 template <> struct RobustArith<float> {    // numpy float32 arithmetic
     typedef float A;
@@ -166,9 +267,15 @@ __global__ void k_transpose(const T *__restrict__ in, u32 rows, u32 cols, T *__r
 }
 
 // calculate_robust_template (preprocessing.py:639-659), one warp per
-// (unit, column): the median and the median absolute deviation by radix
-// select; the values strictly within one MAD of the median are a contiguous
-// range of ranks, whose median is selected directly.
+// (unit, column): the median, the median absolute deviation, and the median of
+// the values strictly within one MAD of the median, which are a contiguous
+// range of ranks.  What bounds it are the passes over a column's values, each
+// with its keys and shared atomics.  One histogram of 256 equal bins serves
+// the medians of the values and one that of the deviations (2 passes with
+// atomics, 7 in all, where four digits of a radix select for each rank took up
+// to 25), and equal bins put few lanes on the same counter where the first
+// digit, sign and exponent, put most.  64 units of 600 spikes, 1616 columns:
+// 1.18 ms, radix selects 2.11 ms.
 template <typename T>
 __global__ void k_robust_template(const T *__restrict__ tr, u32 n_rows, u32 dim, const u32 *__restrict__ off,
                                   u32 n_units, T *__restrict__ out) {
@@ -188,19 +295,37 @@ __global__ void k_robust_template(const T *__restrict__ tr, u32 n_rows, u32 dim,
             if (lane == 0) *dst = x[0];
             continue;
         }
-        auto xk = [&](u32 i) { return fkey((float)x[i]); };
-        auto med_of = [&](u32 a, u32 cnt, auto keyf) -> A {   // median of ranks [a, a + cnt)
-            if (cnt & 1u) return (A)kfloat(warp_select(m, a + (cnt - 1) / 2, keyf, hist));
-            const A lo = (A)kfloat(warp_select(m, a + cnt / 2 - 1, keyf, hist));
-            const A hi = (A)kfloat(warp_select(m, a + cnt / 2, keyf, hist));
-            return R::half_sum(lo, hi);
+        auto xv = [&](u32 i) { return (float)x[i]; };
+        u32 kmin = 0xffffffffu, kmax = 0;
+#pragma unroll 4
+        for (u32 i = lane; i < m; i += 32) {
+            const u32 k = fkey(xv(i));
+            kmin = min(kmin, k);
+            kmax = max(kmax, k);
+        }
+        const float vmin = kfloat(__reduce_min_sync(0xffffffffu, kmin)), vmax = kfloat(__reduce_max_sync(0xffffffffu, kmax));
+        auto med_of = [&](const WarpBins &b, u32 a, u32 cnt, auto val) -> A {   // median of ranks [a, a + cnt)
+            const u32 k0 = a + (cnt - 1) / 2, k1 = a + cnt / 2;
+            float v0, v1;
+            if (!b.ok || !bins_pick(b, m, k0, k1, val, hist, v0, v1)) {
+                auto key = [&](u32 i) { return fkey(val(i)); };
+                v0 = kfloat(warp_select(m, k0, key, hist));
+                v1 = k1 == k0 ? v0 : kfloat(warp_select(m, k1, key, hist));
+            }
+            return k1 == k0 ? (A)v0 : R::half_sum((A)v0, (A)v1);
         };
-        const A med = med_of(0, m, xk);
-        auto dk = [&](u32 i) {
-            const A d = (A)x[i] - med;
-            return fkey((float)(d < (A)0 ? -d : d));    // exact in float32 for both types
+        WarpBins bx, bd;
+        bx.ok = bd.ok = false;
+        if (m <= kBinMax) bins_build(bx, m, vmin, vmax, xv, hist);
+        const A med = med_of(bx, 0, m, xv);
+        auto dv = [&](A y) {
+            const A d = y - med;
+            return (float)(d < (A)0 ? -d : d);          // exact in float32 for both types
         };
-        const A mad = R::mad_scale(med_of(0, m, dk));
+        auto dvi = [&](u32 i) { return dv((A)x[i]); };
+        // the largest deviation is that of the smallest or the largest value
+        if (bx.ok) bins_build(bd, m, 0.0f, fmaxf(dv((A)vmin), dv((A)vmax)), dvi, hist);
+        const A mad = R::mad_scale(med_of(bd, 0, m, dvi));
         const A lo = med - mad, hi = med + mad;
         u32 nle = 0, nlt = 0;                           // #(x <= lo), #(x < hi)
         for (u32 i = lane; i < m; i += 32) {
@@ -214,7 +339,7 @@ __global__ void k_robust_template(const T *__restrict__ tr, u32 n_rows, u32 dim,
             nlt += __shfl_xor_sync(0xffffffffu, nlt, o);
         }
         A res = med;
-        if (nlt > nle) res = med_of(nle, nlt - nle, xk);
+        if (nlt > nle) res = med_of(bx, nle, nlt - nle, xv);
         if (lane == 0) *dst = R::store(res);
     }
 }
@@ -240,47 +365,72 @@ __global__ void k_resid_mean(const T *__restrict__ clips, const T *__restrict__ 
     atomicAdd(&sums[col], s);
 }
 
-constexpr int kCovThreads = 512, kCovPerThread = 24;   // L * L <= 12288: L <= 110
+constexpr u32 kCovMaxLL = 12288;         // L * L: L <= 110
+constexpr u32 kCovT = 4, kCovRows = 32;  // outputs of a thread a side, rows staged at a time
+inline u32 cov_tiles(u32 L) { const u32 t = ceil_div(L, kCovT); return t * (t + 1) / 2; }
+inline u32 cov_threads(u32 L) { return ceil_div(cov_tiles(L), 32) * 32; }
+inline size_t cov_smem_bytes(u32 L) { return ((size_t)kCovRows * ceil_div(L, kCovT) * kCovT + L) * sizeof(double); }
 
 // Per channel c, sum over the selected rows of (x_i - mean_i)(x_j - mean_j),
 // i, j < L; blocks take row ranges and add their partial matrix atomically.
+// FP64 work: a thread holds a 4 x 4 tile of outputs, four 16-byte shared reads
+// for 16 products (an output at a time took two reads for each), and only the
+// tiles on and above the diagonal, the others being the same sums.  16 channels
+// of 101 samples: 0.48 ms, before 1.60 ms.
 template <typename T>
-__global__ void k_resid_cov(const T *__restrict__ clips, const T *__restrict__ tmpl, const u32 *__restrict__ row_unit,
-                            const long long *__restrict__ rows, u32 n_sel, u32 C, u32 L, const double *__restrict__ sums,
-                            double *__restrict__ cov) {
-    extern __shared__ double csm[];                  // [32 rows][L] centred values
-    const u32 c = blockIdx.x, dim = C * L;
+__global__ void __launch_bounds__(416)
+k_resid_cov(const T *__restrict__ clips, const T *__restrict__ tmpl, const u32 *__restrict__ row_unit,
+            const long long *__restrict__ rows, u32 n_sel, u32 C, u32 L, const double *__restrict__ sums,
+            double *__restrict__ cov) {
+    extern __shared__ __align__(16) double csm[];    // [32 rows][L up to a multiple of 4] centred values, [L] means
+    const u32 c = blockIdx.x, dim = C * L, nt = ceil_div(L, kCovT), Lp = nt * kCovT;
     const u32 parts = gridDim.y, part = blockIdx.y;
     const u32 r_begin = (u32)((u64)n_sel * part / parts), r_end = (u32)((u64)n_sel * (part + 1) / parts);
-    const u32 LL = L * L;
-    double acc[kCovPerThread];
+    double *mean = csm + kCovRows * Lp;
+    for (u32 i = threadIdx.x; i < L; i += blockDim.x) mean[i] = sums[c * L + i] / n_sel;
+    // tile threadIdx.x of the upper triangle, row by row
+    u32 ti = 0, tj = threadIdx.x;
+    while (ti < nt && tj >= nt - ti) { tj -= nt - ti; ti++; }
+    const bool mine = ti < nt;
+    tj += ti;
+    double acc[kCovT][kCovT];
 #pragma unroll
-    for (int q = 0; q < kCovPerThread; q++) acc[q] = 0.0;
-    for (u32 r0 = r_begin; r0 < r_end; r0 += 32) {
-        const u32 nr = min(32u, r_end - r0);
-        for (u32 e = threadIdx.x; e < nr * L; e += blockDim.x) {
-            const u32 rr = e / L, i = e % L;
-            const u32 col = c * L + i;
-            csm[rr * L + i] = resid_of(clips, tmpl, row_unit, (u64)rows[r0 + rr], dim, col) - sums[col] / n_sel;
+    for (u32 a = 0; a < kCovT; a++)
+#pragma unroll
+        for (u32 b = 0; b < kCovT; b++) acc[a][b] = 0.0;
+    for (u32 r0 = r_begin; r0 < r_end; r0 += kCovRows) {
+        const u32 nr = min(kCovRows, r_end - r0);
+        __syncthreads();
+        for (u32 e = threadIdx.x; e < nr * Lp; e += blockDim.x) {
+            const u32 rr = e / Lp, i = e % Lp;
+            csm[e] = i < L ? resid_of(clips, tmpl, row_unit, (u64)rows[r0 + rr], dim, c * L + i) - mean[i] : 0.0;
         }
         __syncthreads();
+        if (mine) {
+            const double2 *pa = reinterpret_cast<const double2 *>(csm + ti * kCovT);
+            const double2 *pb = reinterpret_cast<const double2 *>(csm + tj * kCovT);
+#pragma unroll 2
+            for (u32 rr = 0; rr < nr; rr++, pa += Lp / 2, pb += Lp / 2) {
+                const double2 a0 = pa[0], a1 = pa[1], b0 = pb[0], b1 = pb[1];
+                const double av[kCovT] = {a0.x, a0.y, a1.x, a1.y}, bv[kCovT] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-        for (int q = 0; q < kCovPerThread; q++) {
-            const u32 o = threadIdx.x + q * blockDim.x;
-            if (o < LL) {
-                const u32 i = o / L, j = o % L;
-                double a = acc[q];
-                for (u32 rr = 0; rr < nr; rr++) a = fma(csm[rr * L + i], csm[rr * L + j], a);
-                acc[q] = a;
+                for (u32 a = 0; a < kCovT; a++)
+#pragma unroll
+                    for (u32 b = 0; b < kCovT; b++) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
             }
         }
-        __syncthreads();
     }
+    if (!mine) return;
+    double *out = cov + (u64)c * L * L;
 #pragma unroll
-    for (int q = 0; q < kCovPerThread; q++) {
-        const u32 o = threadIdx.x + q * blockDim.x;
-        if (o < LL) atomicAdd(&cov[(u64)c * LL + o], acc[q]);
-    }
+    for (u32 a = 0; a < kCovT; a++)
+#pragma unroll
+        for (u32 b = 0; b < kCovT; b++) {
+            const u32 i = ti * kCovT + a, j = tj * kCovT + b;
+            if (i >= L || j >= L) continue;
+            atomicAdd(&out[i * L + j], acc[a][b]);
+            if (ti != tj) atomicAdd(&out[j * L + i], acc[a][b]);
+        }
 }
 
 __global__ void k_scale(double *__restrict__ x, u64 n, double f) {
@@ -891,7 +1041,7 @@ int fbp_clip_noise_covariance(const void *clips, int dtype, const uint32_t *row_
     if (!clips || !row_unit || !templates || !rows || !cov || !scratch)
         return fail(FBP_ERR_BAD_ARG, "fbp_clip_noise_covariance: null pointer argument");
     if (C == 0 || L == 0 || n_sel == 0) return fail(FBP_ERR_BAD_ARG, "fbp_clip_noise_covariance: empty input");
-    if (L * L > (u32)(kCovThreads * kCovPerThread))
+    if (L * L > kCovMaxLL)
         return fail(FBP_ERR_BAD_ARG, "fbp_clip_noise_covariance: L = %u above 110", L);
     if (scratch_bytes < fbp_noise_cov_scratch_bytes(C, L))
         return fail(FBP_ERR_BAD_ARG, "fbp_clip_noise_covariance: scratch too small");
@@ -902,16 +1052,16 @@ int fbp_clip_noise_covariance(const void *clips, int dtype, const uint32_t *row_
     PP_CUDA(cudaMemsetAsync(cov, 0, (size_t)C * L * L * 8, st));
     const dim3 mb(32, 8), mg(ceil_div(dim, 32), std::min<u32>(64, ceil_div(n_sel, 8)));
     const u32 parts = std::max<u32>(1, std::min<u32>(ceil_div(n_sel, 256), ceil_div(148 * 4, C)));
-    const size_t smem = (size_t)32 * L * sizeof(double);
+    const size_t smem = cov_smem_bytes(L);
     if (dtype == FBP_F32) {
         k_resid_mean<float><<<mg, mb, 0, st>>>((const float *)clips, (const float *)templates, row_unit,
                                                (const long long *)rows, n_sel, dim, sums);
-        k_resid_cov<float><<<dim3(C, parts), kCovThreads, smem, st>>>((const float *)clips, (const float *)templates, row_unit,
+        k_resid_cov<float><<<dim3(C, parts), cov_threads(L), smem, st>>>((const float *)clips, (const float *)templates, row_unit,
                                                               (const long long *)rows, n_sel, C, L, sums, cov);
     } else if (dtype == FBP_I16) {
         k_resid_mean<short><<<mg, mb, 0, st>>>((const short *)clips, (const short *)templates, row_unit,
                                                (const long long *)rows, n_sel, dim, sums);
-        k_resid_cov<short><<<dim3(C, parts), kCovThreads, smem, st>>>((const short *)clips, (const short *)templates, row_unit,
+        k_resid_cov<short><<<dim3(C, parts), cov_threads(L), smem, st>>>((const short *)clips, (const short *)templates, row_unit,
                                                               (const long long *)rows, n_sel, C, L, sums, cov);
     } else {
         return fail(FBP_ERR_BAD_ARG, "fbp_clip_noise_covariance: dtype must be FBP_F32 or FBP_I16");
