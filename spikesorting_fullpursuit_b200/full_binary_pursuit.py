@@ -33,7 +33,7 @@ def pursuit_templates_and_covariance(voltage, unit_spike_indices, sampling_rate,
     lib = _lib.lib()
     # clips of every unit, rows unit by unit (get_clips' edge rule per unit)
     from .parallel.segment_parallel import _valid_range
-    starts, counts, evs = [], [], []
+    counts, evs = [], []
     for ev in unit_spike_indices:
         ev = np.asarray(ev, dtype=np.int64)
         if ev.size == 0:
@@ -41,23 +41,17 @@ def pursuit_templates_and_covariance(voltage, unit_spike_indices, sampling_rate,
         _, a, b = _valid_range(ev, window, n, True)
         if a is None:
             raise ValueError("no clip of a unit lies inside the voltage")
-        starts.append(a)
         counts.append(b - a + 1)
-        evs.append(ev)
+        evs.append(ev[a:b + 1])
     off = np.zeros(len(evs) + 1, np.uint32)
     off[1:] = np.cumsum(counts)
     rows = int(off[-1])
     clips = D.empty((rows, C * L), dt)
     nb = D.to_dev(np.arange(C, dtype=np.int64))
     stream = D.stream()
-    keep = []
-    for u, ev in enumerate(evs):
-        ev_d = D.to_dev(ev)
-        keep.append(ev_d)
-        view = clips[int(off[u]):int(off[u + 1])]
-        _lib.check(lib.fbp_get_clips(_lib.ptr(v), D.code_of(dt), n, C, _lib.ptr(nb), C, _lib.ptr(ev_d),
-                                     int(starts[u]), int(counts[u]), int(window[0]), int(window[1]), _lib.ptr(view),
-                                     stream))
+    ev_d = D.to_dev(np.concatenate(evs) if evs else np.zeros(0, np.int64))
+    _lib.check(lib.fbp_get_clips(_lib.ptr(v), D.code_of(dt), n, C, _lib.ptr(nb), C, _lib.ptr(ev_d), 0, rows,
+                                 int(window[0]), int(window[1]), _lib.ptr(clips), stream))
     from .preprocessing import calculate_robust_templates
     templates = calculate_robust_templates(clips, off, as_tensor=True)
     if n_cov_samples >= rows:
