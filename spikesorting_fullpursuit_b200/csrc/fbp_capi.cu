@@ -716,10 +716,15 @@ int ov_fast_tables(const Workspace &w, const OvArgs &A, Counters *cnt, cudaStrea
                         kTabMThreads, smem, st>>>(A, w.tperm, w.tsup, w.grange32);
         FBP_LAUNCH_CHECK();
     } else {
-        const size_t smem = tables_smem_bytes(S, A.K, A.L);
+        // rows 4 floats apart, so that the staging's stores spread over the
+        // banks, unless that is more than a block can have
+        const size_t plain = tables_smem_bytes(S, A.K, A.L), rows = (size_t)((A.L + 7) & ~7u);
+        const u32 pad = plain + rows * 16 <= 227 * 1024 ? 4u : 0u;
+        const size_t smem = plain + rows * pad * 4;
         if (smem > 48 * 1024)
             FBP_ALLOW_SMEM(k_ov_tables);
-        k_ov_tables<<<grid_for((u64)slots * kTabThreads, kTabThreads, 4), kTabThreads, smem, st>>>(A);
+        const int threads = ceil_div(S, 8) * ceil_div(A.K, 8) <= 128 ? 128 : kTabThreads;
+        k_ov_tables<<<grid_for((u64)slots * threads, threads, 8), threads, smem, st>>>(A, pad);
         FBP_LAUNCH_CHECK();
     }
     *launches = 2;
