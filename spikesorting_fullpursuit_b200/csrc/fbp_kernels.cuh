@@ -442,12 +442,15 @@ k_likelihood_fp32(const float *__restrict__ v, u32 n, u32 C, const float *__rest
 //   0     the stored value is the reference value, or an approximation that
 //         is certainly <= 0 (only its sign is ever read);
 //   1     approximate and certainly > 0; the interval is approx +- lazy_bound;
-//   2, 3  was 1; the reference value was stored by a kernel of the pass with
+//   2, 3  was 1; the reference value was stored by the argmax of a pass with
 //         that parity (tag = 2 + pass % 2).
-// A kernel stores the value before the tag, so a reader in the SAME kernel
+// The argmax stores the value before the tag, so a reader in the SAME kernel
 // that sees its own pass's tag may still read the old approximation: it
 // treats the entry like a 1 (the interval holds both values).  A tag of the
-// other parity was written by an earlier launch and is exact.
+// other parity was written by an earlier launch and is exact.  So is one of
+// the same parity from two or more passes ago; the reader forms that entry
+// again, from the same voltage: an entry whose voltage changes in a window
+// that is not listed next loses its tag first (k_lazy_freeze).
 struct LazyLk {
     u8 *apx;                          // [K][n]; NULL: every entry is exact
     const float *wn, *wa;             // [n] window L2 / L1 norms at computation time (wa NULL: at most wa_f wn)
@@ -556,7 +559,9 @@ __device__ __forceinline__ float warp_lk_exact(const LazyLk &z, const float *Lk,
 // Before the residual subtracts this pass's spikes: an approximate entry
 // that reads a changing sample and whose window is not recomputed next pass
 // keeps, in the reference, the value it was computed with; store that value
-// now, from the voltage it was computed from.
+// now, from the voltage it was computed from.  An entry that an argmax settled
+// before is marked final (0): its tag would have a later argmax form it again,
+// from the changed voltage.
 __global__ void __launch_bounds__(256)
 k_lazy_freeze(u32 n, u32 L, u32 K, const u32 *__restrict__ idx, const u32 *__restrict__ lab,
               const u32 *__restrict__ m_dev, const u8 *__restrict__ next_active, u32 W, float *__restrict__ Lk,
@@ -583,15 +588,17 @@ k_lazy_freeze(u32 n, u32 L, u32 K, const u32 *__restrict__ idx, const u32 *__res
                 // templates without a channel of the spike's read no changing sample
                 if (z.tsup && (z.tsup[2 * t] >= sup_hi || z.tsup[2 * t + 1] <= sup_lo)) continue;
                 const size_t e = (size_t)t * n + s;
-                u32 nm = __ballot_sync(0xffffffffu, cand && z.apx[e] == 1);
+                const u32 f = cand ? z.apx[e] : 0u;
+                if (f > 1) z.apx[e] = 0;             // settled by an argmax: final from here on
+                u32 nm = __ballot_sync(0xffffffffu, f == 1);
                 while (nm) {
                     const u32 src = __ffs(nm) - 1;
                     nm &= nm - 1;
                     const float x = warp_exact_likelihood(z, n, t, __shfl_sync(0xffffffffu, s, src), wbuf);
                     if (lane == src) {
-                        Lk[e] = x;
+                        Lk[e] = x;                   // another spike's warp may store the same value
                         __threadfence();
-                        z.apx[e] = (u8)z.tag;
+                        z.apx[e] = 0;
                         nref++;
                     }
                 }
