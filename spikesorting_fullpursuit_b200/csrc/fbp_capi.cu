@@ -1388,7 +1388,9 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
                   (uint64_t)do_overlap_recheck, (uint64_t)precision, (uint64_t)overlap_method,
                   (uint64_t)(uintptr_t)workspace, (uint64_t)workspace_bytes, (uint64_t)(uintptr_t)spike_idx,
                   (uint64_t)(uintptr_t)spike_lab, spike_cap, (uint64_t)w.masked_tables, (uint64_t)w.tc,
-                  lim_refine, lim_pool, lim_wait, (uint64_t)w.tcw, w.tcw_ns};
+                  lim_refine, lim_pool, lim_wait, (uint64_t)w.tcw, w.tcw_ns,
+                  // the rounding bounds (kappa, gamma, the L1 factor) are arguments of the captured kernels
+                  w.tc_nz, w.tc_cmax};
         for (const TcGroup &g : w.tcg)               // the group plan follows the template supports
             if (w.tc) pg.key.insert(pg.key.end(), {g.t0, g.nt, g.clo, g.Cg, g.nbuf});
         std::lock_guard<std::mutex> lk(g_graph_mu);
