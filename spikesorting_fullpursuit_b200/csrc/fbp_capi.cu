@@ -273,7 +273,7 @@ u32 plan_tcw_groups(const std::vector<u32> &tsup, const std::vector<u32> &tperm,
     if (L < kWMinL || L > 1024) return 0;
     u32 ns = 0;
     for (u32 s = kWProdWarps; s >= 2; s--)
-        if (tcw_smem_layout(L, s).total <= 227 * 1024) { ns = s; break; }
+        if (tcw_px(L) <= kWParts * kWPart && tcw_smem_layout(L, s).total <= 227 * 1024) { ns = s; break; }
     if (ns == 0) return 0;
     size_t off = 0;
     for (u32 t0 = 0; t0 < K; t0 += 16) {

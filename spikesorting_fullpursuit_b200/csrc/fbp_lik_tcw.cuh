@@ -117,6 +117,8 @@ __host__ __device__ inline u32 tcw_entries(u32 L) {
 }
 constexpr u32 kWMaps = 3;                // position maps in flight: built, read by producers, by the epilogue
 constexpr u32 kWLoads = 24;              // voltage loads of a producer lane in flight
+constexpr u32 kWPart = 32 * kWLoads;     // positions a producer warp takes at a time
+constexpr u32 kWParts = 4;               // parts of the staged positions at most (px <= 3072: L <= 1016)
 
 struct TcwInfo {                         // per map: the tile
     u32 g, Cg;
@@ -126,8 +128,9 @@ struct TcwInfo {                         // per map: the tile
     float ck[16], cb[16], css[16], ca[16], tsc[16], tsa[16];
     int texp[16];
 };
+static_assert(sizeof(TcwInfo) % 16 == 0, "what follows it in a map is stored in 8 and 16 bytes");
 struct TcwSmem {
-    size_t ring, stage, a_bytes, map, map_bytes, smap, wrel, tw, es, info, tpos, twin, nrm, um, wl, bars, misc, tcnt, total;
+    size_t ring, stage, a_bytes, map, map_bytes, smap, wrel, tw, info, tpos, twin, ep, es, nrm, um, wl, bars, misc, tcnt, total;
 };
 __host__ __device__ inline TcwSmem tcw_smem_layout(u32 L, u32 ns) {
     const size_t nkc = tcw_nkc(L), px = tcw_px(L), rows = px / 8;
@@ -136,21 +139,22 @@ __host__ __device__ inline TcwSmem tcw_smem_layout(u32 L, u32 ns) {
     m.stage = align_up(m.a_bytes + align_up(px * 2, 16), 128);
     size_t o = 0;
     m.smap = o;  o += px * 4;                             // sample of every staged position, ~0 past the recording
-    m.es = o;    o += rows * 4;                           // energies of the blocks of 8
     m.info = o;  o += sizeof(TcwInfo);
-    m.tw = o;    o += (size_t)kWTwMax * 4;                // window of each table entry
-    m.wrel = o;  o += kWPos;                              // table entry of a kept output, else 0xff
+    m.wrel = o;  o += kWPos;                              // table entry of a kept output, else 0xff (8-byte stores)
+    m.tw = o;    o += (size_t)tcw_entries(L) * 4;         // window of each table entry
     m.map_bytes = align_up(o, 16);
     o = 0;
     m.ring = o;  o += ns * m.stage;                       // A tiles + voltage stream per channel
     m.map = o;   o += kWMaps * m.map_bytes;
-    m.tpos = o;  o += (size_t)(kWTwMax + 1) * 4;          // table warps: stream position and window of each entry
-    m.twin = o;  o += (size_t)(kWTwMax + 1) * 4;
+    m.tpos = o;  o += (size_t)(tcw_entries(L) + 1) * 4;   // table warps: stream position and window of each entry
+    m.twin = o;  o += (size_t)(tcw_entries(L) + 1) * 4;
+    m.ep = o;    o += (size_t)ns * rows * 4;              // energies of the blocks of 8 (scaled samples), per producer
+    m.es = o;    o += 2 * rows * 4;                       // and of all channels, by the tile's parity
     m.nrm = o;   o += 2 * (size_t)kWN * 4;                // epilogue: window norms per block of 8, two spans
     m.um = o;    o += (size_t)16 * tcw_entries(L) * 4;    //           upper bounds per (template, window)
     m.wl = o;    o += (size_t)tcw_entries(L) * 4;         //           lower bounds per window
     o = align_up(o, 8);
-    m.bars = o;  o += (size_t)(2 * ns + 5 + 3 * kWMaps) * 8;
+    m.bars = o;  o += (size_t)(2 * ns + 7 + 3 * kWMaps) * 8;
     m.misc = o;  o += 256;
     m.tcnt = o;  o += 16 * 4;
     m.total = o;
@@ -169,13 +173,23 @@ __device__ __forceinline__ u32 named_bar_popc(u32 id, u32 count, bool v) {
         : "=r"(r) : "r"((u32)v), "r"(id), "r"(count) : "memory");
     return r;
 }
-__device__ __forceinline__ double warp_incl_scan_d(double v, u32 lane) {
+// Sums of squares over each group of 8 lanes, of 8 values per lane: lane l gets
+// the one of z[l & 7] over its group (each step a lane keeps half of its values
+// and takes its partner's for them: 4 + 2 + 1 shuffles).
+__device__ __forceinline__ float octet_energy(const float *z, u32 lane) {
+    float v[8];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double y = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= (u32)o) v += y;
+    for (int i = 0; i < 8; i++) v[i] = __fmul_rn(z[i], z[i]);
+#pragma unroll
+    for (int h = 4; h >= 1; h >>= 1) {
+        const bool hi = (lane & (u32)h) != 0;
+#pragma unroll
+        for (int i = 0; i < h; i++) {
+            const float send = hi ? v[i] : v[i + h], keep = hi ? v[i + h] : v[i];
+            v[i] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, h));
+        }
     }
-    return v;
+    return v[0];
 }
 __device__ __forceinline__ u16 half_bits_clamped(float f) {
     return __half_as_ushort(__float2half_rn(fminf(fmaxf(f, -65504.0f), 65504.0f)));
@@ -184,14 +198,19 @@ __device__ __forceinline__ u16 half_bits_clamped(float f) {
 // Persistent, one CTA per SM, 20 warps.  The tiles of all groups' streams form
 // one sequence; CTA b takes tiles b, b + gridDim, ...
 //   Table warps, per tile, one tile ahead: the windows that meet it, the sample
-//     of every position, the tile's fp16 scale and per-template factors; then,
-//     as each channel of the tile is staged, the energy of every block of 8
-//     positions from the fp16 values themselves (their rounding is bounded and
-//     added).
+//     of every position, the tile's fp16 scale and per-template factors; at the
+//     end of a tile the energies of its blocks of 8 positions, from the
+//     producers' parts.
 //   Producer warp s fills ring stage s: a channel's voltage by coalesced 4-byte
 //     loads (24 in flight per lane, the first ones issued before the wait for
 //     the stage), scaled, rounded to fp16; one bulk copy brings the channel's A
-//     tiles.  No barrier joins the producers.
+//     tiles.  It also sums the energies of its float32 samples over blocks of 8
+//     positions (seven shuffles reduce eight loads of 32 lanes to a block a
+//     lane).  No barrier joins the producers.  (Energies of the fp16 samples,
+//     read from the stages by the table warps, took 17.9 in place of 20.1 ms on
+//     the 384-channel probe's 100 s, and as much on 16 channels; table warps
+//     that load the float32 samples again took 30, since the loads are what
+//     bounds a tile, and a producer that adds its sums to the one before it 20.8.)
 //   The MMA warp issues nkc MMAs per channel.
 //   Epilogue warps (two per TMEM lane quadrant, one half of the columns each)
 //     bound every output's window norm by the blocks that hold its lags,
@@ -204,8 +223,7 @@ __device__ __forceinline__ u16 half_bits_clamped(float f) {
 // tile of 34 channels, against 31,000 of MMA issue.
 // Barriers:
 //   stage_full[s]  the producer arrived and the A copy landed (tx);
-//   stage_empty[s] the MMAs that read stage s are done (tcgen05.commit) and the
-//                  table warps have read it (one arrive each);
+//   stage_empty[s] the MMAs that read stage s are done (tcgen05.commit);
 //   acc_full[b]    the tile's MMAs are done (commit);
 //   acc_empty[b]   the epilogue read accumulator b (one arrive per warp);
 //   map_full[k], norm_full[k]  map k is built, its norms are (one arrive each);
@@ -238,6 +256,8 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
     auto bar_nfull = [&](u32 k) { return smem_u32(&bars[2 * ns + 4 + kWMaps + k]); };
     auto bar_mempty = [&](u32 k) { return smem_u32(&bars[2 * ns + 4 + 2 * kWMaps + k]); };
     const u32 bar_fin = smem_u32(&bars[2 * ns + 4 + 3 * kWMaps]);
+    const u32 bar_efull = smem_u32(&bars[2 * ns + 5 + 3 * kWMaps]), bar_eempty = smem_u32(&bars[2 * ns + 6 + 3 * kWMaps]);
+    const u32 rows = px / 8;                         // blocks of 8 staged positions
     auto aborted = [&]() { return *(volatile u32 *)abort_flag != 0; };
     // a wait of one warp: false when it gave up or another role has
     auto wait_warp = [&](u32 bar, u32 parity, u32 code) -> bool {
@@ -253,7 +273,7 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
     if (tid == 0) {
         for (u32 s = 0; s < ns; s++) {
             mbar_init(bar_sfull(s), 1);
-            mbar_init(bar_sempty(s), 1 + kWTabWarps);
+            mbar_init(bar_sempty(s), 1);
             fills[s] = 0;
         }
         for (u32 b = 0; b < 2; b++) {
@@ -266,6 +286,8 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
             mbar_init(bar_mempty(k), ns + kWEpiWarps);
         }
         mbar_init(bar_fin, 1);
+        mbar_init(bar_efull, ns);
+        mbar_init(bar_eempty, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -280,20 +302,25 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
     const u32 tmem = *tmem_slot;
 
     if (warp < kWTabWarps) {
-        // ======================= tables and norms ========================
+        // ============================ tables =============================
         const u32 tt = tid;                          // 0..127
-        const u32 rows = px / 8;                     // blocks of 8 positions
+        const u32 TW = tcw_entries(L);
         int *tpos = (int *)(wsm + lay.tpos);
         u32 *twin = (u32 *)(wsm + lay.twin);
+        // waits until the tile that had the map of the CTA's it-th tile is done
+        auto map_free = [&](u32 it) -> bool {
+            const u32 k = it % kWMaps, use = it / kWMaps;
+            const bool ok = use == 0 || wait_warp(bar_mempty(k), (use - 1) & 1u, 13u);
+            return !named_bar_or(3, kWTabThreads, !ok);
+        };
         // builds the map of the CTA's it-th tile; false when a role gave up
         auto build = [&](u32 f, u32 it) -> bool {
-            const u32 k = it % kWMaps, use = it / kWMaps;
+            const u32 k = it % kWMaps;
             unsigned char *mp = map_of(k);
             u32 *smap = (u32 *)(mp + lay.smap), *tw = (u32 *)(mp + lay.tw);
             u8 *wrel = mp + lay.wrel;
             TcwInfo &I = *(TcwInfo *)(mp + lay.info);
-            const bool free_map = use == 0 || wait_warp(bar_mempty(k), (use - 1) & 1u, 13u);
-            if (named_bar_or(3, kWTabThreads, !free_map)) return false;
+            if (!map_free(it)) return false;
             // the tile's group and its place in the group's stream.  Group after
             // group: tiles computed together write the rows of 16 templates and
             // read one group's channels (taking every group's tile 0, then tile
@@ -319,10 +346,10 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
             const u32 *gpos = P.pos + (size_t)g * P.wstride, *gwin = P.win + (size_t)g * P.wstride;
             u32 nw = 0;
             float mx = 0.0f;
-            for (u32 b0 = 0; b0 < kWTwMax + 1; b0 += kWTabThreads) {
+            for (u32 b0 = 0; b0 < TW + 1; b0 += kWTabThreads) {
                 const u32 e = b0 + tt, i = i_lo + e;
-                bool in = e <= kWTwMax && i < m && (long long)gpos[i] < Q0 + (long long)px;
-                if (in && e == kWTwMax) {            // cannot happen for L >= kWMinL
+                bool in = e <= TW && i < m && (long long)gpos[i] < Q0 + (long long)px;
+                if (in && e == TW) {                 // cannot happen: windows start at least L positions apart
                     atomicExch(P.err, 15u);
                     atomicExch(abort_flag, 1u);
                     in = false;
@@ -397,46 +424,25 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
             if (tt == 0) mbar_arrive(bar_mfull(k));  // release: the barrier ordered every write
             return true;
         };
-        u32 gs0 = 0, it = 0;                         // ring uses before this tile
+        u32 it = 0;
         bool ok = build(blockIdx.x, 0);
         for (u32 f = blockIdx.x; ok && f < total; f += gridDim.x, it++) {
-            if (f + gridDim.x < total && !build(f + gridDim.x, it + 1)) break;
-            const u32 k = it % kWMaps;
-            unsigned char *mp = map_of(k);
-            const TcwInfo &I = *(const TcwInfo *)(mp + lay.info);
-            const u32 Cg = I.Cg;
-            float e2[3][2];
-#pragma unroll
-            for (int r = 0; r < 3; r++) e2[r][0] = e2[r][1] = 0.0f;
-            for (u32 c = 0; c < Cg; c++) {
-                const u32 gs = gs0 + c, s = gs % ns, u = gs / ns;
-                if (!wait_warp(bar_sfull(s), u & 1u, 17u)) break;    // the barrier below sees the abort flag
-                const unsigned char *B = ring + (size_t)s * lay.stage + lay.a_bytes;
-#pragma unroll
-                for (int r = 0; r < 3; r++) {
-                    const u32 row = tt + 128u * r;
-                    if (row >= rows) continue;
-                    const uint4 h = *reinterpret_cast<const uint4 *>(B + 16 * (size_t)row);
-                    const u32 hw[4] = {h.x, h.y, h.z, h.w};
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const float2 x = __half22float2(*reinterpret_cast<const __half2 *>(&hw[e]));
-                        e2[r][0] = fmaf(x.x, x.x, e2[r][0]);
-                        e2[r][1] = fmaf(x.y, x.y, e2[r][1]);
-                    }
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_sempty(s));
-            }
-            gs0 += Cg;
-            float *es = (float *)(mp + lay.es);
-#pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const u32 row = tt + 128u * r;
-                if (row < rows) es[row] = e2[r][0] + e2[r][1];
+            // once the tile three before the next is done, the one two before this has
+            // had its energies read: their place is free
+            if (f + gridDim.x < total ? !build(f + gridDim.x, it + 1) : !map_free(it + 1)) break;
+            const bool full = wait_warp(bar_efull, it & 1u, 17u);
+            const float *ep = (const float *)(wsm + lay.ep);
+            float *es = (float *)(wsm + lay.es) + (it & 1u) * rows;
+            for (u32 row = tt; full && row < rows; row += kWTabThreads) {
+                float e = ep[row];
+                for (u32 q = 1; q < ns; q++) e = __fadd_rn(e, ep[(size_t)q * rows + row]);
+                es[row] = e;
             }
             if (named_bar_or(3, kWTabThreads, aborted())) break;
-            if (tt == 0) mbar_arrive(bar_nfull(k));
+            if (tt == 0) {
+                mbar_arrive(bar_eempty);
+                mbar_arrive(bar_nfull(it % kWMaps));
+            }
         }
     } else if (warp < kWMmaWarp) {
         // =========================== producers ===========================
@@ -456,10 +462,18 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
             const float *v = T.v;
             const unsigned char *Aw = T.Aw;
             const u32 Cg = I.Cg;
+            // energies of this warp's channels: the lane's block of part p, eight loads j
+            float e2[kWParts][kWLoads / 8];
+#pragma unroll
+            for (u32 j = 0; j < kWLoads / 8; j++)
+#pragma unroll
+                for (u32 q = 0; q < kWParts; q++) e2[q][j] = 0.0f;
             for (u32 c = (s + ns - gs0 % ns) % ns; c < Cg; c += ns) {
                 const u32 u = (gs0 + c) / ns;
                 const float *vc = v + (size_t)c * n;
-                for (u32 x0 = lane; x0 < px; x0 += 32 * kWLoads) {
+#pragma unroll 1
+                for (u32 p = 0; p * kWPart < px; p++) {
+                    const u32 x0 = p * kWPart + lane;
                     float fv[kWLoads];
 #pragma unroll
                     for (u32 i = 0; i < kWLoads; i++) {
@@ -469,7 +483,7 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
                         // output that is not in the zeroed tail multiplies
                         fv[i] = __ldg(vc + min(smap[min(x, px - 1)], n - 1));
                     }
-                    if (x0 == lane) {                // the first loads are in flight
+                    if (p == 0) {                    // the first loads are in flight
                         if (u > 0 && !wait_warp(bar_sempty(s), (u - 1) & 1u, 11u)) { stop = true; break; }
                         if (lane == 0) {
                             fills[s] = u + 1;
@@ -481,15 +495,39 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
                         }
                     }
 #pragma unroll
-                    for (u32 i = 0; i < kWLoads; i++) {
-                        const u32 x = x0 + 32 * i;
-                        if (x < px) B[x] = half_bits_clamped(__fmul_rn(fv[i], kscale));
+                    for (u32 j = 0; j < kWLoads / 8; j++) {
+                        if (p * kWPart + 256 * j >= px) break;       // uniform
+                        float z[8];
+#pragma unroll
+                        for (u32 r = 0; r < 8; r++) {
+                            const u32 x = x0 + 256 * j + 32 * r;
+                            z[r] = fminf(fmaxf(__fmul_rn(fv[8 * j + r], kscale), -65504.0f), 65504.0f);
+                            if (x < px) B[x] = __half_as_ushort(__float2half_rn(z[r]));
+                        }
+                        const float e = octet_energy(z, lane);
+#pragma unroll
+                        for (u32 q = 0; q < kWParts; q++)            // registers: no index that varies
+                            e2[q][j] = __fadd_rn(e2[q][j], q == p ? e : 0.0f);
                     }
                 }
                 if (stop) break;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_sfull(s));
+            }
+            // to the table warps, which have long added the tile before
+            if (!stop && it > 0) stop = !wait_warp(bar_eempty, (it - 1) & 1u, 25u);
+            if (!stop) {
+                float *ep = (float *)(wsm + lay.ep) + (size_t)s * rows;
+#pragma unroll
+                for (u32 q = 0; q < kWParts; q++)
+#pragma unroll
+                    for (u32 j = 0; j < kWLoads / 8; j++) {
+                        const u32 row = q * (kWPart / 8) + 32 * j + 4 * (lane & 7) + (lane >> 3);
+                        if (row < rows) ep[row] = e2[q][j];
+                    }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_efull);
             }
             if (stop) break;
             gs0 += Cg;
@@ -580,18 +618,19 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
             {
                 // norms of the blocks that hold an output's lags: output 8 u + d
                 // reads blocks u .. u + (L - 1) / 8, one more when d + (L - 1) % 8
-                // reaches 8.  The fp16 values round the scaled samples by 2^-11
-                // (2^-25 below the normal range, added as such); the sums' own
-                // rounding (Cg * 4 terms and (L + 14) / 8 blocks in float) is
-                // inside the factor.
-                const float *es = (const float *)(mp + lay.es);
-                const float add = ldexpf(2.98023223876953125e-08f * 1.001f * sqrtf((float)I.Cg * (float)(L + 14)), -I.kexp) +
-                                  1e-30f;
-                float e = 0.0f;
+                // reaches 8.  A block's energy took a product, three adds over
+                // the lanes and one for every channel and warp, each rounded to
+                // float32 (what the products lose below the normal range, 2^-150
+                // each, the added 2^-60 of the scaled samples covers); the blocks
+                // are added in float64.
+                const float *es = (const float *)(wsm + lay.es) + (it & 1u) * rows;
+                const float up = 1.0f + 6.6e-8f * (float)(I.Cg + 32);
+                const float add = ldexpf(8.7e-19f, -I.kexp) + 1e-30f;
+                double e = 0.0;
                 const u32 nb = (L - 1) / 8 + 1;
-                for (u32 q = 0; q < nb; q++) e += es[et + q];
-                nrm_all[et] = ldexpf(sqrtf(e) * 1.001f, -I.kexp) + add;
-                nrm_all[kWN + et] = ldexpf(sqrtf(e + es[et + nb]) * 1.001f, -I.kexp) + add;
+                for (u32 q = 0; q < nb; q++) e += (double)es[et + q];
+                nrm_all[et] = ldexpf(sqrtf((float)e) * up, -I.kexp) + add;
+                nrm_all[kWN + et] = ldexpf(sqrtf((float)(e + (double)es[et + nb])) * up, -I.kexp) + add;
             }
             named_bar(2, kWEpiThreads);
             const float *nrm = nrm_all + span;
