@@ -571,16 +571,17 @@ int launch_check_overlap(u32 n, u32 L, const u32 *cand, const u32 *n_cand_dev, u
     return FBP_OK;
 }
 
+// win: the listed windows (at most max_windows of them); NULL: those marked active.
 int launch_accept(u32 n, u32 C, u32 L, const float *thr, const u32 *win, const u32 *n_win_dev,
                   u32 max_windows, const fbp_window_state &s, const u8 *active, u8 *has, u8 *flags_out,
                   u32 *acc_list, u32 *spk_idx, u32 *spk_lab, u32 *spk_win, u32 *n_spk_dev,
                   u32 *tile_counts, cudaStream_t st, const WinBounds &wb = WinBounds{}, const u32 *grange = nullptr,
                   const u32 *tsup = nullptr, u32 K = 0, const u8 *checked = nullptr) {
-    (void)win; (void)n_win_dev; (void)max_windows;
     const u32 W = ceil_div(n, L);
     const int threads = 256;
-    k_accept_has<<<grid_for(W, threads), threads, 0, st>>>(n, C, L, W, thr, active, s.best_idx, s.best_lab, s.best_ll,
-                                                           s.overlap_recheck, checked, has);
+    if (win) FBP_CUDA(cudaMemsetAsync(has, 0, window_bytes_u8(W), st));
+    k_accept_has<<<grid_for(win ? max_windows : W, threads), threads, 0, st>>>(
+        n, C, L, W, thr, win, n_win_dev, active, s.best_idx, s.best_lab, s.best_ll, s.overlap_recheck, checked, has);
     AcceptView a{n, C, L, W, n / L, thr, s.best_idx, s.best_lab, s.best_ll, active, has, s.flags};
     k_accept_flags<<<grid_for(W, threads), threads, 0, st>>>(a, flags_out);
     FBP_LAUNCH_CHECK();
@@ -1339,7 +1340,7 @@ int fbp_pursuit_chunk(float *voltage, uint32_t n, uint32_t C, const float *templ
         }
         // 5. accept (.py:663-671)
         timer.begin(FBP_STAGE_ACCEPT);
-        if ((rc2 = launch_accept(n, C, L, thresholds, w.win, &w.cnt->n_win, W, s, w.active, w.has,
+        if ((rc2 = launch_accept(n, C, L, thresholds, nullptr, nullptr, W, s, w.active, w.has,
                                  w.flags_out, w.acc_list, w.spk_idx, w.spk_lab, w.spk_win, &w.cnt->n_spk,
                                  w.tile_counts, q, win_bounds(w), w.grange, w.tsup, K,
                                  do_overlap_recheck ? w.ovr2 : nullptr)))

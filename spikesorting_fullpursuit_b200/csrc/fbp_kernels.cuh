@@ -939,15 +939,20 @@ __global__ void k_copy_ovr(const u32 *__restrict__ cand, const u32 *__restrict__
 // k_accept_flags: the flags after the kernel, for every window, reproducing
 // the sequential reads of the neighbours' flags in phase two.
 // ---------------------------------------------------------------------------
-// Windows that are not listed (active) get 0.  checked: the overlap flags
-// after check_overlap_reassignments where they are kept apart (of windows with
-// ovr set; NULL: ovr holds them).
+// win: the listed windows, the others' bytes of `has` being 0 already; NULL:
+// the windows marked active, the others get 0 (the pursuit's own passes, where
+// both say the same: no memset).  checked: the overlap flags after
+// check_overlap_reassignments where they are kept apart (of windows with ovr
+// set; NULL: ovr holds them).
 __global__ void k_accept_has(u32 n, u32 C, u32 L, u32 W, const float *__restrict__ thr,
+                             const u32 *__restrict__ win, const u32 *__restrict__ n_win_dev,
                              const u8 *__restrict__ active, const u32 *__restrict__ best_idx,
                              const u32 *__restrict__ best_lab, const float *__restrict__ best_ll,
                              const u8 *__restrict__ ovr, const u8 *__restrict__ checked, u8 *__restrict__ has) {
-    for (u32 id = blockIdx.x * blockDim.x + threadIdx.x; id < W; id += gridDim.x * blockDim.x) {
-        if (!active[id]) { has[id] = 0; continue; }
+    const u32 m = win ? *n_win_dev : W;
+    for (u32 g = blockIdx.x * blockDim.x + threadIdx.x; g < m; g += gridDim.x * blockDim.x) {
+        const u32 id = win ? win[g] : g;
+        if (!win && !active[id]) { has[id] = 0; continue; }
         const u32 sw = id * L, ew = (id + 1) * L;
         u32 lab = 0, idx = 0;
         float ml = 0.0f;
