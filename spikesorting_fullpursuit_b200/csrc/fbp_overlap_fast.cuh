@@ -1143,7 +1143,7 @@ struct RefItem {                         // one contender, in shared memory
 };
 __host__ __device__ inline size_t ov_refine_smem_bytes() {
     return (size_t)(kRefineThreads / 32) * (2 * kRefRows * kRefStride * 4 + kRefRows * sizeof(RefItem)) +
-           2 * kRefineThreads * 4;
+           kRefineThreads * 4;
 }
 
 // Exact values of the pooled contenders whose upper bound reaches their
@@ -1203,8 +1203,7 @@ k_ov_refine(OvArgs A) {
           if (!A.fallback[g] && !(A.pool_hi[e] < A.cand_lb[g])) list[atomicAdd(&cnt, 1u)] = e;
       }
       __syncthreads();
-      const u32 held = cnt;                          // < 2 * kRefineThreads
-      if (held < kRefineThreads && eb + kRefineThreads < e1) continue;   // gather more
+      const u32 held = cnt;                          // at most kRefineThreads
       if (threadIdx.x == 0 && held) atomicAdd(A.refined, held);
       const u32 per = min(kRefRows, max(1u, (held + kRefineThreads / 32 - 1) / (kRefineThreads / 32)));
       for (u32 base = warp * per; base < held; base += (kRefineThreads / 32) * per) {
