@@ -377,16 +377,25 @@ __global__ void k_resid_mean(const T *__restrict__ clips, const T *__restrict__ 
 constexpr u32 kCovMaxLL = 12288;         // L * L: L <= 110
 constexpr u32 kCovT = 4, kCovRows = 32;  // outputs of a thread a side, rows staged at a time
 inline u32 cov_tiles(u32 L) { const u32 t = ceil_div(L, kCovT); return t * (t + 1) / 2; }
-inline u32 cov_threads(u32 L) { return ceil_div(cov_tiles(L), 32) * 32; }
-inline size_t cov_smem_bytes(u32 L) { return ((size_t)kCovRows * ceil_div(L, kCovT) * kCovT + L) * sizeof(double); }
+// Groups of threads that share a block's rows: few tiles leave a block too small
+// to stage its rows, so there are as many groups as 256 threads hold.
+__host__ __device__ inline u32 cov_groups(u32 tiles) { return tiles >= 128 ? 1u : min(kCovRows, 256u / tiles); }
+inline u32 cov_threads(u32 L) { return ceil_div(cov_tiles(L) * cov_groups(cov_tiles(L)), 32) * 32; }
+inline size_t cov_smem_bytes(u32 L) {
+    const size_t rows = (size_t)kCovRows * ceil_div(L, kCovT) * kCovT + L, g = cov_groups(cov_tiles(L));
+    return std::max(rows, g > 1 ? g * cov_tiles(L) * kCovT * kCovT : (size_t)0) * sizeof(double);
+}
 
 // Per channel c, sum over the selected rows of (x_i - mean_i)(x_j - mean_j),
 // i, j < L; blocks take row ranges and add their partial matrix atomically.
 // FP64 work: a thread holds a 4 x 4 tile of outputs, four 16-byte shared reads
 // for 16 products (an output at a time took two reads for each), and only the
 // tiles on and above the diagonal, the others being the same sums.  16 channels
-// of 101 samples: 0.48 ms, before 1.60 ms.
-template <typename T>
+// of 101 samples: 0.48 ms, before 1.60 ms.  Short templates (up to 60 samples) have
+// fewer than 128 tiles: cov_groups() groups of threads take the rows in turn and
+// add up in shared memory (4 channels x 16 samples of 1,000 clips: 27 us in all, 71
+// with one group, 34 an output at a time).  kGroups: more than one.
+template <typename T, bool kGroups>
 __global__ void __launch_bounds__(416)
 k_resid_cov(const T *__restrict__ clips, const T *__restrict__ tmpl, const u32 *__restrict__ row_unit,
             const long long *__restrict__ rows, u32 n_sel, u32 C, u32 L, const double *__restrict__ sums,
@@ -397,10 +406,12 @@ k_resid_cov(const T *__restrict__ clips, const T *__restrict__ tmpl, const u32 *
     const u32 r_begin = (u32)((u64)n_sel * part / parts), r_end = (u32)((u64)n_sel * (part + 1) / parts);
     double *mean = csm + kCovRows * Lp;
     for (u32 i = threadIdx.x; i < L; i += blockDim.x) mean[i] = sums[c * L + i] / n_sel;
-    // tile threadIdx.x of the upper triangle, row by row
-    u32 ti = 0, tj = threadIdx.x;
-    while (ti < nt && tj >= nt - ti) { tj -= nt - ti; ti++; }
-    const bool mine = ti < nt;
+    // tile (threadIdx.x mod tiles) of the upper triangle, row by row
+    const u32 tiles = nt * (nt + 1) / 2, groups = kGroups ? cov_groups(tiles) : 1u,
+              grp = threadIdx.x / tiles;
+    u32 ti = 0, tj = threadIdx.x - grp * tiles;
+    while (tj >= nt - ti) { tj -= nt - ti; ti++; }
+    const bool mine = grp < groups;
     tj += ti;
     double acc[kCovT][kCovT];
 #pragma unroll
@@ -416,10 +427,11 @@ k_resid_cov(const T *__restrict__ clips, const T *__restrict__ tmpl, const u32 *
         }
         __syncthreads();
         if (mine) {
-            const double2 *pa = reinterpret_cast<const double2 *>(csm + ti * kCovT);
-            const double2 *pb = reinterpret_cast<const double2 *>(csm + tj * kCovT);
+            const u32 r1 = kGroups ? grp : 0u, step = groups * (Lp / 2);
+            const double2 *pa = reinterpret_cast<const double2 *>(csm + r1 * Lp + ti * kCovT);
+            const double2 *pb = reinterpret_cast<const double2 *>(csm + r1 * Lp + tj * kCovT);
 #pragma unroll 2
-            for (u32 rr = 0; rr < nr; rr++, pa += Lp / 2, pb += Lp / 2) {
+            for (u32 rr = r1; rr < nr; rr += groups, pa += step, pb += step) {
                 const double2 a0 = pa[0], a1 = pa[1], b0 = pb[0], b1 = pb[1];
                 const double av[kCovT] = {a0.x, a0.y, a1.x, a1.y}, bv[kCovT] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
@@ -429,8 +441,30 @@ k_resid_cov(const T *__restrict__ clips, const T *__restrict__ tmpl, const u32 *
             }
         }
     }
-    if (!mine) return;
     double *out = cov + (u64)c * L * L;
+    if (kGroups) {
+        __syncthreads();                             // the rows' readers are done
+        if (mine)
+#pragma unroll
+            for (u32 a = 0; a < kCovT; a++)
+#pragma unroll
+                for (u32 b = 0; b < kCovT; b++) csm[(a * kCovT + b) * groups * tiles + threadIdx.x] = acc[a][b];
+        __syncthreads();
+        for (u32 e = threadIdx.x; e < tiles * kCovT * kCovT; e += blockDim.x) {
+            const u32 k = e / tiles, t = e - k * tiles;
+            double s = 0.0;
+            for (u32 g = 0; g < groups; g++) s += csm[(k * groups + g) * tiles + t];
+            u32 i0 = 0, j0 = t;
+            while (j0 >= nt - i0) { j0 -= nt - i0; i0++; }
+            j0 += i0;
+            const u32 i = i0 * kCovT + k / kCovT, j = j0 * kCovT + k % kCovT;
+            if (i >= L || j >= L) continue;
+            atomicAdd(&out[i * L + j], s);
+            if (i0 != j0) atomicAdd(&out[j * L + i], s);
+        }
+        return;
+    }
+    if (!mine) return;
 #pragma unroll
     for (u32 a = 0; a < kCovT; a++)
 #pragma unroll
@@ -1065,16 +1099,19 @@ int fbp_clip_noise_covariance(const void *clips, int dtype, const uint32_t *row_
     const dim3 mb(32, 8), mg(ceil_div(dim, 32), std::min<u32>(64, ceil_div(n_sel, 8)));
     const u32 parts = std::max<u32>(1, std::min<u32>(ceil_div(n_sel, 256), ceil_div(148 * 4, C)));
     const size_t smem = cov_smem_bytes(L);
+    const bool grouped = cov_groups(cov_tiles(L)) > 1;
     if (dtype == FBP_F32) {
         k_resid_mean<float><<<mg, mb, 0, st>>>((const float *)clips, (const float *)templates, row_unit,
                                                (const long long *)rows, n_sel, dim, sums);
-        k_resid_cov<float><<<dim3(C, parts), cov_threads(L), smem, st>>>((const float *)clips, (const float *)templates, row_unit,
-                                                              (const long long *)rows, n_sel, C, L, sums, cov);
+        auto k = grouped ? k_resid_cov<float, true> : k_resid_cov<float, false>;
+        k<<<dim3(C, parts), cov_threads(L), smem, st>>>((const float *)clips, (const float *)templates, row_unit,
+                                                        (const long long *)rows, n_sel, C, L, sums, cov);
     } else if (dtype == FBP_I16) {
         k_resid_mean<short><<<mg, mb, 0, st>>>((const short *)clips, (const short *)templates, row_unit,
                                                (const long long *)rows, n_sel, dim, sums);
-        k_resid_cov<short><<<dim3(C, parts), cov_threads(L), smem, st>>>((const short *)clips, (const short *)templates, row_unit,
-                                                              (const long long *)rows, n_sel, C, L, sums, cov);
+        auto k = grouped ? k_resid_cov<short, true> : k_resid_cov<short, false>;
+        k<<<dim3(C, parts), cov_threads(L), smem, st>>>((const short *)clips, (const short *)templates, row_unit,
+                                                        (const long long *)rows, n_sel, C, L, sums, cov);
     } else {
         return fail(FBP_ERR_BAD_ARG, "fbp_clip_noise_covariance: dtype must be FBP_F32 or FBP_I16");
     }
