@@ -305,14 +305,6 @@ __global__ void k_robust_template(const T *__restrict__ tr, u32 n_rows, u32 dim,
             continue;
         }
         auto xv = [&](u32 i) { return (float)x[i]; };
-        u32 kmin = 0xffffffffu, kmax = 0;
-#pragma unroll 4
-        for (u32 i = lane; i < m; i += 32) {
-            const u32 k = fkey(xv(i));
-            kmin = min(kmin, k);
-            kmax = max(kmax, k);
-        }
-        const float vmin = kfloat(__reduce_min_sync(0xffffffffu, kmin)), vmax = kfloat(__reduce_max_sync(0xffffffffu, kmax));
         auto med_of = [&](const WarpBins &b, u32 a, u32 cnt, auto val) -> A {   // median of ranks [a, a + cnt)
             const u32 k0 = a + (cnt - 1) / 2, k1 = a + cnt / 2;
             float v0, v1;
@@ -325,15 +317,33 @@ __global__ void k_robust_template(const T *__restrict__ tr, u32 n_rows, u32 dim,
         };
         WarpBins bx, bd;
         bx.ok = bd.ok = false;
-        if (m <= kBinMax) bins_build(bx, m, vmin, vmax, xv, hist);
+        float vmin = 0.0f, vmax = 0.0f;
+        if (m <= kBinMax) {
+            u32 kmin = 0xffffffffu, kmax = 0;
+            bool nan = false;
+#pragma unroll 4
+            for (u32 i = lane; i < m; i += 32) {
+                const float v = xv(i);
+                const u32 k = fkey(v);
+                kmin = min(kmin, k);
+                kmax = max(kmax, k);
+                nan |= !(v == v);
+            }
+            vmin = kfloat(__reduce_min_sync(0xffffffffu, kmin));
+            vmax = kfloat(__reduce_max_sync(0xffffffffu, kmax));
+            // a column with NaN, which lies in no bin and has no place among few
+            // values either, is the radix selection's
+            if (!__any_sync(0xffffffffu, nan)) bins_build(bx, m, vmin, vmax, xv, hist);
+        }
         const A med = med_of(bx, 0, m, xv);
         auto dv = [&](A y) {
             const A d = y - med;
             return (float)(d < (A)0 ? -d : d);          // exact in float32 for both types
         };
         auto dvi = [&](u32 i) { return dv((A)x[i]); };
-        // the largest deviation is that of the smallest or the largest value
-        if (bx.ok) bins_build(bd, m, 0.0f, fmaxf(dv((A)vmin), dv((A)vmax)), dvi, hist);
+        // the largest deviation is that of the smallest or the largest value (NaN: the median is infinite)
+        const float dmin = dv((A)vmin), dmax = dv((A)vmax);
+        if (bx.ok && dmin == dmin && dmax == dmax) bins_build(bd, m, 0.0f, fmaxf(dmin, dmax), dvi, hist);
         const A mad = R::mad_scale(med_of(bd, 0, m, dvi));
         const A lo = med - mad, hi = med + mad;
         u32 nle = 0, nlt = 0;                           // #(x <= lo), #(x < hi)
