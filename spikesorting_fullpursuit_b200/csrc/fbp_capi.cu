@@ -816,8 +816,6 @@ int tc_chunk_setup(const Workspace &w, const float *v, u32 n, const float *T, u3
             k_tcw_pack<<<grid_for(total, 256), 256, 0, st>>>(T, C, L, nkc, w.tperm + g.t0, g.nt, g.clo, g.Cg,
                                                               w.tc_texp, (u16 *)(w.Aw + g.tb_off * kWATile));
         }
-        const u32 W = ceil_div(n, L);
-        k_window_vmax<<<grid_for((u64)(W + 2) * 32, 256, 8), 256, 0, st>>>(v, n, C, L, W, w.vwmax);
     }
     FBP_LAUNCH_CHECK();
     return FBP_OK;
@@ -1074,7 +1072,11 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
     FBP_CUDA(cudaMemsetAsync(w.wpos, 0, (size_t)W * w.G16, st));
     FBP_CUDA(cudaMemsetAsync(w.dirty, 0xff, (size_t)W * w.GW * 4, st));   // nothing is computed yet
     k_iota_windows<<<grid_for(W, 256), 256, 0, st>>>(w.win, w.active, W, w.cnt);
-    k_template_ranges<<<(int)std::min(K, 65535u), 256, 0, st>>>(templates, K, C, L, w.tsup);
+    k_template_ranges<<<(int)std::min(K, 65535u), 256, 0, st>>>(templates, K, C, L, w.tsup, neg_half_ss,
+                                                                w.tc ? &w.cnt->no_bounds : nullptr);
+    if (w.tc)
+        k_window_vmax<<<grid_for((u64)(W + 2) * 32, 256, 8), 256, 0, st>>>(voltage, n, C, L, W, w.vwmax,
+                                                                           &w.cnt->no_bounds);
     k_template_support<<<1, 256, 0, st>>>(templates, K, C, L, w.tsup, w.tperm, w.grange, kLikTplPerBlock,
                                           w.grange32, kTabMGroup);
     FBP_LAUNCH_CHECK();
@@ -1083,10 +1085,16 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
         // tensor-core group plan and the choice of overlap-table kernel
         const u32 ng = ceil_div(K, kTabMGroup);
         std::vector<u32> tsup(2 * (size_t)K), tperm(K), gr(2 * (size_t)ng);
+        u32 no_bounds = 0;
         FBP_CUDA(cudaMemcpyAsync(tsup.data(), w.tsup, tsup.size() * 4, cudaMemcpyDeviceToHost, st));
         FBP_CUDA(cudaMemcpyAsync(tperm.data(), w.tperm, tperm.size() * 4, cudaMemcpyDeviceToHost, st));
         FBP_CUDA(cudaMemcpyAsync(gr.data(), w.grange32, gr.size() * 4, cudaMemcpyDeviceToHost, st));
+        if (w.tc) FBP_CUDA(cudaMemcpyAsync(&no_bounds, &w.cnt->no_bounds, 4, cudaMemcpyDeviceToHost, st));
         FBP_CUDA(cudaStreamSynchronize(st));
+        // The intervals of the tensor-core path are for finite values in a safe
+        // range (its operands are clamped to that of fp16): the FP32 kernel takes
+        // a chunk with others.  (The testing output of the bounds is for any.)
+        if (no_bounds && !dbg_bound) w.tc = false;
         // the widest support: adding an exact zero product is exact (in the
         // reference's sum and in any accumulation order), so the tensor-core
         // rounding bounds count its products, not C*L

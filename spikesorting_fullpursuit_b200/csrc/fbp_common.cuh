@@ -33,7 +33,7 @@ struct Counters {
     u32 pad2;
     u32 tc_err;       // non-zero: a bounded wait in the tensor-core kernel gave up
     u32 tc_overflow;  // refinement list overflowed: the exact kernel redoes the pass
-    u32 pad0;
+    u32 no_bounds;    // a voltage or template value is not finite, or too large or small for the intervals
     u64 lazy_ref;     // approximate likelihood entries refined on demand (whole chunk)
     u32 ov_ref;       // overlap contenders evaluated exactly this pass
     u32 pad1;

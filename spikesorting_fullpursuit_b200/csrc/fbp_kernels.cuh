@@ -34,6 +34,12 @@ struct WinBounds {
     u32 *dirty;
     u32 GW;
 };
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) <= 3.402823466e+38f; }
+// What the error bounds of the tensor-core path are for.  With |SS/2| <= 2^100
+// and |v| <= 2^60 no sum of up to 2^24 products overflows (||t|| ||window|| <=
+// 2^50.5 2^60 2^12); with |SS/2| >= 2^-100 what the products and sums lose below
+// the normal range, 2^-150 each, is far inside kappa_s |SS/2|.
+constexpr float kSafeSS = 1.2676506e30f, kSafeV = 1.1529215e18f;
 __device__ __forceinline__ bool win_dirty(const WinBounds &wb, u32 w, u32 g) {
     return !wb.dirty || ((wb.dirty[(size_t)w * wb.GW + (g >> 5)] >> (g & 31)) & 1u);
 }
@@ -181,8 +187,12 @@ constexpr int kLikThreads = 128;
 // template order sorted by (lo, id) (tperm), and per group of kLikTplPerBlock
 // consecutive slots the union of their ranges (grange).  One block.
 // Non-zero channel range of each template: one block per template, warps
-// over channels.
-__global__ void k_template_ranges(const float *__restrict__ T, u32 K, u32 C, u32 L, u32 *__restrict__ tsup) {
+// over channels.  With no_bounds, also whether a template holds a value that is
+// not finite, or its -SS/2 (tss) is so large or small that the reference's own
+// products or sums may leave the normal range, where their rounding is not
+// relative (kSafeSS, kSafeV: see there).
+__global__ void k_template_ranges(const float *__restrict__ T, u32 K, u32 C, u32 L, u32 *__restrict__ tsup,
+                                  const float *__restrict__ tss = nullptr, u32 *__restrict__ no_bounds = nullptr) {
     __shared__ u32 slo, shi;
     const u32 lane = threadIdx.x & 31;
     for (u32 t = blockIdx.x; t < K; t += gridDim.x) {
@@ -191,9 +201,13 @@ __global__ void k_template_ranges(const float *__restrict__ T, u32 K, u32 C, u32
         u32 lo = C, hi = 0;
         for (u32 c = threadIdx.x >> 5; c < C; c += blockDim.x >> 5) {
             const float *tp = T + ((size_t)t * C + c) * L;
-            bool nz = false;
-            for (u32 i = lane; i < L; i += 32) nz |= tp[i] != 0.0f;
+            bool nz = false, bad = false;
+            for (u32 i = lane; i < L; i += 32) {
+                nz |= tp[i] != 0.0f;
+                bad |= !is_finite(tp[i]);
+            }
             if (__any_sync(0xffffffffu, nz)) { lo = min(lo, c); hi = c + 1; }
+            if (bad && no_bounds) *no_bounds = 1;
         }
         if (lane == 0 && hi > 0) {
             atomicMin(&slo, lo);
@@ -203,6 +217,8 @@ __global__ void k_template_ranges(const float *__restrict__ T, u32 K, u32 C, u32
         if (threadIdx.x == 0) {
             tsup[2 * t] = shi == 0 ? 0u : slo;       // all-zero template: empty range
             tsup[2 * t + 1] = shi;
+            const float ss = fabsf(no_bounds ? tss[t] : 0.0f);
+            if (no_bounds && !(ss <= kSafeSS && (shi == 0 || ss >= 1.0f / kSafeSS))) *no_bounds = 1;
         }
         __syncthreads();
     }

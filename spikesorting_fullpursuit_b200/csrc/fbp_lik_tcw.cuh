@@ -826,21 +826,26 @@ __global__ void k_tcw_pack(const float *__restrict__ T, u32 Call, u32 L, u32 nkc
     }
 }
 
-// Largest |v| of each window over all channels; two zero pads past the end.
-__global__ void k_window_vmax(const float *__restrict__ v, u32 n, u32 C, u32 L, u32 W, float *__restrict__ vwmax) {
+// Largest |v| of each window over all channels; two zero pads past the end.  And
+// whether a sample is not finite or above kSafeV.
+__global__ void k_window_vmax(const float *__restrict__ v, u32 n, u32 C, u32 L, u32 W, float *__restrict__ vwmax,
+                              u32 *__restrict__ no_bounds) {
     const u32 lane = threadIdx.x & 31;
     const u32 nwarps = (gridDim.x * blockDim.x) >> 5;
     for (u32 w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < W + 2; w += nwarps) {
-        float m = 0.0f;
+        u32 m = 0;                                   // as bits: in the order of the values, NaN above all
         if (w < W) {
             for (u32 c = 0; c < C; c++) {
                 const float *vc = v + (size_t)c * n + (size_t)w * L;
                 for (u32 i = lane; i < L; i += 32)
-                    if ((size_t)w * L + i < n) m = fmaxf(m, fabsf(vc[i]));
+                    if ((size_t)w * L + i < n) m = max(m, __float_as_uint(vc[i]) & 0x7fffffffu);
             }
         }
-        m = warp_max_float(m);
-        if (lane == 0) vwmax[w] = m;
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0) {
+            vwmax[w] = __uint_as_float(min(m, 0x7f800000u));
+            if (m > __float_as_uint(kSafeV)) *no_bounds = 1;
+        }
     }
 }
 
