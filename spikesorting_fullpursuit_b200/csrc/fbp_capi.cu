@@ -300,9 +300,11 @@ u32 plan_tcw_groups(const std::vector<u32> &tsup, const std::vector<u32> &tperm,
 
 // Bytes a chunk's workspace is planned with.  binary_pursuit() takes chunk
 // lengths from this number and results depend on chunk boundaries, so it is a
-// formula of its own, and layout() fits its buffers into it: the refinement
-// list (tensor cores) or the contender pool takes what the others leave, up
-// to the capacities below.
+// formula of its own, which tests pin, and layout() fits its buffers into it:
+// the refinement list (tensor cores) and then the contender pool give way, down
+// to half of the capacities below, and the buffers that only save time are left
+// out where that is not enough.
+constexpr u32 kPlanTcArgs = 416, kPlanTcwArgs = 336;     // bytes planned for a template group's launch arguments
 size_t planned_bytes(u32 n, u32 K, u32 L, u32 nmax, u32 C, bool want_tc, u32 &pool_cap, u32 &ref_cap) {
     const u64 W = ceil_div(n, L), Wp = W + FBP_WINDOW_PAD, wb = window_bytes_u8((u32)W), S = 2 * (u64)nmax + 1;
     size_t t = 0;
@@ -332,15 +334,18 @@ size_t planned_bytes(u32 n, u32 K, u32 L, u32 nmax, u32 C, bool want_tc, u32 &po
         take((u64)K * n); take(G * n * 4, 2); take((u64)n * 4); take(G * n); take((u64)K * 4, 3);
         take((u64)ref_cap * 4, 2);
         take((u64)((u32)((W * ((L + kTcM - 1) / kTcM) + 16) * G)) * 4, 4);
-        take(G * 12); take((u64)K * 4); take(G * 416, 2);
+        take(G * 12); take((u64)K * 4); take(G * kPlanTcArgs, 2);
         take((W + 2) * 4); take(wb); take(Wp * 4, 2); take((W * (2 * (u64)L) / kWPos + 4) * 4);
-        take(G * C * tcw_nkc(L) * kWATile); take((u64)K * 4); take(G * 12); take(G * 336);
+        take(G * C * tcw_nkc(L) * kWATile); take((u64)K * 4); take(G * 12); take(G * kPlanTcwArgs);
     }
     return t;
 }
 
+static_assert(sizeof(TcArgs) <= kPlanTcArgs && sizeof(TcwArgs) <= kPlanTcwArgs, "the plan holds the arguments");
+
+// extras: XMw (tensor cores) or the dirty bits (FP32).
 Workspace layout_with(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 C, bool want_tc, u32 pool_cap,
-                      u32 ref_cap) {
+                      u32 ref_cap, bool extras) {
     Workspace w{};
     const u32 W = ceil_div(n, L);
     const size_t Wp = (size_t)W + FBP_WINDOW_PAD;
@@ -354,10 +359,10 @@ Workspace layout_with(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast,
     w.snap = (Counters *)take(sizeof(Counters));
     w.G16 = ceil_div(K, 16);
     w.GW = ceil_div(w.G16, 32);
-    w.wlb = (float *)take((size_t)W * w.G16 * 4);
+    w.wlb = want_tc ? (float *)take((size_t)W * w.G16 * 4) : nullptr;
     w.umax = (float *)take((size_t)W * K * 4);
-    w.wpos = (u8 *)take((size_t)W * w.G16);
-    w.dirty = (u32 *)take((size_t)W * w.GW * 4);
+    w.wpos = want_tc ? (u8 *)take((size_t)W * w.G16) : nullptr;
+    w.dirty = want_tc || extras ? (u32 *)take((size_t)W * w.GW * 4) : nullptr;
     w.tsup = (u32 *)take((size_t)K * 8);
     w.tperm = (u32 *)take((size_t)K * 4);
     w.grange = (u32 *)take((size_t)ceil_div(K, kLikTplPerBlock) * 8);
@@ -395,7 +400,7 @@ Workspace layout_with(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast,
         w.tnorm = (float *)take((size_t)K * 4);
         w.Q = (float *)take((size_t)K * K * (2 * L - 1) * (L + 1) * 4);
         w.XMr = (float *)take((size_t)K * K * (2 * L + 1) * 4);
-        w.XMw = want_tc ? (float *)take((size_t)K * K * (2 * L + 32) * 4) : nullptr;
+        w.XMw = want_tc && extras ? (float *)take((size_t)K * K * (2 * L + 32) * 4) : nullptr;
         w.XM = (float *)take((size_t)K * K * 4);
         w.H = (float *)take(sl * K * S * 4);
         w.vn = (float *)take(sl * 4);
@@ -409,7 +414,7 @@ Workspace layout_with(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast,
         w.seed_a1 = (u32 *)take(sl * 4);
         w.pair_mb = (float *)take(sl * K * 4);
         w.pair_mabs = (float *)take(sl * K * 4);     // with wide tables: the largest lower bounds
-        if (want_tc) {
+        if (want_tc && L >= kWMinL) {
             w.pair_b1 = (u16 *)take(sl * K * 2);
             w.slot_tab = (uint4 *)take(sl * sizeof(uint4));
         }
@@ -451,14 +456,16 @@ Workspace layout_with(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast,
         // wide tiles: per-window |v| bound, the pass's stream, A tiles of
         // every group of 16 templates (at most all C channels each)
         w.vwmax = (float *)take(((size_t)W + 2) * 4);
-        w.wl_stride = W;
-        w.wf_stride = (u32)((size_t)W * (2 * (size_t)L) / kWPos + 4);
-        w.wl_win = (u32 *)take((size_t)w.G16 * W * 4);
-        w.wl_pos = (u32 *)take((size_t)w.G16 * W * 4);
-        w.wl_first = (u32 *)take((size_t)w.G16 * w.wf_stride * 4);
-        w.wl_nwin = (u32 *)take((size_t)w.G16 * 4);
-        w.wl_nst = (u32 *)take((size_t)w.G16 * 4);
-        w.wl_counts = (u32 *)take((size_t)w.G16 * ceil_div(W, kCompactTile) * 4);
+        if (L >= kWMinL) {
+            w.wl_stride = W;
+            w.wf_stride = (u32)((size_t)W * (2 * (size_t)L) / kWPos + 4);
+            w.wl_win = (u32 *)take((size_t)w.G16 * W * 4);
+            w.wl_pos = (u32 *)take((size_t)w.G16 * W * 4);
+            w.wl_first = (u32 *)take((size_t)w.G16 * w.wf_stride * 4);
+            w.wl_nwin = (u32 *)take((size_t)w.G16 * 4);
+            w.wl_nst = (u32 *)take((size_t)w.G16 * 4);
+            w.wl_counts = (u32 *)take((size_t)w.G16 * ceil_div(W, kCompactTile) * 4);
+        }
         w.Aw = (unsigned char *)take((size_t)w.tc_gmax * C * tcw_nkc(L) * kWATile);
         w.tgrp_w = (u32 *)take((size_t)K * 4);
         w.tcw_gdesc = (u32 *)take((size_t)w.tc_gmax * 12);
@@ -472,15 +479,25 @@ Workspace layout_with(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast,
 Workspace layout(char *base, u32 n, u32 K, u32 L, u32 nmax, bool want_fast, u32 C = 0, bool want_tc = false) {
     u32 pool = 0, ref = 0;
     const size_t plan = planned_bytes(n, K, L, nmax, C, want_tc, pool, ref);
-    // with the fast overlap's buffers, whether or not this call uses them
-    const size_t need = layout_with(nullptr, n, K, L, nmax, true, C, want_tc, pool, ref).bytes;
-    if (need > plan) {
-        const size_t over = need - plan + 1024;      // alignment of the shrunken buffers
-        if (ref) ref = (u32)std::max<u64>(std::min<u64>(ref, 1u << 16), ref - std::min<u64>(ref, ceil_div64(over, 8)));
-        else if (pool) pool = (u32)std::max<u64>(std::min<u64>(pool, 1u << 20), pool - std::min<u64>(pool, ceil_div64(over, 12)));
+    const u32 pool0 = pool, ref0 = ref;
+    bool extras = true;
+    for (;; extras = false) {
+        // with the fast overlap's buffers, whether or not this call uses them
+        const size_t need = layout_with(nullptr, n, K, L, nmax, true, C, want_tc, pool0, ref0, extras).bytes;
+        if (need <= plan) break;
+        // Half the list is 12 % of the chunk's entries; 1 to 2 % are queued on a
+        // dense probe, and a list that overflows costs a pass by the FP32 kernel.
+        // XMw for 300 templates of 61 samples is 55 MB, as much as the list of
+        // three seconds; without it k_ov_scan bounds a pair's lags by XM.
+        const u64 over = need - plan + 2048;         // 2048: alignment of the shrunken buffers
+        const u32 from_ref = (u32)std::min<u64>(ref0 / 2, ceil_div64(over, 8));
+        const u64 rest = over - std::min<u64>(over, (u64)from_ref * 8);
+        const u32 from_pool = (u32)std::min<u64>(pool0 / 2, ceil_div64(rest, 12));
+        ref = ref0 - from_ref;
+        pool = pool0 - from_pool;
+        if ((u64)from_pool * 12 >= rest || !extras) break;   // (else: templates of one sample, the workspace grows)
     }
-    Workspace w = layout_with(base, n, K, L, nmax, want_fast, C, want_tc, pool, ref);
-    return w;
+    return layout_with(base, n, K, L, nmax, want_fast, C, want_tc, pool, ref, extras);
 }
 
 int grid_for(u64 items, int threads, int per_sm = 8) {
@@ -1067,10 +1084,10 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
     FBP_CUDA(cudaMemsetAsync(w.ovr, 0, wb, st));
     FBP_CUDA(cudaMemsetAsync(w.ovr2, 0, wb, st));
     FBP_CUDA(cudaMemsetAsync(w.active, 0, wb, st));
-    FBP_CUDA(cudaMemsetAsync(w.wlb, 0, (size_t)W * w.G16 * 4, st));
+    if (w.wlb) FBP_CUDA(cudaMemsetAsync(w.wlb, 0, (size_t)W * w.G16 * 4, st));
     FBP_CUDA(cudaMemsetAsync(w.umax, 0, (size_t)W * K * 4, st));
-    FBP_CUDA(cudaMemsetAsync(w.wpos, 0, (size_t)W * w.G16, st));
-    FBP_CUDA(cudaMemsetAsync(w.dirty, 0xff, (size_t)W * w.GW * 4, st));   // nothing is computed yet
+    if (w.wpos) FBP_CUDA(cudaMemsetAsync(w.wpos, 0, (size_t)W * w.G16, st));
+    if (w.dirty) FBP_CUDA(cudaMemsetAsync(w.dirty, 0xff, (size_t)W * w.GW * 4, st));   // nothing is computed yet
     k_iota_windows<<<grid_for(W, 256), 256, 0, st>>>(w.win, w.active, W, w.cnt);
     k_template_ranges<<<(int)std::min(K, 65535u), 256, 0, st>>>(templates, K, C, L, w.tsup, neg_half_ss,
                                                                 w.tc ? &w.cnt->no_bounds : nullptr);

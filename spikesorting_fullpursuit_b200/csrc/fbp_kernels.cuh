@@ -20,7 +20,8 @@ namespace fbp {
 // wlb[w][g] the largest lower bound of an entry of window w, umax[w][t] the
 // largest upper bound of template t's entries there (>= 0), wpos[w][g]
 // whether any entry is > 0.  Reset when the (window, group) is recomputed;
-// entries only move inside their intervals later.
+// entries only move inside their intervals later.  In FP32 mode, where umax is the
+// largest entry itself, wlb and wpos are NULL.
 // dirty: one bit per (window, group), GW words a window: the voltage the
 // group's entries of the window read has changed since they were computed
 // (k_gather_spikes), so a listed window recomputes them; the others keep the
@@ -154,7 +155,7 @@ __global__ void k_mark_active(const u8 *__restrict__ flags, u8 *__restrict__ act
             const u32 w = i0 + __ffs(m) - 1;
             m &= m - 1;
             for (u32 g = lane; g < wb.G; g += 32) {
-                if (!win_dirty(wb, w, g)) continue;
+                if (!wb.wlb || !win_dirty(wb, w, g)) continue;
                 wb.wlb[(size_t)w * wb.G + g] = 0.0f;
                 wb.wpos[(size_t)w * wb.G + g] = 0;
             }
@@ -426,10 +427,11 @@ k_likelihood_fp32(const float *__restrict__ v, u32 n, u32 C, const float *__rest
                     anypos |= mq > 0.0f;
                     if (lane == 0 && mq > 0.0f && slot0 + q < K) {
                         atomicMax(reinterpret_cast<int *>(wb.umax) + (size_t)w * K + tq[q], __float_as_int(mq));
-                        atomicMax(reinterpret_cast<int *>(wb.wlb) + (size_t)w * wb.G + kg, __float_as_int(mq));
+                        if (wb.wlb)
+                            atomicMax(reinterpret_cast<int *>(wb.wlb) + (size_t)w * wb.G + kg, __float_as_int(mq));
                     }
                 }
-                if (lane == 0 && anypos) wb.wpos[(size_t)w * wb.G + kg] = 1;
+                if (lane == 0 && anypos && wb.wpos) wb.wpos[(size_t)w * wb.G + kg] = 1;
             }
 #pragma unroll
             for (int q = 0; q < kLikQ; q++) {
@@ -667,6 +669,11 @@ k_window_argmax(u32 n, u32 L, u32 K, const u32 *__restrict__ win,
             const u32 glo = (id > 0 ? id - 1 : 0) * wb.G, ghi = min(id + 2, W) * wb.G;
             for (u32 k = glo + lane; k < ghi; k += 32) lb = fmaxf(lb, wb.wlb[k]);
             for (u32 k = lane; k < wb.G; k += 32) check |= wb.wpos[(size_t)id * wb.G + k] != 0;
+            lb = warp_max_float(lb);
+        } else if (wb.umax) {                            // exact entries: the upper bounds are the largest entries
+            const size_t ulo = (size_t)(id > 0 ? id - 1 : 0) * K, uhi = (size_t)min(id + 2, W) * K;
+            for (size_t k = ulo + lane; k < uhi; k += 32) lb = fmaxf(lb, wb.umax[k]);
+            for (u32 k = lane; k < K; k += 32) check |= wb.umax[(size_t)id * K + k] > 0.0f;
             lb = warp_max_float(lb);
         }
         // With window bounds only templates whose upper bound over windows
