@@ -92,6 +92,15 @@ __device__ __forceinline__ float kfloat(u32 k) {
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
 
+// The key of a stored value, from its bits as an integer: fkey() of a value that the
+// compiler knows as a float may lose the sign of a NaN.
+__device__ __forceinline__ u32 stored_key(const float *p) {
+    const u32 b = *reinterpret_cast<const u32 *>(p);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ u32 stored_key(const short *p) { return fkey((float)*p); }
+constexpr u32 kKeyLow = 0x007fffffu, kKeyHigh = 0xff800000u;     // of the infinities: NaN lies outside
+
 // Products rounded on their own (no contraction into a following add), as
 // numpy forms an array of squares before it sums them.
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
@@ -320,20 +329,19 @@ __global__ void k_robust_template(const T *__restrict__ tr, u32 n_rows, u32 dim,
         float vmin = 0.0f, vmax = 0.0f;
         if (m <= kBinMax) {
             u32 kmin = 0xffffffffu, kmax = 0;
-            bool nan = false;
 #pragma unroll 4
             for (u32 i = lane; i < m; i += 32) {
-                const float v = xv(i);
-                const u32 k = fkey(v);
+                const u32 k = stored_key(x + i);
                 kmin = min(kmin, k);
                 kmax = max(kmax, k);
-                nan |= !(v == v);
             }
-            vmin = kfloat(__reduce_min_sync(0xffffffffu, kmin));
-            vmax = kfloat(__reduce_max_sync(0xffffffffu, kmax));
+            kmin = __reduce_min_sync(0xffffffffu, kmin);
+            kmax = __reduce_max_sync(0xffffffffu, kmax);
+            vmin = kfloat(kmin);
+            vmax = kfloat(kmax);
             // a column with NaN, which lies in no bin and has no place among few
             // values either, is the radix selection's
-            if (!__any_sync(0xffffffffu, nan)) bins_build(bx, m, vmin, vmax, xv, hist);
+            if (kmin >= kKeyLow && kmax <= kKeyHigh) bins_build(bx, m, vmin, vmax, xv, hist);
         }
         const A med = med_of(bx, 0, m, xv);
         auto dv = [&](A y) {
