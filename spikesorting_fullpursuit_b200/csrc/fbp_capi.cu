@@ -266,7 +266,14 @@ bool plan_tc_groups(const std::vector<u32> &tsup, const std::vector<u32> &tperm,
 // Wide-tile groups (fbp_lik_tcw.cuh): templates in support order (tperm)
 // cut into groups of 16 (M = 16 templates x 8 sample shifts); a group's
 // channels are the union of its templates' supports.  Returns the ring
-// stages that fit shared memory, 0 when the wide layout does not apply.
+// stages that fit shared memory, 0 when the wide layout does not apply (below
+// 16 samples a tile meets too many windows, above 329 two stages do not fit).
+// There are seven stages up to 73 samples and two or three above 153, which is
+// still the better layout.  Likelihood and refinement of a pursuit here and with
+// 128-sample tiles, templates of 191, 260 and 329 samples: 16 channels x 32
+// templates 3.2, 6.1, 8.7 against 3.1, 7.9, 9.8 ms; 4 x 8 0.8, 1.3, 1.3 against
+// 1.5, 2.7, 2.9 ms; 96 x 100 on 12 channels each, 191 samples, 6.1 against 40 ms
+// (longer ones have no plan of 128-sample tiles).
 u32 plan_tcw_groups(const std::vector<u32> &tsup, const std::vector<u32> &tperm, u32 K, u32 C, u32 L,
                     std::vector<TcGroup> &out) {
     out.clear();
@@ -842,7 +849,7 @@ int tc_chunk_setup(const Workspace &w, const float *v, u32 n, const float *T, u3
 TcwParams tcw_params(const Workspace &w, u32 n, u32 K, u32 L, const float *tss, float *Lk, Counters *cnt,
                      float *dbg_bound) {
     TcwParams A{};
-    A.n = n; A.L = L; A.ns = w.tcw_ns; A.G = (u32)w.tcwg.size(); A.Kall = K; A.W = ceil_div(n, L);
+    A.n = n; A.L = L; A.ns = w.tcw_ns; A.G = (u32)w.tcwg.size(); A.Kall = K;
     A.wstride = w.wl_stride; A.fstride = w.wf_stride;
     A.groups = w.tcw_args;
     A.kappa_b = tc_kappa(w.tc_nz, L, ceil_div(w.tc_nz, 8));

@@ -71,7 +71,7 @@ struct TcwArgs {
     const unsigned char *Aw;         // [Cg][nkc] A tiles
 };
 struct TcwParams {
-    u32 n, L, ns, G, Kall, W, wstride, fstride;
+    u32 n, L, ns, G, Kall, wstride, fstride;
     const TcwArgs *groups;           // [G]
     float kappa_b, kappa_s;
     const float *tss, *tnorm, *tabs;
