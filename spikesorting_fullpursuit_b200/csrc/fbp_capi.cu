@@ -1108,13 +1108,18 @@ int prepare_chunk(Workspace &w, float *voltage, u32 n, u32 C, const float *templ
         // template supports on the host (one small read-back per chunk): the
         // tensor-core group plan and the choice of overlap-table kernel
         const u32 ng = ceil_div(K, kTabMGroup);
-        std::vector<u32> tsup(2 * (size_t)K), tperm(K), gr(2 * (size_t)ng);
+        // (tsup, tperm, grange and grange32 follow one another)
+        std::vector<u32> head((size_t)(w.grange32 - w.tsup) + 2 * (size_t)ng);
         u32 no_bounds = 0;
-        FBP_CUDA(cudaMemcpyAsync(tsup.data(), w.tsup, tsup.size() * 4, cudaMemcpyDeviceToHost, st));
-        FBP_CUDA(cudaMemcpyAsync(tperm.data(), w.tperm, tperm.size() * 4, cudaMemcpyDeviceToHost, st));
-        FBP_CUDA(cudaMemcpyAsync(gr.data(), w.grange32, gr.size() * 4, cudaMemcpyDeviceToHost, st));
+        FBP_CUDA(cudaMemcpyAsync(head.data(), w.tsup, head.size() * 4, cudaMemcpyDeviceToHost, st));
         if (w.tc) FBP_CUDA(cudaMemcpyAsync(&no_bounds, &w.cnt->no_bounds, 4, cudaMemcpyDeviceToHost, st));
         FBP_CUDA(cudaStreamSynchronize(st));
+        auto part = [&](const u32 *from, size_t count) {
+            const u32 *p = head.data() + (from - w.tsup);
+            return std::vector<u32>(p, p + count);
+        };
+        const std::vector<u32> tsup = part(w.tsup, 2 * (size_t)K), tperm = part(w.tperm, K),
+                               gr = part(w.grange32, 2 * (size_t)ng);
         // The intervals of the tensor-core path are for finite values in a safe
         // range (its operands are clamped to that of fp16): the FP32 kernel takes
         // a chunk with others.  (The testing output of the bounds is for any.)
