@@ -151,9 +151,9 @@ class ClockSampler:
 # DRAM bytes (read + write) per unit of algorithmic work of the tensor-core
 # likelihood kernel of each layout, from one ncu capture of pass 1 of a 10 s
 # slice of each workload (every window listed; dram__bytes_read.sum +
-# dram__bytes_write.sum over sample x templates of the pass); see the
-# k_lik_tc* summaries in profiles/.
-LIK_TC_DRAM_BYTES_PER_ST = {("hd384_300u", "wide"): 12.23, ("linear16_64u", "wide"): None,
+# dram__bytes_write.sum over sample x templates of the pass); see
+# k_tcw_hd384_10s.md and the k_lik_tc* summaries in profiles/.
+LIK_TC_DRAM_BYTES_PER_ST = {("hd384_300u", "wide"): 10.76, ("linear16_64u", "wide"): None,
                             ("hd384_300u", "samples"): 11.5, ("linear16_64u", "samples"): None}
 LIK_KERNEL = {"wide": "k_lik_tcw", "samples": "k_lik_tc<0>"}
 

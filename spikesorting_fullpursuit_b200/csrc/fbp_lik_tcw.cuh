@@ -325,7 +325,7 @@ k_lik_tcw(const __grid_constant__ TcwParams P) {
             // group: tiles computed together write the rows of 16 templates and
             // read one group's channels (taking every group's tile 0, then tile
             // 1, ... spreads them over all rows, 1,000 pages of 2 MB on the
-            // 384-channel probe: 17.9 against 10.6 ms for its first pass of 100 s)
+            // 384-channel probe: its first pass of 100 s took 1.7 times as long)
             u32 g = 0, q = f;
             for (u32 g0 = 0; g0 < G; g0 += 32) {
                 const u32 t = g0 + lane < G ? P.n_stiles[g0 + lane] : 0u;
